@@ -378,8 +378,8 @@ int mpsgpu_launch_count(long long* n);
  *    call returns MPSGPU_ERR_ARG naming the first such row, with x untouched;
  *  - b = 0 gives x = 0, 0 iterations and relres 0 (Eigen's CG returns the same);
  *  - each call clears the array's control words itself; nothing needs zeroing first;
- *  - the array is shared by every call on a device: calls that overlap on the GPU
- *    (two streams, two host threads) race and corrupt each other;
+ *  - the array is shared by every call on a device: calls of several host threads take
+ *    turns;
  *  - the first call on a device looks the array's address up with that device
  *    current; make it before any stream capture begins.
  * The call synchronises `stream` (cudaStream_t as void*, may be NULL) to poll
