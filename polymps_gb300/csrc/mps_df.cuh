@@ -62,6 +62,12 @@ __device__ __forceinline__ df operator*(df a, float b) {
 }
 __device__ __forceinline__ df& operator+=(df& a, df b) { a = a + b; return a; }
 __device__ __forceinline__ df& operator-=(df& a, df b) { a = a - b; return a; }
+// a / b: the FP32 quotient and one correction of the remainder (about 2^-45 relative)
+__device__ __forceinline__ df divDF(df a, df b) {
+    const float y = 1.0f / b.h, q = fM(a.h, y);
+    const df r = a - b * q;
+    return quick2(q, fM(r.h, y));
+}
 // ordering of normalised values (|l| <= ulp(h)/2)
 __device__ __forceinline__ bool operator<(df a, df b) { return a.h < b.h || (a.h == b.h && a.l < b.l); }
 __device__ __forceinline__ bool operator>(df a, df b) { return b < a; }

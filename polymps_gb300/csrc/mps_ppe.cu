@@ -17,7 +17,9 @@
 // and all dot products, and runs the inner CG on FP32 matrix values and vectors.
 #include "mps_df.cuh"
 #include "mps_internal.h"
+#include <algorithm>
 #include "mps_bulk.cuh"
+#include "mps_grid.cuh"
 
 #define PBLK 256
 
@@ -450,12 +452,12 @@ int ppeSolveMixed(const Dev& d, const PpeBuffers& B, double tol, int maxIter, cu
 //   x += alpha p, r -= alpha Ap, z = M^-1 r
 // so the only vector every block gathers (z) is complete at the reduction before it.
 // A reduction is one barrier: every block stores its partial sums, adds one to the
-// arrival counter (release) and waits until the counter reaches the generation's target
-// (acquire); then every block sums all partials in block order and derives the solver's
+// arrival counter (release) and polls it until it reaches the generation's target; then
+// every block sums all partials in block order and derives the solver's
 // scalars itself.  Identical inputs in identical order give every block identical
 // scalars, so no block has to publish them and release the others.  The scalars and flags
 // live in shared memory per block; block 0 stores its copy for the host at the end.  Waits are
-// bounded: a block that waits longer than QSPIN polls sets the abort word and every
+// bounded: a block that waits longer than GRID_SPIN polls sets the abort word and every
 // block returns.
 // Block sizes: one block per SM (1024 threads for the mixed solvers at <= 64 registers,
 // 768 for the FP64 solvers at <= 80), so a reduction reads 152 partials per value
@@ -464,7 +466,6 @@ int ppeSolveMixed(const Dev& d, const PpeBuffers& B, double tol, int maxIter, cu
 #define QB 256
 #define QBX 1024
 #define QBC 768
-#define QSPIN (1 << 21)
 // barrier words, each on its own 128-byte line (the arrival counter is 64-bit and only
 // grows within a launch; it is zeroed before each launch): arrivals, unused, abort
 #define QB_ARR 0
@@ -501,70 +502,83 @@ __device__ __forceinline__ void qStore(const PpeBuffers& B, const QLocal& L) {
     }
 }
 
+__device__ __forceinline__ GridBar qBar(const PpeBuffers& B, const QCtl& c) {
+    return {reinterpret_cast<unsigned long long*>(B.bar + QB_ARR), B.bar + QB_ABT, c.gen};
+}
 // Grid barrier: all writes of the block before it are visible to every block after it.
 __device__ __forceinline__ bool qBarrier(const PpeBuffers& B, QCtl& c) {
-    __shared__ int sOk;
-    __syncthreads();
+    GridBar g = qBar(B, c);
     c.gen++;
-    if (threadIdx.x == 0) {
-        unsigned long long* cnt = reinterpret_cast<unsigned long long*>(B.bar + QB_ARR);
-        const unsigned long long target = (unsigned long long)c.gen * gridDim.x;
-        asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(cnt) : "memory");
-        int ok = 1;
-        long long spins = 0;
-        while (true) {
-            unsigned long long v;
-            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(cnt) : "memory");
-            if (v >= target) break;
-            if (++spins > QSPIN) { atomicExch(B.bar + QB_ABT, 1u); ok = 0; break; }
-            if ((spins & 15) == 0 && *(volatile unsigned int*)(B.bar + QB_ABT)) { ok = 0; break; }
-            if (spins > 4) __nanosleep(32);
-        }
-        __threadfence();
-        if (ok && *(volatile unsigned int*)(B.bar + QB_ABT)) ok = 0;
-        sOk = ok;
-    }
-    __syncthreads();
-    return sOk;
+    return gridBarrier(g);
 }
-// Grid sum of NV (<= 4) FP64 values per thread; fin(tot) runs on thread 0 of every block
-// with the same totals, and its writes to the block-local scalars are visible to the
-// block's threads on return.  The partials of consecutive reductions alternate between
-// two buffers: a block can be at most one reduction ahead of the slowest block's reads.
+// The grid's sum of NV (<= 4) values from the blocks' partials pv (thread 0's), by warp 0 of
+// every block in the same order: got(word) turns a partial's word into a T, which add
+// sums; fin(tot) runs on thread 0 with the totals, and its writes to the block-local scalars
+// are visible to the block's threads on return.  The block has passed a __syncthreads since
+// its last global write.  The partials of consecutive reductions alternate between two
+// buffers: a block can be at most one reduction ahead of the slowest block's reads.
+template <int NV, class T, class Got, class Xor, class Fin>
+__device__ __forceinline__ bool qCollect(const unsigned long long (&pv)[NV], const PpeBuffers& B, QCtl& c, Got&& got,
+                                         Xor&& xorLane, Fin&& fin) {
+    c.gen++;
+    int ok = 1;
+    if (threadIdx.x < 32) {
+        GridBar g = qBar(B, c);
+        unsigned long long* const set = reinterpret_cast<unsigned long long*>(B.partials) + (size_t)(c.gen & 1u) * 4u * gridDim.x;
+        if (threadIdx.x == 0)
+#pragma unroll
+            for (int q = 0; q < NV; q++)
+                asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(set + q * gridDim.x + blockIdx.x), "l"(pv[q]) : "memory");
+        ok = gridWaitWarp0(g);
+        if (ok) {
+            T tot[NV];
+#pragma unroll
+            for (int q = 0; q < NV; q++) tot[q] = got(0ull);
+            // five partials of a lane (160 blocks) in flight at a time
+            for (unsigned b0 = 0; b0 < gridDim.x; b0 += 160) {
+                unsigned long long w[NV][5];
+#pragma unroll
+                for (int q = 0; q < NV; q++)
+#pragma unroll
+                    for (int m = 0; m < 5; m++) {
+                        const unsigned b = b0 + threadIdx.x + 32 * m;
+                        w[q][m] = b < gridDim.x ? ldRelaxed(set + q * gridDim.x + b) : 0ull;
+                    }
+#pragma unroll
+                for (int q = 0; q < NV; q++)
+                    tot[q] += ((got(w[q][0]) + got(w[q][1])) + (got(w[q][2]) + got(w[q][3]))) + got(w[q][4]);
+            }
+#pragma unroll
+            for (int q = 0; q < NV; q++)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) tot[q] += xorLane(tot[q], o);
+            if (threadIdx.x == 0) fin(tot);
+        }
+    }
+    return __syncthreads_and(ok) != 0;
+}
+// Grid sum of NV FP64 values per thread.
 template <int NV, class Fin>
 __device__ __forceinline__ bool qSum(double (&v)[NV], const PpeBuffers& B, QCtl& c, Fin fin) {
     __shared__ double sm[NV * 32];
     blockSum<NV>(v, sm);
-    double* part = B.partials + (size_t)(c.gen & 1u) * 4u * gridDim.x;
-    if (threadIdx.x == 0)
+    unsigned long long pv[NV];
 #pragma unroll
-        for (int q = 0; q < NV; q++) part[q * gridDim.x + blockIdx.x] = v[q];
-    if (!qBarrier(B, c)) return false;
-    if (threadIdx.x < 32) {   // warp 0: lane-strided partial sums, then a fixed shuffle tree
-        double acc[NV];
-#pragma unroll
-        for (int q = 0; q < NV; q++) {
-            double s = 0.0;
-            for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) s += ((volatile double*)part)[q * gridDim.x + b];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            acc[q] = s;
-        }
-        if (threadIdx.x == 0) fin(acc);
-    }
-    __syncthreads();
-    return true;
+    for (int q = 0; q < NV; q++) pv[q] = (unsigned long long)__double_as_longlong(v[q]);
+    return qCollect<NV, double>(
+        pv, B, c, [](unsigned long long w) { return __longlong_as_double((long long)w); },
+        [](double x, int o) { return __shfl_xor_sync(0xffffffffu, x, o); }, fin);
 }
 // The same with float-float per-thread partials (FP32 vectors), reduced in float-float all
 // the way: the warps' shuffle trees, the block's sum of its warps, the block partials (two
-// floats in the same partial slots) and the final sum over the blocks, converted to FP64
-// once for fin.  In FP64 the shuffle trees of every warp and the final sum ran on the FP64
-// pipe (1/64 of the FP32 rate) between the last arrival and the release of every barrier.
+// floats in the same partial slots) and the final sum over the blocks; fin takes the
+// float-float totals.  In FP64 the shuffle trees of every warp and the final sum ran on the
+// FP64 pipe (1/64 of the FP32 rate) between the last arrival and the release of every barrier.
 __device__ __forceinline__ df shflXorDF(df a, int o) {
     return {__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)};
 }
 template <int NV, class Fin>
-__device__ __forceinline__ bool qSumDF(df (&a)[NV], const PpeBuffers& B, QCtl& c, Fin fin) {
+__device__ __forceinline__ bool qSumF2(df (&a)[NV], const PpeBuffers& B, QCtl& c, Fin fin) {
     __shared__ float2 sm[NV * 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
@@ -574,7 +588,7 @@ __device__ __forceinline__ bool qSumDF(df (&a)[NV], const PpeBuffers& B, QCtl& c
         if (lane == 0) sm[q * 32 + w] = make_float2(a[q].h, a[q].l);
     }
     __syncthreads();
-    float2* part = reinterpret_cast<float2*>(B.partials + (size_t)(c.gen & 1u) * 4u * gridDim.x);
+    unsigned long long pv[NV];
     if (w == 0) {
 #pragma unroll
         for (int q = 0; q < NV; q++) {
@@ -582,28 +596,22 @@ __device__ __forceinline__ bool qSumDF(df (&a)[NV], const PpeBuffers& B, QCtl& c
             df s = {x.x, x.y};
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) s += shflXorDF(s, o);
-            if (lane == 0) part[q * gridDim.x + blockIdx.x] = make_float2(s.h, s.l);
+            pv[q] = (unsigned long long)__float_as_uint(s.h) | ((unsigned long long)__float_as_uint(s.l) << 32);
         }
     }
-    if (!qBarrier(B, c)) return false;
-    if (threadIdx.x < 32) {   // warp 0: lane-strided partial sums, then a fixed shuffle tree
+    return qCollect<NV, df>(
+        pv, B, c, [](unsigned long long u) { return df{__uint_as_float((unsigned)u), __uint_as_float((unsigned)(u >> 32))}; },
+        [](df x, int o) { return shflXorDF(x, o); }, fin);
+}
+// ... with the totals in FP64 for fin
+template <int NV, class Fin>
+__device__ __forceinline__ bool qSumDF(df (&a)[NV], const PpeBuffers& B, QCtl& c, Fin fin) {
+    return qSumF2<NV>(a, B, c, [&](const df* t) {
         double tot[NV];
 #pragma unroll
-        for (int q = 0; q < NV; q++) {
-            df s = dfF(0.f);
-            for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) {
-                // both floats in one volatile 8-byte load (x at the lower address)
-                const unsigned long long u = ((volatile unsigned long long*)part)[q * gridDim.x + b];
-                s += df{__uint_as_float((unsigned)u), __uint_as_float((unsigned)(u >> 32))};
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += shflXorDF(s, o);
-            tot[q] = dD(s);
-        }
-        if (threadIdx.x == 0) fin(tot);
-    }
-    __syncthreads();
-    return true;
+        for (int q = 0; q < NV; q++) tot[q] = dD(t[q]);
+        fin(tot);
+    });
 }
 
 // FP64 per-thread partials summed as float-float from the warp level on (each partial split
@@ -805,7 +813,7 @@ __device__ __forceinline__ float h16Row(const PpeBuffers& B, const float* y, int
 // TS_CH slices into a TS_NS-stage ring, up to TS_NS - 1 chunks ahead of the threads, which
 // read their row's entries from shared memory and gather z.  The engine keeps the HBM
 // stream in flight independently of the threads' gather latencies.  Every mbarrier wait
-// is bounded; a wait that runs out sets the abort word (see qBarrier) and the block stops
+// is bounded; a wait that runs out sets the abort word (mps_grid.cuh) and the block stops
 // consuming, drains the copies it issued (again bounded) and returns at the next barrier.
 #define TS_CH 8
 #define TS_NS 3
@@ -1136,6 +1144,35 @@ __device__ __forceinline__ void forOwnL(const RowSet& s, F&& f) {
     for (int m = 0; m < cnt; m++) f(m * (int)blockDim.x + (int)threadIdx.x, rowAt(s, m));
 }
 
+// Scalars of a mixed solve from the sums r.r, b.b (LEARNED: also r.q and q.q) of its start.
+template <bool LEARNED>
+__device__ __forceinline__ void mxStart(QLocal& qL, const double* t, double tol, double eta2) {
+    double* const qS = qL.scal;
+    int* const qF = qL.flag;
+    double th = 0.0, rr = t[0];
+    if (LEARNED) {
+        // a non-finite correction keeps the start x (theta = 0, its residual as is)
+        const double rq = t[LEARNED ? 2 : 0], qq = t[LEARNED ? 3 : 0];
+        if (qq > 0.0 && qq < 1.0 / 0.0 && rq == rq && fabs(rq) < 1.0 / 0.0) {
+            th = rq / qq;
+            rr = fmax(t[0] - th * rq, 0.0);
+        }
+    }
+    qS[S_OMEGA] = th;
+    qS[S_RR] = rr;
+    qS[S_BB] = t[1];
+    double thr = tol * tol * t[1];
+    if (thr < 2.2250738585072014e-308) thr = 2.2250738585072014e-308;
+    qS[S_THR] = thr;
+    qS[S_SCALE] = sqrt(rr / (t[1] > 0 ? t[1] : 1.0));
+    qS[S_SQRT] = sqrt(rr);
+    qS[S_INV] = 1.0 / sqrt(rr);
+    qS[S_ETA2] = fmax(eta2, 0.25 * thr / rr);
+    qF[0] = (t[1] == 0.0 || rr < thr) ? 1 : 0;
+    qF[1] = 0;
+    qF[3] = 0;
+    if (!(rr == rr)) { qF[0] = 1; qF[2] = 1; }
+}
 // Set-up of the shared-memory mixed solve: FP64 residual of the warm start, ||r||^2 and
 // ||b||^2 and the solver scalars; with a learned correction c (B.cdir, with q = A c in
 // B.cq) the residual r_e of the start x_e is already in B.r (the learned start's features
@@ -1167,31 +1204,7 @@ __device__ __forceinline__ bool mxSetup(const PpeBuffers& B, const RowSet& rs, Q
             v[1] += bi * bi;
         });
     }
-    if (!qSum<LEARNED ? 4 : 2>(v, B, c, [&](const double* t) {
-            double th = 0.0, rr = t[0];
-            if (LEARNED) {
-                // a non-finite correction keeps the start x (theta = 0, its residual as is)
-                const double rq = t[LEARNED ? 2 : 0], qq = t[LEARNED ? 3 : 0];
-                if (qq > 0.0 && qq < 1.0 / 0.0 && rq == rq && fabs(rq) < 1.0 / 0.0) {
-                    th = rq / qq;
-                    rr = fmax(t[0] - th * rq, 0.0);
-                }
-            }
-            qS[S_OMEGA] = th;
-            qS[S_RR] = rr;
-            qS[S_BB] = t[1];
-            double thr = tol * tol * t[1];
-            if (thr < 2.2250738585072014e-308) thr = 2.2250738585072014e-308;
-            qS[S_THR] = thr;
-            qS[S_SCALE] = sqrt(rr / (t[1] > 0 ? t[1] : 1.0));
-            qS[S_SQRT] = sqrt(rr);
-            qS[S_INV] = 1.0 / sqrt(rr);
-            qS[S_ETA2] = fmax(eta2, 0.25 * thr / rr);
-            qF[0] = (t[1] == 0.0 || rr < thr) ? 1 : 0;
-            qF[1] = 0;
-            qF[3] = 0;
-            if (!(rr == rr)) { qF[0] = 1; qF[2] = 1; }
-        }))
+    if (!qSum<LEARNED ? 4 : 2>(v, B, c, [&](const double* t) { mxStart<LEARNED>(qL, t, tol, eta2); }))
         return false;
     if (LEARNED && vd(qS + S_OMEGA) != 0.0) {   // x += theta c, r -= theta q on the thread's own rows
         const double th = vd(qS + S_OMEGA);
@@ -1688,6 +1701,331 @@ __global__ void __launch_bounds__(QBC, 1) k_cg_own(Dev d, PpeBuffers B, double t
     qStore(B, qL);
 }
 
+// ------------------------------------------------------------------ resident matrices
+// The solvers of systems with at most one row per thread of the grid (152 x RBS = 116,736
+// rows): L lanes (1, 2, 4 or 8: as many as fit) share a row, lane l holding the entries l,
+// l + L, ..., and the first `cap` entries of every lane stay in the block's shared memory from the
+// first iteration to the last (slot e RBS + thread), the others, if any, are streamed.  A
+// row's vector elements are registers of its lanes.  An iteration then reads nothing but z, in
+// one trip to the L2 for all entries of a lane, where the streaming kernels take two dependent
+// trips per eight entries; below a few thousand rows per SM these latencies and the grid
+// sums are the whole time.  More than four lanes would lengthen the FP64 solver: its vector
+// operations cost a warp the same for one row as for 32.
+// Whole solves per step, k_cg_own / k_mx_own before and now: plain FP64 CG at 2,000 rows (27
+// iterations) 0.355 -> 0.242 ms, at 6,912 (25) 0.391 -> 0.252 ms, mixed solver to 1e-10 at
+// 108,000 rows (39 iterations, 1.75 refinements) 0.65 -> 0.38 ms.  Above one row per
+// thread the matrix of a block no longer fits: k_cg_own and k_mx_own stream it.
+#define RBS 768
+#define RES_CAP32 36   // entries per lane: 36 x 768 x 8 B = 216 KB
+#define RES_CAP64 24   // 24 x 768 x 12 B = 216 KB
+
+struct ResRow {
+    int i, l, L, len;   // row (-1: none), lane of the row, lanes per row, entries of the row
+    int most;           // entries of the busiest lane of the warp
+    bool any;           // the warp has a row
+    size_t base, stride;
+};
+__device__ __forceinline__ ResRow resRow(const PpeBuffers& B, int n, int L) {
+    ResRow r;
+    const int G = gridDim.x, R = (n + G - 1) / G, g = threadIdx.x / L;
+    r.L = L;
+    r.l = threadIdx.x & (L - 1);
+    const int i = blockIdx.x * R + g;
+    r.i = (g < R && i < n) ? i : -1;
+    r.len = r.i >= 0 ? __ldg(B.rowLen + r.i) : 0;
+    r.any = __any_sync(0xffffffffu, r.i >= 0);
+    r.most = __reduce_max_sync(0xffffffffu, (r.len - r.l + L - 1) / L);
+    r.base = r.i >= 0 ? ellBase(B, r.i) : 0;
+    r.stride = B.ellStride;
+    return r;
+}
+// Sum of the row's off-diagonal products with x over all its lanes (the same in each): lane
+// entries [0, cap) from shared memory (sc, sv), the others from the ELL arrays.
+template <class T>
+__device__ __forceinline__ T resDot(const ResRow& r, const int* sc, const T* sv, int cap, const int* col, const T* val,
+                                    const T* x) {
+    T a[4] = {T(0), T(0), T(0), T(0)};
+    const int held = (min(r.most, cap) + 3) & ~3;   // cap is a multiple of 4; slots past a row's end hold zeros
+    int e = 0;
+    for (; e + 8 <= held; e += 8) {
+        int c[8];
+        T v[8], g[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) { c[u] = sc[(e + u) * RBS + threadIdx.x]; v[u] = sv[(e + u) * RBS + threadIdx.x]; }
+#pragma unroll
+        for (int u = 0; u < 8; u++) g[u] = x[c[u]];
+#pragma unroll
+        for (int u = 0; u < 8; u++) a[u & 3] += v[u] * g[u];
+    }
+    if (e < held) {
+        int c[4];
+        T v[4], g[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) { c[u] = sc[(e + u) * RBS + threadIdx.x]; v[u] = sv[(e + u) * RBS + threadIdx.x]; }
+#pragma unroll
+        for (int u = 0; u < 4; u++) g[u] = x[c[u]];
+#pragma unroll
+        for (int u = 0; u < 4; u++) a[u] += v[u] * g[u];
+        e += 4;
+    }
+    for (; e < r.most; e += 4) {
+        int c[4];
+        T v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int k = r.l + (e + u) * r.L;
+            const bool ok = k < r.len;
+            c[u] = ok ? ldStream(col + r.base + (size_t)k * r.stride) : -1;
+            v[u] = ok ? ldStream(val + r.base + (size_t)k * r.stride) : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (c[u] >= 0) a[u] += v[u] * x[c[u]];
+    }
+    T s = (a[0] + a[1]) + (a[2] + a[3]);
+    for (int o = r.L >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+template <class T>
+__device__ __forceinline__ void resLoad(const ResRow& r, int* sc, T* sv, int cap, const int* col, const T* val) {
+    const int held = min((r.most + 3) & ~3, cap);
+    for (int e = 0; e < held; e++) {
+        const int k = r.l + e * r.L;
+        const bool ok = k < r.len;
+        sc[e * RBS + threadIdx.x] = ok ? ldStream(col + r.base + (size_t)k * r.stride) : max(r.i, 0);
+        sv[e * RBS + threadIdx.x] = ok ? ldStream(val + r.base + (size_t)k * r.stride) : T(0);
+    }
+}
+
+// Plain FP64 Jacobi-PCG: method, stopping rule and reports of k_cg_own.
+__global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double tol, int maxIter, int L, int cap) {
+    __shared__ QLocal qL;
+    qInit(qL);
+    double* const qS = qL.scal;
+    int* const qF = qL.flag;
+    extern __shared__ __align__(128) unsigned char dynSmem[];
+    double* const sv = reinterpret_cast<double*>(dynSmem);
+    int* const sc = reinterpret_cast<int*>(sv + (size_t)cap * RBS);
+    const ResRow R = resRow(B, liveN(d), L);
+    const bool own = R.i >= 0 && R.l == 0;
+    QCtl c = {0u};
+    resLoad(R, sc, sv, cap, B.col, B.val);
+    double x = 0.0, r = 0.0, z = 0.0, p = 0.0, ap = 0.0, di = 0.0, dg = 0.0;
+    {
+        double v[3] = {0.0, 0.0, 0.0};
+        if (R.any) {
+            const double q = resDot<double>(R, sc, sv, cap, B.col, B.val, B.x);
+            if (R.i >= 0) {
+                dg = __ldg(B.diag + R.i);
+                di = 1.0 / dg;
+                x = B.x[R.i];
+                const double bi = B.b[R.i];
+                r = bi - (dg * x + q);
+                z = r * di;
+                if (own) {
+                    B.z[R.i] = z;
+                    v[0] = r * z; v[1] = r * r; v[2] = bi * bi;
+                }
+            }
+        }
+        if (!qSum<3>(v, B, c, [&](const double* t) {
+                qS[S_RZ] = t[0]; qS[S_RR] = t[1]; qS[S_BB] = t[2];
+                double thr = tol * tol * t[2];
+                if (thr < 2.2250738585072014e-308) thr = 2.2250738585072014e-308;
+                qS[S_THR] = thr;
+                qS[S_SCALE] = sqrt(t[1] / (t[2] > 0 ? t[2] : 1.0));
+                qF[0] = (t[2] == 0.0 || t[1] < thr) ? 1 : 0;
+                qF[1] = 0;
+                if (!(t[0] == t[0]) || !(t[1] == t[1])) { qF[0] = 1; qF[2] = 1; }
+            }))
+            return;
+    }
+    int it = 0;
+    while (!vi(qF) && it < maxIter) {
+        {   // Ap = A z + beta Ap, p = z + beta p, p.Ap
+            double v[1] = {0.0};
+            if (R.any) {
+                const double beta = it ? vd(qS + S_BETA) : 0.0;
+                const double q = dg * z + resDot<double>(R, sc, sv, cap, B.col, B.val, B.z);
+                ap = it ? q + beta * ap : q;
+                p = it ? z + beta * p : z;
+                if (own) v[0] = p * ap;
+            }
+            if (!qSumD<1>(v, B, c, [&](const double* t) { qS[S_PAP] = t[0]; qS[S_ALPHA] = qS[S_RZ] / t[0]; }))
+                return;
+        }
+        {   // x += alpha p, r -= alpha Ap, z = M^-1 r; r.z, r.r
+            double v[2] = {0.0, 0.0};
+            if (R.any) {
+                const double alpha = vd(qS + S_ALPHA);
+                x += alpha * p;
+                r -= alpha * ap;
+                z = r * di;
+                if (own) {
+                    B.z[R.i] = z;
+                    v[0] = r * z; v[1] = r * r;
+                }
+            }
+            if (!qSumD<2>(v, B, c, [&](const double* t) {
+                    qF[1] += 1;
+                    qS[S_RR] = t[1];
+                    qS[S_BETA] = t[0] / qS[S_RZ];
+                    qS[S_RZ] = t[0];
+                    if (t[1] < qS[S_THR]) qF[0] = 1;
+                    if (!(t[1] == t[1])) { qF[0] = 1; qF[2] = 1; }
+                }))
+                return;
+        }
+        it++;
+    }
+    if (own) B.x[R.i] = x;
+    if (!qBarrier(B, c)) return;
+    {   // FP64 residual of the result
+        double v[1] = {0.0};
+        if (R.any) {
+            const double q = resDot<double>(R, sc, sv, cap, B.col, B.val, B.x);
+            if (own) {
+                const double t = B.b[R.i] - (dg * x + q);
+                v[0] = t * t;
+            }
+        }
+        qSum<1>(v, B, c, [&](const double* t) { qS[S_RR] = t[0]; });
+    }
+    qStore(B, qL);
+}
+
+// Mixed FP32/FP64 solver: method, stopping rules and reports of k_mx_own (LEARNED as there:
+// the residual of the start is in B.r, its correction and their product in B.cdir and B.cq).
+template <bool LEARNED>
+__global__ void __launch_bounds__(RBS, 1) k_mx_res(Dev d, PpeBuffers B, double tol, int maxIter, double eta2, int L, int cap) {
+    __shared__ QLocal qL;
+    __shared__ df rz, stop2;   // inner solve: r.z, and the squared residual norm that ends it
+    qInit(qL);
+    double* const qS = qL.scal;
+    int* const qF = qL.flag;
+    extern __shared__ __align__(128) unsigned char dynSmem[];
+    float* const sv = reinterpret_cast<float*>(dynSmem);
+    int* const sc = reinterpret_cast<int*>(sv + (size_t)cap * RBS);
+    const ResRow R = resRow(B, liveN(d), L);
+    const bool own = R.i >= 0 && R.l == 0;
+    QCtl c = {0u};
+    resLoad(R, sc, sv, cap, B.col, B.valf);
+    // FP64 residual of B.x, whose element of the row is x
+    double x = 0.0, r = 0.0;
+    auto residual = [&]() {
+        const double q = resDot<double>(R, nullptr, nullptr, 0, B.col, B.val, B.x);
+        return R.i >= 0 ? B.b[R.i] - (__ldg(B.diag + R.i) * x + q) : 0.0;
+    };
+    float dgf = 0.f, dif = 0.f;
+    {
+        double v[LEARNED ? 4 : 2] = {};
+        if (R.any) {
+            if (R.i >= 0) { x = B.x[R.i]; dgf = __ldg(B.diagf + R.i); dif = __ldg(B.diagInvf + R.i); }
+            if (LEARNED) r = R.i >= 0 ? B.r[R.i] : 0.0;
+            else r = residual();
+            if (own) {
+                const double bi = B.b[R.i];
+                v[0] = r * r;
+                v[1] = bi * bi;
+                if (LEARNED) {
+                    const double q = (double)__ldg(B.cq + R.i);
+                    v[LEARNED ? 2 : 0] = r * q;
+                    v[LEARNED ? 3 : 0] = q * q;
+                }
+            }
+        }
+        if (!qSum<LEARNED ? 4 : 2>(v, B, c, [&](const double* t) { mxStart<LEARNED>(qL, t, tol, eta2); })) return;
+        if (LEARNED) {
+            const double th = vd(qS + S_OMEGA);
+            if (R.i >= 0 && th != 0.0) {
+                x += th * (double)__ldg(B.cdir + R.i);
+                r -= th * (double)__ldg(B.cq + R.i);
+                if (own) B.x[R.i] = x;
+            }
+        }
+    }
+    int total = 0, refine = 0;
+    while (!vi(qF) && total < maxIter && refine <= 20) {
+        float xf = 0.f, rf = 0.f, zf = 0.f, pf = 0.f, apf = 0.f;
+        {   // inner start: r_f = r / ||r||, z = M^-1 r_f, x_f = 0
+            df a[2] = {dfF(0.f), dfF(0.f)};
+            if (R.any) {
+                rf = (float)(r * vd(qS + S_INV));
+                zf = rf * dif;
+                if (own) {
+                    B.zf[R.i] = zf;
+                    a[0] = prod2(rf, zf);
+                    a[1] = prod2(rf, rf);
+                }
+            }
+            if (!qSumF2<2>(a, B, c, [&](const df* t) {
+                    rz = t[0];
+                    stop2 = t[1] * dfD(qS[S_ETA2]);
+                    qF[3] = 0;
+                }))
+                return;
+        }
+        int inner = 0;
+        while (true) {
+            {   // Ap = A z + beta Ap, p = z + beta p, p.Ap
+                df a[1] = {dfF(0.f)};
+                if (R.any) {
+                    const float beta = inner ? vf(qL.scalf + SF_BETA) : 0.f;
+                    const float q = dgf * zf + resDot<float>(R, sc, sv, cap, B.col, B.valf, B.zf);
+                    apf = inner ? q + beta * apf : q;
+                    pf = inner ? zf + beta * pf : zf;
+                    if (own) a[0] = prod2(pf, apf);
+                }
+                if (!qSumF2<1>(a, B, c, [&](const df* t) { qL.scalf[SF_ALPHA] = divDF(rz, t[0]).h; })) return;
+            }
+            {   // x_f += alpha p, r -= alpha Ap, z = M^-1 r; r.z, r.r
+                const float alpha = vf(qL.scalf + SF_ALPHA);
+                df a[2] = {dfF(0.f), dfF(0.f)};
+                xf += alpha * pf;
+                rf -= alpha * apf;
+                zf = rf * dif;
+                if (own) {
+                    B.zf[R.i] = zf;
+                    a[0] = prod2(rf, zf);
+                    a[1] = prod2(rf, rf);
+                }
+                if (!qSumF2<2>(a, B, c, [&](const df* t) {
+                        qF[1] += 1;
+                        qL.scalf[SF_BETA] = divDF(t[0], rz).h;
+                        rz = t[0];
+                        if (t[1] < stop2 || !(t[1].h == t[1].h)) qF[3] = 1;
+                    }))
+                    return;
+            }
+            inner++;
+            if (vi(qF + 3) || total + inner >= maxIter || inner >= 400) break;
+        }
+        total += inner;
+        {   // x += ||r|| x_f (FP64), then the FP64 residual r = b - A x
+            if (R.any) x += vd(qS + S_SQRT) * (double)xf;
+            if (own) B.x[R.i] = x;
+            if (!qBarrier(B, c)) return;
+            double v[1] = {0.0};
+            if (R.any) {
+                r = residual();
+                if (own) v[0] = r * r;
+            }
+            if (!qSum<1>(v, B, c, [&](const double* t) {
+                    qS[S_RR] = t[0];
+                    qS[S_SQRT] = sqrt(t[0]);
+                    qS[S_INV] = 1.0 / sqrt(t[0]);
+                    qS[S_ETA2] = fmax(eta2, 0.25 * qS[S_THR] / t[0]);
+                    if (t[0] < qS[S_THR]) qF[0] = 1;
+                    if (!(t[0] == t[0])) { qF[0] = 1; qF[2] = 1; }
+                    qF[4] += 1;
+                }))
+                return;
+        }
+        refine++;
+    }
+    qStore(B, qL);
+}
+
 // Jacobi-preconditioned BiCGSTAB (solver_type 1: Eigen::BiCGSTAB, src/MpsPressure.cpp:448-468;
 // van der Vorst 1992 with the preconditioner on the right), in one cooperative launch: per
 // iteration two SpMVs and five grid synchronisations (y and z must be complete before their
@@ -1818,7 +2156,7 @@ __global__ void __launch_bounds__(QBC, 1) k_bicgstab(Dev d, PpeBuffers B, double
 // kind: 0 plain FP64, 1 mixed, 2 mixed with the matrix-free inner operator, 3 mixed with
 // the compact scaled inner operator, 4 mixed with the staged tiles, 5 mixed with the
 // pipelined inner CG, 6 BiCGSTAB, 7 mixed with block-owned rows (one block per SM), 8 plain
-// FP64 with block-owned rows (one block per SM)
+// FP64 with block-owned rows (one block per SM), 9 resident matrices (one block per SM)
 int ppePersistentGrid(int kind) {
     int dev = 0, sms = 0, coop = 0, per = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
@@ -1837,6 +2175,14 @@ int ppePersistentGrid(int kind) {
         const int dyn = OWN64_CAPMAX * 24;
         if (cudaFuncSetAttribute(k_cg_own, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess) return 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cg_own, QBC, dyn) != cudaSuccess || per <= 0) return 0;
+        return sms;
+    }
+    if (kind == 9) {   // resident matrices, one block per SM
+        for (const void* f : {(const void*)k_cg_res, (const void*)k_mx_res<false>, (const void*)k_mx_res<true>}) {
+            const int dyn = f == (const void*)k_cg_res ? RES_CAP64 * RBS * 12 : RES_CAP32 * RBS * 8;
+            if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess) return 0;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, RBS, dyn) != cudaSuccess || per <= 0) return 0;
+        }
         return sms;
     }
     if (kind == 4) {
@@ -1897,6 +2243,14 @@ int ppeSolveBicgstab(const Dev& d, const PpeBuffers& B, double tol, int maxIter,
     return finishPersistent(B, s, iters, nullptr, relres, relres0);
 }
 
+// Lanes per row of the resident solvers: 4, 2 or 1, as many as give every row of `rows` its
+// lanes in one round of the grid; 0: too many rows.
+static int resLanes(int rows, int grid) {
+    for (int L = 4; L; L >>= 1)
+        if (rows <= grid * (RBS / L)) return L;
+    return 0;
+}
+
 int ppeSolvePersistent(const Dev& d, const PpeBuffers& B, int mixed, double tol, int maxIter, cudaStream_t s,
                        int* iters, int* refinements, double* relres, double* relres0, Prof* prof) {
     int grid = !mixed ? B.pgridCg
@@ -1921,6 +2275,24 @@ int ppeSolvePersistent(const Dev& d, const PpeBuffers& B, int mixed, double tol,
     double t = tol, eta2 = 1e-6 * 1e-6;
     int mi = maxIter;
     void* args[6] = {&dd, &bb, &t, &mi, &eta2, nullptr};
+    const int lanes = B.matfree == 0 && !B.ownOff && B.pgridRes > 0 ? resLanes(d.N0, B.pgridRes) : 0;
+    if (lanes) {
+        // at most one row per thread: the matrix stays in shared memory.  The rows are spread
+        // over all SMs (the FP64 pipe and the latencies are per SM), 16 to a block at least
+        const int need = (B.K + lanes - 1) / lanes;
+        int L = lanes, cap = std::min((need + 3) / 4 * 4, mixed ? RES_CAP32 : RES_CAP64);
+        const int g = std::min(B.pgridRes, (d.N0 + 15) / 16);
+        void* aPlain[6] = {&dd, &bb, &t, &mi, &L, &cap};
+        void* aMixed[7] = {&dd, &bb, &t, &mi, &eta2, &L, &cap};
+        const void* fn = !mixed ? (const void*)k_cg_res : B.cdir ? (const void*)k_mx_res<true> : (const void*)k_mx_res<false>;
+        if (pr) prof->begin(PROF_PPE_SOLVE, s);
+        cudaError_t e = cudaLaunchCooperativeKernel(fn, g, RBS, mixed ? aMixed : aPlain,
+                                                    (size_t)cap * RBS * (mixed ? 8 : 12), s);
+        if (pr) prof->end(s);
+        if (e != cudaSuccess) return MPSGPU_ERR_CUDA;
+        countLaunch(1);
+        return finishPersistent(B, s, iters, refinements, relres, relres0);
+    }
     if (!mixed && !B.ownOff && B.pgridOwn64 > 0 && B.ownCap64 > 0) {
         // block-owned rows: r, p, Ap of each block in its shared memory
         int cap = B.ownCap64;
