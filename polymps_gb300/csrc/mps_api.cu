@@ -179,9 +179,8 @@ static void ensureList(mpsgpu_t h) {
     if (h->listValid) return;
     if (h->prof.on) h->prof.begin(PROF_NEIGHBOR_LIST, h->s);
     if (h->skinValid) {
-        if (df32(h)) launchNeighborFilterDF(h->d, h->s);
-        else launchNeighborFilter(h->d, h->s);
-        countLaunch(df32(h) ? 5 : 4);   // FP32 copies (2), skin check, filter (DF32: listed + unlisted particles)
+        launchNeighborFilter(h->d, h->s, !df32(h));
+        countLaunch(5);   // FP32 copies (2), skin check, filter, scan of the particles it left
     } else {
         if (df32(h)) launchNeighborListDF(h->d, h->s);
         else launchNeighborList(h->d, h->s);
@@ -470,7 +469,7 @@ static int runOpBody(mpsgpu_t h, int op) {
                 // particle that moved out of its skin or scan window, or any particle after a
                 // removal, scans the buckets), its masks, then list sweeps
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(PROF_NEIGHBOR_LIST, s, false); }
-                launchNeighborFilterDF(d, s);
+                launchNeighborFilter(d, s, false);
                 launchSideMasksDF(d, s);
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(MPS_OP_SHIFTING, s, false); }
                 launchShiftingListDF(d, s);
@@ -485,8 +484,8 @@ static int runOpBody(mpsgpu_t h, int op) {
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(MPS_OP_SHIFTING, s, false); }
                 launchShifting(d, s, true);
                 invalidate();
-                // posf + cell copy, skin check, filter; then the sweeps and applies
-                countLaunch(4 + (P.shiftingType == 1 ? 2 : (P.wallType == 1 ? 6 : 3)));
+                // posf + cell copy, skin check, filter (2); then the sweeps and applies
+                countLaunch(5 + (P.shiftingType == 1 ? 2 : (P.wallType == 1 ? 6 : 3)));
                 h->opSkipped = true;
             } else {
                 if (x) launchShiftingDF(d, s); else launchShifting(d, s, false);
@@ -772,6 +771,7 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
     A(d.posSkin, n);
     A(d.skinCell, n);
     A(d.skinFlag, 2);
+    d.rescan = d.skinFlag + 1;
     A(d.corrDF, (size_t)9 * n);
     A(d.corrDFn, (size_t)9 * n);
     A(d.c1n, n);
@@ -814,6 +814,9 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
         d.bandHi = (float)(d.reMax2 + band(d.reMax2));
         d.bandHiS = (float)(p->reS2 + band(p->reS2));
         d.bandHiL = (float)(p->reL2 + band(p->reL2));
+        d.bandLoS = (float)(p->reS2 - band(p->reS2));
+        d.bandLoL = (float)(p->reL2 - band(p->reL2));
+        d.sideBand = (float)(band(d.reMax2) + band(3.3 * 3.3 * d.reMax2));
         d.bandHiColl = (float)(p->distCollisionLimit2 + band(p->distCollisionLimit2));
         // start-of-step skin list: reMax + 0.15 l0 (covers steps that move no particle by
         // more than 0.075 l0 from its start position; otherwise the list is rebuilt)
@@ -847,6 +850,8 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
         k.reS2 = hd(p->reS2); k.reL2 = hd(p->reL2); k.reMax2 = hd(d.reMax2);
         k.coll2 = hd(p->distCollisionLimit2);
         double mu = p->KNM_VS1 * p->DNS_FL1, rho = p->DNS_FL1;
+        d.neuWall64 = (2.0 * mu) / rho;
+        d.neuFluid64 = (2.0 * mu * mu / (mu + mu)) / rho;
         k.neuW = hd((2.0 * mu) / rho);
         k.neuF = hd((2.0 * mu * mu / (mu + mu)) / rho);
         k.neuWall = hd(((mu + mu) > p->epsilonZero ? 2.0 * mu * mu / (mu + mu) : 0.0) / p->DNS_FL1);

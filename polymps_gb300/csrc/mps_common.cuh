@@ -112,6 +112,7 @@ struct Dev {
     float4* posSkin;                // start positions (hi parts)
     long long* skinCell;            // bucket coordinates of the start position (scan window)
     int* skinFlag;                  // [0] set: the skin list no longer covers the list
+    int* rescan;                    // particles the list filter left to the bucket scan
     float skinR2;                   // FP32 squared radius of the skin list (with the band)
     float skinMove2;                // FP32 squared displacement bound (half the skin, less the band)
     float invSidef, epsf;           // FP32 copies of invBucketSide and epsilonZero (bucket fast path)
@@ -141,6 +142,9 @@ struct Dev {
     int *nearList, *nearCount;      // fluid particles near the polygon wall (compacted)
     double reMax2;                  // list radius^2 = max(reS^2, reL^2)
     float bandHiS, bandHiL;         // FP32 prefilter upper bounds for the reS / reL balls
+    float bandLoS, bandLoL;         // ... and the lower bounds below which an entry is inside
+    float sideBand;                 // FP32 mirror-side test: certain beyond this difference
+    double neuWall64, neuFluid64;   // kinematic factors of a wall and of a fluid neighbour
     float bandHiColl;               // ... and for the collision distance
     // polygon mesh and wall tables
     int ntri;

@@ -44,10 +44,10 @@ void launchFillCache(const Dev& d, cudaStream_t s);
 
 // mps_ops.cu
 void launchViscosity(const Dev& d, cudaStream_t s);
-// FP64 tier over the start-of-step skin list (built by launchSkinListDF): the viscosity
-// sweep, and the list of the current positions with its weights filtered from it
+// over the start-of-step skin list (built by launchSkinListDF): the FP64 viscosity sweep, and
+// the list of the current positions filtered from it (weights: the FP64 tier's cache)
 void launchViscosityList(const Dev& d, cudaStream_t s);
-void launchNeighborFilter(const Dev& d, cudaStream_t s, bool weights = true);   // the FP64 list from the skin list
+void launchNeighborFilter(const Dev& d, cudaStream_t s, bool weights);
 void launchAddGravity(const Dev& d, cudaStream_t s);
 void launchPredict(const Dev& d, cudaStream_t s);
 void launchOutOfDomain(const Dev& d, int* flags, int* counter, cudaStream_t s);
@@ -92,11 +92,9 @@ void launchUpdateBCArc(const Dev& d, cudaStream_t s);
 void launchCollisionDPC(const Dev& d, cudaStream_t s);
 // velocity divergence of the PND + div u source (list based, FP64; + the polygon-wall term)
 void launchVelDivergence(const Dev& d, cudaStream_t s);
-// start-of-step list with a skin: build, viscosity over it, and the list of the current
-// positions filtered from it
+// start-of-step list with a skin: build, and the DF32 viscosity over it
 void launchSkinListDF(const Dev& d, cudaStream_t s);
 void launchViscosityListDF(const Dev& d, cudaStream_t s);
-void launchNeighborFilterDF(const Dev& d, cudaStream_t s);
 // the skin list's validity flag for the current positions (moved more than half the skin)
 void launchSkinCheck(const Dev& d, cudaStream_t s);
 void launchShiftVelApply(const Dev& d, cudaStream_t s);

@@ -1,0 +1,179 @@
+// mps_lanes.cuh — L lanes of a warp per particle for the neighbour sweeps, and the FP32 tests
+// that settle most of a sweep's decisions before any FP64 operation.
+//
+// GB300 issues FP64 at 1/64 of the FP32 rate, so an FP64 sweep is bound by the FP64
+// operations its warps issue, whether one lane or all 32 need them.  The sweeps therefore run
+// in two phases: the FP32 copies decide each row entry (an entry inside the rounding band of
+// a decision takes the reference's FP64 expression, out of line) and leave a bit mask; then
+// the FP64 sums walk the set bits, so the lanes of a warp stay in step through them.
+#pragma once
+#include "mps_common.cuh"
+
+// Lanes per particle for n particles.  From 40k particles on the sweeps are bound by the FP64
+// pipe and one lane per particle keeps its lanes busiest; below, the chip is not full and a
+// row's chain of gathers and FP64 sums is the time of the sweep, which L lanes shorten.  The
+// viscosity sweep with 1, 4 and 8 lanes: 6.9k particles 64 / 28 / 22 us, 18.5k 63 / 44 / 51 us,
+// 32k 74 / 68 / 77 us, 55k 94 / 110 / 122 us, 108k 166 / 200 / 231 us.
+static inline int lanesFor(int n) { return n >= 40000 ? 1 : (n >= 12000 ? 4 : 8); }
+// Launch a kernel template over its lane count: KERNEL(L) expands to the launch for L lanes.
+#define MPS_FOR_LANES(n, KERNEL)                                                                  \
+    do {                                                                                          \
+        switch (lanesFor(n)) {                                                                    \
+            case 1: KERNEL(1); break;                                                             \
+            case 4: KERNEL(4); break;                                                             \
+            default: KERNEL(8); break;                                                            \
+        }                                                                                         \
+    } while (0)
+
+// Row and lane of the calling thread; the lanes of a row are neighbours within one warp.
+template <int L>
+__device__ __forceinline__ int laneRow() { return (int)((blockIdx.x * blockDim.x + threadIdx.x) / L); }
+template <int L>
+__device__ __forceinline__ int laneOf() { return (int)(threadIdx.x & (L - 1)); }
+template <int L>
+__device__ __forceinline__ unsigned laneGroup() {
+    return L == 1 ? 1u << (threadIdx.x & 31) : ((1u << L) - 1u) << (threadIdx.x & 31 & ~(L - 1));
+}
+// Sums over the lanes of a row: every lane of the group gets the same bits (a symmetric tree).
+template <int L>
+__device__ __forceinline__ double laneSum(double v) {
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1) v += __shfl_xor_sync(laneGroup<L>(), v, o);
+    return v;
+}
+template <int L>
+__device__ __forceinline__ int laneSum(int v) {
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1) v += __shfl_xor_sync(laneGroup<L>(), v, o);
+    return v;
+}
+template <int L>
+__device__ __forceinline__ Mask laneOr(Mask m) {
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1) {
+        m.lo |= __shfl_xor_sync(laneGroup<L>(), m.lo, o);
+        m.hi |= __shfl_xor_sync(laneGroup<L>(), m.hi, o);
+    }
+    return m;
+}
+// The entries of a mask that lane l takes: k with k mod L == l.
+template <int L>
+__device__ __forceinline__ Mask laneShare(Mask m, int l) {
+    if (L == 1) return m;
+    const unsigned long long p = (L == 2 ? 0x5555555555555555ull : L == 4 ? 0x1111111111111111ull : 0x0101010101010101ull) << l;
+    m.lo &= p; m.hi &= p;
+    return m;
+}
+// Set bits below bit k.
+__device__ __forceinline__ int maskRank(const Mask& m, int k) {
+    if (k < 64) return __popcll(m.lo & ((1ull << k) - 1ull));
+    return __popcll(m.lo) + __popcll(m.hi & ((1ull << (k - 64)) - 1ull));
+}
+
+// a < b for non-negative doubles by their bits (NaN compares false, as in FP64): two integer
+// comparisons instead of one on the FP64 pipe.
+__device__ __forceinline__ bool lessPos(double a, double b) {
+    return (unsigned long long)__double_as_longlong(a) < (unsigned long long)__double_as_longlong(b);
+}
+
+// The reference's FP64 decisions, out of line: inlined, the compiler predicates them into every
+// entry and their FP64 operations then run for all of them.
+static __device__ __noinline__ bool pairInsideExact(const dvec4* pos, int j, int i, double R2) {
+    return pairOf(pos[j], pos[i]).d2 < R2;
+}
+static __device__ __noinline__ bool pairSideExact(const dvec4* pos, const dvec4* mirror, int j, int i) {
+    const dvec4 pj = pos[j];
+    return pairOf(pj, pos[i]).d2 < pairMirror(pj, mirror[i]).dm2;
+}
+
+// FP32 squared distance of two position copies
+__device__ __forceinline__ float dist2f(float4 a, float4 b) {
+    const float ex = a.x - b.x, ey = a.y - b.y, ez = a.z - b.z;
+    return ex * ex + ey * ey + ez * ez;
+}
+// The mirror-side test of particle i (SideCtx) with the mirror's FP32 copy: |x_j - x_i|^2 and
+// |x_j - m_i|^2 in FP32 are each within their band of the FP64 values (the second up to
+// 3.3 reMax, beyond which the test is off), so a difference above the sum of both bands
+// (sideBand) decides.
+struct SideF {
+    float4 m;
+    bool check;
+};
+__device__ __forceinline__ float4 posfOf(dvec4 p, const MpsParams& P) {
+    return make_float4(d2fRN(p.x - P.domainMin[0]), d2fRN(p.y - P.domainMin[1]), d2fRN(p.z - P.domainMin[2]), 0.f);
+}
+__device__ __forceinline__ SideF sideF(const Dev& d, int i, dvec4 pi) {
+    const SideCtx sc = sideCtx(d, i, pi);
+    SideF s;
+    s.check = sc.check;
+    s.m = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (sc.check) s.m = posfOf(sc.mi, d.P);
+    return s;
+}
+__device__ __forceinline__ bool sideOKF(const Dev& d, const SideF& s, float4 hj, float d2f, int i, int j) {
+    if (!s.check) return true;
+    const float t = dist2f(hj, s.m) - d2f;
+    if (t > d.sideBand) return true;
+    if (t < -d.sideBand) return false;
+    return pairSideExact(d.pos, d.mirror, j, i);
+}
+// |x_j - x_i|^2 < R2 from the FP32 squared distance: certain outside [lo, hi]
+__device__ __forceinline__ bool insideF(const Dev& d, float d2f, float lo, float hi, double R2, int i, int j) {
+    if (d2f < lo) return true;
+    if (d2f > hi) return false;
+    return pairInsideExact(d.pos, j, i, R2);
+}
+
+// A pair vector and its squared norm for the sums (decisions are made before): the products
+// are fused, one rounding less per term than the decision's expression.
+__device__ __forceinline__ PairG pairSum(dvec4 pj, dvec4 pi) {
+    PairG q;
+    q.v0 = pj.x - pi.x; q.v1 = pj.y - pi.y; q.v2 = pj.z - pi.z;
+    q.d2 = fma(q.v2, q.v2, fma(q.v1, q.v1, q.v0 * q.v0));
+    return q;
+}
+
+// Bits of the entries k = l, l + L, ... < c of a list row that pass test(j, posf[j]); four
+// entries' indices and FP32 copies are loaded ahead of their tests.
+template <int L, class T>
+__device__ __forceinline__ Mask rowMask(const Dev& d, const int* row, int l, int c, T&& test) {
+    Mask m = maskNone();
+    for (int k = l; k < c; k += 4 * L) {
+        int jj[4];
+        float4 hh[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) jj[u] = k + u * L < c ? ldStream(row + (size_t)(k + u * L) * d.N0) : -1;
+#pragma unroll
+        for (int u = 0; u < 4; u++) hh[u] = jj[u] >= 0 ? __ldg(&d.posf[jj[u]]) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (jj[u] >= 0 && test(jj[u], hh[u])) maskSet(m, k + u * L);
+    }
+    return m;
+}
+// f(j, k) for the set bits of m in ascending order, the next entry's index loaded ahead.
+template <class F>
+__device__ __forceinline__ void forBits(const int* row, size_t N0, Mask m, F&& f) {
+    int k = maskPop(m);
+    if (k < 0) return;
+    int j = ldStream(row + (size_t)k * N0);
+    for (;;) {
+        const int kn = maskPop(m);
+        int jn = 0;
+        if (kn >= 0) jn = ldStream(row + (size_t)kn * N0);
+        f(j, k);
+        if (kn < 0) break;
+        k = kn; j = jn;
+    }
+}
+
+// The per-entry weights of a list entry (element e) at squared distance d2: w(r; reS), w/r^2
+// and, when the radii differ, w(r; reL).
+__device__ __forceinline__ void storeWeights(const Dev& d, size_t e, double d2) {
+    const MpsParams& P = d.P;
+    double w, wd;
+    weightR(d2, P.reS, P.weightType, w, wd);
+    d.cw[e] = w;
+    d.cwd[e] = wd;
+    if (d.cwL) { double wl, wdl; weightR(d2, P.reL, P.weightType, wl, wdl); d.cwL[e] = wl; }
+}

@@ -8,6 +8,7 @@
 // with the distance comparisons evaluated in exact FP64 (see mps_common.cuh).
 #include "mps_df.cuh"
 #include "mps_internal.h"
+#include "mps_lanes.cuh"
 
 #define BLK 128
 
@@ -15,128 +16,197 @@
 // MpsViscosity::calcViscosity, src/MpsViscosity.cpp:20-100 (Newtonian: MEU and RHO are
 // uniform, src/MpsInputOutput.cpp:833-838, so the harmonic mean is hoisted).  Staged scan
 // at the start-of-step positions; FP32 prefilter, exact FP64 radius/side tests.
+// The kinematic factors of a wall and of a fluid neighbour, (2 mu)/rho and
+// (2 mu mu / (mu + mu))/rho (src/MpsViscosity.cpp:55-62), are run constants (Dev).
+struct ViscSum {
+    dvec4 vi;
+    double ax, ay, az;
+    __device__ __forceinline__ void add(const Dev& d, dvec4 pi, int j) {
+        const MpsParams& P = d.P;
+        const PairG q = pairSum(d.pos[j], pi);
+        double wL, wd;
+        weightR(q.d2, P.reL, P.weightType, wL, wd);
+        const double f = wL * ((d.type[j] == P.wall) ? d.neuWall64 : d.neuFluid64);
+        const dvec4 vj = d.vel[j];
+        ax += (vj.x - vi.x) * f; ay += (vj.y - vi.y) * f; az += (vj.z - vi.z) * f;
+    }
+};
 struct OpViscosity {
-    // the kinematic factors of a wall and of a fluid neighbour, (2 mu)/rho and
-    // (2 mu mu / (mu + mu))/rho (src/MpsViscosity.cpp:55-62), are the same for every pair of
-    // the run: formed once per particle with the reference's operations (same bits)
-    struct State { dvec4 vi; SideCtx sc; double ax, ay, az, neuWall, neuFluid; };
+    struct State { ViscSum v; SideCtx sc; dvec4 pi; };
     __device__ float hi(const Dev& d) const { return d.bandHiL; }
     __device__ bool active(const Dev&, const State&) const { return true; }
     __device__ void begin(const Dev& d, int i, State& st) const {
-        st.vi = d.vel[i];
-        st.sc = sideCtx(d, i, d.pos[i]);
-        st.ax = st.ay = st.az = 0.0;
-        const double mu = d.P.KNM_VS1 * d.P.DNS_FL1, rho = d.P.DNS_FL1;
-        st.neuWall = (2.0 * mu) / rho;
-        st.neuFluid = (2.0 * mu * mu / (mu + mu)) / rho;
+        st.v = {d.vel[i], 0.0, 0.0, 0.0};
+        st.pi = d.pos[i];
+        st.sc = sideCtx(d, i, st.pi);
     }
     __device__ void visit(const Dev& d, int i, State& st, int j, dvec4 pj, PairG q) const {
-        const MpsParams& P = d.P;
-        if (!(q.d2 < P.reL2) || !sideOK(st.sc, pj, q.d2)) return;
-        const double neu = (d.type[j] == P.wall) ? st.neuWall : st.neuFluid;
-        double wL, wd;
-        weightR(q.d2, P.reL, P.weightType, wL, wd);
-        dvec4 vj = d.vel[j];
-        st.ax += (vj.x - st.vi.x) * wL * neu;
-        st.ay += (vj.y - st.vi.y) * wL * neu;
-        st.az += (vj.z - st.vi.z) * wL * neu;
+        if (!(q.d2 < d.P.reL2) || !sideOK(st.sc, pj, q.d2)) return;
+        st.v.add(d, st.pi, j);
     }
     __device__ void end(const Dev& d, int i, State& st) const {
         double c = d.P.coeffViscMultiphase;
-        d.acc[i] = make_dvec4(c * st.ax, c * st.ay, c * st.az, 0.0);
+        d.acc[i] = make_dvec4(c * st.v.ax, c * st.v.ay, c * st.v.az, 0.0);
     }
 };
 void launchViscosity(const Dev& d, cudaStream_t s) {
     launchScan(d, OpViscosity(), s);
 }
 // The same sweep over the start-of-step skin list (built just before from the same FP32
-// copies): its entries within the reL band, in scan order, are exactly the candidates the
-// 27-bucket scan passes to the exact FP64 test, so the sums are the scan's bit for bit.
-// A row that overflowed the list capacity (count K + 1) scans the buckets.
+// copies), L lanes per particle.  The list holds about 56 entries a row for the 32 inside
+// reL: the FP32 copies decide them first, and the FP64 sums (bound by the FP64 pipe, about 20
+// operations an entry) walk only those inside: 2,252 -> 1,066 us at 864k particles, 114 -> 22
+// at 6.9k.  A row that overflowed the list capacity
+// (count K + 1) scans the buckets with its first lane.
+template <int L>
 __global__ void __launch_bounds__(128) k_visc_list(Dev d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
-    const OpViscosity op;
-    OpViscosity::State st;
-    op.begin(d, i, st);
     const dvec4 pi = d.pos[i];
     const float4 fi = d.posf[i];
-    const float hi = op.hi(d);
+    ViscSum v = {d.vel[i], 0.0, 0.0, 0.0};
     const int c = d.nbrCount[i];
     if (c <= d.K) {
         const int* row = d.nbr + i;
-        for (int k = 0; k < c; k++) {
-            const int j = ldStream(row + (size_t)k * d.N0);
-            const float4 fj = d.posf[j];
-            const float ex = fj.x - fi.x, ey = fj.y - fi.y, ez = fj.z - fi.z;
-            if (ex * ex + ey * ey + ez * ez > hi) continue;
-            const dvec4 pj = d.pos[j];
-            op.visit(d, i, st, j, pj, pairOf(pj, pi));
-        }
-    } else {
-        forCellsNear(d, pi, fi, hi, [&](int j, dvec4 pj, PairG q) {
-            if (j != i) op.visit(d, i, st, j, pj, q);
+        const SideF sd = sideF(d, i, pi);
+        const Mask m = rowMask<L>(d, row, l, c, [&](int j, float4 hj) {
+            const float d2f = dist2f(hj, fi);
+            return insideF(d, d2f, d.bandLoL, d.bandHiL, d.P.reL2, i, j) && sideOKF(d, sd, hj, d2f, i, j);
+        });
+        forBits(row, d.N0, m, [&](int j, int) { v.add(d, pi, j); });
+    } else if (l == 0) {
+        const SideCtx sc = sideCtx(d, i, pi);
+        forCellsNear(d, pi, fi, d.bandHiL, [&](int j, dvec4 pj, PairG q) {
+            if (j != i && q.d2 < d.P.reL2 && sideOK(sc, pj, q.d2)) v.add(d, pi, j);
         });
     }
-    op.end(d, i, st);
+    const double ax = laneSum<L>(v.ax), ay = laneSum<L>(v.ay), az = laneSum<L>(v.az);
+    const double cv = d.P.coeffViscMultiphase;
+    if (l == 0) d.acc[i] = make_dvec4(cv * ax, cv * ay, cv * az, 0.0);
 }
 void launchViscosityList(const Dev& d, cudaStream_t s) {
-    k_visc_list<<<gridFor(d.N0, 128), 128, 0, s>>>(d);
+#define LAUNCH(L) k_visc_list<L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
 }
 
-// FP64 list of the current positions filtered from the skin list: the set, order and
-// (WEIGHTS) per-entry weights of k_build_nbr (candidates within the FP32 band, exact FP64
-// test d^2 < reMax^2).  A particle whose scan window changed or whose skin row overflowed,
-// or every particle once the skin list went stale, scans the 27 buckets as k_build_nbr does.
-template <bool WEIGHTS>
+// List of the current positions filtered from the skin list: the set, order and (WEIGHTS, the
+// FP64 tier) per-entry weights of k_build_nbr, L lanes per particle.  Membership (d^2 <
+// reMax^2) comes from the FP32 copies outside their rounding band; the weights, the FP64
+// part, are then formed over the members only (864k particles: 1,699 -> 992 us; decided and
+// formed entry by entry, every warp issued the weights for 56 entries instead of 33).  A
+// particle whose scan window changed or whose skin row overflowed, or every particle once the
+// skin list went stale, is left to k_rescan: a few particles cross a bucket face in every
+// step, and scanned in place one lane's walk of 27 buckets was the time of the whole kernel
+// (108k particles with weights 226 us, without them 98; now 130 + 14 and 32 + 13 us).
+template <bool WEIGHTS, int L>
 __global__ void __launch_bounds__(128) k_filter_nbr(Dev d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
-    const MpsParams& P = d.P;
     const dvec4 pi = d.pos[i];
     const float4 fi = d.posf[i];
     const size_t N0 = d.N0;
+    const int c = d.skinCnt[i];
     int cnt = 0;
-    auto keep = [&](int j, PairG q) {
-        if (!(q.d2 < d.reMax2)) return;
-        if (cnt < d.K) {
-            const size_t e = (size_t)cnt * N0 + i;
+    if (!*(volatile int*)d.skinFlag && c <= d.K && d.skinCell[i] == cellKeyOf(d, pi, fi)) {
+        const int* row = d.skinNbr + i;
+        // without weights one lane appends as it decides: 393 us at 2.8M particles against
+        // 672 with the second walk of the row (124 / 205 us at 864k)
+        const bool direct = !WEIGHTS && L == 1;
+        const Mask m = rowMask<L>(d, row, l, c, [&](int j, float4 hj) {
+            const bool in = insideF(d, dist2f(hj, fi), d.bandLo, d.bandHi, d.reMax2, i, j);
+            if (direct && in) d.nbr[(size_t)cnt++ * N0 + i] = j;
+            return in && !direct;
+        });
+        const Mask all = laneOr<L>(m);
+        if (!direct) cnt = maskCount(all);
+        if (l == 0) d.nbrCount[i] = cnt;
+        forBits(row, N0, m, [&](int j, int k) {
+            const size_t e = (size_t)maskRank(all, k) * N0 + i;
             d.nbr[e] = j;
-            if (WEIGHTS) {
-                double w, wd;
-                weightR(q.d2, P.reS, P.weightType, w, wd);
-                d.cw[e] = w;
-                d.cwd[e] = wd;
-                if (d.cwL) { double wl, wdl; weightR(q.d2, P.reL, P.weightType, wl, wdl); d.cwL[e] = wl; }
+            if (WEIGHTS) storeWeights(d, e, pairSum(d.pos[j], pi).d2);
+        });
+    } else if (l == 0) {
+        d.nearList[atomicAdd(d.rescan, 1)] = i;   // the near-wall list is written later (masks)
+    }
+    warpCount(d.counters, l == 0 ? (unsigned)cnt : 0u);
+}
+// The particles the filter left: the 27-bucket scan of k_build_nbr by one warp each.  The
+// window's nine rows of three buckets are ranges of the bucket order of about 28 particles, one
+// pass of the warp's lanes each; their bounds are loaded by nine lanes at once.
+template <bool WEIGHTS>
+__global__ void __launch_bounds__(128) k_rescan(Dev d) {
+    const int lane = threadIdx.x & 31;
+    const int n = *(volatile int*)d.rescan;
+    const MpsParams& P = d.P;
+    const size_t N0 = d.N0;
+    for (int w = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += (int)(gridDim.x * blockDim.x) >> 5) {
+        const int i = d.nearList[w];
+        const dvec4 pi = d.pos[i];
+        const float4 fi = d.posf[i];
+        int ix, iy, iz;
+        bucketCoordsHi(d, pi, fi, ix, iy, iz);
+        int a = 0, b = 0;
+        if (lane < (d.dz3 ? 9 : 3)) {
+            const long long jb = (long long)((iz - 1) * d.dz3 + lane / 3) * P.numBucketsXY +
+                                 (long long)(iy - 1 + lane % 3) * P.numBucketsX + ix;
+            const long long lo = jb - 1 > 0 ? jb - 1 : 0, hi = jb + 1 < d.nB - 1 ? jb + 1 : d.nB - 1;
+            if (lo <= hi) { a = d.cellStart[lo]; b = d.cellStart[hi + 1]; }
+        }
+        float4 f[9];   // the first pass over every range, loaded at once
+#pragma unroll
+        for (int r = 0; r < 9; r++) {
+            const int s0 = __shfl_sync(0xffffffffu, a, r), s1 = __shfl_sync(0xffffffffu, b, r);
+            if (s0 + lane < s1) f[r] = __ldg(&d.posfCell[s0 + lane]);
+        }
+        int cnt = 0;
+#pragma unroll
+        for (int r = 0; r < 9; r++) {
+            const int s0 = __shfl_sync(0xffffffffu, a, r), s1 = __shfl_sync(0xffffffffu, b, r);
+            for (int t = s0; t < s1; t += 32) {
+                const int s = t + lane;
+                int j = i;
+                bool in = false;
+                if (s < s1) {
+                    const float d2f = dist2f(t == s0 ? f[r] : __ldg(&d.posfCell[s]), fi);
+                    if (!(d2f > d.bandHi)) {
+                        j = __ldg(d.cellSorted + s);
+                        in = j != i && insideF(d, d2f, d.bandLo, d.bandHi, d.reMax2, i, j);
+                    }
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, in);
+                const int k = cnt + __popc(m & ((1u << lane) - 1u));
+                if (in && k < d.K) d.nbr[(size_t)k * N0 + i] = j;
+                cnt += __popc(m);
             }
         }
-        cnt++;
-    };
-    const int c = d.skinCnt[i];
-    if (!*(volatile int*)d.skinFlag && c <= d.K && d.skinCell[i] == cellKeyOf(d, pi, fi)) {
-        for (int k = 0; k < c; k++) {
-            const int j = ldStream(d.skinNbr + (size_t)k * N0 + i);
-            const float4 fj = d.posf[j];
-            const float ex = fj.x - fi.x, ey = fj.y - fi.y, ez = fj.z - fi.z;
-            if (ex * ex + ey * ey + ez * ez > d.bandHi) continue;
-            const dvec4 pj = d.pos[j];
-            keep(j, pairOf(pj, pi));
+        if (WEIGHTS) {
+            __syncwarp();
+            for (int k = lane; k < cnt && k < d.K; k += 32) {
+                const size_t e = (size_t)k * N0 + i;
+                storeWeights(d, e, pairSum(d.pos[d.nbr[e]], pi).d2);
+            }
         }
-    } else {
-        forCellsNear(d, pi, fi, d.bandHi, [&](int j, dvec4, PairG q) {
-            if (j != i) keep(j, q);
-        });
+        if (lane == 0) {
+            if (cnt > d.K) { setErr(d, MPSE_CAPACITY); cnt = d.K; }
+            d.nbrCount[i] = cnt;
+            if (cnt) atomicAdd(d.counters, (unsigned long long)cnt);
+        }
     }
-    if (cnt > d.K) { setErr(d, MPSE_CAPACITY); cnt = d.K; }
-    d.nbrCount[i] = cnt;
-    warpCount(d.counters, (unsigned)cnt);
 }
 void launchNeighborFilter(const Dev& d, cudaStream_t s, bool weights) {
     cudaMemsetAsync(d.counters, 0, sizeof(unsigned long long), s);
     launchPosf(d, s);
-    launchSkinCheck(d, s);
-    if (weights) k_filter_nbr<true><<<gridFor(d.N0, 128), 128, 0, s>>>(d);
-    else k_filter_nbr<false><<<gridFor(d.N0, 128), 128, 0, s>>>(d);
+    launchSkinCheck(d, s);   // also clears the rescan count
+#define LAUNCH(L)                                                                        \
+    if (weights) k_filter_nbr<true, L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d);        \
+    else k_filter_nbr<false, L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
+    // the list's length is on the device: enough warps to fill the chip, at most one each
+    const int grid = gridFor(d.N0, 4) < 1216 ? gridFor(d.N0, 4) : 1216;
+    if (weights) k_rescan<true><<<grid, 128, 0, s>>>(d);
+    else k_rescan<false><<<grid, 128, 0, s>>>(d);
 }
 
 // MpsParticle::addGravity, src/MpsParticle.cpp:111-130

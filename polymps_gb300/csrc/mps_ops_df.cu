@@ -1005,72 +1005,12 @@ void launchViscosityListDF(const Dev& d, cudaStream_t s) {
 // half the skin of its start position (FP32 test with margin).
 __global__ void k_skin_check(Dev d) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *d.rescan = 0;   // read by the filter that follows
     if (i >= liveN(d)) return;
     float4 a = d.posf[i], b = d.posSkin[i];
     float ex = a.x - b.x, ey = a.y - b.y, ez = a.z - b.z;
     if (!(ex * ex + ey * ey + ez * ez <= d.skinMove2)) d.skinFlag[0] = 1;
 }
-// List of the current positions (the set and order of k_build_nbr_df) filtered from the
-// skin list; a particle whose scan window changed, whose skin row overflowed, or any
-// particle after the skin list went stale, scans the 27 buckets as k_build_nbr_df does.
-template <bool STRAY>
-__global__ void __launch_bounds__(128) k_filter_nbr_df(Dev d) {
-    const int i = scanParticle<STRAY>(d);
-    if (i < 0) return;
-    const dvec4 pi = d.pos[i];
-    const float4 hi = d.posf[i], li = d.posLo[i];
-    const df R2 = K(d.k.reMax2);
-    const size_t N0 = d.N0;
-    int cnt = 0;
-    // the lo part (lo: where it sits) is read only for pairs in the uncertain band
-    auto keep = [&](int j, float4 hj, const float4* lo) {
-        float ex = hj.x - hi.x, ey = hj.y - hi.y, ez = hj.z - hi.z;
-        float d2f = ex * ex + ey * ey + ez * ez;
-        if (d2f > d.bandHi) return;
-        if (!(d2f < d.bandLo)) {
-            PairF q = pairDF(hj, __ldg(lo), hi, li);
-            if (!inBallDF(d, q.d2, R2, d.mgMax, d.reMax2, i, j)) return;
-        }
-        if (cnt < d.K) d.nbr[(size_t)cnt * N0 + i] = j;
-        cnt++;
-    };
-    const int c = d.skinCnt[i];
-    if (!*(volatile int*)d.skinFlag && c <= d.K && d.skinCell[i] == cellKeyOf(d, pi, hi)) {
-        // the skin list stays intact (a later sweep filters it again); four entries' loads
-        // are issued before their tests (the list stores would otherwise order each gather
-        // after the previous entry's store)
-        const int* row = d.skinNbr + i;
-        int k = 0;
-        for (; k + 4 <= c; k += 4) {
-            int jj[4];
-            float4 hh[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) jj[u] = ldStream(row + (size_t)(k + u) * N0);
-#pragma unroll
-            for (int u = 0; u < 4; u++) hh[u] = __ldg(&d.posf[jj[u]]);
-#pragma unroll
-            for (int u = 0; u < 4; u++) keep(jj[u], hh[u], d.posLo + jj[u]);
-        }
-        for (; k < c; k++) {
-            const int j = ldStream(row + (size_t)k * N0);
-            keep(j, __ldg(&d.posf[j]), d.posLo + j);
-        }
-    } else {
-        forCellsDF(d, pi, hi, d.bandHi, [&](int j, int s, float4 hj) {
-            if (j != i) keep(j, hj, d.posLoCell + s);
-        });
-    }
-    if (cnt > d.K) { setErr(d, MPSE_CAPACITY); cnt = d.K; }
-    d.nbrCount[i] = cnt;
-    warpCount(d.counters, (unsigned)cnt);
-}
 void launchSkinCheck(const Dev& d, cudaStream_t s) {
     k_skin_check<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
-}
-void launchNeighborFilterDF(const Dev& d, cudaStream_t s) {
-    cudaMemsetAsync(d.counters, 0, sizeof(unsigned long long), s);
-    launchPosf(d, s);
-    k_skin_check<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
-    k_filter_nbr_df<false><<<gridFor(d.N0, 128), 128, 0, s>>>(d);
-    k_filter_nbr_df<true><<<gridFor(d.N0, 128), 128, 0, s>>>(d);
 }
