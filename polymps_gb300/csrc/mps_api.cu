@@ -44,6 +44,7 @@ struct mpsgpu_s {
     int *nbrAlt = nullptr, *cntAlt = nullptr;   // second list arrays (the skin list keeps its own)
     int skinOn = 1;            // viscosity and the post-prediction list from the start-of-step skin list
     bool corrFresh = false;    // the correction matrix of the current positions and masks is written
+    bool pAuxFresh = false;    // the last operator was the pressure gradient: its p_min still stand
     bool opSkipped = false;    // the last operator had nothing left to launch
     void* vtuDev = nullptr;    // staging of the binary .vtu block (device, page-locked host)
     void* vtuHost = nullptr;
@@ -208,8 +209,7 @@ static void ensureMasks(mpsgpu_t h) {
     ensureList(h);
     if (h->masksValid) return;
     if (h->prof.on) h->prof.begin(PROF_NEIGHBOR_LIST, h->s);
-    if (df32(h)) launchSideMasksDF(h->d, h->s);
-    else launchSideMasks(h->d, h->s);
+    launchSideMasks(h->d, h->s);
     if (h->prof.on) h->prof.end(h->s);
     countLaunch(1);
     h->masksValid = true;
@@ -373,6 +373,8 @@ static int runOpBody(mpsgpu_t h, int op) {
         h->listValid = false; h->masksValid = false; h->cacheValid = false; h->corrFresh = false;
     };
     const bool x = df32(h);
+    const bool pAuxFresh = h->pAuxFresh;
+    h->pAuxFresh = false;
     switch (op) {
         case MPS_OP_UPDATE_BUCKETS: {
             bool rn = h->renumberEvery > 0 && h->renumberCountdown <= 0;
@@ -430,7 +432,7 @@ static int runOpBody(mpsgpu_t h, int op) {
         case MPS_OP_WALL_NPCD: ensureMasks(h); if (x) launchWallNpcdDF(d, s); else launchWallNpcd(d, s); break;
         case MPS_OP_CORRECTION_MATRIX:
             ensureMasks(h);
-            if (x && h->corrFresh && h->masksValid) {   // formed by the PND sweep: publish it
+            if (h->corrFresh && h->masksValid) {   // formed by the PND sweep: publish it
                 std::swap(d.c1, d.c1n); std::swap(d.c2, d.c2n); std::swap(d.c3, d.c3n);
                 std::swap(d.corrDF, d.corrDFn);
                 h->corrFresh = false;
@@ -443,8 +445,8 @@ static int runOpBody(mpsgpu_t h, int op) {
             ensureMasks(h);
             // the correction matrix of the step (read after the pressure solve, positions and
             // masks unchanged in between) is formed in the same pass
-            bool corr = x && P.gradientCorrection && P.pndType != 2;
-            if (x) launchPndNeighNpcdDF(d, s, corr); else launchPndNeighNpcd(d, s);
+            bool corr = P.gradientCorrection && P.pndType != 2;
+            if (x) launchPndNeighNpcdDF(d, s, corr); else launchPndNeighNpcd(d, s, corr);
             h->corrFresh = corr;
             break;
         }
@@ -456,11 +458,18 @@ static int runOpBody(mpsgpu_t h, int op) {
             break;
         case MPS_OP_CALC_PRESS: { int e = calcPress(h); if (e) return e; break; }
         case MPS_OP_EXTRAPOLATE_PRESS: ensureMasks(h); ensureCache(h); launchExtrapolatePress(d, s); break;
-        case MPS_OP_PRESS_GRADIENT: ensureMasks(h); if (x) launchPressGradientDF(d, s); else launchPressGradient(d, s); break;
-        case MPS_OP_WALL_PRESS_GRADIENT:
+        case MPS_OP_PRESS_GRADIENT:
             ensureMasks(h);
-            if (x) launchWallPressGradientDF(d, s); else launchWallPressGradient(d, s);
+            if (x) launchPressGradientDF(d, s); else launchPressGradient(d, s);
+            h->pAuxFresh = true;
             break;
+        case MPS_OP_WALL_PRESS_GRADIENT: {
+            // p_min over the same entries (maskS) as the pressure gradient's, when that ran last
+            const bool fresh = pAuxFresh && h->masksValid;
+            ensureMasks(h);
+            if (x) launchWallPressGradientDF(d, s, fresh); else launchWallPressGradient(d, s, fresh);
+            break;
+        }
         case MPS_OP_WALL_VISCOSITY: ensureMasks(h); if (x) launchWallViscosityDF(d, s); else launchWallViscosity(d, s); break;
         case MPS_OP_CORRECT: launchCorrect(d, s); invalidate(); break;
         case MPS_OP_SHIFTING:
@@ -470,7 +479,7 @@ static int runOpBody(mpsgpu_t h, int op) {
                 // removal, scans the buckets), its masks, then list sweeps
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(PROF_NEIGHBOR_LIST, s, false); }
                 launchNeighborFilter(d, s, false);
-                launchSideMasksDF(d, s);
+                launchSideMasks(d, s);
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(MPS_OP_SHIFTING, s, false); }
                 launchShiftingListDF(d, s);
                 invalidate();
@@ -788,6 +797,10 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
     if (p->reS2 != p->reL2) A(d.cwL, (size_t)d.K * n);
     A(d.maskS, n);
     A(d.maskL, n);
+    A(d.mirrorS, n);
+    if (p->reS2 != p->reL2) A(d.mirrorL, n);
+    else d.mirrorL = d.mirrorS;
+    A(d.pAux, n);
     A(d.nearList, n);
     A(d.nearCount, 1);
     A(d.velMax, 1);
@@ -850,6 +863,7 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
         k.reS2 = hd(p->reS2); k.reL2 = hd(p->reL2); k.reMax2 = hd(d.reMax2);
         k.coll2 = hd(p->distCollisionLimit2);
         double mu = p->KNM_VS1 * p->DNS_FL1, rho = p->DNS_FL1;
+        d.cPG = p->relaxPress * p->coeffPressGrad / p->DNS_FL1;
         d.neuWall64 = (2.0 * mu) / rho;
         d.neuFluid64 = (2.0 * mu * mu / (mu + mu)) / rho;
         k.neuW = hd((2.0 * mu) / rho);
@@ -1083,6 +1097,7 @@ int mpsgpu_set_precision(mpsgpu_t h, int precision) {
         h->d.prec = precision;
         h->listValid = false;
         h->skinValid = false;
+        h->pAuxFresh = false;
         h->corrFresh = false;
         h->masksValid = false;
         h->cacheValid = false;
@@ -1319,6 +1334,7 @@ int mpsgpu_set_field(mpsgpu_t h, int f, const void* host) {
     h->listValid = false;
     h->skinValid = false;
     h->corrFresh = false;
+    h->pAuxFresh = false;
     h->masksValid = false;
     h->cacheValid = false;
     if (f == MPS_F_POS) launchPosf(h->d, h->s);

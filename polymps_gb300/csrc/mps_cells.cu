@@ -381,40 +381,74 @@ void launchNeighborList(const Dev& d, cudaStream_t s) {
 
 // ------------------------------------------------------------------ entry masks
 // After the wall pass: for each particle, which entries are inside the reS / reL ball and
-// not on the mirror side (dstij2 < dstimj2, e.g. src/MpsPndNeigh.cpp:249), all in exact
-// FP64.  Particles whose mirror is far (see SideCtx) and whose list radius equals the
-// ball radius take every entry without per-entry work.  Fluid particles near the wall
-// are appended to nearList for the wall-only sweeps.
+// not on the mirror side (dstij2 < dstimj2, e.g. src/MpsPndNeigh.cpp:249), with the
+// reference's decisions: from the FP32 copies outside their rounding bands, in FP64 inside
+// them.  Particles whose mirror is far (see SideCtx) and whose list radius equals the ball
+// radius take every entry without per-entry work.  Fluid particles near the wall also get
+// their mirror entries and are appended to nearList for the wall-only sweeps, which walk the
+// masks instead of testing the list again.
+static __device__ __noinline__ bool mirrorInsideExact(const dvec4* pos, const dvec4* mirror, int j, int i, double R2) {
+    return pairMirror(pos[j], mirror[i]).dm2 < R2;
+}
+template <int L>
 __global__ void __launch_bounds__(128) k_side_masks(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
-    int c = d.nbrCount[i];
+    const int c = d.nbrCount[i];
     const Mask all = maskFirst(c);
-    dvec4 pi = d.pos[i];
-    SideCtx sc = sideCtx(d, i, pi);
-    bool fullS = P.reS2 >= d.reMax2, fullL = P.reL2 >= d.reMax2;
+    const dvec4 pi = d.pos[i];
+    const bool near = P.wallType == 1 && d.type[i] == P.fluid && d.nearWall[i];
+    SideF sd = sideF(d, i, pi);
+    if (near && !sd.check) sd.m = posfOf(d.mirror[i], P);
+    const bool fullS = P.reS2 >= d.reMax2, fullL = P.reL2 >= d.reMax2;
+    const bool two = d.mirrorL != d.mirrorS;
     Mask mS = all, mL = all;
-    if (sc.check || !fullS || !fullL) {
+    if (sd.check || near || !fullS || !fullL) {
         mS = maskNone(); mL = maskNone();
+        Mask rS = maskNone(), rL = maskNone();
+        const float4 fi = d.posf[i];
         const int* row = d.nbr + i;
-        for (int k = 0; k < c; k++) {
-            dvec4 pj = d.pos[__ldg(row + (size_t)k * d.N0)];
-            PairG q = pairOf(pj, pi);
-            bool side = sideOK(sc, pj, q.d2);
-            if (side && q.d2 < P.reS2) maskSet(mS, k);
-            if (side && q.d2 < P.reL2) maskSet(mL, k);
+        auto mirrorIn = [&](float dm2f, float lo, float hi, double R2, int j) {
+            if (dm2f < lo) return true;
+            if (dm2f > hi) return false;
+            return mirrorInsideExact(d.pos, d.mirror, j, i, R2);
+        };
+        for (int k = l; k < c; k += L) {
+            const int j = ldStream(row + (size_t)k * d.N0);
+            const float4 fj = __ldg(&d.posf[j]);
+            const float d2f = dist2f(fj, fi);
+            if (!sideOKF(d, sd, fj, d2f, i, j)) continue;
+            const bool inS = fullS || insideF(d, d2f, d.bandLoS, d.bandHiS, P.reS2, i, j);
+            const bool inL = fullL || insideF(d, d2f, d.bandLoL, d.bandHiL, P.reL2, i, j);
+            if (inS) maskSet(mS, k);
+            if (inL) maskSet(mL, k);
+            if (near) {
+                const float dm2f = dist2f(fj, sd.m);
+                if (inS && mirrorIn(dm2f, d.bandLoS, d.bandHiS, P.reS2, j)) maskSet(rS, k);
+                if (two && inL && mirrorIn(dm2f, d.bandLoL, d.bandHiL, P.reL2, j)) maskSet(rL, k);
+            }
+        }
+        mS = laneOr<L>(mS); mL = laneOr<L>(mL);
+        if (near) {
+            rS = laneOr<L>(rS);
+            if (two) rL = laneOr<L>(rL);
+            if (l == 0) {
+                d.mirrorS[i] = rS;
+                if (two) d.mirrorL[i] = rL;
+            }
         }
     }
-    d.maskS[i] = mS;
-    d.maskL[i] = mL;
-    if (P.wallType == 1 && d.type[i] == P.fluid && d.nearWall[i]) {
-        int slot = atomicAdd(d.nearCount, 1);
-        d.nearList[slot] = i;
+    if (l == 0) {
+        d.maskS[i] = mS;
+        d.maskL[i] = mL;
+        if (near) d.nearList[atomicAdd(d.nearCount, 1)] = i;
     }
 }
 
 void launchSideMasks(const Dev& d, cudaStream_t s) {
     cudaMemsetAsync(d.nearCount, 0, sizeof(int), s);
-    k_side_masks<<<gridFor(d.N0, 128), 128, 0, s>>>(d);
+#define LAUNCH(L) k_side_masks<L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
 }

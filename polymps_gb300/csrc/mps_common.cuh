@@ -139,12 +139,19 @@ struct Dev {
     // per-particle entry masks after the wall pass: bit k set when entry k is inside the
     // reS (maskS) / reL (maskL) ball and not on the mirror side
     Mask *maskS, *maskL;
+    // and, for the fluid particles near the wall, the entries whose image counts in the wall
+    // sweeps: inside the ball, the mirror-side distance inside it too, not on the mirror side
+    Mask *mirrorS, *mirrorL;        // the reS and the reL ball (one array when the radii agree)
     int *nearList, *nearCount;      // fluid particles near the polygon wall (compacted)
     double reMax2;                  // list radius^2 = max(reS^2, reL^2)
     float bandHiS, bandHiL;         // FP32 prefilter upper bounds for the reS / reL balls
     float bandLoS, bandLoL;         // ... and the lower bounds below which an entry is inside
     float sideBand;                 // FP32 mirror-side test: certain beyond this difference
     double neuWall64, neuFluid64;   // kinematic factors of a wall and of a fluid neighbour
+    double cPG;                     // relaxPress * coeffPressGrad / DNS_FL1
+    // per particle, written by the pressure gradient: p_min of its entries (gradient types 0
+    // and 2; FP64 or a float-float pair, by tier) or p / n (type 3; 0 where n <= epsilonZero)
+    double* pAux;
     float bandHiColl;               // ... and for the collision distance
     // polygon mesh and wall tables
     int ntri;
@@ -589,29 +596,31 @@ __device__ __forceinline__ void wallRepulsion(const MpsParams& P, const ReflG& r
     }
 }
 
-// MpsVectorMatrix::correctionMatrix + inverseMatrix (Gauss-Jordan without pivoting,
-// identity when det <= eps), src/MpsVectorMatrix.cpp:20-166
-__device__ __forceinline__ void invert3(double* m, int dim, double eps) {
-    double A[9], M[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) { A[k] = m[k]; M[k] = (k % 4 == 0) ? 1.0 : 0.0; }
-    if (dim == 2) { A[2] = A[5] = A[6] = A[7] = 0.0; A[8] = 1.0; }
-    double det = (A[0] * A[4] * A[8] + A[1] * A[5] * A[6] + A[2] * A[3] * A[7]) -
-                 (A[2] * A[4] * A[6] + A[1] * A[3] * A[8] + A[0] * A[5] * A[7]);
+// MpsVectorMatrix::inverseMatrix (elimination without pivoting, identity when det <= eps),
+// src/MpsVectorMatrix.cpp:20-166, of the symmetric moment matrix m (xx, xy, xz, yy, yz, zz):
+// its L D L^T factors have the reference's pivots, and the inverse follows from them with 6
+// divisions instead of the 15 of a full Gauss-Jordan (an FP64 division is about ten FP64
+// operations).  Against an 80-bit inverse both are off alike (mean 1.0e-16 and 1.1e-16 of the
+// largest entry on well-spread neighbourhoods, 2.0e-15 and 2.0e-15 on flat ones).
+__device__ __forceinline__ void invertSym3(double m[6], int dim, double eps) {
+    const double a = m[0], b = m[1], d = m[3];
+    const double c = dim == 2 ? 0.0 : m[2], e = dim == 2 ? 0.0 : m[4], f = dim == 2 ? 1.0 : m[5];
+    const double det = (a * d * f + b * e * c + c * b * e) - (c * d * c + b * b * f + a * e * e);
     if (det <= eps) {
-#pragma unroll
-        for (int k = 0; k < 9; k++) m[k] = (k % 4 == 0) ? 1.0 : 0.0;
+        m[0] = m[3] = m[5] = 1.0;
+        m[1] = m[2] = m[4] = 0.0;
         return;
     }
-    for (int k = 0; k < dim; k++)
-        for (int r = 0; r < dim; r++) {
-            if (r == k) continue;
-            double f = A[r * 3 + k] / A[k * 3 + k];
-            for (int c = 0; c < dim; c++) { A[r * 3 + c] -= f * A[k * 3 + c]; M[r * 3 + c] -= f * M[k * 3 + c]; }
-        }
-    for (int r = 0; r < dim; r++)
-        for (int c = 0; c < dim; c++) M[r * 3 + c] /= A[r * 3 + r];
-#pragma unroll
-    for (int k = 0; k < 9; k++) m[k] = M[k];
+    const double l1 = b / a, l2 = c / a;
+    const double d1 = d - l1 * b, e1 = e - l1 * c, l3 = e1 / d1;
+    const double d2 = f - l2 * c - l3 * e1;
+    const double i0 = 1.0 / a, i1 = 1.0 / d1, i2 = 1.0 / d2;
+    const double g = l1 * l3 - l2;
+    m[5] = i2;
+    m[4] = -l3 * i2;
+    m[2] = g * i2;
+    m[3] = i1 - l3 * m[4];
+    m[1] = -l1 * i1 - l3 * m[2];
+    m[0] = i0 + l1 * (l1 * i1) + g * m[2];
 }
 static inline int gridFor(int n, int block) { return (n + block - 1) / block; }

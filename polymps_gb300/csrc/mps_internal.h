@@ -55,7 +55,8 @@ void launchCollision(const Dev& d, cudaStream_t s);
 void launchCollisionApply(const Dev& d, cudaStream_t s);
 void launchWallNpcd(const Dev& d, cudaStream_t s);
 void launchCorrectionMatrix(const Dev& d, cudaStream_t s);
-void launchPndNeighNpcd(const Dev& d, cudaStream_t s);
+// withCorrection: also the correction matrix of the same positions and masks
+void launchPndNeighNpcd(const Dev& d, cudaStream_t s, bool withCorrection);
 void launchPndDiffusive(const Dev& d, cudaStream_t s);
 void launchPndMean(const Dev& d, cudaStream_t s);
 void launchInitPnd(const Dev& d, cudaStream_t s);
@@ -63,7 +64,8 @@ void launchUpdateBC(const Dev& d, cudaStream_t s);
 void launchEOS(const Dev& d, cudaStream_t s);
 void launchExtrapolatePress(const Dev& d, cudaStream_t s);
 void launchPressGradient(const Dev& d, cudaStream_t s);
-void launchWallPressGradient(const Dev& d, cudaStream_t s);
+// fresh: the pressure gradient has just written p_min (Dev::pAux)
+void launchWallPressGradient(const Dev& d, cudaStream_t s, bool fresh);
 void launchPredictPressGradient(const Dev& d, bool skin, cudaStream_t s);   // relax_fact < 1, before PREDICT
 void launchWallViscosity(const Dev& d, cudaStream_t s);
 void launchCorrect(const Dev& d, cudaStream_t s);
@@ -72,16 +74,14 @@ void launchDummyVelocity(const Dev& d, cudaStream_t s);
 
 // mps_ops_df.cu (DF32 tier)
 void launchNeighborListDF(const Dev& d, cudaStream_t s);
-void launchSideMasksDF(const Dev& d, cudaStream_t s);
 void launchViscosityDF(const Dev& d, cudaStream_t s);
 void launchCollisionDF(const Dev& d, cudaStream_t s);
 void launchWallNpcdDF(const Dev& d, cudaStream_t s);
 void launchCorrectionMatrixDF(const Dev& d, cudaStream_t s);
 void launchCorrDF(const Dev& d, cudaStream_t s);
-// withCorrection: also the correction matrix of the same positions and masks
 void launchPndNeighNpcdDF(const Dev& d, cudaStream_t s, bool withCorrection = false);
 void launchPressGradientDF(const Dev& d, cudaStream_t s);
-void launchWallPressGradientDF(const Dev& d, cudaStream_t s);
+void launchWallPressGradientDF(const Dev& d, cudaStream_t s, bool fresh);
 void launchWallViscosityDF(const Dev& d, cudaStream_t s);
 void launchShiftingDF(const Dev& d, cudaStream_t s);
 // the same from the list of the current positions (filtered from the skin list, masks built)

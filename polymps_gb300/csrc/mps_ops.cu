@@ -455,38 +455,39 @@ __device__ __forceinline__ int nearIndex(const Dev& d) {
     return (t < *d.nearCount) ? d.nearList[t] : -1;
 }
 // MpsPndNeigh::calcWallNPCD, src/MpsPndNeigh.cpp:105-195
-__global__ void __launch_bounds__(BLK) k_wall_npcd(Dev d) {
-    int i = nearIndex(d);
-    if (i < 0) return;
+__global__ void __launch_bounds__(WALL_BLK) k_wall_npcd(Dev d) {
+    __shared__ double sm[3][32];
     const MpsParams& P = d.P;
-    dvec4 pi = d.pos[i], mi = d.mirror[i];
-    ReflG r = makeRefl(pi, mi, P.epsilonZero, true);
-    double dx = 0, dy = 0, dz = 0;
-    forNbrs(d, i, [&](int j) {
-        dvec4 pj = d.pos[j];
-        PairG q = pairOf(pj, pi);
-        if (q.d2 < P.reS2) {
-            PairM m = pairMirror(pj, mi);
-            if (m.dm2 < P.reS2 && q.d2 < m.dm2) {
-                double wS = wfun(sqrt(m.dm2), P.reS, P.weightType);
-                dx += m.m0 * wS; dy += m.m1 * wS; dz += m.m2 * wS;
-            }
+    forNearWall(d, [](int, int) {}, [&](int i, int g, int l) {
+        const dvec4 mi = d.mirror[i];
+        double dx = 0, dy = 0, dz = 0;
+        forBitsShared<WALL_L>(d.nbr + i, d.N0, d.mirrorS[i], l, [&](int j, int) {
+            const PairG m = pairSum(d.pos[j], mi);
+            double wS, wd;
+            weightR(m.d2, P.reS, P.weightType, wS, wd);
+            dx += m.v0 * wS; dy += m.v1 * wS; dz += m.v2 * wS;
+        });
+        dx = laneSum<WALL_L>(dx); dy = laneSum<WALL_L>(dy); dz = laneSum<WALL_L>(dz);
+        if (l == 0) { sm[0][g] = dx; sm[1][g] = dy; sm[2][g] = dz; }
+    }, [&](int i, int g) {
+        const dvec4 pi = d.pos[i], mi = d.mirror[i];
+        const ReflG r = makeRefl(pi, mi, P.epsilonZero, true);
+        double dx = sm[0][g], dy = sm[1][g], dz = sm[2][g];
+        PairM s = pairMirror(pi, mi);
+        if (s.dm2 < P.reS2) {
+            double wS = wfun(sqrt(s.dm2), P.reS, P.weightType);
+            dx += s.m0 * wS; dy += s.m1 * wS; dz += s.m2 * wS;
         }
+        dvec4 n = d.npcd[i];
+        n.x += r.R[0] * dx + r.R[1] * dy + r.R[2] * dz;
+        n.y += r.R[3] * dx + r.R[4] * dy + r.R[5] * dz;
+        n.z += r.R[6] * dx + r.R[7] * dy + r.R[8] * dz;
+        d.npcd[i] = n;
     });
-    PairM s = pairMirror(pi, mi);
-    if (s.dm2 < P.reS2) {
-        double wS = wfun(sqrt(s.dm2), P.reS, P.weightType);
-        dx += s.m0 * wS; dy += s.m1 * wS; dz += s.m2 * wS;
-    }
-    dvec4 n = d.npcd[i];
-    n.x += r.R[0] * dx + r.R[1] * dy + r.R[2] * dz;
-    n.y += r.R[3] * dx + r.R[4] * dy + r.R[5] * dz;
-    n.z += r.R[6] * dx + r.R[7] * dy + r.R[8] * dz;
-    d.npcd[i] = n;
 }
 void launchWallNpcd(const Dev& d, cudaStream_t s) {
     if (d.P.wallType != 1) return;
-    k_wall_npcd<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
+    k_wall_npcd<<<wallGrid(d.N0), WALL_BLK, 0, s>>>(d);
 }
 
 // ------------------------------------------------------------------ velocity divergence
@@ -572,56 +573,85 @@ void launchVelDivergence(const Dev& d, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------ correction matrix
-// MpsVectorMatrix::correctionMatrix + inverseMatrix (Gauss-Jordan without pivoting,
-// identity when det <= eps or numNeigh < 4), src/MpsVectorMatrix.cpp:20-166
-__global__ void __launch_bounds__(BLK) k_corr_matrix(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= liveN(d)) return;
-    const MpsParams& P = d.P;
-    dvec4 pi = d.pos[i];
-    double m[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    forMask(d, i, d.maskS[i], [&](int j, size_t e) {
-        dvec4 pj = d.pos[j];
-        double v[3] = {pj.x - pi.x, pj.y - pi.y, pj.z - pi.z};
-        double wd = d.cwd[e];   // w / r^2
-#pragma unroll
-        for (int a = 0; a < 3; a++)
-#pragma unroll
-            for (int b = 0; b < 3; b++) m[a * 3 + b] += wd * v[a] * v[b];
-    });
-#pragma unroll
-    for (int k = 0; k < 9; k++) m[k] *= -P.coeffPressGrad;
-    invert3(m, (int)P.dim, P.epsilonZero);
-    if (d.numNeigh[i] < 4) {
-#pragma unroll
-        for (int k = 0; k < 9; k++) m[k] = (k % 4 == 0) ? 1.0 : 0.0;
+// MpsVectorMatrix::correctionMatrix + inverseMatrix (identity when det <= eps or numNeigh < 4),
+// src/MpsVectorMatrix.cpp:20-166, from the sums of w / r^2 r r^T over the reS entries.
+struct Moments {
+    double xx = 0, xy = 0, xz = 0, yy = 0, yz = 0, zz = 0;
+    __device__ __forceinline__ void add(double v0, double v1, double v2, double wd) {
+        const double t0 = wd * v0, t1 = wd * v1, t2 = wd * v2;
+        xx += t0 * v0; xy += t0 * v1; xz += t0 * v2;
+        yy += t1 * v1; yz += t1 * v2; zz += t2 * v2;
     }
-    d.c1[i] = make_dvec4(m[0], m[1], m[2], 0.0);
-    d.c2[i] = make_dvec4(m[3], m[4], m[5], 0.0);
-    d.c3[i] = make_dvec4(m[6], m[7], m[8], 0.0);
+    template <int L>
+    __device__ __forceinline__ void sum() {
+        xx = laneSum<L>(xx); xy = laneSum<L>(xy); xz = laneSum<L>(xz);
+        yy = laneSum<L>(yy); yz = laneSum<L>(yz); zz = laneSum<L>(zz);
+    }
+    __device__ __forceinline__ void store(const Dev& d, int i, int numNeigh, dvec4* c1, dvec4* c2, dvec4* c3) const {
+        const MpsParams& P = d.P;
+        const double c = -P.coeffPressGrad;
+        double m[6] = {xx * c, xy * c, xz * c, yy * c, yz * c, zz * c};
+        invertSym3(m, (int)P.dim, P.epsilonZero);
+        if (numNeigh < 4) {
+            m[0] = m[3] = m[5] = 1.0;
+            m[1] = m[2] = m[4] = 0.0;
+        }
+        c1[i] = make_dvec4(m[0], m[1], m[2], 0.0);
+        c2[i] = make_dvec4(m[1], m[3], m[4], 0.0);
+        c3[i] = make_dvec4(m[2], m[4], m[5], 0.0);
+    }
+};
+template <int L>
+__global__ void __launch_bounds__(BLK) k_corr_matrix(Dev d) {
+    const int i = laneRow<L>(), l = laneOf<L>();
+    if (i >= liveN(d)) return;
+    const dvec4 pi = d.pos[i];
+    Moments M;
+    forMaskLane<L>(d, i, d.maskS[i], l, [&](int j, size_t e, int) {
+        const dvec4 pj = d.pos[j];
+        M.add(pj.x - pi.x, pj.y - pi.y, pj.z - pi.z, d.cwd[e]);
+    });
+    M.sum<L>();
+    if (l == 0) M.store(d, i, d.numNeigh[i], d.c1, d.c2, d.c3);
 }
-void launchCorrectionMatrix(const Dev& d, cudaStream_t s) { k_corr_matrix<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d); }
+void launchCorrectionMatrix(const Dev& d, cudaStream_t s) {
+#define LAUNCH(L) k_corr_matrix<L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
+}
 
 // ------------------------------------------------------------------ PND / NPCD
 // MpsPndNeigh::calcPndnNeighNPCD, src/MpsPndNeigh.cpp:199-331 (init == 0), and
-// setInitialPndNumberOfNeighNPCD, src/MpsPndNeigh.cpp:21-101 (init == 1)
-template <int INIT>
+// setInitialPndNumberOfNeighNPCD, src/MpsPndNeigh.cpp:21-101 (init == 1).
+// CORR: the correction matrix's moment sums over the reS entries in the same pass (it shares
+// the entries, their gathers and their pair vectors), into the staging arrays that the
+// correction-matrix operator publishes.  FP64-pipe bound: 864k particles 951 us (463 for the
+// PND sums and 1,003 for the matrix when each had its own pass).
+template <int INIT, bool CORR, int L>
 __global__ void __launch_bounds__(BLK) k_pnd_npcd(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
-    dvec4 pi = d.pos[i];
-    double ni = 0.0, wSum = 0.0;
-    const Mask mL = d.maskL[i];
+    const dvec4 pi = d.pos[i];
+    double ni = 0.0, nx = 0.0, ny = 0.0, nz = 0.0;
+    Moments M;
+    const Mask mL = d.maskL[i], mS = d.maskS[i];
+    forMaskLane<L>(d, i, CORR ? mS : (mL & mS), l, [&](int j, size_t e, int k) {
+        const dvec4 pj = d.pos[j];
+        const double v0 = pj.x - pi.x, v1 = pj.y - pi.y, v2 = pj.z - pi.z;
+        if (!CORR || maskHas(mL, k)) {
+            const double wS = d.cw[e];
+            ni += wS;
+            nx += v0 * wS; ny += v1 * wS; nz += v2 * wS;
+        }
+        if (CORR) M.add(v0, v1, v2, d.cwd[e]);
+    });
+    ni = laneSum<L>(ni); nx = laneSum<L>(nx); ny = laneSum<L>(ny); nz = laneSum<L>(nz);
+    if (CORR) M.sum<L>();
+    if (l != 0) return;
     int nn = (INIT ? 0 : d.nNeighWall[i]) + maskCount(mL);
     dvec4 np = INIT ? make_dvec4(0, 0, 0, 0) : d.npcd[i];
-    forMask(d, i, mL & d.maskS[i], [&](int j, size_t e) {
-        dvec4 pj = d.pos[j];
-        double wS = d.cw[e];
-        ni += wS;
-        np.x += (pj.x - pi.x) * wS; np.y += (pj.y - pi.y) * wS; np.z += (pj.z - pi.z) * wS;
-        wSum += wS;
-    });
+    np.x += nx; np.y += ny; np.z += nz;
     double pndSmall;
     if (INIT) {
         double pn = d.pndi[i] + ni;     // pndi accumulates onto its initial value
@@ -640,104 +670,124 @@ __global__ void __launch_bounds__(BLK) k_pnd_npcd(Dev d) {
     }
     d.pndSmall[i] = pndSmall;
     d.numNeigh[i] = nn;
-    if (wSum > P.epsilonZero) { np.x /= pndSmall; np.y /= pndSmall; np.z /= pndSmall; }
+    if (ni > P.epsilonZero) { np.x /= pndSmall; np.y /= pndSmall; np.z /= pndSmall; }
     d.npcd[i] = np;
     d.npcd2[i] = np.x * np.x + np.y * np.y + np.z * np.z;
     dvec4 nw = d.polyNormal[i];
     d.devDot[i] = (np.x * nw.x + np.y * nw.y + np.z * nw.z < 0.0) ? 1.0 : -1.0;
+    if (CORR) M.store(d, i, nn, d.c1n, d.c2n, d.c3n);
 }
-void launchPndNeighNpcd(const Dev& d, cudaStream_t s) { k_pnd_npcd<0><<<gridFor(d.N0, BLK), BLK, 0, s>>>(d); }
+template <int INIT, bool CORR>
+static void launchPndNpcd(const Dev& d, cudaStream_t s) {
+#define LAUNCH(L) k_pnd_npcd<INIT, CORR, L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
+}
+void launchPndNeighNpcd(const Dev& d, cudaStream_t s, bool withCorrection) {
+    if (withCorrection) launchPndNpcd<0, true>(d, s);
+    else launchPndNpcd<0, false>(d, s);
+}
 
 // ------------------------------------------------------------------ diffusive PND (pnd type 2)
-// MpsPndNeigh::calcPndDiffusiveTerm, src/MpsPndNeigh.cpp:334-489
+// MpsPndNeigh::calcPndDiffusiveTerm, src/MpsPndNeigh.cpp:334-489.  What is constant per
+// particle (the time step and density factors, n0 and n_i) multiplies the sums once (108k
+// particles: 161 -> 136 us).
+template <int L>
 __global__ void __launch_bounds__(BLK) k_pnd_diffusive(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
-    double ni = d.pndi[i];
+    const double ni = d.pndi[i];
     if (ni < P.epsilonZero) return;
-    dvec4 pi = d.pos[i], vi = d.vel[i];
-    dvec4 C1 = d.c1[i], C2 = d.c2[i], C3 = d.c3[i];
-    double Pi = d.press[i];
-    double rho = P.DNS_FL1;
-    bool fi = d.type[i] == P.fluid;
+    const dvec4 pi = d.pos[i], vi = d.vel[i];
+    const dvec4 C1 = d.c1[i], C2 = d.c2[i], C3 = d.c3[i];
+    const double Pi = d.press[i], rho = P.DNS_FL1;
+    const bool fi = d.type[i] == P.fluid;
+    // hydrostatic part: -2 rho rho / (rho + rho) g . r
+    const double kg = -2.0 * (rho * rho / (rho + rho));
+    const double gx = kg * P.gravity[0], gy = kg * P.gravity[1], gz = kg * P.gravity[2];
     double Di = 0.0, DivV = 0.0;
-    double cdiv = P.dim / P.pndSmallZero;
-    double invNi = 1.0 / ni;
     const Mask mL = d.maskL[i], mS = d.maskS[i] & mL;
     const double* wLc = d.cwL ? d.cwL : d.cw;
-    forMaskK(d, i, mL, [&](int j, size_t e, int k) {
-        dvec4 pj = d.pos[j];
-        double v0 = pj.x - pi.x, v1 = pj.y - pi.y, v2 = pj.z - pi.z;
-        double wL = wLc[e];
-        if (fi && d.type[j] == P.fluid) {
-            double pgh = -2.0 * (rho * rho / (rho + rho)) * (P.gravity[0] * v0 + P.gravity[1] * v1 + P.gravity[2] * v2);
-            Di += P.timeStep / rho * P.coeffViscMultiphase * (d.press[j] - Pi - pgh) * wL;
-        }
+    forMaskLane<L>(d, i, mL, l, [&](int j, size_t e, int k) {
+        const dvec4 pj = d.pos[j];
+        const double v0 = pj.x - pi.x, v1 = pj.y - pi.y, v2 = pj.z - pi.z;
+        if (fi && d.type[j] == P.fluid) Di += (d.press[j] - Pi - (gx * v0 + gy * v1 + gz * v2)) * wLc[e];
         if (maskHas(mS, k)) {
-            dvec4 vj = d.vel[j];
-            double vx = vj.x - vi.x, vy = vj.y - vi.y, vz = vj.z - vi.z;
-            double wd = d.cwd[e];   // wS / r^2
+            const dvec4 vj = d.vel[j];
+            const double vx = vj.x - vi.x, vy = vj.y - vi.y, vz = vj.z - vi.z;
+            const double wd = d.cwd[e];   // wS / r^2
             if (!P.gradientCorrection) {
-                DivV += cdiv * (d.pndi[j] * invNi) * (vx * v0 + vy * v1 + vz * v2) * wd;
+                DivV += d.pndi[j] * (vx * v0 + vy * v1 + vz * v2) * wd;
             } else {
-                double a0 = v0 * C1.x + v1 * C1.y + v2 * C1.z;
-                double a1 = v0 * C2.x + v1 * C2.y + v2 * C2.z;
-                double a2 = v0 * C3.x + v1 * C3.y + v2 * C3.z;
-                DivV += cdiv * (vx * a0 + vy * a1 + vz * a2) * wd;
+                const double a0 = v0 * C1.x + v1 * C1.y + v2 * C1.z;
+                const double a1 = v0 * C2.x + v1 * C2.y + v2 * C2.z;
+                const double a2 = v0 * C3.x + v1 * C3.y + v2 * C3.z;
+                DivV += (vx * a0 + vy * a1 + vz * a2) * wd;
             }
         }
     });
-    d.aux1[i] = d.pndi[i] * (1.0 + P.timeStep * (-DivV + Di * 1.0));
+    Di = laneSum<L>(Di); DivV = laneSum<L>(DivV);
+    if (l != 0) return;
+    Di *= P.timeStep / rho * P.coeffViscMultiphase;
+    DivV *= P.dim / P.pndSmallZero;
+    if (!P.gradientCorrection) DivV /= ni;
+    d.aux1[i] = ni * (1.0 + P.timeStep * (-DivV + Di * 1.0));
     d.velDiv[i] = DivV;
     d.diffTerm[i] = Di;
 }
 
 // MpsPndNeigh::calcWallSlipPndDiffusiveTerm / calcWallNoSlipPndDiffusiveTerm,
 // src/MpsPndNeigh.cpp:492-744 (fixed wall: wall velocity zero)
-__global__ void __launch_bounds__(BLK) k_wall_pnd_diffusive(Dev d) {
-    int i = nearIndex(d);
-    if (i < 0) return;
+__global__ void __launch_bounds__(WALL_BLK) k_wall_pnd_diffusive(Dev d) {
+    __shared__ double sm[32], R[9][32], vm[3][32];
     const MpsParams& P = d.P;
-    double ni = d.pndi[i];
-    if (!(ni > P.epsilonZero)) return;
-    bool noslip = P.slipCondition == 0;
-    dvec4 pi = d.pos[i], vi = d.vel[i], mi = d.mirror[i];
-    ReflG r = makeRefl(pi, mi, P.epsilonZero, false);
-    double vm[3];
-    if (noslip) { vm[0] = -vi.x; vm[1] = -vi.y; vm[2] = -vi.z; }
-    else {
-        vm[0] = r.R[0] * vi.x + r.R[1] * vi.y + r.R[2] * vi.z;
-        vm[1] = r.R[3] * vi.x + r.R[4] * vi.y + r.R[5] * vi.z;
-        vm[2] = r.R[6] * vi.x + r.R[7] * vi.y + r.R[8] * vi.z;
-    }
-    double cdiv = P.dim / P.pndSmallZero;
-    double DivV = 0.0;
-    auto term = [&](double vx, double vy, double vz, double m0, double m1, double m2, double dm2, double pj) {
-        double wS = wfun(sqrt(dm2), P.reS, P.weightType);
-        if (noslip) {
-            vx = -vx; vy = -vy; vz = -vz;
-            double a0 = r.R[0] * m0 + r.R[1] * m1 + r.R[2] * m2;
-            double a1 = r.R[3] * m0 + r.R[4] * m1 + r.R[5] * m2;
-            double a2 = r.R[6] * m0 + r.R[7] * m1 + r.R[8] * m2;
-            return cdiv * (pj / ni) * (vx * a0 + vy * a1 + vz * a2) * wS / dm2;
-        }
-        return cdiv * (pj / ni) * (vx * m0 + vy * m1 + vz * m2) * wS / dm2;
+    const bool noslip = P.slipCondition == 0;
+    const double cdiv = P.dim / P.pndSmallZero;
+    // cdiv (n_j / n_i) (v . m) w / |m|^2, the no-slip pair vectors reflected by R
+    auto term = [&](int g, double ni, double vx, double vy, double vz, const PairG& m, double wd, double nj) {
+        if (!noslip) return cdiv * (nj / ni) * (vx * m.v0 + vy * m.v1 + vz * m.v2) * wd;
+        const double a0 = R[0][g] * m.v0 + R[1][g] * m.v1 + R[2][g] * m.v2;
+        const double a1 = R[3][g] * m.v0 + R[4][g] * m.v1 + R[5][g] * m.v2;
+        const double a2 = R[6][g] * m.v0 + R[7][g] * m.v1 + R[8][g] * m.v2;
+        return -(cdiv * (nj / ni) * (vx * a0 + vy * a1 + vz * a2) * wd);
     };
-    forNbrs(d, i, [&](int j) {
-        dvec4 pj = d.pos[j];
-        PairG q = pairOf(pj, pi);
-        if (q.d2 < P.reS2) {
-            PairM m = pairMirror(pj, mi);
-            if (m.dm2 < P.reS2 && q.d2 < m.dm2) {
-                dvec4 vj = d.vel[j];
-                DivV += term(vj.x - vm[0], vj.y - vm[1], vj.z - vm[2], m.m0, m.m1, m.m2, m.dm2, d.pndi[j]);
-            }
+    forNearWall(d, [&](int i, int g) {
+        const dvec4 vi = d.vel[i];
+        const ReflG r = makeRefl(d.pos[i], d.mirror[i], P.epsilonZero, false);
+#pragma unroll
+        for (int k = 0; k < 9; k++) R[k][g] = r.R[k];
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+            vm[a][g] = noslip ? -(a == 0 ? vi.x : a == 1 ? vi.y : vi.z)
+                              : r.R[3 * a] * vi.x + r.R[3 * a + 1] * vi.y + r.R[3 * a + 2] * vi.z;
+    }, [&](int i, int g, int l) {
+        const double ni = d.pndi[i];
+        const dvec4 mi = d.mirror[i];
+        double div = 0.0;
+        if (ni > P.epsilonZero)
+            forBitsShared<WALL_L>(d.nbr + i, d.N0, d.mirrorS[i], l, [&](int j, int) {
+                const PairG m = pairSum(d.pos[j], mi);
+                double wS, wd;
+                weightR(m.d2, P.reS, P.weightType, wS, wd);
+                const dvec4 vj = d.vel[j];
+                div += term(g, ni, vj.x - vm[0][g], vj.y - vm[1][g], vj.z - vm[2][g], m, wd, d.pndi[j]);
+            });
+        div = laneSum<WALL_L>(div);
+        if (l == 0) sm[g] = div;
+    }, [&](int i, int g) {
+        const double ni = d.pndi[i];
+        if (!(ni > P.epsilonZero)) return;
+        const dvec4 pi = d.pos[i], vi = d.vel[i], mi = d.mirror[i];
+        double div = sm[g];
+        if (pairMirror(pi, mi).dm2 < P.reS2) {
+            const PairG m = pairSum(pi, mi);
+            double wS, wd;
+            weightR(m.d2, P.reS, P.weightType, wS, wd);
+            div += term(g, ni, vi.x - vm[0][g], vi.y - vm[1][g], vi.z - vm[2][g], m, wd, ni);
         }
+        d.aux1[i] += -ni * P.timeStep * div;
     });
-    PairM s = pairMirror(pi, mi);
-    if (s.dm2 < P.reS2) DivV += term(vi.x - vm[0], vi.y - vm[1], vi.z - vm[2], s.m0, s.m1, s.m2, s.dm2, ni);
-    d.aux1[i] += -ni * P.timeStep * DivV;
 }
 
 // MpsPndNeigh::updatePnd, src/MpsPndNeigh.cpp:747-774
@@ -774,8 +824,10 @@ __global__ void k_mean_pnd_wds_apply(Dev d) {
 }
 
 void launchPndDiffusive(const Dev& d, cudaStream_t s) {
-    k_pnd_diffusive<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
-    if (d.P.wallType == 1) k_wall_pnd_diffusive<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
+#define LAUNCH(L) k_pnd_diffusive<L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
+    if (d.P.wallType == 1) k_wall_pnd_diffusive<<<wallGrid(d.N0), WALL_BLK, 0, s>>>(d);
     k_update_pnd<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
     k_mean_pnd_wds<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
     k_mean_pnd_wds_apply<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
@@ -847,7 +899,7 @@ void launchPndMean(const Dev& d, cudaStream_t s) {
 }
 // step-0 sequence, src/main.cpp:158-166
 void launchInitPnd(const Dev& d, cudaStream_t s) {
-    k_pnd_npcd<1><<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
+    launchPndNpcd<1, false>(d, s);
     launchPndMean(d, s);
     k_mean_neigh_fluid_pnd<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
 }
@@ -1010,15 +1062,16 @@ __global__ void k_eos(Dev d) {
 void launchEOS(const Dev& d, cudaStream_t s) { k_eos<<<gridFor(d.N0, 256), 256, 0, s>>>(d); }
 
 // MpsPressure::extrapolatePressParticlesWallDummy, src/MpsPressure.cpp:792-846
+template <int L>
 __global__ void __launch_bounds__(BLK) k_extrapolate(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
     if (!(d.type[i] == P.dummyWall || (P.mpsType == 1 && d.type[i] == P.wall))) return;
-    dvec4 pi = d.pos[i];
+    const dvec4 pi = d.pos[i];
     double ni = 0.0, pr = 0.0;
     // particle walls: maskS is exactly dst^2 < reS^2 (no mirror side test)
-    forMask(d, i, d.maskS[i], [&](int j, size_t e) {
+    forMaskLane<L>(d, i, d.maskS[i], l, [&](int j, size_t e, int) {
         if (d.type[j] != P.fluid) return;
         dvec4 pj = d.pos[j];
         double v0 = pj.x - pi.x, v1 = pj.y - pi.y, v2 = pj.z - pi.z;
@@ -1026,60 +1079,81 @@ __global__ void __launch_bounds__(BLK) k_extrapolate(Dev d) {
         ni += wS;
         pr += (d.press[j] - P.DNS_FL1 * (P.gravity[0] * v0 + P.gravity[1] * v1 + P.gravity[2] * v2)) * wS;
     });
-    if (pr < 0.0) return;
+    ni = laneSum<L>(ni); pr = laneSum<L>(pr);
+    if (pr < 0.0 || l != 0) return;
     d.press[i] = (ni > 0) ? pr / ni : pr;
 }
-void launchExtrapolatePress(const Dev& d, cudaStream_t s) { k_extrapolate<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d); }
+void launchExtrapolatePress(const Dev& d, cudaStream_t s) {
+#define LAUNCH(L) k_extrapolate<L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
+}
 
 // ------------------------------------------------------------------ pressure gradient
-// MpsPressure::calcPressGradient, src/MpsPressure.cpp:1217-1338 (p_min sweep, then sum)
+__host__ __device__ __forceinline__ bool ratioGradient(int gt) { return gt != 0 && gt != 1 && gt != 2; }
+// p / n of every particle for gradient type 3 (a division per particle instead of one per pair)
+__global__ void k_press_ratio(Dev d) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= d.N0) return;
+    const double n = d.pndi[i];
+    d.pAux[i] = n > d.P.epsilonZero ? d.press[i] / n : 0.0;
+}
+// MpsPressure::calcPressGradient, src/MpsPressure.cpp:1217-1338 (p_min sweep, then sum).  The
+// correction matrix, constant per particle, multiplies the sum once: sum (C r) f = C (sum r f)
+// leaves 8 FP64 operations an entry for 17 (864k particles: 952 -> 450 us, type 3 at 108k:
+// 386 -> 90 us).
+template <int L>
 __global__ void __launch_bounds__(BLK) k_press_grad(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
-    dvec4 pi = d.pos[i];
-    double Pi = d.press[i], pmin = Pi, ni = d.pndi[i];
-    int gt = P.gradientType;
+    const dvec4 pi = d.pos[i];
+    const double Pi = d.press[i], ni = d.pndi[i];
+    const int gt = P.gradientType;
     const Mask mS = d.maskS[i];
+    double base = Pi;
     if (gt == 0 || gt == 2) {
-        forMask(d, i, mS, [&](int j, size_t e) {
-            double pj_ = d.press[j];
-            if (pmin > pj_) pmin = pj_;
-        });
+        double pmin = Pi;
+        forMaskLane<L>(d, i, mS, l, [&](int j, size_t, int) { minBits(pmin, d.press[j]); });
+#pragma unroll
+        for (int o = 1; o < L; o <<= 1) minBits(pmin, __shfl_xor_sync(laneGroup<L>(), pmin, o));
+        if (l == 0) d.pAux[i] = pmin;
+        base = gt == 0 ? -pmin : Pi - 2.0 * pmin;
     }
-    dvec4 C1 = d.c1[i], C2 = d.c2[i], C3 = d.c3[i];
+    const bool ratio = ratioGradient(gt);
+    const double qi = ratio ? d.pAux[i] : 0.0;
     double ax = 0, ay = 0, az = 0;
-    forMask(d, i, mS, [&](int j, size_t e) {
-        dvec4 pj = d.pos[j];
-        double v0 = pj.x - pi.x, v1 = pj.y - pi.y, v2 = pj.z - pi.z;
-        double Pj = d.press[j];
-        double wd = d.cwd[e];   // wS / r^2
+    forMaskLane<L>(d, i, mS, l, [&](int j, size_t e, int) {
+        const dvec4 pj = d.pos[j];
         double f;
-        if (gt == 0) f = (Pj - pmin) * wd;
-        else if (gt == 1) f = (Pj + Pi) * wd;
-        else if (gt == 2) f = (Pj + Pi - 2.0 * pmin) * wd;
+        if (!ratio) f = (d.press[j] + base) * d.cwd[e];   // cwd: wS / r^2
         else {
-            double nj = d.pndi[j];
-            f = (ni > P.epsilonZero && nj > P.epsilonZero) ? (ni * Pj / nj + nj * Pi / ni) * wd : d.cw[e];
+            const double nj = d.pndi[j];
+            f = (ni > P.epsilonZero && nj > P.epsilonZero) ? (ni * d.pAux[j] + nj * qi) * d.cwd[e] : d.cw[e];
         }
-        if (!P.gradientCorrection) { ax += v0 * f; ay += v1 * f; az += v2 * f; }
-        else {
-            ax += (v0 * C1.x + v1 * C1.y + v2 * C1.z) * f;
-            ay += (v0 * C2.x + v1 * C2.y + v2 * C2.z) * f;
-            az += (v0 * C3.x + v1 * C3.y + v2 * C3.z) * f;
-        }
+        ax += (pj.x - pi.x) * f; ay += (pj.y - pi.y) * f; az += (pj.z - pi.z) * f;
     });
-    d.acc[i] = make_dvec4(P.relaxPress * ax * P.coeffPressGrad / P.DNS_FL1,
-                          P.relaxPress * ay * P.coeffPressGrad / P.DNS_FL1,
-                          P.relaxPress * az * P.coeffPressGrad / P.DNS_FL1, 0.0);
+    ax = laneSum<L>(ax); ay = laneSum<L>(ay); az = laneSum<L>(az);
+    if (l != 0) return;
+    if (P.gradientCorrection) {
+        const dvec4 C1 = d.c1[i], C2 = d.c2[i], C3 = d.c3[i];
+        const double bx = C1.x * ax + C1.y * ay + C1.z * az, by = C2.x * ax + C2.y * ay + C2.z * az,
+                     bz = C3.x * ax + C3.y * ay + C3.z * az;
+        ax = bx; ay = by; az = bz;
+    }
+    d.acc[i] = make_dvec4(d.cPG * ax, d.cPG * ay, d.cPG * az, 0.0);
 }
-void launchPressGradient(const Dev& d, cudaStream_t s) { k_press_grad<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d); }
+void launchPressGradient(const Dev& d, cudaStream_t s) {
+    if (ratioGradient(d.P.gradientType)) k_press_ratio<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
+#define LAUNCH(L) k_press_grad<L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
+}
 
-// Wall term of the pressure gradient at a fluid particle near the polygon wall (Mitsume's
-// mirror model and the repulsive force), src/MpsPressure.cpp:1341-1611: the sums over the
-// candidates that forCand passes as f(j, pj, q), j != i, returned as
-// fac * R a * coeffPressGrad - f_rep (fac = relax_fact after the solve, 1 - relax_fact in
-// the prediction, src/MpsPressure.cpp:1031-1214).
+// Wall term of the prediction's pressure gradient at a fluid particle near the polygon wall
+// (Mitsume's mirror model and the repulsive force), src/MpsPressure.cpp:1031-1214: the sums
+// over the candidates that forCand passes as f(j, pj, q), j != i, returned as
+// fac * R a * coeffPressGrad - f_rep (fac = 1 - relax_fact).
 template <class C>
 __device__ __forceinline__ void wallGradTerm(const Dev& d, int i, dvec4 pi, double fac, C&& forCand, double g[3]) {
     const MpsParams& P = d.P;
@@ -1129,28 +1203,77 @@ __device__ __forceinline__ void wallGradTerm(const Dev& d, int i, dvec4 pi, doub
     g[2] = fac * (r.R[6] * ax + r.R[7] * ay + r.R[8] * az) * P.coeffPressGrad - f[2];
 }
 
-// MpsPressure::calcWallPressGradient + repulsive forces, src/MpsPressure.cpp:1341-1611,
-// over the post-prediction neighbour list.
-__global__ void __launch_bounds__(BLK) k_wall_press_grad(Dev d) {
-    int i = nearIndex(d);
-    if (i < 0) return;
+// MpsPressure::calcWallPressGradient + repulsive forces, src/MpsPressure.cpp:1341-1611, over
+// the entry masks of the post-prediction list: p_min over the entries inside reS off the
+// mirror side (maskS), the sums over the mirror entries.
+// fresh: p_min of those entries is the pressure gradient's, just written (pAux); type 3 finds
+// p / n there.
+__global__ void __launch_bounds__(WALL_BLK) k_wall_press_grad(Dev d, bool fresh) {
+    __shared__ double sm[3][32], pmn[32];
     const MpsParams& P = d.P;
-    dvec4 pi = d.pos[i];
-    double g[3];
-    wallGradTerm(d, i, pi, P.relaxPress, [&](auto&& f) {
-        forNbrs(d, i, [&](int j) { dvec4 pj = d.pos[j]; f(j, pj, pairOf(pj, pi)); });
-    }, g);
-    dvec4 a = d.acc[i];
-    a.x += g[0] / P.DNS_FL1; a.y += g[1] / P.DNS_FL1; a.z += g[2] / P.DNS_FL1;
-    d.acc[i] = a;
-    double vf = (P.dim == 3) ? P.partDist * P.partDist * P.partDist : P.partDist * P.partDist;
-    dvec4 fw = d.forceWall[i];
-    fw.x += -g[0] * vf; fw.y += -g[1] * vf; fw.z += -g[2] * vf;
-    d.forceWall[i] = fw;
+    const int gt = P.gradientType;
+    // min(velMax of the last corrector, expected maximum velocity)^2 (src/MpsPressure.cpp:1342-1344)
+    const double vm = fmin(*d.velMax, P.expectMaxVelocity);
+    // the gradient type's factor of the mirror pair, times w / |m|^2 (type 3 without PND: w)
+    auto phi = [&](int i, int j, double Pi, double ni, double pmin, double wS, double wd) {
+        if (gt == 0) return wd * (d.press[j] - pmin);
+        if (gt == 1) return wd * (d.press[j] + Pi);
+        if (gt == 2) return wd * (d.press[j] + Pi - 2.0 * pmin);
+        const double nj = d.pndi[j];
+        if (gt == 3 && ni > P.epsilonZero && nj > P.epsilonZero) return wd * (ni * d.pAux[j] + nj * d.pAux[i]);
+        return wS;
+    };
+    forNearWall(d, [](int, int) {}, [&](int i, int g, int l) {
+        const dvec4 mi = d.mirror[i];
+        const double Pi = d.press[i], ni = d.pndi[i];
+        double pmin = Pi;
+        if ((gt == 0 || gt == 2) && fresh) pmin = d.pAux[i];
+        else if (gt == 0 || gt == 2) {
+            forMaskLane<WALL_L>(d, i, d.maskS[i], l, [&](int j, size_t, int) { minBits(pmin, d.press[j]); });
+#pragma unroll
+            for (int o = 1; o < WALL_L; o <<= 1) minBits(pmin, __shfl_xor_sync(laneGroup<WALL_L>(), pmin, o));
+        }
+        double ax = 0, ay = 0, az = 0;
+        forBitsShared<WALL_L>(d.nbr + i, d.N0, d.mirrorS[i], l, [&](int j, int) {
+            const PairG m = pairSum(d.pos[j], mi);
+            double wS, wd;
+            weightR(m.d2, P.reS, P.weightType, wS, wd);
+            const double f = phi(i, j, Pi, ni, pmin, wS, wd);
+            ax += m.v0 * f; ay += m.v1 * f; az += m.v2 * f;
+        });
+        ax = laneSum<WALL_L>(ax); ay = laneSum<WALL_L>(ay); az = laneSum<WALL_L>(az);
+        if (l == 0) { sm[0][g] = ax; sm[1][g] = ay; sm[2][g] = az; pmn[g] = pmin; }
+    }, [&](int i, int g) {
+        const dvec4 pi = d.pos[i], mi = d.mirror[i];
+        const double Pi = d.press[i], ni = d.pndi[i];
+        const ReflG r = makeRefl(pi, mi, P.epsilonZero, true);
+        double ax = sm[0][g], ay = sm[1][g], az = sm[2][g];
+        if (pairMirror(pi, mi).dm2 < P.reS2) {
+            const PairG m = pairSum(pi, mi);
+            double wS, wd;
+            weightR(m.d2, P.reS, P.weightType, wS, wd);
+            const double f = phi(i, i, Pi, ni, pmn[g], wS, wd);
+            ax += m.v0 * f; ay += m.v1 * f; az += m.v2 * f;
+        }
+        double fr[3];
+        wallRepulsion(P, r, vm * vm, fr);
+        double gr[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+            gr[a] = P.relaxPress * (r.R[3 * a] * ax + r.R[3 * a + 1] * ay + r.R[3 * a + 2] * az) * P.coeffPressGrad - fr[a];
+        dvec4 a = d.acc[i];
+        a.x += gr[0] / P.DNS_FL1; a.y += gr[1] / P.DNS_FL1; a.z += gr[2] / P.DNS_FL1;
+        d.acc[i] = a;
+        const double vf = (P.dim == 3) ? P.partDist * P.partDist * P.partDist : P.partDist * P.partDist;
+        dvec4 fw = d.forceWall[i];
+        fw.x += -gr[0] * vf; fw.y += -gr[1] * vf; fw.z += -gr[2] * vf;
+        d.forceWall[i] = fw;
+    });
 }
-void launchWallPressGradient(const Dev& d, cudaStream_t s) {
+void launchWallPressGradient(const Dev& d, cudaStream_t s, bool fresh) {
     if (d.P.wallType != 1) return;
-    k_wall_press_grad<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
+    if (d.P.gradientType == 3 && !fresh) k_press_ratio<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
+    k_wall_press_grad<<<wallGrid(d.N0), WALL_BLK, 0, s>>>(d, fresh);
 }
 
 // ------------------------------------------------------------------ prediction-step pressure gradient
@@ -1246,63 +1369,67 @@ void launchPredictPressGradient(const Dev& d, bool skin, cudaStream_t s) {
 // ------------------------------------------------------------------ wall viscosity
 // MpsViscosity::calcWallNoSlipViscosity / calcWallSlipViscosity (Newtonian, fixed wall),
 // src/MpsViscosity.cpp:1527-1910
-__global__ void __launch_bounds__(BLK) k_wall_visc(Dev d) {
-    int i = nearIndex(d);
-    if (i < 0) return;
-    const MpsParams& P = d.P;
-    bool noslip = P.slipCondition == 0;
-    dvec4 pi = d.pos[i], vi = d.vel[i], mi = d.mirror[i];
-    ReflG r = makeRefl(pi, mi, P.epsilonZero, false);
-    double M[9];
-    if (noslip) {
+__device__ __forceinline__ void wallViscMatrix(const MpsParams& P, dvec4 pi, dvec4 mi, double M[9]) {
+    if (P.slipCondition == 0) {   // no-slip: -I
 #pragma unroll
         for (int k = 0; k < 9; k++) M[k] = (k % 4 == 0) ? -1.0 : 0.0;
-    } else {
+        return;
+    }
+    const ReflG r = makeRefl(pi, mi, P.epsilonZero, false);
 #pragma unroll
-        for (int k = 0; k < 9; k++) M[k] = r.R[k];
-    }
-    double vm0 = M[0] * vi.x + M[1] * vi.y + M[2] * vi.z;
-    double vm1 = M[3] * vi.x + M[4] * vi.y + M[5] * vi.z;
-    double vm2 = M[6] * vi.x + M[7] * vi.y + M[8] * vi.z;
-    double mu = P.KNM_VS1 * P.DNS_FL1;
-    double neu = ((mu + mu) > P.epsilonZero ? 2.0 * mu * mu / (mu + mu) : 0.0) / P.DNS_FL1;
-    double ax = 0, ay = 0, az = 0;
-    forNbrs(d, i, [&](int j) {
-        dvec4 pj = d.pos[j];
-        PairG q = pairOf(pj, pi);
-        if (q.d2 < P.reL2) {
-            PairM m = pairMirror(pj, mi);
-            if (m.dm2 < P.reL2 && q.d2 < m.dm2) {
-                double wL = wfun(sqrt(m.dm2), P.reL, P.weightType);
-                dvec4 vj = d.vel[j];
-                ax += (vj.x - vm0) * wL * neu;
-                ay += (vj.y - vm1) * wL * neu;
-                az += (vj.z - vm2) * wL * neu;
-            }
+    for (int k = 0; k < 9; k++) M[k] = r.R[k];
+}
+__global__ void __launch_bounds__(WALL_BLK) k_wall_visc(Dev d) {
+    __shared__ double sm[3][32], vm[3][32];
+    const MpsParams& P = d.P;
+    const double mu = P.KNM_VS1 * P.DNS_FL1;
+    const double neu = ((mu + mu) > P.epsilonZero ? 2.0 * mu * mu / (mu + mu) : 0.0) / P.DNS_FL1;
+    forNearWall(d, [&](int i, int g) {
+        const dvec4 vi = d.vel[i];
+        double M[9];
+        wallViscMatrix(P, d.pos[i], d.mirror[i], M);
+#pragma unroll
+        for (int a = 0; a < 3; a++) vm[a][g] = M[3 * a] * vi.x + M[3 * a + 1] * vi.y + M[3 * a + 2] * vi.z;
+    }, [&](int i, int g, int l) {
+        const dvec4 mi = d.mirror[i];
+        double ax = 0, ay = 0, az = 0;
+        forBitsShared<WALL_L>(d.nbr + i, d.N0, d.mirrorL[i], l, [&](int j, int) {
+            double wL, wd;
+            weightR(pairSum(d.pos[j], mi).d2, P.reL, P.weightType, wL, wd);
+            const dvec4 vj = d.vel[j];
+            const double f = wL * neu;
+            ax += (vj.x - vm[0][g]) * f; ay += (vj.y - vm[1][g]) * f; az += (vj.z - vm[2][g]) * f;
+        });
+        ax = laneSum<WALL_L>(ax); ay = laneSum<WALL_L>(ay); az = laneSum<WALL_L>(az);
+        if (l == 0) { sm[0][g] = ax; sm[1][g] = ay; sm[2][g] = az; }
+    }, [&](int i, int g) {
+        const dvec4 pi = d.pos[i], vi = d.vel[i], mi = d.mirror[i];
+        double M[9];
+        wallViscMatrix(P, pi, mi, M);
+        double ax = sm[0][g], ay = sm[1][g], az = sm[2][g];
+        PairM s = pairMirror(pi, mi);
+        if (s.dm2 < P.reL2) {
+            double wL = wfun(sqrt(s.dm2), P.reL, P.weightType);
+            double neuS = (mu > P.epsilonZero ? 2.0 * mu * mu / (mu + mu) : 0.0) / P.DNS_FL1;
+            ax += (vi.x - vm[0][g]) * wL * neuS;
+            ay += (vi.y - vm[1][g]) * wL * neuS;
+            az += (vi.z - vm[2][g]) * wL * neuS;
         }
+        double f0 = (M[0] * ax + M[1] * ay + M[2] * az) * P.coeffViscMultiphase;
+        double f1 = (M[3] * ax + M[4] * ay + M[5] * az) * P.coeffViscMultiphase;
+        double f2 = (M[6] * ax + M[7] * ay + M[8] * az) * P.coeffViscMultiphase;
+        dvec4 a = d.acc[i];
+        a.x += f0; a.y += f1; a.z += f2;
+        d.acc[i] = a;
+        double vf = (P.dim == 3) ? P.partDist * P.partDist * P.partDist : P.partDist * P.partDist;
+        dvec4 fw = d.forceWall[i];
+        fw.x += -f0 * vf * P.DNS_FL1; fw.y += -f1 * vf * P.DNS_FL1; fw.z += -f2 * vf * P.DNS_FL1;
+        d.forceWall[i] = fw;
     });
-    PairM s = pairMirror(pi, mi);
-    if (s.dm2 < P.reL2) {
-        double wL = wfun(sqrt(s.dm2), P.reL, P.weightType);
-        double neuS = (mu > P.epsilonZero ? 2.0 * mu * mu / (mu + mu) : 0.0) / P.DNS_FL1;
-        ax += (vi.x - vm0) * wL * neuS;
-        ay += (vi.y - vm1) * wL * neuS;
-        az += (vi.z - vm2) * wL * neuS;
-    }
-    double f0 = (M[0] * ax + M[1] * ay + M[2] * az) * P.coeffViscMultiphase;
-    double f1 = (M[3] * ax + M[4] * ay + M[5] * az) * P.coeffViscMultiphase;
-    double f2 = (M[6] * ax + M[7] * ay + M[8] * az) * P.coeffViscMultiphase;
-    dvec4 a = d.acc[i];
-    a.x += f0; a.y += f1; a.z += f2;
-    d.acc[i] = a;
-    double vf = (P.dim == 3) ? P.partDist * P.partDist * P.partDist : P.partDist * P.partDist;
-    dvec4 fw = d.forceWall[i];
-    fw.x += -f0 * vf * P.DNS_FL1; fw.y += -f1 * vf * P.DNS_FL1; fw.z += -f2 * vf * P.DNS_FL1;
-    d.forceWall[i] = fw;
 }
 void launchWallViscosity(const Dev& d, cudaStream_t s) {
     if (d.P.wallType != 1) return;
-    k_wall_visc<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
+    k_wall_visc<<<wallGrid(d.N0), WALL_BLK, 0, s>>>(d);
 }
 
 // ------------------------------------------------------------------ corrector

@@ -9,6 +9,7 @@
 // the reference's FP64 expression, so entry sets, masks and flags equal the FP64 tier's.
 #include "mps_df.cuh"
 #include "mps_internal.h"
+#include "mps_lanes.cuh"
 
 #define BLK 128
 
@@ -69,43 +70,6 @@ void launchNeighborListDF(const Dev& d, cudaStream_t s) {
     launchPosf(d, s);
     k_build_nbr_df<false><<<gridFor(d.N0, 128), 128, 0, s>>>(d);
     k_build_nbr_df<true><<<gridFor(d.N0, 128), 128, 0, s>>>(d);
-}
-
-// ------------------------------------------------------------------ entry masks
-__global__ void __launch_bounds__(128, 10) k_side_masks_df(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= liveN(d)) return;
-    const MpsParams& P = d.P;
-    int c = d.nbrCount[i];
-    const Mask all = maskFirst(c);
-    dvec4 pi = d.pos[i];
-    SideDF sc = sideDF(d, i, pi);
-    bool fullS = P.reS2 >= d.reMax2, fullL = P.reL2 >= d.reMax2;
-    Mask mS = all, mL = all;
-    if (sc.check || !fullS || !fullL) {
-        mS = maskNone(); mL = maskNone();
-        float4 hi = d.posf[i], li = d.posLo[i];
-        const df RS = K(d.k.reS2), RL = K(d.k.reL2);
-        const int* row = d.nbr + i;
-        for (int k = 0; k < c; k++) {
-            int j = ldStream(row + (size_t)k * d.N0);
-            float4 hj = d.posf[j], lj = d.posLo[j];
-            df d2 = norm2(diff3(hj, lj, hi, li));
-            if (!sideOkDF(d, sc, hj, lj, d2, i, j)) continue;
-            if (fullS || inBallDF(d, d2, RS, d.mgS, P.reS2, i, j)) maskSet(mS, k);
-            if (fullL || inBallDF(d, d2, RL, d.mgL, P.reL2, i, j)) maskSet(mL, k);
-        }
-    }
-    d.maskS[i] = mS;
-    d.maskL[i] = mL;
-    if (P.wallType == 1 && d.type[i] == P.fluid && d.nearWall[i]) {
-        int slot = atomicAdd(d.nearCount, 1);
-        d.nearList[slot] = i;
-    }
-}
-void launchSideMasksDF(const Dev& d, cudaStream_t s) {
-    cudaMemsetAsync(d.nearCount, 0, sizeof(int), s);
-    k_side_masks_df<<<gridFor(d.N0, 128), 128, 0, s>>>(d);
 }
 
 // ------------------------------------------------------------------ viscosity
@@ -240,9 +204,14 @@ void launchCollisionDF(const Dev& d, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------ wall sweeps
-__device__ __forceinline__ int nearIndexDF(const Dev& d) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    return (t < *d.nearCount) ? d.nearList[t] : -1;
+template <int L>
+__device__ __forceinline__ df laneSumDF(df v) {
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1) {
+        const df q = {__shfl_xor_sync(laneGroup<L>(), v.h, o), __shfl_xor_sync(laneGroup<L>(), v.l, o)};
+        v += q;
+    }
+    return v;
 }
 struct MirrorDF {
     float4 mh, ml;
@@ -254,59 +223,40 @@ __device__ __forceinline__ MirrorDF mirrorDF(const Dev& d, dvec4 m) {
     o.ml = posLoOf(m, o.mh, P);
     return o;
 }
-// One wall-sweep entry: j within R of i, its mirror image within R of the mirror of i
-// and j not on the mirror side (e.g. src/MpsPndNeigh.cpp:140-160).  Returns the mirror
-// pair (x_j - m_i, |x_j - m_i|^2) through m.
-// hj: the entry's FP32 copy (posf[j]); band: the FP32 upper bound of the radius R (an
-// entry above it is outside the ball, and its lo part is never read)
-__device__ __forceinline__ bool wallEntryDF(const Dev& d, int i, int j, float4 hj, float4 hi, float4 li,
-                                            const MirrorDF& M, df R2f, float mg, double R2, float band, PairF& m) {
-    const float ex = hj.x - hi.x, ey = hj.y - hi.y, ez = hj.z - hi.z;
-    if (ex * ex + ey * ey + ez * ez > band) return false;
-    const float4 lj = __ldg(&d.posLo[j]);
-    PairF q = pairDF(hj, lj, hi, li);
-    if (!inBallDF(d, q.d2, R2f, mg, R2, i, j)) return false;
-    m = pairDF(hj, lj, M.mh, M.ml);
-    if (!lessDF(m.d2, R2f, mg, [&] { return pairMirror(d.pos[j], d.mirror[i]).dm2 < R2; })) return false;
-    return lessDF(q.d2, m.d2, d.mgSide, [&] {
-        dvec4 pj = d.pos[j];
-        return pairOf(pj, d.pos[i]).d2 < pairMirror(pj, d.mirror[i]).dm2;
-    });
-}
-
 // MpsPndNeigh::calcWallNPCD, src/MpsPndNeigh.cpp:105-195
-__global__ void __launch_bounds__(BLK) k_wall_npcd_df(Dev d) {
-    int i = nearIndexDF(d);
-    if (i < 0) return;
+__global__ void __launch_bounds__(WALL_BLK) k_wall_npcd_df(Dev d) {
+    __shared__ double sm[3][32];
     const MpsParams& P = d.P;
-    dvec4 pi = d.pos[i], mi = d.mirror[i];
-    ReflG r = makeRefl(pi, mi, P.epsilonZero, true);
-    float4 hi = d.posf[i], li = d.posLo[i];
-    MirrorDF M = mirrorDF(d, mi);
-    const df R2 = K(d.k.reS2);
     const RadiusDF RS = {K(d.k.reS), K(d.k.invReS)};
-    df sx = dfF(0.f), sy = dfF(0.f), sz = dfF(0.f);
-    forNbrsPosf(d, i, [&](int j, float4 hj) {
-        PairF m;
-        if (!wallEntryDF(d, i, j, hj, hi, li, M, R2, d.mgS, P.reS2, d.bandHiS, m)) return;
-        df wS = weightDF(m.d2, RS, P.weightType).w;
-        sx += m.v.x * wS; sy += m.v.y * wS; sz += m.v.z * wS;
+    forNearWall(d, [](int, int) {}, [&](int i, int g, int l) {
+        const MirrorDF M = mirrorDF(d, d.mirror[i]);
+        df sx = dfF(0.f), sy = dfF(0.f), sz = dfF(0.f);
+        forBitsShared<WALL_L>(d.nbr + i, d.N0, d.mirrorS[i], l, [&](int j, int) {
+            const PairF m = pairDF(__ldg(&d.posf[j]), __ldg(&d.posLo[j]), M.mh, M.ml);
+            const df wS = weightDF(m.d2, RS, P.weightType).w;
+            sx += m.v.x * wS; sy += m.v.y * wS; sz += m.v.z * wS;
+        });
+        sx = laneSumDF<WALL_L>(sx); sy = laneSumDF<WALL_L>(sy); sz = laneSumDF<WALL_L>(sz);
+        if (l == 0) { sm[0][g] = dD(sx); sm[1][g] = dD(sy); sm[2][g] = dD(sz); }
+    }, [&](int i, int g) {
+        const dvec4 pi = d.pos[i], mi = d.mirror[i];
+        const ReflG r = makeRefl(pi, mi, P.epsilonZero, true);
+        double dx = sm[0][g], dy = sm[1][g], dz = sm[2][g];
+        PairM s = pairMirror(pi, mi);
+        if (s.dm2 < P.reS2) {
+            double wS = wfun(sqrt(s.dm2), P.reS, P.weightType);
+            dx += s.m0 * wS; dy += s.m1 * wS; dz += s.m2 * wS;
+        }
+        dvec4 n = d.npcd[i];
+        n.x += r.R[0] * dx + r.R[1] * dy + r.R[2] * dz;
+        n.y += r.R[3] * dx + r.R[4] * dy + r.R[5] * dz;
+        n.z += r.R[6] * dx + r.R[7] * dy + r.R[8] * dz;
+        d.npcd[i] = n;
     });
-    double dx = dD(sx), dy = dD(sy), dz = dD(sz);
-    PairM s = pairMirror(pi, mi);
-    if (s.dm2 < P.reS2) {
-        double wS = wfun(sqrt(s.dm2), P.reS, P.weightType);
-        dx += s.m0 * wS; dy += s.m1 * wS; dz += s.m2 * wS;
-    }
-    dvec4 n = d.npcd[i];
-    n.x += r.R[0] * dx + r.R[1] * dy + r.R[2] * dz;
-    n.y += r.R[3] * dx + r.R[4] * dy + r.R[5] * dz;
-    n.z += r.R[6] * dx + r.R[7] * dy + r.R[8] * dz;
-    d.npcd[i] = n;
 }
 void launchWallNpcdDF(const Dev& d, cudaStream_t s) {
     if (d.P.wallType != 1) return;
-    k_wall_npcd_df<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
+    k_wall_npcd_df<<<wallGrid(d.N0), WALL_BLK, 0, s>>>(d);
 }
 
 // ------------------------------------------------------------------ correction matrix
@@ -521,6 +471,7 @@ __global__ void __launch_bounds__(BLK, 9) k_press_grad_df(Dev d) {
             df pj = loadDF(d.pressDF, j);
             if (pmin > pj) pmin = pj;
         });
+        ((float2*)d.pAux)[i] = make_float2(pmin.h, pmin.l);   // for the wall term
     }
     df base = (gt == 0) ? -pmin : (gt == 1 ? Pi : Pi - pmin - pmin);
     // sum of r_ij f_ij; with gradient correction C (constant per particle) is applied to
@@ -555,143 +506,147 @@ void launchPressGradientDF(const Dev& d, cudaStream_t s) {
 }
 
 // MpsPressure::calcWallPressGradient + repulsive forces, src/MpsPressure.cpp:1341-1611
-__global__ void __launch_bounds__(BLK) k_wall_press_grad_df(Dev d) {
-    int i = nearIndexDF(d);
-    if (i < 0) return;
+__global__ void __launch_bounds__(WALL_BLK) k_wall_press_grad_df(Dev d, bool fresh) {
+    __shared__ double sm[3][32], pmn[32];
     const MpsParams& P = d.P;
-    double vm = fmin(*d.velMax, P.expectMaxVelocity);
-    double vMax2 = vm * vm;
-    dvec4 pi = d.pos[i], mi = d.mirror[i];
-    float4 hi = d.posf[i], li = d.posLo[i];
-    MirrorDF M = mirrorDF(d, mi);
-    const df R2 = K(d.k.reS2);
+    const int gt = P.gradientType;
+    const double vm = fmin(*d.velMax, P.expectMaxVelocity);
     const RadiusDF RS = {K(d.k.reS), K(d.k.invReS)};
-    double Pid = d.press[i], ni = d.pndi[i];
-    df Pi = loadDF(d.pressDF, i), pmin = Pi;
-    int gt = P.gradientType;
-    ReflG r = makeRefl(pi, mi, P.epsilonZero, true);
-    if (gt == 0 || gt == 2) {
-        forNbrs(d, i, [&](int j) {
-            float4 hj = d.posf[j], lj = d.posLo[j];
-            PairF q = pairDF(hj, lj, hi, li);
-            if (!inBallDF(d, q.d2, R2, d.mgS, P.reS2, i, j)) return;
-            df dm2 = norm2(diff3(hj, lj, M.mh, M.ml));
-            bool side = lessDF(q.d2, dm2, d.mgSide, [&] {
-                dvec4 pj = d.pos[j];
-                return pairOf(pj, pi).d2 < pairMirror(pj, mi).dm2;
+    forNearWall(d, [](int, int) {}, [&](int i, int g, int l) {
+        const MirrorDF M = mirrorDF(d, d.mirror[i]);
+        const double Pid = d.press[i], ni = d.pndi[i];
+        const df Pi = loadDF(d.pressDF, i);
+        df pmin = Pi;
+        if ((gt == 0 || gt == 2) && fresh) pmin = loadDF((const float2*)d.pAux, i);
+        else if (gt == 0 || gt == 2) {
+            forMaskLane<WALL_L>(d, i, d.maskS[i], l, [&](int j, size_t, int) {
+                const df pj = loadDF(d.pressDF, j);
+                if (pmin > pj) pmin = pj;
             });
-            if (side) { df pj = loadDF(d.pressDF, j); if (pmin > pj) pmin = pj; }
-        });
-    }
-    df base = (gt == 0) ? -pmin : (gt == 1 ? Pi : Pi - pmin - pmin);
-    df sx = dfF(0.f), sy = sx, sz = sx;
-    forNbrs(d, i, [&](int j) {
-        PairF m;
-        if (!wallEntryDF(d, i, j, d.posf[j], hi, li, M, R2, d.mgS, P.reS2, d.bandHiS, m)) return;
-        WeightDF w = weightDF(m.d2, RS, P.weightType);
-        df f;
-        if (gt <= 2) f = (loadDF(d.pressDF, j) + base) * w.wr2;
-        else {
-            double nj = d.pndi[j], Pj = d.press[j];
-            f = (ni > P.epsilonZero && nj > P.epsilonZero) ? dfD(ni * Pj / nj + nj * Pid / ni) * w.wr2 : w.w;
+#pragma unroll
+            for (int o = 1; o < WALL_L; o <<= 1) {
+                const df q = {__shfl_xor_sync(laneGroup<WALL_L>(), pmin.h, o), __shfl_xor_sync(laneGroup<WALL_L>(), pmin.l, o)};
+                if (pmin > q) pmin = q;
+            }
         }
-        sx += m.v.x * f; sy += m.v.y * f; sz += m.v.z * f;
+        const df base = (gt == 0) ? -pmin : (gt == 1 ? Pi : Pi - pmin - pmin);
+        df sx = dfF(0.f), sy = sx, sz = sx;
+        forBitsShared<WALL_L>(d.nbr + i, d.N0, d.mirrorS[i], l, [&](int j, int) {
+            const PairF m = pairDF(__ldg(&d.posf[j]), __ldg(&d.posLo[j]), M.mh, M.ml);
+            const WeightDF w = weightDF(m.d2, RS, P.weightType);
+            df f;
+            if (gt <= 2) f = (loadDF(d.pressDF, j) + base) * w.wr2;
+            else {
+                double nj = d.pndi[j], Pj = d.press[j];
+                f = (ni > P.epsilonZero && nj > P.epsilonZero) ? dfD(ni * Pj / nj + nj * Pid / ni) * w.wr2 : w.w;
+            }
+            sx += m.v.x * f; sy += m.v.y * f; sz += m.v.z * f;
+        });
+        sx = laneSumDF<WALL_L>(sx); sy = laneSumDF<WALL_L>(sy); sz = laneSumDF<WALL_L>(sz);
+        if (l == 0) { sm[0][g] = dD(sx); sm[1][g] = dD(sy); sm[2][g] = dD(sz); pmn[g] = dD(pmin); }
+    }, [&](int i, int g) {
+        const dvec4 pi = d.pos[i], mi = d.mirror[i];
+        const double Pid = d.press[i], ni = d.pndi[i], pmind = pmn[g];
+        const ReflG r = makeRefl(pi, mi, P.epsilonZero, true);
+        double ax = sm[0][g], ay = sm[1][g], az = sm[2][g];
+        PairM s = pairMirror(pi, mi);
+        if (s.dm2 < P.reS2) {
+            double wS = wfun(sqrt(s.dm2), P.reS, P.weightType);
+            if (gt == 0) wS = wS * ((Pid - pmind) / s.dm2);
+            else if (gt == 1) wS = wS * ((Pid + Pid) / s.dm2);
+            else if (gt == 2) wS = wS * ((Pid + Pid - 2.0 * pmind) / s.dm2);
+            else if (gt == 3 && ni > P.epsilonZero) wS = wS * ((ni * Pid / ni + ni * Pid / ni) / s.dm2);
+            ax += s.m0 * wS; ay += s.m1 * wS; az += s.m2 * wS;
+        }
+        double f[3];
+        wallRepulsion(P, r, vm * vm, f);
+        double gr[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+            gr[a] = P.relaxPress * (r.R[3 * a] * ax + r.R[3 * a + 1] * ay + r.R[3 * a + 2] * az) * P.coeffPressGrad - f[a];
+        dvec4 a = d.acc[i];
+        a.x += gr[0] / P.DNS_FL1; a.y += gr[1] / P.DNS_FL1; a.z += gr[2] / P.DNS_FL1;
+        d.acc[i] = a;
+        double vf = (P.dim == 3) ? P.partDist * P.partDist * P.partDist : P.partDist * P.partDist;
+        dvec4 fw = d.forceWall[i];
+        fw.x += -gr[0] * vf; fw.y += -gr[1] * vf; fw.z += -gr[2] * vf;
+        d.forceWall[i] = fw;
     });
-    double ax = dD(sx), ay = dD(sy), az = dD(sz);
-    double pmind = dD(pmin);
-    auto phi = [&](double Pj, double nj, double dm2, double wS) {
-        if (gt == 0) return wS * ((Pj - pmind) / dm2);
-        if (gt == 1) return wS * ((Pj + Pid) / dm2);
-        if (gt == 2) return wS * ((Pj + Pid - 2.0 * pmind) / dm2);
-        if (gt == 3 && ni > P.epsilonZero && nj > P.epsilonZero) return wS * ((ni * Pj / nj + nj * Pid / ni) / dm2);
-        return wS;
-    };
-    PairM s = pairMirror(pi, mi);
-    if (s.dm2 < P.reS2) {
-        double wS = wfun(sqrt(s.dm2), P.reS, P.weightType);
-        wS = phi(Pid, ni, s.dm2, wS);
-        ax += s.m0 * wS; ay += s.m1 * wS; az += s.m2 * wS;
-    }
-    double f[3];
-    wallRepulsion(P, r, vMax2, f);
-    double g0 = P.relaxPress * (r.R[0] * ax + r.R[1] * ay + r.R[2] * az) * P.coeffPressGrad - f[0];
-    double g1 = P.relaxPress * (r.R[3] * ax + r.R[4] * ay + r.R[5] * az) * P.coeffPressGrad - f[1];
-    double g2 = P.relaxPress * (r.R[6] * ax + r.R[7] * ay + r.R[8] * az) * P.coeffPressGrad - f[2];
-    dvec4 a = d.acc[i];
-    a.x += g0 / P.DNS_FL1; a.y += g1 / P.DNS_FL1; a.z += g2 / P.DNS_FL1;
-    d.acc[i] = a;
-    double vf = (P.dim == 3) ? P.partDist * P.partDist * P.partDist : P.partDist * P.partDist;
-    dvec4 fw = d.forceWall[i];
-    fw.x += -g0 * vf; fw.y += -g1 * vf; fw.z += -g2 * vf;
-    d.forceWall[i] = fw;
 }
-void launchWallPressGradientDF(const Dev& d, cudaStream_t s) {
+void launchWallPressGradientDF(const Dev& d, cudaStream_t s, bool fresh) {
     if (d.P.wallType != 1) return;
-    launchPressDF(d, s);
-    k_wall_press_grad_df<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
+    if (!fresh) launchPressDF(d, s);
+    k_wall_press_grad_df<<<wallGrid(d.N0), WALL_BLK, 0, s>>>(d, fresh);
 }
 
 // ------------------------------------------------------------------ wall viscosity
 // MpsViscosity::calcWallNoSlipViscosity / calcWallSlipViscosity, src/MpsViscosity.cpp:1527-1910
-__global__ void __launch_bounds__(BLK) k_wall_visc_df(Dev d) {
-    int i = nearIndexDF(d);
-    if (i < 0) return;
+__global__ void __launch_bounds__(WALL_BLK) k_wall_visc_df(Dev d) {
+    __shared__ double sm[3][32], vm[3][32];
     const MpsParams& P = d.P;
-    bool noslip = P.slipCondition == 0;
-    dvec4 pi = d.pos[i], vi = d.vel[i], mi = d.mirror[i];
-    ReflG r = makeRefl(pi, mi, P.epsilonZero, false);
-    double M[9];
-    if (noslip) {
+    const bool noslip = P.slipCondition == 0;
+    const double mu = P.KNM_VS1 * P.DNS_FL1;
+    const df neuF = K(d.k.neuWall);
+    const RadiusDF RL = {K(d.k.reL), K(d.k.invReL)};
+    auto matrix = [&](int i, double M[9]) {
+        if (noslip) {
 #pragma unroll
-        for (int k = 0; k < 9; k++) M[k] = (k % 4 == 0) ? -1.0 : 0.0;
-    } else {
+            for (int k = 0; k < 9; k++) M[k] = (k % 4 == 0) ? -1.0 : 0.0;
+            return;
+        }
+        const ReflG r = makeRefl(d.pos[i], d.mirror[i], P.epsilonZero, false);
 #pragma unroll
         for (int k = 0; k < 9; k++) M[k] = r.R[k];
-    }
-    double vm0 = M[0] * vi.x + M[1] * vi.y + M[2] * vi.z;
-    double vm1 = M[3] * vi.x + M[4] * vi.y + M[5] * vi.z;
-    double vm2 = M[6] * vi.x + M[7] * vi.y + M[8] * vi.z;
-    df vmx = dfD(vm0), vmy = dfD(vm1), vmz = dfD(vm2);
-    double mu = P.KNM_VS1 * P.DNS_FL1;
-    const df neuF = K(d.k.neuWall);
-    float4 hi = d.posf[i], li = d.posLo[i];
-    MirrorDF Mi = mirrorDF(d, mi);
-    const df R2 = K(d.k.reL2);
-    const RadiusDF RL = {K(d.k.reL), K(d.k.invReL)};
-    df sx = dfF(0.f), sy = sx, sz = sx;
-    forNbrsPosf(d, i, [&](int j, float4 hj) {
-        PairF m;
-        if (!wallEntryDF(d, i, j, hj, hi, li, Mi, R2, d.mgL, P.reL2, d.bandHiL, m)) return;
-        df c = weightDF(m.d2, RL, P.weightType).w * neuF;
-        float4 vhj = d.velHi[j], vlj = d.velLo[j];
-        sx += (dfOf(vhj.x, vlj.x) - vmx) * c;
-        sy += (dfOf(vhj.y, vlj.y) - vmy) * c;
-        sz += (dfOf(vhj.z, vlj.z) - vmz) * c;
+    };
+    forNearWall(d, [&](int i, int g) {
+        const dvec4 vi = d.vel[i];
+        double M[9];
+        matrix(i, M);
+#pragma unroll
+        for (int a = 0; a < 3; a++) vm[a][g] = M[3 * a] * vi.x + M[3 * a + 1] * vi.y + M[3 * a + 2] * vi.z;
+    }, [&](int i, int g, int l) {
+        const MirrorDF Mi = mirrorDF(d, d.mirror[i]);
+        const df vmx = dfD(vm[0][g]), vmy = dfD(vm[1][g]), vmz = dfD(vm[2][g]);
+        df sx = dfF(0.f), sy = sx, sz = sx;
+        forBitsShared<WALL_L>(d.nbr + i, d.N0, d.mirrorL[i], l, [&](int j, int) {
+            const PairF m = pairDF(__ldg(&d.posf[j]), __ldg(&d.posLo[j]), Mi.mh, Mi.ml);
+            const df c = weightDF(m.d2, RL, P.weightType).w * neuF;
+            float4 vhj = d.velHi[j], vlj = d.velLo[j];
+            sx += (dfOf(vhj.x, vlj.x) - vmx) * c;
+            sy += (dfOf(vhj.y, vlj.y) - vmy) * c;
+            sz += (dfOf(vhj.z, vlj.z) - vmz) * c;
+        });
+        sx = laneSumDF<WALL_L>(sx); sy = laneSumDF<WALL_L>(sy); sz = laneSumDF<WALL_L>(sz);
+        if (l == 0) { sm[0][g] = dD(sx); sm[1][g] = dD(sy); sm[2][g] = dD(sz); }
+    }, [&](int i, int g) {
+        const dvec4 pi = d.pos[i], vi = d.vel[i], mi = d.mirror[i];
+        double M[9];
+        matrix(i, M);
+        double ax = sm[0][g], ay = sm[1][g], az = sm[2][g];
+        PairM s = pairMirror(pi, mi);
+        if (s.dm2 < P.reL2) {
+            double wL = wfun(sqrt(s.dm2), P.reL, P.weightType);
+            double neuS = (mu > P.epsilonZero ? 2.0 * mu * mu / (mu + mu) : 0.0) / P.DNS_FL1;
+            ax += (vi.x - vm[0][g]) * wL * neuS;
+            ay += (vi.y - vm[1][g]) * wL * neuS;
+            az += (vi.z - vm[2][g]) * wL * neuS;
+        }
+        double f0 = (M[0] * ax + M[1] * ay + M[2] * az) * P.coeffViscMultiphase;
+        double f1 = (M[3] * ax + M[4] * ay + M[5] * az) * P.coeffViscMultiphase;
+        double f2 = (M[6] * ax + M[7] * ay + M[8] * az) * P.coeffViscMultiphase;
+        dvec4 a = d.acc[i];
+        a.x += f0; a.y += f1; a.z += f2;
+        d.acc[i] = a;
+        double vf = (P.dim == 3) ? P.partDist * P.partDist * P.partDist : P.partDist * P.partDist;
+        dvec4 fw = d.forceWall[i];
+        fw.x += -f0 * vf * P.DNS_FL1; fw.y += -f1 * vf * P.DNS_FL1; fw.z += -f2 * vf * P.DNS_FL1;
+        d.forceWall[i] = fw;
     });
-    double ax = dD(sx), ay = dD(sy), az = dD(sz);
-    PairM s = pairMirror(pi, mi);
-    if (s.dm2 < P.reL2) {
-        double wL = wfun(sqrt(s.dm2), P.reL, P.weightType);
-        double neuS = (mu > P.epsilonZero ? 2.0 * mu * mu / (mu + mu) : 0.0) / P.DNS_FL1;
-        ax += (vi.x - vm0) * wL * neuS;
-        ay += (vi.y - vm1) * wL * neuS;
-        az += (vi.z - vm2) * wL * neuS;
-    }
-    double f0 = (M[0] * ax + M[1] * ay + M[2] * az) * P.coeffViscMultiphase;
-    double f1 = (M[3] * ax + M[4] * ay + M[5] * az) * P.coeffViscMultiphase;
-    double f2 = (M[6] * ax + M[7] * ay + M[8] * az) * P.coeffViscMultiphase;
-    dvec4 a = d.acc[i];
-    a.x += f0; a.y += f1; a.z += f2;
-    d.acc[i] = a;
-    double vf = (P.dim == 3) ? P.partDist * P.partDist * P.partDist : P.partDist * P.partDist;
-    dvec4 fw = d.forceWall[i];
-    fw.x += -f0 * vf * P.DNS_FL1; fw.y += -f1 * vf * P.DNS_FL1; fw.z += -f2 * vf * P.DNS_FL1;
-    d.forceWall[i] = fw;
 }
 void launchWallViscosityDF(const Dev& d, cudaStream_t s) {
     if (d.P.wallType != 1) return;
     launchVelDF(d, s);
-    k_wall_visc_df<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
+    k_wall_visc_df<<<wallGrid(d.N0), WALL_BLK, 0, s>>>(d);
 }
 
 // ------------------------------------------------------------------ shifting

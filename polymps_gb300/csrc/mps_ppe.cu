@@ -20,6 +20,7 @@
 #include <algorithm>
 #include "mps_bulk.cuh"
 #include "mps_grid.cuh"
+#include "mps_lanes.cuh"
 
 #define PBLK 256
 
@@ -28,51 +29,71 @@ enum { S_RZ = 0, S_RR, S_BB, S_ALPHA, S_BETA, S_PAP, S_THR, S_RZNEW, S_SCALE, S_
        S_RHO, S_RHOOLD, S_OMEGA, S_R0N2, S_COUNT };
 
 // ------------------------------------------------------------------ assembly
+// The row of particle i by L lanes.  Dummy-wall neighbours (their hydrostatic source term, 12
+// FP64 operations) are left to a second walk over the few there are: in the loop, every entry
+// of every particle paid for them (864k particles without any: 596 -> 172 us).
+template <int L>
 __global__ void __launch_bounds__(128) k_ppe_assemble(Dev d, PpeBuffers B) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
-    int bci = d.bc[i];
+    const int bci = d.bc[i];
     if (bci == P.other || bci == P.surface) {
-        B.diag[i] = 1.0; B.rowLen[i] = 0; B.b[i] = 0.0; B.mfMask[i] = maskNone();
+        if (l == 0) { B.diag[i] = 1.0; B.rowLen[i] = 0; B.b[i] = 0.0; B.mfMask[i] = maskNone(); }
         warpCount(d.counters + 1, 0u);
         return;
     }
-    dvec4 pi = d.pos[i];
     double sum = 0.0, src = 0.0;
-    int len = 0;
-    Mask mm = maskNone();
+    Mask mm = maskNone(), dm = maskNone();
     const double* wLc = d.cwL ? d.cwL : d.cw;
-    forMaskK(d, i, d.maskL[i], [&](int j, size_t e, int ke) {
-        double wL = wLc[e];
-        double mij = wL * P.coeffPPE;
-        if (d.type[j] == P.dummyWall) {
-            dvec4 pj = d.pos[j];
-            double v0 = pj.x - pi.x, v1 = pj.y - pi.y, v2 = pj.z - pi.z;
-            double pgh = P.DNS_FL1 * (v0 * P.gravity[0] + v1 * P.gravity[1] + v2 * P.gravity[2]) * wL;
-            src -= P.coeffPPE * pgh;
-        } else {
-            sum -= mij;
-            if (d.bc[j] == P.inner) {
-                size_t k = ellBase(B, i) + (size_t)len * B.ellStride;
-                B.val[k] = mij;
-                B.col[k] = j;
-                len++;
-                maskSet(mm, ke);
-            }
-        }
+    const Mask mL = d.maskL[i];
+    const size_t base = ellBase(B, i);
+    int len = 0;
+    if (L > 1) {   // the matrix entries of the whole row first: an entry's place is its rank
+        forMaskLane<L>(d, i, mL, l, [&](int j, size_t, int k) {
+            if (d.type[j] != P.dummyWall && d.bc[j] == P.inner) maskSet(mm, k);
+        });
+        mm = laneOr<L>(mm);
+        len = maskCount(mm);
+    }
+    forMaskLane<L>(d, i, mL, l, [&](int j, size_t e, int k) {
+        if (d.type[j] == P.dummyWall) { maskSet(dm, k); return; }
+        const double mij = wLc[e] * P.coeffPPE;
+        sum -= mij;
+        if (d.bc[j] != P.inner) return;
+        int at;
+        if (L > 1) at = maskRank(mm, k);
+        else { at = len++; maskSet(mm, k); }
+        B.val[base + (size_t)at * B.ellStride] = mij;
+        B.col[base + (size_t)at * B.ellStride] = j;
     });
-    double rho = P.DNS_FL1;
-    sum -= P.alphaCompressibility * rho / (P.timeStep * P.timeStep);
-    B.diag[i] = sum;
-    B.rowLen[i] = len;
-    B.mfMask[i] = mm;
-    B.b[i] = src + ppeSource(d, i, rho);
-    warpCount(d.counters + 1, (unsigned)len);
+    if (dm.lo | dm.hi) {
+        const dvec4 pi = d.pos[i];
+        forBits(d.nbr + i, d.N0, dm, [&](int j, int k) {
+            const dvec4 pj = d.pos[j];
+            const double v0 = pj.x - pi.x, v1 = pj.y - pi.y, v2 = pj.z - pi.z;
+            const double pgh = P.DNS_FL1 * (v0 * P.gravity[0] + v1 * P.gravity[1] + v2 * P.gravity[2]) *
+                               wLc[(size_t)k * d.N0 + i];
+            src -= P.coeffPPE * pgh;
+        });
+    }
+    sum = laneSum<L>(sum);
+    src = laneSum<L>(src);
+    if (l == 0) {
+        const double rho = P.DNS_FL1;
+        sum -= P.alphaCompressibility * rho / (P.timeStep * P.timeStep);
+        B.diag[i] = sum;
+        B.rowLen[i] = len;
+        B.mfMask[i] = mm;
+        B.b[i] = src + ppeSource(d, i, rho);
+    }
+    warpCount(d.counters + 1, l == 0 ? (unsigned)len : 0u);
 }
 void launchPpeAssemble(const Dev& d, const PpeBuffers& B, cudaStream_t s) {
     cudaMemsetAsync(d.counters + 1, 0, sizeof(unsigned long long), s);
-    k_ppe_assemble<<<gridFor(d.N0, 128), 128, 0, s>>>(d, B);
+#define LAUNCH(L) k_ppe_assemble<L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d, B)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
 }
 
 // press = max(x, 0) (setZeroOnNegativePressure, src/MpsPressure.cpp:471-476); x is kept
