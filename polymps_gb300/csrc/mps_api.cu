@@ -487,14 +487,15 @@ static int runOpBody(mpsgpu_t h, int op) {
                 countLaunch(6 + (P.shiftingType == 1 ? 3 : (P.wallType == 1 ? 7 : 4)));
                 h->opSkipped = true;
             } else if (!x && h->skinShift && (P.shiftingType == 1 || P.shiftingType == 2)) {
-                // FP64: the same list (no weight cache), then the operators' sweeps over it
+                // FP64: the same list, with its weights (type 2), and the operators' sweeps over it
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(PROF_NEIGHBOR_LIST, s, false); }
-                launchNeighborFilter(d, s, false);
+                launchNeighborFilter(d, s, P.shiftingType == 2);
+                launchSideMasks(d, s);
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(MPS_OP_SHIFTING, s, false); }
                 launchShifting(d, s, true);
                 invalidate();
-                // posf + cell copy, skin check, filter (2); then the sweeps and applies
-                countLaunch(5 + (P.shiftingType == 1 ? 2 : (P.wallType == 1 ? 6 : 3)));
+                // posf + cell copy, skin check, filter (2), masks; then the sweeps and applies
+                countLaunch(6 + (P.shiftingType == 1 ? 2 : (P.wallType == 1 ? 6 : 3)));
                 h->opSkipped = true;
             } else {
                 if (x) launchShiftingDF(d, s); else launchShifting(d, s, false);

@@ -387,9 +387,6 @@ void launchNeighborList(const Dev& d, cudaStream_t s) {
 // radius take every entry without per-entry work.  Fluid particles near the wall also get
 // their mirror entries and are appended to nearList for the wall-only sweeps, which walk the
 // masks instead of testing the list again.
-static __device__ __noinline__ bool mirrorInsideExact(const dvec4* pos, const dvec4* mirror, int j, int i, double R2) {
-    return pairMirror(pos[j], mirror[i]).dm2 < R2;
-}
 template <int L>
 __global__ void __launch_bounds__(128) k_side_masks(Dev d) {
     const int i = laneRow<L>(), l = laneOf<L>();
@@ -451,4 +448,14 @@ void launchSideMasks(const Dev& d, cudaStream_t s) {
 #define LAUNCH(L) k_side_masks<L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d)
     MPS_FOR_LANES(d.N0, LAUNCH);
 #undef LAUNCH
+}
+
+// nearList for the current positions, where no list and no masks are built
+__global__ void k_near_list(Dev d) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < liveN(d) && d.type[i] == d.P.fluid && d.nearWall[i]) d.nearList[atomicAdd(d.nearCount, 1)] = i;
+}
+void launchNearList(const Dev& d, cudaStream_t s) {
+    cudaMemsetAsync(d.nearCount, 0, sizeof(int), s);
+    k_near_list<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
 }

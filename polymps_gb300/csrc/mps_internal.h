@@ -39,7 +39,8 @@ int renumberLaunches();
 void launchNeighborList(const Dev& d, cudaStream_t s);
 void launchPosf(const Dev& d, cudaStream_t s);       // FP32 copy, then its bucket-ordered copy
 void launchPosfCell(const Dev& d, cudaStream_t s);   // bucket-ordered copy only
-void launchSideMasks(const Dev& d, cudaStream_t s);
+void launchSideMasks(const Dev& d, cudaStream_t s);   // also nearList and the mirror masks
+void launchNearList(const Dev& d, cudaStream_t s);
 void launchFillCache(const Dev& d, cudaStream_t s);
 
 // mps_ops.cu
@@ -69,7 +70,7 @@ void launchWallPressGradient(const Dev& d, cudaStream_t s, bool fresh);
 void launchPredictPressGradient(const Dev& d, bool skin, cudaStream_t s);   // relax_fact < 1, before PREDICT
 void launchWallViscosity(const Dev& d, cudaStream_t s);
 void launchCorrect(const Dev& d, cudaStream_t s);
-void launchShifting(const Dev& d, cudaStream_t s, bool list);   // list: filter the kept skin list first
+void launchShifting(const Dev& d, cudaStream_t s, bool list);   // list: filter and masks of these positions are built
 void launchDummyVelocity(const Dev& d, cudaStream_t s);
 
 // mps_ops_df.cu (DF32 tier)
@@ -99,6 +100,7 @@ void launchViscosityListDF(const Dev& d, cudaStream_t s);
 void launchSkinCheck(const Dev& d, cudaStream_t s);
 void launchShiftVelApply(const Dev& d, cudaStream_t s);
 void launchApplyShift(const Dev& d, cudaStream_t s);
+void launchApplyShiftNear(const Dev& d, cudaStream_t s);   // the particles of nearList
 
 // mps_wall.cu
 void launchWallDistance(const Dev& d, cudaStream_t s);

@@ -7,7 +7,7 @@
 // a decision takes the reference's FP64 expression, out of line) and leave a bit mask; then
 // the FP64 sums walk the set bits, so the lanes of a warp stay in step through them.
 #pragma once
-#include "mps_common.cuh"
+#include "mps_df.cuh"
 
 // Lanes per particle for n particles.  From 40k particles on the sweeps are bound by the FP64
 // pipe and one lane per particle keeps its lanes busiest; below, the chip is not full and a
@@ -80,6 +80,9 @@ __device__ __forceinline__ bool lessPos(double a, double b) {
 // entry and their FP64 operations then run for all of them.
 static __device__ __noinline__ bool pairInsideExact(const dvec4* pos, int j, int i, double R2) {
     return pairOf(pos[j], pos[i]).d2 < R2;
+}
+static __device__ __noinline__ bool mirrorInsideExact(const dvec4* pos, const dvec4* mirror, int j, int i, double R2) {
+    return pairMirror(pos[j], mirror[i]).dm2 < R2;
 }
 static __device__ __noinline__ bool pairSideExact(const dvec4* pos, const dvec4* mirror, int j, int i) {
     const dvec4 pj = pos[j];
@@ -232,4 +235,119 @@ __device__ __forceinline__ void forNearWall(const Dev& d, Pre&& pre, Sum&& sum, 
         if (head) post(d.nearList[own], (int)threadIdx.x);
         __syncthreads();
     }
+}
+
+// Mirror entries of the near-wall particles at positions that have no list (the shifting's wall
+// term, whose first sweep has just moved them).  A warp takes 8 of the block's 32 particles one
+// after another and tests a particle's candidates with all its lanes: the start-of-step skin
+// list while that covers the particle (skin: the flag of the last k_skin_check), else the nine
+// bucket rows of its window.  The entries are left in cand[g] in scan order, their number in
+// num[g] (-1: more than WALL_CAND); the caller synchronises, then forWallCand walks them.
+#define WALL_CAND 128
+struct WallCand {
+    int cand[32][WALL_CAND];
+    int num[32];
+};
+__device__ __forceinline__ void wallCandidates(const Dev& d, WallCand& W, int base, int nn, bool skin) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const MpsParams& P = d.P;
+    for (int q = 0; q < 8; q++) {
+        const int g = warp * 8 + q;
+        if (base + g >= nn) break;
+        const int i = d.nearList[base + g];
+        const dvec4 pi = d.pos[i];
+        const float4 fi = d.posf[i], mf = posfOf(d.mirror[i], P);
+        int cnt = 0;
+        auto test = [&](int j, float4 fj) {
+            const float d2f = dist2f(fj, fi);
+            if (d2f > d.bandHiS || j == i) return false;
+            const float dm2f = dist2f(fj, mf);
+            if (dm2f > d.bandHiS) return false;
+            if (!insideF(d, d2f, d.bandLoS, d.bandHiS, P.reS2, i, j)) return false;
+            if (!(dm2f < d.bandLoS) && !mirrorInsideExact(d.pos, d.mirror, j, i, P.reS2)) return false;
+            const float t = dm2f - d2f;
+            if (t > d.sideBand) return true;
+            if (t < -d.sideBand) return false;
+            return pairSideExact(d.pos, d.mirror, j, i);
+        };
+        auto append = [&](bool in, int j) {
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            const int k = cnt + __popc(m & ((1u << lane) - 1u));
+            if (in && k < WALL_CAND) W.cand[g][k] = j;
+            cnt += __popc(m);
+        };
+        const int c = skin ? d.skinCnt[i] : d.K + 1;
+        if (c <= d.K && d.skinCell[i] == cellKeyOf(d, pi, fi)) {
+            for (int k0 = 0; k0 < c; k0 += 32) {
+                bool in = false;
+                int j = i;
+                if (k0 + lane < c) {
+                    j = ldStream(d.skinNbr + (size_t)(k0 + lane) * d.N0 + i);
+                    in = test(j, __ldg(&d.posf[j]));
+                }
+                append(in, j);
+            }
+        } else {
+            int ix, iy, iz;
+            bucketCoordsHi(d, pi, fi, ix, iy, iz);
+            const int nr = d.dz3 ? 9 : 3;
+            int a = 0, b = 0;
+            if (lane < nr) {
+                const long long jb = (long long)((iz - 1) * d.dz3 + lane / 3) * P.numBucketsXY +
+                                     (long long)(iy - 1 + lane % 3) * P.numBucketsX + ix;
+                const long long lo = jb - 1 > 0 ? jb - 1 : 0, hi = jb + 1 < d.nB - 1 ? jb + 1 : d.nB - 1;
+                if (lo <= hi) { a = d.cellStart[lo]; b = d.cellStart[hi + 1]; }
+            }
+            for (int r = 0; r < nr; r++) {
+                const int s0 = __shfl_sync(0xffffffffu, a, r), s1 = __shfl_sync(0xffffffffu, b, r);
+                for (int t = s0; t < s1; t += 32) {
+                    bool in = false;
+                    int j = i;
+                    if (t + lane < s1) {
+                        j = __ldg(d.cellSorted + t + lane);
+                        in = test(j, __ldg(&d.posf[j]));
+                    }
+                    append(in, j);
+                }
+            }
+        }
+        if (lane == 0) W.num[g] = cnt <= WALL_CAND ? cnt : -1;
+    }
+}
+// f(j) for lane l's share of the mirror entries of particle i = the block's g-th; one lane scans
+// the buckets for a particle with more entries than were kept.
+template <class F>
+__device__ __forceinline__ void forWallCand(const Dev& d, const WallCand& W, int i, int g, int l, F&& f) {
+    const int n = W.num[g];
+    for (int t = l; t < n; t += WALL_L) f(W.cand[g][t]);
+    if (n >= 0 || l != 0) return;
+    const dvec4 pi = d.pos[i], mi = d.mirror[i];
+    forCells(d, pi, [&](int j) {
+        const dvec4 pj = d.pos[j];
+        const double d2 = pairOf(pj, pi).d2, dm2 = pairMirror(pj, mi).dm2;
+        if (j != i && d2 < d.P.reS2 && dm2 < d.P.reS2 && d2 < dm2) f(j);
+    });
+}
+
+// End of the shifting's wall term at particle i (src/MpsShifting.cpp:640-691): its own image,
+// the reflection, and the shift of inner particles.
+__device__ __forceinline__ void wallGradConcEnd(const Dev& d, int i, double dx, double dy, double dz) {
+    const MpsParams& P = d.P;
+    const dvec4 pi = d.pos[i], mi = d.mirror[i];
+    const ReflG r = makeRefl(pi, mi, P.epsilonZero, true);
+    const double ci = d.conc[i];
+    const PairM s = pairMirror(pi, mi);
+    if (s.dm2 < P.reS2) {
+        const double f = (ci + ci) * wfun(sqrt(s.dm2), P.reS, P.weightType) / s.dm2;
+        dx += f * s.m0; dy += f * s.m1; dz += f * s.m2;
+    }
+    const double g0 = -(r.R[0] * dx + r.R[1] * dy + r.R[2] * dz) * P.coeffPressGrad;
+    const double g1 = -(r.R[3] * dx + r.R[4] * dy + r.R[5] * dz) * P.coeffPressGrad;
+    const double g2 = -(r.R[6] * dx + r.R[7] * dy + r.R[8] * dz) * P.coeffPressGrad;
+    dvec4 g = d.gradC[i];
+    g.x += g0; g.y += g1; g.z += g2;
+    d.gradC[i] = g;
+    d.shift[i] = d.bc[i] == P.inner
+                     ? make_dvec4(-P.coeffShifting2 * g0, -P.coeffShifting2 * g1, -P.coeffShifting2 * g2, 0.0)
+                     : make_dvec4(0, 0, 0, 0);
 }

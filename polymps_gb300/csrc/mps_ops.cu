@@ -1493,8 +1493,10 @@ struct OpShiftVel {
         st.vi = d.vel[i]; st.ux = st.uy = st.uz = 0.0;
     }
     __device__ void visit(const Dev& d, int i, State& st, int j, dvec4 pj, PairG q) const {
-        if (!E2Base::accept(d, st.c, pj, q)) return;
-        double dw = dwfun(sqrt(q.d2), d.P.reS, d.P.weightType);
+        if (E2Base::accept(d, st.c, pj, q)) add(d, st, j, q.d2);
+    }
+    __device__ __forceinline__ void add(const Dev& d, State& st, int j, double d2) const {
+        double dw = dwfun(sqrt(d2), d.P.reS, d.P.weightType);
         dvec4 vj = d.vel[j];
         st.ux += dw * (vj.x - st.vi.x); st.uy += dw * (vj.y - st.vi.y); st.uz += dw * (vj.z - st.vi.z);
     }
@@ -1553,47 +1555,42 @@ struct OpGradConc {
         d.shift[i] = sh;
     }
 };
-// MpsShifting::calcWallConcAndConcGradient, src/MpsShifting.cpp:578-691
-__global__ void __launch_bounds__(BLK) k_wall_grad_conc(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= liveN(d)) return;
+// MpsShifting::calcWallConcAndConcGradient, src/MpsShifting.cpp:578-691, at the shifted
+// positions: 40 us at 108k particles (449 as a 27-bucket FP64 scan of one thread each; float-
+// float at 2.8M 427 -> 218).
+__global__ void __launch_bounds__(WALL_BLK) k_wall_grad_conc(Dev d, bool skin) {
+    __shared__ WallCand W;
+    __shared__ double sm[3][32];
     const MpsParams& P = d.P;
-    dvec4 sh = make_dvec4(0, 0, 0, 0);
-    if (d.type[i] == P.fluid && d.nearWall[i]) {
-        dvec4 pi = d.pos[i], mi = d.mirror[i];
-        double ci = d.conc[i];
-        ReflG r = makeRefl(pi, mi, P.epsilonZero, true);
-        double dx = 0, dy = 0, dz = 0;
-        forCellsNear(d, pi, d.posf[i], d.bandHiS, [&](int j, dvec4 pj, PairG q) {
-            if (q.d2 < P.reS2 && j != i) {
-                PairM m = pairMirror(pj, mi);
-                if (m.dm2 < P.reS2 && q.d2 < m.dm2) {
-                    double wS = wfun(sqrt(m.dm2), P.reS, P.weightType);
-                    double cc = ci + d.conc[j];
-                    dx += cc * m.m0 * wS / m.dm2; dy += cc * m.m1 * wS / m.dm2; dz += cc * m.m2 * wS / m.dm2;
-                }
-            }
-        });
-        PairM s = pairMirror(pi, mi);
-        if (s.dm2 < P.reS2) {
-            double wS = wfun(sqrt(s.dm2), P.reS, P.weightType);
-            dx += (ci + ci) * s.m0 * wS / s.dm2; dy += (ci + ci) * s.m1 * wS / s.dm2; dz += (ci + ci) * s.m2 * wS / s.dm2;
+    const int nn = *d.nearCount;
+    const bool useSkin = skin && !*(volatile int*)d.skinFlag;
+    for (int base = blockIdx.x * 32; base < nn; base += gridDim.x * 32) {
+        wallCandidates(d, W, base, nn, useSkin);
+        __syncthreads();
+        const int g = threadIdx.x / WALL_L, l = threadIdx.x & (WALL_L - 1);
+        if (base + g < nn) {
+            const int i = d.nearList[base + g];
+            const dvec4 mi = d.mirror[i];
+            const double ci = d.conc[i];
+            double dx = 0, dy = 0, dz = 0;
+            forWallCand(d, W, i, g, l, [&](int j) {
+                const PairG m = pairSum(d.pos[j], mi);
+                double wS, wd;
+                weightR(m.d2, P.reS, P.weightType, wS, wd);
+                const double cc = (ci + d.conc[j]) * wd;
+                dx += cc * m.v0; dy += cc * m.v1; dz += cc * m.v2;
+            });
+            dx = laneSum<WALL_L>(dx); dy = laneSum<WALL_L>(dy); dz = laneSum<WALL_L>(dz);
+            if (l == 0) { sm[0][g] = dx; sm[1][g] = dy; sm[2][g] = dz; }
         }
-        double g0 = -(r.R[0] * dx + r.R[1] * dy + r.R[2] * dz) * P.coeffPressGrad;
-        double g1 = -(r.R[3] * dx + r.R[4] * dy + r.R[5] * dz) * P.coeffPressGrad;
-        double g2 = -(r.R[6] * dx + r.R[7] * dy + r.R[8] * dz) * P.coeffPressGrad;
-        dvec4 g = d.gradC[i];
-        g.x += g0; g.y += g1; g.z += g2;
-        d.gradC[i] = g;
-        if (d.bc[i] == P.inner)
-            sh = make_dvec4(-P.coeffShifting2 * g0, -P.coeffShifting2 * g1, -P.coeffShifting2 * g2, 0.0);
+        __syncthreads();
+        if (threadIdx.x < 32 && base + (int)threadIdx.x < nn)
+            wallGradConcEnd(d, d.nearList[base + threadIdx.x], sm[0][threadIdx.x], sm[1][threadIdx.x], sm[2][threadIdx.x]);
+        __syncthreads();
     }
-    d.shift[i] = sh;
 }
 // x += shift; the FP32 copy follows the new positions (next prefiltered scan)
-__global__ void k_apply_shift(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= liveN(d)) return;
+__device__ __forceinline__ void applyShift(const Dev& d, int i) {
     dvec4 x = d.pos[i], s = d.shift[i];
     x.x += s.x; x.y += s.y; x.z += s.z;
     d.pos[i] = x;
@@ -1602,56 +1599,96 @@ __global__ void k_apply_shift(Dev d) {
     d.posf[i] = hi;
     d.posLo[i] = posLoOf(x, hi, d.P);
 }
+__global__ void k_apply_shift(Dev d) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < liveN(d)) applyShift(d, i);
+}
+// the same for the particles near the wall
+__global__ void k_apply_shift_near(Dev d) {
+    const int n = *d.nearCount;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) applyShift(d, d.nearList[t]);
+}
 void launchShiftVelApply(const Dev& d, cudaStream_t s) { k_shift_vel_apply<<<gridFor(d.N0, 256), 256, 0, s>>>(d); }
 void launchApplyShift(const Dev& d, cudaStream_t s) { k_apply_shift<<<gridFor(d.N0, 256), 256, 0, s>>>(d); }
-// A 27-bucket sweep over the list of the current positions instead of the buckets: the
-// list holds every candidate within reMax of the scan, in the scan's order, and each
-// operator applies its own exact radius and side tests, so it sees the same neighbours in
-// the same order (the same sums).
-template <class Op>
-__global__ void __launch_bounds__(128) k_list_scan(Dev d, Op op) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= liveN(d)) return;
-    typename Op::State st;
-    op.begin(d, i, st);
-    if (op.active(d, st)) {
-        const dvec4 pi = d.pos[i];
-        const int c = d.nbrCount[i];
-        const int* row = d.nbr + i;
-        for (int k = 0; k < c; k++) {
-            const int j = ldStream(row + (size_t)k * d.N0);
-            const dvec4 pj = d.pos[j];
-            op.visit(d, i, st, j, pj, pairOf(pj, pi));
-        }
-    }
-    op.end(d, i, st);
+void launchApplyShiftNear(const Dev& d, cudaStream_t s) {
+    const int grid = gridFor(d.N0, 256) < 608 ? gridFor(d.N0, 256) : 608;
+    k_apply_shift_near<<<grid, 256, 0, s>>>(d);
 }
-template <class Op>
-static void launchSweep(const Dev& d, const Op& op, bool list, cudaStream_t s) {
-    if (list) k_list_scan<Op><<<gridFor(d.N0, 128), 128, 0, s>>>(d, op);
-    else launchScan(d, op, s);
+// The 27-bucket sweeps over the list of the post-corrector positions instead: its maskS
+// entries (inside reS, off the mirror side) are the scan's neighbours in the scan's order.
+template <int L>
+__global__ void __launch_bounds__(128) k_shift_vel_list(Dev d) {
+    const int i = laneRow<L>(), l = laneOf<L>();
+    if (i >= liveN(d)) return;
+    const OpShiftVel op;
+    OpShiftVel::State st;
+    const bool on = d.type[i] == d.P.fluid;
+    st.c.on = on;
+    st.vi = d.vel[i]; st.ux = st.uy = st.uz = 0.0;
+    const dvec4 pi = d.pos[i];
+    if (on) forMaskLane<L>(d, i, d.maskS[i], l, [&](int j, size_t, int) { op.add(d, st, j, pairSum(d.pos[j], pi).d2); });
+    st.ux = laneSum<L>(st.ux); st.uy = laneSum<L>(st.uy); st.uz = laneSum<L>(st.uz);
+    if (l == 0) op.end(d, i, st);
+}
+template <int L>
+__global__ void __launch_bounds__(128) k_conc_list(Dev d) {
+    const int i = laneRow<L>(), l = laneOf<L>();
+    if (i >= liveN(d)) return;
+    double sum = 0.0;
+    forMaskLane<L>(d, i, d.maskS[i], l, [&](int, size_t e, int) { sum += d.cw[e]; });
+    sum = laneSum<L>(sum);
+    if (l == 0) d.conc[i] = (sum + d.pndWall[i]) / d.P.pndSmallZero;
+}
+template <int L>
+__global__ void __launch_bounds__(128) k_grad_conc_list(Dev d) {
+    const int i = laneRow<L>(), l = laneOf<L>();
+    if (i >= liveN(d)) return;
+    OpGradConc::State st;
+    st.c.on = d.type[i] == d.P.fluid;
+    st.ci = d.conc[i]; st.gx = st.gy = st.gz = 0.0;
+    const dvec4 pi = d.pos[i];
+    if (st.c.on)
+        forMaskLane<L>(d, i, d.maskS[i], l, [&](int j, size_t e, int) {
+            const dvec4 pj = d.pos[j];
+            const double cc = (st.ci + d.conc[j]) * d.cwd[e];
+            st.gx += cc * (pj.x - pi.x); st.gy += cc * (pj.y - pi.y); st.gz += cc * (pj.z - pi.z);
+        });
+    st.gx = laneSum<L>(st.gx); st.gy = laneSum<L>(st.gy); st.gz = laneSum<L>(st.gz);
+    if (l == 0) OpGradConc().end(d, i, st);
 }
 
-// list: the sweeps read the list of the post-corrector positions, filtered from the kept
-// start-of-step skin list (launchNeighborFilter without the weight cache, which also
-// refreshes the FP32 copies) just before; else they scan the buckets
+// list: the sweeps read the list of the post-corrector positions with its weights and masks,
+// filtered from the kept start-of-step skin list just before (108k particles: concentration
+// and gradient 22 + 67 us beside a filter of 130, for 165 + 210 with the weights formed in
+// each beside one of 24); else they scan the buckets
 void launchShifting(const Dev& d, cudaStream_t s, bool list) {
     const MpsParams& P = d.P;
     if (P.shiftingType != 1 && P.shiftingType != 2) return;
     if (!list) launchPosf(d, s);   // post-corrector positions
+#define LAUNCH_VEL(L) k_shift_vel_list<L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d)
+#define LAUNCH_CONC(L)                                          \
+    k_conc_list<L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d);   \
+    k_grad_conc_list<L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d)
     if (P.shiftingType == 1) {
-        launchSweep(d, OpShiftVel(), list, s);
+        if (list) MPS_FOR_LANES(d.N0, LAUNCH_VEL);
+        else launchScan(d, OpShiftVel(), s);
         k_shift_vel_apply<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
     } else {
-        launchSweep(d, OpConc(), list, s);
-        launchSweep(d, OpGradConc(), list, s);
+        if (list) MPS_FOR_LANES(d.N0, LAUNCH_CONC);
+        else {
+            launchScan(d, OpConc(), s);
+            launchScan(d, OpGradConc(), s);
+        }
         k_apply_shift<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
-        if (P.wallType == 1) {
-            launchPosfCell(d, s);   // the wall sweep sees the shifted positions
-            k_wall_grad_conc<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
-            k_apply_shift<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
+        if (P.wallType == 1) {   // the wall sweep sees the shifted positions
+            if (list) launchSkinCheck(d, s);
+            else launchNearList(d, s);
+            k_wall_grad_conc<<<wallGrid(d.N0), WALL_BLK, 0, s>>>(d, list);
+            launchApplyShiftNear(d, s);
         }
     }
+#undef LAUNCH_VEL
+#undef LAUNCH_CONC
 }
 
 // ------------------------------------------------------------------ dummy velocity

@@ -763,52 +763,41 @@ struct GradConcDF {
 };
 // type 2, wall contribution (src/MpsShifting.cpp:578-691) at the shifted positions:
 // mirror entries of near-wall fluid particles, reflected by the wall plane of i.
-__global__ void __launch_bounds__(BLK) k_wall_grad_conc_df(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= liveN(d)) return;
+__global__ void __launch_bounds__(WALL_BLK) k_wall_grad_conc_df(Dev d, bool skin) {
+    __shared__ WallCand W;
+    __shared__ double sm[3][32];
     const MpsParams& P = d.P;
-    dvec4 sh = make_dvec4(0, 0, 0, 0);
-    if (d.type[i] == P.fluid && d.nearWall[i]) {
-        dvec4 pi = d.pos[i], mi = d.mirror[i];
-        ReflG r = makeRefl(pi, mi, P.epsilonZero, true);
-        const float4 hi = d.posf[i], li = d.posLo[i];
-        const MirrorDF M = mirrorDF(d, mi);
-        const df R2 = K(d.k.reS2);
-        const RadiusDF RS = {K(d.k.reS), K(d.k.invReS)};
-        const df ci = loadDF(d.concDF, i);
-        df sx = dfF(0.f), sy = dfF(0.f), sz = dfF(0.f);
-        forCellsDF(d, pi, hi, d.bandHiS, [&](int j, int s, float4 hj) {
-            if (j == i) return;
-            const float4 lj = __ldg(&d.posLoCell[s]);
-            PairF q = pairDF(hj, lj, hi, li);
-            if (!inBallDF(d, q.d2, R2, d.mgS, P.reS2, i, j)) return;
-            PairF m = pairDF(hj, lj, M.mh, M.ml);
-            if (!lessDF(m.d2, R2, d.mgS, [&] { return pairMirror(d.pos[j], mi).dm2 < P.reS2; })) return;
-            if (!lessDF(q.d2, m.d2, d.mgSide, [&] {
-                    dvec4 pj = d.pos[j];
-                    return pairOf(pj, pi).d2 < pairMirror(pj, mi).dm2;
-                }))
-                return;
-            df cc = (ci + loadDF(d.concDF, j)) * weightDF(m.d2, RS, P.weightType).wr2;
-            sx += m.v.x * cc; sy += m.v.y * cc; sz += m.v.z * cc;
-        });
-        double dx = dD(sx), dy = dD(sy), dz = dD(sz);
-        double cI = d.conc[i];
-        PairM s = pairMirror(pi, mi);
-        if (s.dm2 < P.reS2) {
-            double wS = wfun(sqrt(s.dm2), P.reS, P.weightType);
-            dx += (cI + cI) * s.m0 * wS / s.dm2; dy += (cI + cI) * s.m1 * wS / s.dm2; dz += (cI + cI) * s.m2 * wS / s.dm2;
+    const RadiusDF RS = {K(d.k.reS), K(d.k.invReS)};
+    const int nn = *d.nearCount;
+    const bool useSkin = skin && !*(volatile int*)d.skinFlag;
+    for (int base = blockIdx.x * 32; base < nn; base += gridDim.x * 32) {
+        wallCandidates(d, W, base, nn, useSkin);
+        __syncthreads();
+        const int g = threadIdx.x / WALL_L, l = threadIdx.x & (WALL_L - 1);
+        if (base + g < nn) {
+            const int i = d.nearList[base + g];
+            const MirrorDF M = mirrorDF(d, d.mirror[i]);
+            const df ci = loadDF(d.concDF, i);
+            df sx = dfF(0.f), sy = sx, sz = sx;
+            forWallCand(d, W, i, g, l, [&](int j) {
+                const PairF m = pairDF(__ldg(&d.posf[j]), __ldg(&d.posLo[j]), M.mh, M.ml);
+                const df cc = (ci + loadDF(d.concDF, j)) * weightDF(m.d2, RS, P.weightType).wr2;
+                sx += m.v.x * cc; sy += m.v.y * cc; sz += m.v.z * cc;
+            });
+            sx = laneSumDF<WALL_L>(sx); sy = laneSumDF<WALL_L>(sy); sz = laneSumDF<WALL_L>(sz);
+            if (l == 0) { sm[0][g] = dD(sx); sm[1][g] = dD(sy); sm[2][g] = dD(sz); }
         }
-        double g0 = -(r.R[0] * dx + r.R[1] * dy + r.R[2] * dz) * P.coeffPressGrad;
-        double g1 = -(r.R[3] * dx + r.R[4] * dy + r.R[5] * dz) * P.coeffPressGrad;
-        double g2 = -(r.R[6] * dx + r.R[7] * dy + r.R[8] * dz) * P.coeffPressGrad;
-        dvec4 g = d.gradC[i];
-        g.x += g0; g.y += g1; g.z += g2;
-        d.gradC[i] = g;
-        if (d.bc[i] == P.inner)
-            sh = make_dvec4(-P.coeffShifting2 * g0, -P.coeffShifting2 * g1, -P.coeffShifting2 * g2, 0.0);
+        __syncthreads();
+        if (threadIdx.x < 32 && base + (int)threadIdx.x < nn)
+            wallGradConcEnd(d, d.nearList[base + threadIdx.x], sm[0][threadIdx.x], sm[1][threadIdx.x], sm[2][threadIdx.x]);
+        __syncthreads();
     }
-    d.shift[i] = sh;
+}
+static void launchWallGradConcDF(const Dev& d, cudaStream_t s, bool list) {
+    if (list) launchSkinCheck(d, s);
+    else launchNearList(d, s);
+    k_wall_grad_conc_df<<<wallGrid(d.N0), WALL_BLK, 0, s>>>(d, list);
+    launchApplyShiftNear(d, s);
 }
 // The shifting sums over the list of the post-corrector positions (filtered from the skin
 // list) instead of the 27-bucket scan: the reS-ball entries off the mirror side are the
@@ -841,11 +830,7 @@ void launchShiftingListDF(const Dev& d, cudaStream_t s) {
     k_df_conc<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
     k_shift_list_df<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d, GradConcDF());
     launchApplyShift(d, s);
-    if (P.wallType == 1) {
-        launchPosfCell(d, s);
-        k_wall_grad_conc_df<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
-        launchApplyShift(d, s);
-    }
+    if (P.wallType == 1) launchWallGradConcDF(d, s, true);
 }
 void launchShiftingDF(const Dev& d, cudaStream_t s) {
     const MpsParams& P = d.P;
@@ -861,11 +846,7 @@ void launchShiftingDF(const Dev& d, cudaStream_t s) {
     k_df_conc<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
     launchShiftScanDF(d, GradConcDF(), s);
     launchApplyShift(d, s);
-    if (P.wallType == 1) {
-        launchPosfCell(d, s);   // the wall sweep sees the shifted positions
-        k_wall_grad_conc_df<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
-        launchApplyShift(d, s);
-    }
+    if (P.wallType == 1) launchWallGradConcDF(d, s, false);
 }
 
 // ------------------------------------------------------------------ start-of-step list
