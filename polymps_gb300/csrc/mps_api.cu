@@ -113,7 +113,7 @@ void Prof::destroy() {
 // Kernels launched by one operator (fixed by the configuration; the solvers count theirs).
 static int opLaunches(int op, const MpsParams& P, bool x) {
     switch (op) {
-        case MPS_OP_UPDATE_BUCKETS: return 8;   // key, 3 scan, scatter, sort, list positions, bucket-ordered copy
+        case MPS_OP_UPDATE_BUCKETS: return 5;   // key, 2 scan, scatter, rank (small grids: 1 scan)
         case MPS_OP_VISCOSITY: return x ? 3 : 1;   // (DF32: velocity copy) + sweep (+ unlisted particles)
         case MPS_OP_OUT_OF_DOMAIN: return 2;
         case MPS_OP_COLLISION: return P.collisionType == 1 ? 2 : (x ? 3 : 2);
@@ -183,9 +183,8 @@ static void ensureList(mpsgpu_t h) {
         launchNeighborFilter(h->d, h->s, !df32(h));
         countLaunch(5);   // FP32 copies (2), skin check, filter, scan of the particles it left
     } else {
-        if (df32(h)) launchNeighborListDF(h->d, h->s);
-        else launchNeighborList(h->d, h->s);
-        countLaunch(df32(h) ? 4 : 3);   // FP32 copies (2), list build (DF32: + unlisted particles)
+        launchNeighborList(h->d, h->s, !df32(h));
+        countLaunch(3);   // FP32 copies (2), list build
     }
     h->skinValid = false;
     if (h->prof.on) h->prof.end(h->s);
@@ -392,7 +391,7 @@ static int runOpBody(mpsgpu_t h, int op) {
                 // the predicted positions is filtered from it (ensureList); in the FP64 tier
                 // the sweep and the filter keep the bucket scan's FP64 arithmetic and order
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(PROF_NEIGHBOR_LIST, s, false); }
-                launchSkinListDF(d, s);
+                launchSkinList(d, s);
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(MPS_OP_VISCOSITY, s, false); }
                 if (x) launchViscosityListDF(d, s);
                 else launchViscosityList(d, s);
@@ -404,7 +403,7 @@ static int runOpBody(mpsgpu_t h, int op) {
                 std::swap(d.nbrCount, h->cntAlt);
                 h->skinValid = true;
                 h->skinShift = true;   // the shifting sweeps filter the kept skin list again
-                countLaunch(2);   // skin list (listed + unlisted particles); the sweep is counted below
+                countLaunch(1);   // skin list; the sweep is counted below
             } else if (x) launchViscosityDF(d, s);
             else launchViscosity(d, s);
             break;
@@ -758,10 +757,11 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
     A(d.pressPPEprev2, n);
     A(d.cellOf, n);
     A(d.cellStart, d.nB + 2);
-    A(d.cellCount, d.nB + 2);
-    A(d.cellCursor, d.nB + 2);
+    A(d.cellCount, 2 * ((size_t)d.nB + 2));   // counters, then cursors
+    d.cellCursor = d.cellCount + d.nB + 2;
     A(d.orig, n);
     A(d.slotOf, n);
+    A(d.cellRec, n);
     A(d.cellPos, n);
     A(h->perm, n);
     {

@@ -4,7 +4,7 @@
 //
 // Both are HBM/L2-latency bound integer work: one coalesced pass over the particles for
 // the bucket keys, atomics into the per-bucket counters, a device-wide scan, a scatter
-// and a per-bucket insertion sort that restores ascending particle order (the
+// and a ranking within each bucket that restores ascending particle order (the
 // reference's linked lists are filled in ascending index order).
 #include <atomic>
 #include "mps_df.cuh"
@@ -86,30 +86,41 @@ __global__ void k_cell_key(Dev d) {
     if (i < d.N0) d.cellOf[i] = key;
 }
 
+// The records (reference index, slot) of each bucket in arrival order.
 __global__ void k_cell_scatter(Dev d) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int c = (i < d.N0) ? d.cellOf[i] : -1;
     const int r = warpGroupAdd(d.cellCursor, c, c >= 0);
-    if (c >= 0) d.cellSorted[d.cellStart[c] + r] = i;
+    if (c >= 0) d.cellRec[d.cellStart[c] + r] = make_int2(d.orig[i], i);
+    else if (i < d.N0) d.cellPos[i] = -1;
 }
 
-// Order each bucket by reference index (the reference's linked-list order; buckets hold
-// ~16 particles).  The range after the last bucket is ordered the same way.
-__global__ void k_cell_sort(Dev d) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c > d.nB) return;
-    int s0 = d.cellStart[c], s1 = d.cellStart[c + 1];
-    for (int a = s0 + 1; a < s1; a++) {
-        int v = d.cellSorted[a];
-        int ov = d.orig[v];
-        int b = a - 1;
-        while (b >= s0 && d.orig[d.cellSorted[b]] > ov) { d.cellSorted[b + 1] = d.cellSorted[b]; b--; }
-        d.cellSorted[b + 1] = v;
+// Each bucket ordered by reference index (the reference's linked-list order; buckets hold ~10
+// particles), the range after the last bucket the same way: a record's place is the number of
+// smaller reference indices in its bucket, so every particle finds its own with a few reads
+// of neighbouring records: 6 us at 6.9k particles and 15 at 864k, with the inverse list and the
+// copies below (one thread sorting each bucket by insertion walked dependent loads: 28 and 52
+// us, and two more launches).  place: also the inverse list and the FP32 copies in
+// bucket order (the renumbering, which moves the slots, writes them after it).
+__global__ void k_cell_rank(Dev d, bool place) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= d.cellStart[d.nB + 1]) return;
+    const int2 me = d.cellRec[p];
+    const int c = d.cellOf[me.y];
+    const int s0 = d.cellStart[c], s1 = d.cellStart[c + 1];
+    int at = s0;
+    for (int q = s0; q < s1; q++) at += d.cellRec[q].x < me.x ? 1 : 0;
+    d.cellSorted[at] = me.y;
+    if (!place) return;
+    d.cellPos[me.y] = at;
+    if (c < d.nB) {
+        d.posfCell[at] = d.posf[me.y];
+        d.posLoCell[at] = d.posLo[me.y];
     }
 }
 
 // ------------------------------------------------------------------ exclusive scan
-// Three-phase block scan for int arrays (n <= 4096 * 4096).
+// Block scan for int arrays: tiles, then each tile's offset from the tile sums before it.
 #define SCAN_BLOCK 1024
 #define SCAN_PER_THREAD 4
 #define SCAN_TILE (SCAN_BLOCK * SCAN_PER_THREAD)
@@ -160,26 +171,49 @@ __global__ void k_scan_tiles(const int* in, int* out, int* tileSums, int n) {
     if (threadIdx.x == 0 && tileSums) tileSums[blockIdx.x] = total;
 }
 
-__global__ void k_scan_add(int* out, const int* tileOffsets, int n, int* totalOut) {
-    int base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_PER_THREAD;
-    int add = tileOffsets[blockIdx.x];
+// out += the sums of the tiles before this block's; the last block writes the total to out[n].
+__global__ void k_scan_add(int* out, const int* tileSums, int n) {
+    __shared__ int smem[32];
+    int add = 0;
+    for (int t = threadIdx.x; t < (int)blockIdx.x; t += SCAN_BLOCK) add += tileSums[t];
+    int total;
+    blockExclusiveScan(add, smem, total);
+    const int base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_PER_THREAD;
 #pragma unroll
     for (int k = 0; k < SCAN_PER_THREAD; k++)
-        if (base + k < n) out[base + k] += add;
-    (void)totalOut;
+        if (base + k < n) out[base + k] += total;
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = total + tileSums[blockIdx.x];
+}
+// Up to SCAN_SMALL tiles by one block, a tile after the other (one launch for three).
+#define SCAN_SMALL 4
+__global__ void k_scan_small(const int* in, int* out, int n) {
+    __shared__ int smem[32];
+    int carry = 0;
+    for (int t = 0; t < n; t += SCAN_TILE) {
+        const int base = t + threadIdx.x * SCAN_PER_THREAD;
+        int v[SCAN_PER_THREAD], s = 0, total;
+#pragma unroll
+        for (int k = 0; k < SCAN_PER_THREAD; k++) { v[k] = (base + k < n) ? in[base + k] : 0; s += v[k]; }
+        int pre = carry + blockExclusiveScan(s, smem, total);
+#pragma unroll
+        for (int k = 0; k < SCAN_PER_THREAD; k++) {
+            if (base + k < n) out[base + k] = pre;
+            pre += v[k];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) out[n] = carry;
 }
 
-// out[0..n) = exclusive scan of in; out[n] = total.  scratch holds >= 2*tiles+2 ints.
+// out[0..n) = exclusive scan of in; out[n] = total.  scratch holds >= tiles ints.
 void scanExclusive(const int* in, int* out, int n, int* scratch, cudaStream_t s) {
     int tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-    int* tileSums = scratch;
-    int* tileOffsets = scratch + tiles + 1;
-    k_scan_tiles<<<tiles, SCAN_BLOCK, 0, s>>>(in, out, tileSums, n);
-    // second level: one tile covers up to 4096 tiles
-    k_scan_tiles<<<1, SCAN_BLOCK, 0, s>>>(tileSums, tileOffsets, tileOffsets + tiles, tiles);
-    k_scan_add<<<tiles, SCAN_BLOCK, 0, s>>>(out, tileOffsets, n, nullptr);
-    // total = offset of last tile + its sum
-    cudaMemcpyAsync(out + n, tileOffsets + tiles, sizeof(int), cudaMemcpyDeviceToDevice, s);
+    if (tiles <= SCAN_SMALL) {
+        k_scan_small<<<1, SCAN_BLOCK, 0, s>>>(in, out, n);
+        return;
+    }
+    k_scan_tiles<<<tiles, SCAN_BLOCK, 0, s>>>(in, out, scratch, n);
+    k_scan_add<<<tiles, SCAN_BLOCK, 0, s>>>(out, scratch, n);
 }
 int scanScratchInts(int n) { return 2 * ((n + SCAN_TILE - 1) / SCAN_TILE) + 4; }
 
@@ -213,7 +247,7 @@ static void permute(T* a, const int* perm, void* scratch, int n, cudaStream_t s)
     k_gather<T><<<gridFor(n, 256), 256, 0, s>>>(a, (T*)scratch, perm, n);
     cudaMemcpyAsync(a, scratch, sizeof(T) * n, cudaMemcpyDeviceToDevice, s);
 }
-int renumberLaunches() { return 1 + (15 + 17 + 5 + 3) + 1; }
+int renumberLaunches() { return 1 + (15 + 17 + 5 + 3) + 1 + 2; }
 static void launchRenumber(const Dev& d, int* perm, void* scratch, cudaStream_t s) {
     const int n = d.N0;
     k_perm_build<<<gridFor(n, 256), 256, 0, s>>>(d, perm);
@@ -238,13 +272,13 @@ __global__ void k_cell_pos(Dev d) {
 }
 
 void launchBuckets(const Dev& d, int* scanScratch, cudaStream_t s, int* perm, void* permScratch) {
-    cudaMemsetAsync(d.cellCount, 0, sizeof(int) * (d.nB + 2), s);
-    cudaMemsetAsync(d.cellCursor, 0, sizeof(int) * (d.nB + 2), s);
+    cudaMemsetAsync(d.cellCount, 0, sizeof(int) * 2 * (d.nB + 2), s);   // counters and cursors
     k_cell_key<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
     scanExclusive(d.cellCount, d.cellStart, d.nB + 1, scanScratch, s);
     k_cell_scatter<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
-    k_cell_sort<<<gridFor(d.nB + 1, 256), 256, 0, s>>>(d);
-    if (perm) launchRenumber(d, perm, permScratch, s);
+    k_cell_rank<<<gridFor(d.N0, 256), 256, 0, s>>>(d, perm == nullptr);
+    if (!perm) return;
+    launchRenumber(d, perm, permScratch, s);
     cudaMemsetAsync(d.cellPos, 0xff, sizeof(int) * d.N0, s);
     k_cell_pos<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
     k_posf_cell<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
@@ -278,25 +312,29 @@ void launchPosf(const Dev& d, cudaStream_t s) {
     launchPosfCell(d, s);
 }
 
-// Candidates are decided in FP32 first; only those whose FP32 squared distance falls in the
-// rounding band around the list radius^2 are re-tested in exact FP64, so membership equals
-// the reference's FP64 test dst^2 < re^2 bit for bit.  Each accepted entry then gets its
-// weights for the epoch: w(r; reS), w/r^2 and, when the radii differ, w(r; reL) — the FP64
-// divisions and square roots of all later sweeps happen here once.  L lanes per particle walk
-// the candidates (the three buckets of a row of the window are one range of the bucket order)
-// and append the members in scan order; the weights, which are the FP64 part, follow in a
-// second pass over the members only: formed where a candidate is accepted, every warp issues
-// them for nearly all of its ~250 candidates, as its lanes accept at different places
-// (108k particles: 721 -> 158 us).
-template <int L>
-__global__ void __launch_bounds__(128) k_build_nbr(Dev d) {
+// The 27-bucket scan into list rows, L lanes per particle: the three buckets of a row of the
+// window are one range of the bucket order (about 28 particles), tested 32 candidates at a time
+// into a bit mask whose set bits are then appended in scan order (appended where they are
+// found, every warp issued the append for nearly every candidate).  The skin list: 74 -> 19 us
+// at 6.9k particles (8 lanes), 98 -> 71 at 108k, 1,675 -> 1,311 at 2.8M (366 and 394 at 864k).
+//   MODE 0: the start-of-step skin list: candidates within reMax + skin (FP32 test against a
+//     radius that includes the rounding band: a superset of every list the step's sweeps can
+//     need while the particles stay within half the skin), start position and scan window.
+//   MODE 1: the list of the current positions.  Candidates are decided in FP32 first; only
+//     those whose FP32 squared distance falls in the rounding band around the list radius^2 are
+//     re-tested in exact FP64, so membership equals the reference's test dst^2 < re^2.
+//   MODE 2: the same with the entries' weights for the epoch, in a second pass over the members
+//     (formed where a candidate is accepted, they took 721 us for 158 at 108k particles): the
+//     FP64 divisions and square roots of all later sweeps happen here once.
+template <int MODE, int L>
+__global__ void __launch_bounds__(128) k_build_list(Dev d) {
     const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
-    const unsigned grp = laneGroup<L>(), below = ((1u << (threadIdx.x & 31)) - 1u) & grp;
     const dvec4 pi = d.pos[i];
     const float4 fi = d.posf[i];
     const size_t N0 = d.N0;
+    const int me = d.cellPos[i];   // the particle is no neighbour of itself
     int cnt = 0;
     int ix, iy, iz;
     bucketCoordsHi(d, pi, fi, ix, iy, iz);
@@ -310,48 +348,66 @@ __global__ void __launch_bounds__(128) k_build_nbr(Dev d) {
             if (lo > hi) continue;
             const int s1 = d.cellStart[hi + 1];
 #pragma unroll 1
-            for (int s0 = d.cellStart[lo]; s0 < s1; s0 += 4 * L) {
-                float4 f[4];
+            for (int s0 = d.cellStart[lo]; s0 < s1; s0 += 32) {
+                const int w = s1 - s0 < 32 ? s1 - s0 : 32;
+                unsigned m = 0u;
+#pragma unroll 1
+                for (int t = l; t < w; t += 4 * L) {
+                    float4 f[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++)
-                    if (s0 + u * L + l < s1) f[u] = __ldg(&d.posfCell[s0 + u * L + l]);
+                    for (int u = 0; u < 4; u++)
+                        f[u] = t + u * L < w ? __ldg(&d.posfCell[s0 + t + u * L]) : make_float4(3e38f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int s = s0 + u * L + l;
-                    int j = i;
-                    bool in = false;
-                    if (s < s1) {
+                    for (int u = 0; u < 4; u++) {
                         const float d2f = dist2f(f[u], fi);
-                        if (!(d2f > d.bandHi)) {
-                            j = __ldg(d.cellSorted + s);
-                            in = j != i && insideF(d, d2f, d.bandLo, d.bandHi, d.reMax2, i, j);
+                        bool in = t + u * L < w && s0 + t + u * L != me;
+                        if (MODE == 0) in = in && !(d2f > d.skinR2);
+                        else {
+                            in = in && !(d2f > d.bandHi);
+                            if (in && !(d2f < d.bandLo))
+                                in = pairInsideExact(d.pos, __ldg(d.cellSorted + s0 + t + u * L), i, d.reMax2);
                         }
-                    }
-                    if (L == 1) {
-                        if (in) {
-                            if (cnt < d.K) d.nbr[(size_t)cnt * N0 + i] = j;
-                            cnt++;
-                        }
-                    } else {
-                        const unsigned b = __ballot_sync(grp, in) & grp;
-                        const int k = cnt + __popc(b & below);
-                        if (in && k < d.K) d.nbr[(size_t)k * N0 + i] = j;
-                        cnt += __popc(b);
+                        if (in) m |= 1u << (t + u * L);
                     }
                 }
+                unsigned all = m;
+#pragma unroll
+                for (int o = 1; o < L; o <<= 1) all |= __shfl_xor_sync(laneGroup<L>(), all, o);
+                for (unsigned r = m; r; r &= r - 1u) {
+                    const int b = __ffs((int)r) - 1;
+                    const int k = cnt + __popc(all & ((1u << b) - 1u));
+                    if (k < d.K) d.nbr[(size_t)k * N0 + i] = __ldg(d.cellSorted + s0 + b);
+                }
+                cnt += __popc(all);
             }
         }
-    __syncwarp(grp);
+    if (MODE == 0) {
+        if (l == 0) {
+            d.nbrCount[i] = cnt > d.K ? d.K + 1 : cnt;   // K + 1: the row overflowed, rescanned where read
+            d.posSkin[i] = fi;
+            d.skinCell[i] = cellKeyOf(d, pi, fi);
+        }
+        return;
+    }
     const int c = cnt < d.K ? cnt : d.K;
     if (l == 0) {
         if (cnt > d.K) setErr(d, MPSE_CAPACITY);
         d.nbrCount[i] = c;
     }
     warpCount(d.counters, l == 0 ? (unsigned)c : 0u);
-    for (int k = l; k < c; k += L) {
-        const size_t e = (size_t)k * N0 + i;
-        storeWeights(d, e, pairSum(d.pos[d.nbr[e]], pi).d2);
+    if (MODE == 2) {
+        __syncwarp(laneGroup<L>());
+        for (int k = l; k < c; k += L) {
+            const size_t e = (size_t)k * N0 + i;
+            storeWeights(d, e, pairSum(d.pos[d.nbr[e]], pi).d2);
+        }
     }
+}
+template <int MODE>
+static void launchBuild(const Dev& d, cudaStream_t s) {
+#define LAUNCH(L) k_build_list<MODE, L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
 }
 
 // Per-entry weights of the current list for the FP64 sweeps, when the list was built by
@@ -370,13 +426,15 @@ void launchFillCache(const Dev& d, cudaStream_t s) {
     k_fill_cache<<<gridFor(d.N0, 128), 128, 0, s>>>(d);
 }
 
-void launchNeighborList(const Dev& d, cudaStream_t s) {
+void launchNeighborList(const Dev& d, cudaStream_t s, bool weights) {
     cudaMemsetAsync(d.counters, 0, sizeof(unsigned long long), s);
     launchPosf(d, s);
-    // 8 lanes against one: 35 / 84 us at 6.9k particles, 79 / 100 at 32k, 114 / 111 at 55k
-    // (the lanes' ballots cost more than they share), 209 / 158 at 108k
-    if (lanesFor(d.N0) > 1) k_build_nbr<8><<<gridFor(d.N0 * 8, 128), 128, 0, s>>>(d);
-    else k_build_nbr<1><<<gridFor(d.N0, 128), 128, 0, s>>>(d);
+    if (weights) launchBuild<2>(d, s);
+    else launchBuild<1>(d, s);
+}
+void launchSkinList(const Dev& d, cudaStream_t s) {
+    cudaMemsetAsync(d.skinFlag, 0, sizeof(int), s);
+    launchBuild<0>(d, s);
 }
 
 // ------------------------------------------------------------------ entry masks

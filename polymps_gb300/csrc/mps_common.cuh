@@ -85,6 +85,7 @@ struct Dev {
     // bucket (ghost type), -1 beyond the live count; cellStart has nB + 2 entries, the
     // range [cellStart[nB], cellStart[nB+1]) lists the live particles in no bucket
     int *cellOf, *cellStart, *cellCount, *cellSorted, *cellCursor;
+    int2* cellRec;     // (reference index, slot) by bucket, before the ordering
     int* cellPos;      // inverse of cellSorted over the list (-1: slot not listed)
     // FP32 positions in bucket order (posfCell[s] = posf[cellSorted[s]]): the prefilter of
     // the 27-bucket scans reads contiguous 16-byte records and fetches the particle index

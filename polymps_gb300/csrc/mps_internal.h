@@ -36,7 +36,9 @@ int scanScratchInts(int n);
 // perm != NULL: renumber the storage into bucket order (perm: N0 ints, permScratch: 32 N0 bytes)
 void launchBuckets(const Dev& d, int* scanScratch, cudaStream_t s, int* perm, void* permScratch);
 int renumberLaunches();
-void launchNeighborList(const Dev& d, cudaStream_t s);
+void launchNeighborList(const Dev& d, cudaStream_t s, bool weights);   // weights: the FP64 tier's cache
+// start-of-step list with a skin (both tiers)
+void launchSkinList(const Dev& d, cudaStream_t s);
 void launchPosf(const Dev& d, cudaStream_t s);       // FP32 copy, then its bucket-ordered copy
 void launchPosfCell(const Dev& d, cudaStream_t s);   // bucket-ordered copy only
 void launchSideMasks(const Dev& d, cudaStream_t s);   // also nearList and the mirror masks
@@ -45,7 +47,7 @@ void launchFillCache(const Dev& d, cudaStream_t s);
 
 // mps_ops.cu
 void launchViscosity(const Dev& d, cudaStream_t s);
-// over the start-of-step skin list (built by launchSkinListDF): the FP64 viscosity sweep, and
+// over the start-of-step skin list (built by launchSkinList): the FP64 viscosity sweep, and
 // the list of the current positions filtered from it (weights: the FP64 tier's cache)
 void launchViscosityList(const Dev& d, cudaStream_t s);
 void launchNeighborFilter(const Dev& d, cudaStream_t s, bool weights);
@@ -74,7 +76,6 @@ void launchShifting(const Dev& d, cudaStream_t s, bool list);   // list: filter 
 void launchDummyVelocity(const Dev& d, cudaStream_t s);
 
 // mps_ops_df.cu (DF32 tier)
-void launchNeighborListDF(const Dev& d, cudaStream_t s);
 void launchViscosityDF(const Dev& d, cudaStream_t s);
 void launchCollisionDF(const Dev& d, cudaStream_t s);
 void launchWallNpcdDF(const Dev& d, cudaStream_t s);
@@ -93,8 +94,7 @@ void launchUpdateBCArc(const Dev& d, cudaStream_t s);
 void launchCollisionDPC(const Dev& d, cudaStream_t s);
 // velocity divergence of the PND + div u source (list based, FP64; + the polygon-wall term)
 void launchVelDivergence(const Dev& d, cudaStream_t s);
-// start-of-step list with a skin: build, and the DF32 viscosity over it
-void launchSkinListDF(const Dev& d, cudaStream_t s);
+// DF32 viscosity over the start-of-step list
 void launchViscosityListDF(const Dev& d, cudaStream_t s);
 // the skin list's validity flag for the current positions (moved more than half the skin)
 void launchSkinCheck(const Dev& d, cudaStream_t s);

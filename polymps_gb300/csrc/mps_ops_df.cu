@@ -37,41 +37,6 @@ __device__ __forceinline__ df loadDF(const float2* p, int j) {
     return {v.x, v.y};
 }
 
-// ------------------------------------------------------------------ neighbour list
-// The list of the current positions through the stale buckets: candidates whose FP32
-// squared distance is below the band are members, those above it were never seen by the
-// prefilter, and only the band's few candidates are decided in float-float (and, inside
-// the float-float margin, in FP64).  No per-entry weights: the DF32 sweeps recompute them.
-template <bool STRAY>
-__global__ void __launch_bounds__(128) k_build_nbr_df(Dev d) {
-    const int i = scanParticle<STRAY>(d);
-    if (i < 0) return;
-    dvec4 pi = d.pos[i];
-    float4 hi = d.posf[i], li = d.posLo[i];
-    const df R2 = K(d.k.reMax2);
-    int cnt = 0;
-    const size_t N0 = d.N0;
-    forCellsDF(d, pi, hi, d.bandHi, [&](int j, int s, float4 hj) {
-        if (j == i) return;
-        float ex = hj.x - hi.x, ey = hj.y - hi.y, ez = hj.z - hi.z;
-        if (!(ex * ex + ey * ey + ez * ez < d.bandLo)) {
-            PairF q = pairDF(hj, __ldg(&d.posLoCell[s]), hi, li);
-            if (!inBallDF(d, q.d2, R2, d.mgMax, d.reMax2, i, j)) return;
-        }
-        if (cnt < d.K) d.nbr[(size_t)cnt * N0 + i] = j;
-        cnt++;
-    });
-    if (cnt > d.K) { setErr(d, MPSE_CAPACITY); cnt = d.K; }
-    d.nbrCount[i] = cnt;
-    warpCount(d.counters, (unsigned)cnt);
-}
-void launchNeighborListDF(const Dev& d, cudaStream_t s) {
-    cudaMemsetAsync(d.counters, 0, sizeof(unsigned long long), s);
-    launchPosf(d, s);
-    k_build_nbr_df<false><<<gridFor(d.N0, 128), 128, 0, s>>>(d);
-    k_build_nbr_df<true><<<gridFor(d.N0, 128), 128, 0, s>>>(d);
-}
-
 // ------------------------------------------------------------------ viscosity
 // MpsViscosity::calcViscosity, src/MpsViscosity.cpp:20-100, at the start-of-step
 // positions through the 27 buckets (Newtonian: uniform MEU and RHO).  Two phases per
@@ -850,32 +815,6 @@ void launchShiftingDF(const Dev& d, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------ start-of-step list
-// Candidates of the 27-bucket scan within reMax + skin of the start positions (FP32 test
-// against a radius that includes the rounding band: a superset of every list the step's
-// sweeps can need while the particles stay within half the skin), in scan order.
-template <bool STRAY>
-__global__ void __launch_bounds__(128) k_build_skin_df(Dev d) {
-    const int i = scanParticle<STRAY>(d);
-    if (i < 0) return;
-    const dvec4 pi = d.pos[i];
-    const float4 hi = d.posf[i];
-    int cnt = 0;
-    const size_t N0 = d.N0;
-    forCellsDF(d, pi, hi, d.skinR2, [&](int j, int, float4) {
-        if (j == i) return;
-        if (cnt < d.K) d.nbr[(size_t)cnt * N0 + i] = j;
-        cnt++;
-    });
-    d.nbrCount[i] = cnt > d.K ? d.K + 1 : cnt;   // K + 1: the row overflowed, rescanned where read
-    d.posSkin[i] = hi;
-    d.skinCell[i] = cellKeyOf(d, pi, hi);
-}
-void launchSkinListDF(const Dev& d, cudaStream_t s) {
-    cudaMemsetAsync(d.skinFlag, 0, sizeof(int), s);
-    k_build_skin_df<false><<<gridFor(d.N0, 128), 128, 0, s>>>(d);
-    k_build_skin_df<true><<<gridFor(d.N0, 128), 128, 0, s>>>(d);
-}
-
 // Viscosity (the sweep of k_visc_df: same entries in the same scan order, same float-float
 // arithmetic, so the same sums) over the start-of-step list instead of the 27 buckets.
 __global__ void __launch_bounds__(128) k_visc_list_df(Dev d) {
