@@ -37,6 +37,21 @@ __device__ __forceinline__ df loadDF(const float2* p, int j) {
     return {v.x, v.y};
 }
 
+template <int L>
+__device__ __forceinline__ df laneSumDF(df v) {
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1) {
+        const df q = {__shfl_xor_sync(laneGroup<L>(), v.h, o), __shfl_xor_sync(laneGroup<L>(), v.l, o)};
+        v += q;
+    }
+    return v;
+}
+// What a pair needs of its neighbour: the position's hi and lo parts (and X, the sweep's own).
+struct NbrPos {
+    float4 h, l;
+};
+__device__ __forceinline__ NbrPos loadPos(const Dev& d, int j) { return {__ldg(&d.posf[j]), __ldg(&d.posLo[j])}; }
+
 // ------------------------------------------------------------------ viscosity
 // MpsViscosity::calcViscosity, src/MpsViscosity.cpp:20-100, at the start-of-step
 // positions through the 27 buckets (Newtonian: uniform MEU and RHO).  Two phases per
@@ -169,15 +184,6 @@ void launchCollisionDF(const Dev& d, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------ wall sweeps
-template <int L>
-__device__ __forceinline__ df laneSumDF(df v) {
-#pragma unroll
-    for (int o = 1; o < L; o <<= 1) {
-        const df q = {__shfl_xor_sync(laneGroup<L>(), v.h, o), __shfl_xor_sync(laneGroup<L>(), v.l, o)};
-        v += q;
-    }
-    return v;
-}
 struct MirrorDF {
     float4 mh, ml;
 };
@@ -238,21 +244,34 @@ __device__ __forceinline__ df recipDF(df a) {
 }
 __device__ __forceinline__ void corrFinish(const Dev& d, int i, int numNeigh, df m00, df m01, df m02, df m11,
                                            df m12, df m22, dvec4* c1, dvec4* c2, dvec4* c3, float2* cdf);
+struct MomentsDF {
+    df xx = {0.f, 0.f}, xy = {0.f, 0.f}, xz = {0.f, 0.f}, yy = {0.f, 0.f}, yz = {0.f, 0.f}, zz = {0.f, 0.f};
+    __device__ __forceinline__ void add(const V3& v, df wr2) {
+        const df t0 = v.x * wr2, t1 = v.y * wr2, t2 = v.z * wr2;
+        xx += t0 * v.x; xy += t0 * v.y; xz += t0 * v.z;
+        yy += t1 * v.y; yz += t1 * v.z; zz += t2 * v.z;
+    }
+    template <int L>
+    __device__ __forceinline__ void sum() {
+        xx = laneSumDF<L>(xx); xy = laneSumDF<L>(xy); xz = laneSumDF<L>(xz);
+        yy = laneSumDF<L>(yy); yz = laneSumDF<L>(yz); zz = laneSumDF<L>(zz);
+    }
+};
+template <int L>
 __global__ void __launch_bounds__(BLK) k_corr_matrix_df(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
     float4 hi = d.posf[i], li = d.posLo[i];
     const RadiusDF RS = {K(d.k.reS), K(d.k.invReS)};
-    df m00 = dfF(0.f), m01 = m00, m02 = m00, m11 = m00, m12 = m00, m22 = m00;
-    forMask(d, i, d.maskS[i], [&](int j, size_t) {
-        PairF q = pairDF(d.posf[j], d.posLo[j], hi, li);
-        df wd = weightDF(q.d2, RS, P.weightType).wr2;
-        df t0 = q.v.x * wd, t1 = q.v.y * wd, t2 = q.v.z * wd;
-        m00 += t0 * q.v.x; m01 += t0 * q.v.y; m02 += t0 * q.v.z;
-        m11 += t1 * q.v.y; m12 += t1 * q.v.z; m22 += t2 * q.v.z;
-    });
-    corrFinish(d, i, d.numNeigh[i], m00, m01, m02, m11, m12, m22, d.c1, d.c2, d.c3, d.corrDF);
+    MomentsDF M;
+    forBitsOne(d.nbr + i, d.N0, laneShare<L>(d.maskS[i], l), [&](int j) { return loadPos(d, j); },
+                 [&](int, int, const NbrPos& n) {
+                     PairF q = pairDF(n.h, n.l, hi, li);
+                     M.add(q.v, weightDF(q.d2, RS, P.weightType).wr2);
+                 });
+    M.sum<L>();
+    if (l == 0) corrFinish(d, i, d.numNeigh[i], M.xx, M.xy, M.xz, M.yy, M.yz, M.zz, d.c1, d.c2, d.c3, d.corrDF);
 }
 // inverse of -coeffPressGrad * the moment matrix (identity when det <= eps or fewer than
 // four neighbours), written as the FP64 rows and the float-float copy
@@ -300,48 +319,41 @@ __global__ void k_df_corr(Dev d) {
     }
 }
 void launchCorrDF(const Dev& d, cudaStream_t s) { k_df_corr<<<gridFor(d.N0, 256), 256, 0, s>>>(d); }
-void launchCorrectionMatrixDF(const Dev& d, cudaStream_t s) { k_corr_matrix_df<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d); }
+void launchCorrectionMatrixDF(const Dev& d, cudaStream_t s) {
+#define LAUNCH(L) k_corr_matrix_df<L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
+}
 
 // ------------------------------------------------------------------ PND / NPCD
 // MpsPndNeigh::calcPndnNeighNPCD, src/MpsPndNeigh.cpp:199-331
 // CORR: the correction matrix's moment sums over the reS entries in the same pass (one
 // pair evaluation serves both; the PND sums take the entries also inside reL, in the same
 // ascending order as the plain sweep, so both results equal the separate kernels').
-template <bool CORR>
+template <bool CORR, int L>
 __global__ void __launch_bounds__(BLK, 9) k_pnd_npcd_df(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
     float4 hi = d.posf[i], li = d.posLo[i];
     const RadiusDF RS = {K(d.k.reS), K(d.k.invReS)};
-    const Mask mL = d.maskL[i];
-    int nn = d.nNeighWall[i] + maskCount(mL);
+    const Mask mL = d.maskL[i], mS = d.maskS[i];
     df ni = dfF(0.f), nx = ni, ny = ni, nz = ni;
-    df m00 = dfF(0.f), m01 = m00, m02 = m00, m11 = m00, m12 = m00, m22 = m00;
-    if (CORR) {
-        Mask m = d.maskS[i];
-        const int* row = d.nbr + i;
-        int k;
-        while ((k = maskPop(m)) >= 0) {
-            const int j = ldStream(row + (size_t)k * d.N0);
-            PairF q = pairDF(d.posf[j], d.posLo[j], hi, li);
-            WeightDF w = weightDF(q.d2, RS, P.weightType);
-            df t0 = q.v.x * w.wr2, t1 = q.v.y * w.wr2, t2 = q.v.z * w.wr2;
-            m00 += t0 * q.v.x; m01 += t0 * q.v.y; m02 += t0 * q.v.z;
-            m11 += t1 * q.v.y; m12 += t1 * q.v.z; m22 += t2 * q.v.z;
-            if (maskHas(mL, k)) {
-                ni += w.w;
-                nx += q.v.x * w.w; ny += q.v.y * w.w; nz += q.v.z * w.w;
-            }
-        }
-    } else {
-        forMask(d, i, mL & d.maskS[i], [&](int j, size_t) {
-            PairF q = pairDF(d.posf[j], d.posLo[j], hi, li);
-            df wS = weightDF(q.d2, RS, P.weightType).w;
-            ni += wS;
-            nx += q.v.x * wS; ny += q.v.y * wS; nz += q.v.z * wS;
-        });
-    }
+    MomentsDF M;
+    forBitsOne(d.nbr + i, d.N0, laneShare<L>(CORR ? mS : (mL & mS), l), [&](int j) { return loadPos(d, j); },
+                 [&](int, int k, const NbrPos& n) {
+                     PairF q = pairDF(n.h, n.l, hi, li);
+                     WeightDF w = weightDF(q.d2, RS, P.weightType);
+                     if (CORR) M.add(q.v, w.wr2);
+                     if (!CORR || maskHas(mL, k)) {
+                         ni += w.w;
+                         nx += q.v.x * w.w; ny += q.v.y * w.w; nz += q.v.z * w.w;
+                     }
+                 });
+    ni = laneSumDF<L>(ni); nx = laneSumDF<L>(nx); ny = laneSumDF<L>(ny); nz = laneSumDF<L>(nz);
+    if (CORR) M.sum<L>();
+    if (l != 0) return;
+    const int nn = d.nNeighWall[i] + maskCount(mL);
     double nd = dD(ni);
     dvec4 np = d.npcd[i];
     np.x += dD(nx); np.y += dD(ny); np.z += dD(nz);
@@ -359,70 +371,96 @@ __global__ void __launch_bounds__(BLK, 9) k_pnd_npcd_df(Dev d) {
     d.devDot[i] = (np.x * nw.x + np.y * nw.y + np.z * nw.z < 0.0) ? 1.0 : -1.0;
     // into the staging arrays: the correction-matrix operator publishes them (the reference
     // writes the matrix there, not in this sweep)
-    if (CORR) corrFinish(d, i, nn, m00, m01, m02, m11, m12, m22, d.c1n, d.c2n, d.c3n, d.corrDFn);
+    if (CORR) corrFinish(d, i, nn, M.xx, M.xy, M.xz, M.yy, M.yz, M.zz, d.c1n, d.c2n, d.c3n, d.corrDFn);
 }
 void launchPndNeighNpcdDF(const Dev& d, cudaStream_t s, bool withCorrection) {
-    if (withCorrection) k_pnd_npcd_df<true><<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
-    else k_pnd_npcd_df<false><<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
+#define LAUNCH(L)                                                                            \
+    if (withCorrection) k_pnd_npcd_df<true, L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d);    \
+    else k_pnd_npcd_df<false, L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
 }
 
 // ------------------------------------------------------------------ PPE assembly
 // MpsPressure::solvePressurePoissonPnd, src/MpsPressure.cpp:169-286 (matrix values are
 // assembled in float-float and stored in FP64)
-__global__ void __launch_bounds__(128, 12) k_ppe_assemble_df(Dev d, PpeBuffers B) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+template <int L>
+__global__ void __launch_bounds__(128, 9) k_ppe_assemble_df(Dev d, PpeBuffers B) {
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
     int bci = d.bc[i];
     if (bci == P.other || bci == P.surface) {
-        B.diag[i] = 1.0; B.diagf[i] = 1.0f; B.diagInvf[i] = 1.0f; B.rowLen[i] = 0; B.b[i] = 0.0; B.mfMask[i] = maskNone();
+        if (l == 0) {
+            B.diag[i] = 1.0; B.diagf[i] = 1.0f; B.diagInvf[i] = 1.0f; B.rowLen[i] = 0; B.b[i] = 0.0;
+            B.mfMask[i] = maskNone();
+        }
         warpCount(d.counters + 1, 0u);
         return;
     }
     float4 hi = d.posf[i], li = d.posLo[i];
     const RadiusDF RL = {K(d.k.reL), K(d.k.invReL)};
-    const df cP = K(d.k.cPPE), cG = K(d.k.cPPEg);
-    const df gx = K(d.k.g[0]), gy = K(d.k.g[1]), gz = K(d.k.g[2]);
+    const df cP = K(d.k.cPPE);
     df sum = dfF(0.f), src = dfF(0.f);
+    const Mask mL = d.maskL[i];
+    const int* row = d.nbr + i;
+    const size_t base = ellBase(B, i);
     int len = 0;
     Mask mm = maskNone();
-    forMaskK(d, i, d.maskL[i], [&](int j, size_t, int ke) {
-        PairF q = pairDF(d.posf[j], d.posLo[j], hi, li);
-        df wL = weightDF(q.d2, RL, P.weightType).w;
-        if (d.type[j] == P.dummyWall) {
-            src -= (q.v.x * gx + q.v.y * gy + q.v.z * gz) * wL * cG;
-        } else {
-            df mij = wL * cP;
-            sum -= mij;
-            if (d.bc[j] == P.inner) {
-                size_t k = ellBase(B, i) + (size_t)len * B.ellStride;
-                B.val[k] = dD(mij);
-                B.valf[k] = mij.h;   // the FP32 copy of the mixed solver (hi part = fl32)
-                B.col[k] = j;
-                len++;
-                maskSet(mm, ke);
-            }
-        }
-    });
-    B.mfMask[i] = mm;
-    double rho = P.DNS_FL1;
-    double dg = dD(sum) - P.alphaCompressibility * rho / (P.timeStep * P.timeStep);
-    B.diag[i] = dg;
-    B.diagf[i] = (float)dg;
-    B.diagInvf[i] = 1.0f / (float)dg;
-    B.rowLen[i] = len;
-    B.b[i] = dD(src) + ppeSource(d, i, rho);
-    warpCount(d.counters + 1, (unsigned)len);
+    if (L > 1) {   // the matrix entries of the whole row first: an entry's place is its rank
+        forMaskLane<L>(d, i, mL, l, [&](int j, size_t, int k) {
+            if (d.type[j] != P.dummyWall && d.bc[j] == P.inner) maskSet(mm, k);
+        });
+        mm = laneOr<L>(mm);
+        len = maskCount(mm);
+    }
+    struct Nbr { NbrPos p; int type, bc; };
+    forBitsTwo(row, d.N0, laneShare<L>(mL, l),
+                 [&](int j) { return Nbr{loadPos(d, j), __ldg(&d.type[j]), __ldg(&d.bc[j])}; },
+                 [&](int j, int k, const Nbr& n) {
+                     PairF q = pairDF(n.p.h, n.p.l, hi, li);
+                     df wL = weightDF(q.d2, RL, P.weightType).w;
+                     if (n.type == P.dummyWall) {
+                         src -= (q.v.x * K(d.k.g[0]) + q.v.y * K(d.k.g[1]) + q.v.z * K(d.k.g[2])) * wL * K(d.k.cPPEg);
+                         return;
+                     }
+                     df mij = wL * cP;
+                     sum -= mij;
+                     if (n.bc != P.inner) return;
+                     int at;
+                     if (L > 1) at = maskRank(mm, k);
+                     else { at = len++; maskSet(mm, k); }
+                     const size_t e = base + (size_t)at * B.ellStride;
+                     B.val[e] = dD(mij);
+                     B.valf[e] = mij.h;   // the FP32 copy of the mixed solver (hi part = fl32)
+                     B.col[e] = j;
+                 });
+    sum = laneSumDF<L>(sum);
+    src = laneSumDF<L>(src);
+    if (l == 0) {
+        B.mfMask[i] = mm;
+        double rho = P.DNS_FL1;
+        double dg = dD(sum) - P.alphaCompressibility * rho / (P.timeStep * P.timeStep);
+        B.diag[i] = dg;
+        B.diagf[i] = (float)dg;
+        B.diagInvf[i] = 1.0f / (float)dg;
+        B.rowLen[i] = len;
+        B.b[i] = dD(src) + ppeSource(d, i, rho);
+    }
+    warpCount(d.counters + 1, l == 0 ? (unsigned)len : 0u);
 }
 void launchPpeAssembleDF(const Dev& d, const PpeBuffers& B, cudaStream_t s) {
     cudaMemsetAsync(d.counters + 1, 0, sizeof(unsigned long long), s);
-    k_ppe_assemble_df<<<gridFor(d.N0, 128), 128, 0, s>>>(d, B);
+#define LAUNCH(L) k_ppe_assemble_df<L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d, B)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
 }
 
 // ------------------------------------------------------------------ pressure gradient
 // MpsPressure::calcPressGradient, src/MpsPressure.cpp:1217-1338
-__global__ void __launch_bounds__(BLK, 9) k_press_grad_df(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+template <int L>
+__global__ void __launch_bounds__(BLK, 8) k_press_grad_df(Dev d) {
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
     float4 hi = d.posf[i], li = d.posLo[i];
@@ -430,29 +468,39 @@ __global__ void __launch_bounds__(BLK, 9) k_press_grad_df(Dev d) {
     df Pi = loadDF(d.pressDF, i), pmin = Pi;
     double ni = d.pndi[i];
     int gt = P.gradientType;
-    const Mask mS = d.maskS[i];
+    const Mask mS = laneShare<L>(d.maskS[i], l);
+    const int* row = d.nbr + i;
     if (gt == 0 || gt == 2) {
-        forMask(d, i, mS, [&](int j, size_t) {
-            df pj = loadDF(d.pressDF, j);
+        forBitsTwo(row, d.N0, mS, [&](int j) { return __ldg(d.pressDF + j); }, [&](int, int, float2 p) {
+            const df pj = {p.x, p.y};
             if (pmin > pj) pmin = pj;
         });
-        ((float2*)d.pAux)[i] = make_float2(pmin.h, pmin.l);   // for the wall term
+#pragma unroll
+        for (int o = 1; o < L; o <<= 1) {
+            const df q = {__shfl_xor_sync(laneGroup<L>(), pmin.h, o), __shfl_xor_sync(laneGroup<L>(), pmin.l, o)};
+            if (pmin > q) pmin = q;
+        }
+        if (l == 0) ((float2*)d.pAux)[i] = make_float2(pmin.h, pmin.l);   // for the wall term
     }
     df base = (gt == 0) ? -pmin : (gt == 1 ? Pi : Pi - pmin - pmin);
     // sum of r_ij f_ij; with gradient correction C (constant per particle) is applied to
     // the sum once: sum (C r) f = C (sum r f)
     df ax = dfF(0.f), ay = ax, az = ax;
-    forMask(d, i, mS, [&](int j, size_t) {
-        PairF q = pairDF(d.posf[j], d.posLo[j], hi, li);
-        WeightDF w = weightDF(q.d2, RS, P.weightType);
-        df f;
-        if (gt <= 2) f = (loadDF(d.pressDF, j) + base) * w.wr2;
-        else {
-            double nj = d.pndi[j], Pj = d.press[j], Pid = d.press[i];
-            f = (ni > P.epsilonZero && nj > P.epsilonZero) ? dfD(ni * Pj / nj + nj * Pid / ni) * w.wr2 : w.w;
-        }
-        ax += q.v.x * f; ay += q.v.y * f; az += q.v.z * f;
-    });
+    struct Nbr { NbrPos p; float2 pr; };
+    forBitsTwo(row, d.N0, mS, [&](int j) { return Nbr{loadPos(d, j), __ldg(d.pressDF + j)}; },
+                 [&](int j, int, const Nbr& n) {
+                     PairF q = pairDF(n.p.h, n.p.l, hi, li);
+                     WeightDF w = weightDF(q.d2, RS, P.weightType);
+                     df f;
+                     if (gt <= 2) f = (df{n.pr.x, n.pr.y} + base) * w.wr2;
+                     else {
+                         double nj = d.pndi[j], Pj = d.press[j], Pid = d.press[i];
+                         f = (ni > P.epsilonZero && nj > P.epsilonZero) ? dfD(ni * Pj / nj + nj * Pid / ni) * w.wr2 : w.w;
+                     }
+                     ax += q.v.x * f; ay += q.v.y * f; az += q.v.z * f;
+                 });
+    ax = laneSumDF<L>(ax); ay = laneSumDF<L>(ay); az = laneSumDF<L>(az);
+    if (l != 0) return;
     if (P.gradientCorrection) {
         df C[9];
 #pragma unroll
@@ -462,12 +510,13 @@ __global__ void __launch_bounds__(BLK, 9) k_press_grad_df(Dev d) {
         df bz = C[6] * ax + C[7] * ay + C[8] * az;
         ax = bx; ay = by; az = bz;
     }
-    double c = P.relaxPress * P.coeffPressGrad / P.DNS_FL1;
-    d.acc[i] = make_dvec4(dD(ax) * c, dD(ay) * c, dD(az) * c, 0.0);
+    d.acc[i] = make_dvec4(dD(ax) * d.cPG, dD(ay) * d.cPG, dD(az) * d.cPG, 0.0);
 }
 void launchPressGradientDF(const Dev& d, cudaStream_t s) {
     launchPressDF(d, s);
-    k_press_grad_df<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
+#define LAUNCH(L) k_press_grad_df<L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
 }
 
 // MpsPressure::calcWallPressGradient + repulsive forces, src/MpsPressure.cpp:1341-1611
@@ -775,10 +824,8 @@ __global__ void __launch_bounds__(BLK) k_shift_list_df(Dev d, Op op) {
     const bool on = op.begin(d, i, st);
     if (on) {
         const float4 hi = d.posf[i], li = d.posLo[i];
-        forMask(d, i, d.maskS[i], [&](int j, size_t) {
-            const PairF q = pairDF(__ldg(d.posf + j), __ldg(d.posLo + j), hi, li);
-            op.visit(d, st, j, q);
-        });
+        forBitsTwo(d.nbr + i, d.N0, d.maskS[i], [&](int j) { return loadPos(d, j); },
+                     [&](int j, int, const NbrPos& n) { op.visit(d, st, j, pairDF(n.h, n.l, hi, li)); });
     }
     op.end(d, i, st, on);
 }
@@ -815,65 +862,57 @@ void launchShiftingDF(const Dev& d, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------ start-of-step list
-// Viscosity (the sweep of k_visc_df: same entries in the same scan order, same float-float
-// arithmetic, so the same sums) over the start-of-step list instead of the 27 buckets.
+// Viscosity over the start-of-step list instead of the 27 buckets (k_visc_df's entries, in the
+// scan order within a lane), L lanes per particle: the FP32 copies decide the 56 entries of a
+// row first (mps_lanes.cuh), the float-float sums walk the 32 inside (559 -> 369 us at 864k
+// particles).
+template <int L>
 __global__ void __launch_bounds__(128) k_visc_list_df(Dev d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
-    const dvec4 pi = d.pos[i];
     const float4 hi = d.posf[i], li = d.posLo[i];
     const float4 vh = d.velHi[i], vl = d.velLo[i];
-    const SideDF sc = sideDF(d, i, pi);
-    const df R2 = K(d.k.reL2), neuW = K(d.k.neuW), neuF = K(d.k.neuF);
     const RadiusDF RL = {K(d.k.reL), K(d.k.invReL)};
     df ax = dfF(0.f), ay = dfF(0.f), az = dfF(0.f);
-    auto pair = [&](int j, float4 hj, float4 lj) {
-        PairF q = pairDF(hj, lj, hi, li);
-        if (!inBallDF(d, q.d2, R2, d.mgL, P.reL2, i, j)) return;
-        if (!sideOkDF(d, sc, hj, lj, q.d2, i, j)) return;
-        WeightDF w = weightDF(q.d2, RL, P.weightType);
-        df c = w.w * ((d.type[j] == P.wall) ? neuW : neuF);
-        float4 vhj = d.velHi[j], vlj = d.velLo[j];
-        ax += diffDF(vhj.x, vlj.x, vh.x, vl.x) * c;
-        ay += diffDF(vhj.y, vlj.y, vh.y, vl.y) * c;
-        az += diffDF(vhj.z, vlj.z, vh.z, vl.z) * c;
+    struct Nbr { NbrPos p; float4 vh, vl; int type; };
+    auto load = [&](int j) { return Nbr{loadPos(d, j), __ldg(&d.velHi[j]), __ldg(&d.velLo[j]), __ldg(&d.type[j])}; };
+    auto add = [&](int, int, const Nbr& n) {
+        const PairF q = pairDF(n.p.h, n.p.l, hi, li);
+        const df c = weightDF(q.d2, RL, P.weightType).w * (n.type == P.wall ? K(d.k.neuW) : K(d.k.neuF));
+        ax += diffDF(n.vh.x, n.vl.x, vh.x, vl.x) * c;
+        ay += diffDF(n.vh.y, n.vl.y, vh.y, vl.y) * c;
+        az += diffDF(n.vh.z, n.vl.z, vh.z, vl.z) * c;
     };
     const int c = d.nbrCount[i];
     if (c <= d.K) {
-        // four entries' indices and FP32 copies ahead of their tests (forNbrsPosf's order)
-        auto entry = [&](int j, float4 hj) {
-            float ex = hj.x - hi.x, ey = hj.y - hi.y, ez = hj.z - hi.z;
-            if (ex * ex + ey * ey + ez * ez > d.bandHiL) return;   // outside the reL band
-            pair(j, hj, __ldg(&d.posLo[j]));
-        };
         const int* row = d.nbr + i;
-        int k = 0;
-        for (; k + 4 <= c; k += 4) {
-            int jj[4];
-            float4 hh[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) jj[u] = ldStream(row + (size_t)(k + u) * d.N0);
-#pragma unroll
-            for (int u = 0; u < 4; u++) hh[u] = __ldg(&d.posf[jj[u]]);
-#pragma unroll
-            for (int u = 0; u < 4; u++) entry(jj[u], hh[u]);
-        }
-        for (; k < c; k++) {
-            const int j = ldStream(row + (size_t)k * d.N0);
-            entry(j, __ldg(&d.posf[j]));
-        }
-    } else {
+        const SideF sd = sideF(d, i, d.pos[i]);
+        const Mask m = rowMask<L>(d, row, l, c, [&](int j, float4 hj) {
+            const float d2f = dist2f(hj, hi);
+            return insideF(d, d2f, d.bandLoL, d.bandHiL, P.reL2, i, j) && sideOKF(d, sd, hj, d2f, i, j);
+        });
+        forBitsTwo(row, d.N0, m, load, add);
+    } else if (l == 0) {   // the row overflowed: scan the buckets
+        const dvec4 pi = d.pos[i];
+        const SideDF sc = sideDF(d, i, pi);
+        const df R2 = K(d.k.reL2);
         forCellsDF(d, pi, hi, d.bandHiL, [&](int j, int s, float4 hj) {
-            if (j != i) pair(j, hj, __ldg(&d.posLoCell[s]));
+            if (j == i) return;
+            const float4 lj = __ldg(&d.posLoCell[s]);
+            const df d2 = pairDF(hj, lj, hi, li).d2;
+            if (inBallDF(d, d2, R2, d.mgL, P.reL2, i, j) && sideOkDF(d, sc, hj, lj, d2, i, j)) add(j, 0, load(j));
         });
     }
-    double cv = P.coeffViscMultiphase;
-    d.acc[i] = make_dvec4(cv * dD(ax), cv * dD(ay), cv * dD(az), 0.0);
+    ax = laneSumDF<L>(ax); ay = laneSumDF<L>(ay); az = laneSumDF<L>(az);
+    const double cv = P.coeffViscMultiphase;
+    if (l == 0) d.acc[i] = make_dvec4(cv * dD(ax), cv * dD(ay), cv * dD(az), 0.0);
 }
 void launchViscosityListDF(const Dev& d, cudaStream_t s) {
     launchVelDF(d, s);
-    k_visc_list_df<<<gridFor(d.N0, 128), 128, 0, s>>>(d);
+#define LAUNCH(L) k_visc_list_df<L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
 }
 
 // The skin list covers the list of the current positions while every particle is within
