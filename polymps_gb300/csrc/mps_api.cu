@@ -983,6 +983,7 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
             else B.pgridOwn = 0;
         }
         B.pgridRes = ppePersistentGrid(9);
+        B.cluster = ppePersistentGrid(10);
         B.pgridOwn64 = ppePersistentGrid(8);
         if (B.pgridOwn64 > 0) {
             const long long slots = ((long long)n / ((long long)B.pgridOwn64 * 768) + 1) * 768;

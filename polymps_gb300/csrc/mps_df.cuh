@@ -72,12 +72,22 @@ __device__ __forceinline__ df divDF(df a, df b) {
 __device__ __forceinline__ bool operator<(df a, df b) { return a.h < b.h || (a.h == b.h && a.l < b.l); }
 __device__ __forceinline__ bool operator>(df a, df b) { return b < a; }
 
-// conversions (per particle and per stored value; one FP64 addition each, the FP32 <-> FP64
-// conversions in integer operations)
-__device__ __forceinline__ df dfD(double x) {
-    float h = d2fRN(x);
+// conversions (per particle and per stored value).  dfD: the significand's upper 24 bits and its
+// lower 29 bits as two floats, normalised by a fast two-sum, without an FP64 operation; values
+// outside the normal range of FP32 are rounded and subtracted in FP64.
+static __device__ __noinline__ df dfWide(double x) {
+    const float h = d2fRN(x);
     return {h, d2fRN(x - f2dExact(h))};
 }
+__device__ __forceinline__ df dfD(double x) {
+    const unsigned xh = (unsigned)__double2hiint(x), xl = (unsigned)__double2loint(x);
+    const unsigned s = xh & 0x80000000u, e = (xh >> 20) & 0x7ffu;
+    if (e - 897u >= 253u) return (x == 0.0) ? df{(float)0.f, 0.f} : dfWide(x);
+    const float h = __uint_as_float(s | __funnelshift_l(xl, (xh & 0x7fffffffu) - 0x38000000u, 3));
+    const float l = (float)(xl & 0x1fffffffu) * 0x1p-52f * __uint_as_float(s | ((e - 896u) << 23));
+    return quick2(h, l);
+}
+// one FP64 addition
 __device__ __forceinline__ double dD(df a) { return f2dExact(a.h) + f2dExact(a.l); }
 
 // 1/sqrt(a) for a > 0: FP32 estimate refined by one Newton step in float-float

@@ -147,6 +147,7 @@ struct PpeBuffers {
     // vector in global memory instead
     int pgridOwn, ownCap, ownOff;
     int pgridOwn64, ownCap64;
+    int cluster;             // 1: the one-cluster solver of small systems is available
     int pgridRes;            // blocks of the solvers with resident matrices at most (0: unavailable)
     // learned warm start: the network's correction c of the start x (nullptr: none); the
     // shared-memory mixed solver takes the residual-minimising step x + theta c in its set-up

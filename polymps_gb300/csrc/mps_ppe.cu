@@ -1915,6 +1915,260 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
     qStore(B, qL);
 }
 
+// ------------------------------------------------------------------ one cluster
+// The plain FP64 solver of systems of a few thousand rows by one cluster of 16 blocks, one row
+// per thread.  At that size an iteration over the whole grid is its two grid sums (arrival
+// counter, poll and partials: three trips to the L2 each); inside a cluster a barrier and the
+// exchange of partials stay in distributed shared memory, every block keeps its own copy of z
+// (an owner writes its element into all 16), and the matrix stays in shared memory with 16-bit
+// columns.  One reduction an iteration (Chronopoulos and Gear, s-step methods, J. Comput. Appl.
+// Math. 25, 1989): with q = A z,
+//   gamma = r.z, delta = z.q, rho = r.r;  beta = gamma / gamma_old,
+//   alpha = gamma / (delta - gamma^2 / (gamma_old alpha_old)),
+//   p = z + beta p,  Ap = q + beta Ap,  x += alpha p,  r -= alpha Ap,  z = M^-1 r,
+// the same vectors as k_cg_res, whose p.Ap it forms by linearity too.  The first warp has no
+// rows: it sums the warps' partials and forms the step scalars.
+#define CLB 16                 // blocks of the cluster
+#define CL_ROWS 256            // rows of a block at most
+struct ClShared {
+    float2 part[3][CL_ROWS / 32][CLB];   // the warps' partials (every warp writes its own into all blocks)
+    double alpha, beta;
+    int stop;
+};
+__device__ __forceinline__ void clArrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void clWait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ unsigned clAddr(const void* p, unsigned rank) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void clStore(const void* p, unsigned rank, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(clAddr(p, rank)), "d"(v) : "memory");
+}
+__device__ __forceinline__ void clStore(const void* p, unsigned rank, float2 v) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(clAddr(p, rank)), "f"(v.x), "f"(v.y) : "memory");
+}
+// The cluster's sums of NV values per thread, in float-float from the warp level on (as qSumD):
+// every warp writes its partials into all blocks, the first warp of each sums them in the same
+// order; fin(totals) on its thread 0; the caller synchronises the block before reading what it
+// wrote.  One cluster barrier.
+template <int NV, class Fin>
+__device__ __forceinline__ void clSum(const double (&v)[NV], ClShared& S, unsigned rank, Fin&& fin) {
+    const int lane = threadIdx.x & 31, w = (int)threadIdx.x >> 5, nw = ((int)blockDim.x >> 5) - 1;
+    if (w > 0) {
+#pragma unroll
+        for (int q = 0; q < NV; q++) {
+            df a = dfD(v[q]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a += shflXorDF(a, o);
+            if (lane < CLB) clStore(&S.part[q][w - 1][rank], lane, make_float2(a.h, a.l));
+        }
+    }
+    clArrive();
+    clWait();
+    if (w == 0) {
+        df a[NV];
+#pragma unroll
+        for (int q = 0; q < NV; q++) a[q] = dfF(0.f);
+        for (int m = lane; m < nw * CLB; m += 32)
+#pragma unroll
+            for (int q = 0; q < NV; q++) {
+                const float2 x = S.part[q][0][m];
+                a[q] += df{x.x, x.y};
+            }
+#pragma unroll
+        for (int q = 0; q < NV; q++)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a[q] += shflXorDF(a[q], o);
+        if (lane == 0) fin(a);
+    }
+}
+// a / b to the last bits of the pair: the quotient of divDF corrected by its remainder
+__device__ __forceinline__ df divDF2(df a, df b) {
+    const df q = divDF(a, b);
+    return q + divDF(a - b * q, b);
+}
+__global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffers B, double tol, int maxIter, int cap) {
+    __shared__ QLocal qL;
+    __shared__ ClShared S;
+    extern __shared__ __align__(128) unsigned char dynSmem[];
+    double* const zc = reinterpret_cast<double*>(dynSmem);
+    const int n = liveN(d), T = (int)blockDim.x - 32;
+    double* const sv = zc + CLB * T;
+    unsigned short* const sc = reinterpret_cast<unsigned short*>(sv + (size_t)cap * T);
+    unsigned rank;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    qInit(qL);
+    double* const qS = qL.scal;
+    int* const qF = qL.flag;
+    const int t = (int)threadIdx.x - 32;                                  // row of the block, negative: none
+    const int i = t >= 0 && (int)rank * T + t < n ? (int)rank * T + t : -1;
+    const bool own = i >= 0;
+    const int len = own ? __ldg(B.rowLen + i) : 0;
+    const int most = __reduce_max_sync(0xffffffffu, len);
+    const size_t base = own ? ellBase(B, i) : 0;
+    const int held = min((most + 3) & ~3, cap);   // cap is a multiple of 4
+    if (t >= 0)
+        for (int e = 0; e < held; e++) {
+            const bool ok = e < len;
+            sc[e * T + t] = ok ? (unsigned short)ldStream(B.col + base + (size_t)e * B.ellStride) : (unsigned short)0;
+            sv[e * T + t] = ok ? ldStream(B.val + base + (size_t)e * B.ellStride) : 0.0;
+        }
+    for (int k = threadIdx.x; k < n; k += blockDim.x) zc[k] = B.x[k];
+    __syncthreads();
+    double dg = 1.0, x = 0.0, r = 0.0, z = 0.0, p = 0.0, ap = 0.0, di = 1.0, bi = 0.0;
+    // (A v)_i of the vector in zc, v its own element
+    auto product = [&](double v) {
+        double a[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int e = 0; e < held; e += 4) {
+            double g[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) g[u] = zc[sc[(e + u) * T + t]];
+#pragma unroll
+            for (int u = 0; u < 4; u++) a[u] += sv[(e + u) * T + t] * g[u];
+        }
+        for (int e = held; e < len; e++)
+            a[0] += ldStream(B.val + base + (size_t)e * B.ellStride) * zc[ldStream(B.col + base + (size_t)e * B.ellStride)];
+        return dg * v + ((a[0] + a[1]) + (a[2] + a[3]));
+    };
+    auto publish = [&](double v) {   // into every block's copy
+#pragma unroll
+        for (unsigned q = 0; q < CLB; q++) clStore(zc + i, q, v);
+    };
+    if (own) {
+        dg = __ldg(B.diag + i);
+        di = 1.0 / dg;
+        x = B.x[i];
+        bi = B.b[i];
+        r = bi - product(x);
+        z = r * di;
+    }
+    {
+        const double v[2] = {bi * bi, r * r};
+        clSum<2>(v, S, rank, [&](const df* sums) {   // its barrier also ends every block's reads of x
+            const double s[2] = {dD(sums[0]), dD(sums[1])};
+            qS[S_BB] = s[0];
+            double thr = tol * tol * s[0];
+            if (thr < 2.2250738585072014e-308) thr = 2.2250738585072014e-308;
+            qS[S_THR] = thr;
+            qS[S_RR] = s[1];
+            qS[S_SCALE] = sqrt(s[1] / (s[0] > 0 ? s[0] : 1.0));
+            qF[0] = (s[0] == 0.0 || s[1] < thr) ? 1 : 0;
+            qF[1] = 0;
+            if (!(s[1] == s[1])) { qF[0] = 1; qF[2] = 1; }
+            S.stop = qF[0] || maxIter <= 0;
+        });
+    }
+    if (own) publish(z);
+    clArrive();
+    clWait();
+    // thread 0: gamma_old and gamma_old alpha_old, and the squared residual norm that ends it
+    df gammaOld = dfF(0.f), step = dfF(0.f);
+    const df stop2 = dfD(qS[S_THR]);
+    __syncthreads();
+    while (!S.stop) {
+        double v[3] = {0.0, 0.0, 0.0}, q = 0.0;
+        if (own) {
+            q = product(z);
+            v[0] = r * z; v[1] = z * q; v[2] = r * r;
+        }
+        df gamma = dfF(0.f), rr = dfF(0.f), alpha2 = dfF(0.f);
+        clSum<3>(v, S, rank, [&](const df* s) {
+            // (step scalars in float-float like the sums they come from: a chain of FP64
+            // divisions on one thread would be a third of the iteration)
+            const bool first = qF[1] == 0;
+            gamma = s[0];
+            rr = s[2];
+            if (rr < stop2) qF[0] = 1;
+            if (!(rr.h == rr.h) || !(gamma.h == gamma.h)) { qF[0] = 1; qF[2] = 1; }
+            S.stop = qF[0] || qF[1] >= maxIter;
+            S.beta = first ? 0.0 : dD(divDF2(gamma, gammaOld));
+            alpha2 = divDF2(gamma, first ? s[1] : s[1] - divDF2(gamma * gamma, step));
+            S.alpha = dD(alpha2);
+        });
+        __syncthreads();
+        if (S.stop) {
+            if (threadIdx.x == 0) qS[S_RR] = dD(rr);
+            break;
+        }
+        if (own) {
+            const double alpha = S.alpha, beta = S.beta;
+            p = z + beta * p;
+            ap = q + beta * ap;
+            x += alpha * p;
+            r -= alpha * ap;
+            z = r * di;
+            publish(z);
+        }
+        clArrive();
+        if (threadIdx.x == 0) {
+            qF[1] += 1;
+            gammaOld = gamma;
+            step = gamma * alpha2;
+        }
+        clWait();
+    }
+    // FP64 residual of the result
+    clArrive();
+    clWait();   // every block has left its last product
+    if (own) { B.x[i] = x; publish(x); }
+    clArrive();
+    clWait();
+    {
+        double v[1] = {0.0};
+        if (own) {
+            const double e = bi - product(x);
+            v[0] = e * e;
+        }
+        clSum<1>(v, S, rank, [&](const df* s) { qS[S_RR] = dD(s[0]); });
+    }
+    __syncthreads();
+    if (rank == 0) qStore(B, qL);
+}
+// Shared memory of k_cg_cluster for a system of `rows` rows (T threads with rows per block, cap
+// entries of each held), 0 where a block's part does not fit.
+static size_t clusterShape(const PpeBuffers& B, int rows, int* T, int* cap) {
+    *T = ((rows + CLB - 1) / CLB + 31) / 32 * 32;
+    if (rows <= 0 || *T > CL_ROWS) return 0;
+    const size_t room = 220 * 1024 - (size_t)CLB * *T * 8;
+    *cap = std::min((B.K + 3) / 4 * 4, (int)(room / ((size_t)*T * 10)) / 4 * 4);
+    return (size_t)CLB * *T * 8 + (size_t)*cap * *T * 10;
+}
+static cudaError_t launchCluster(const Dev& d, const PpeBuffers& B, double tol, int maxIter, int T, int cap, size_t dyn,
+                                 cudaStream_t s) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(CLB);
+    c.blockDim = dim3(T + 32);
+    c.dynamicSmemBytes = dyn;
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CLB; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, k_cg_cluster, d, B, tol, maxIter, cap);
+}
+// 1 when this GPU can hold a cluster of the largest shape.
+static int clusterAvailable() {
+    if (cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(CLB);
+    c.blockDim = dim3(CL_ROWS + 32);
+    c.dynamicSmemBytes = 220 * 1024;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CLB; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k_cg_cluster, &c) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return clusters > 0;
+}
+
 // Mixed FP32/FP64 solver: method, stopping rules and reports of k_mx_own (LEARNED as there:
 // the residual of the start is in B.r, its correction and their product in B.cdir and B.cq).
 template <bool LEARNED>
@@ -2198,6 +2452,7 @@ int ppePersistentGrid(int kind) {
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cg_own, QBC, dyn) != cudaSuccess || per <= 0) return 0;
         return sms;
     }
+    if (kind == 10) return clusterAvailable();
     if (kind == 9) {   // resident matrices, one block per SM
         for (const void* f : {(const void*)k_cg_res, (const void*)k_mx_res<false>, (const void*)k_mx_res<true>}) {
             const int dyn = f == (const void*)k_cg_res ? RES_CAP64 * RBS * 12 : RES_CAP32 * RBS * 8;
@@ -2264,6 +2519,10 @@ int ppeSolveBicgstab(const Dev& d, const PpeBuffers& B, double tol, int maxIter,
     return finishPersistent(B, s, iters, nullptr, relres, relres0);
 }
 
+// Rows up to which one cluster takes the plain FP64 solve (its 16 SMs' FP64 pipes bound it above):
+// whole solves by k_cg_cluster and k_cg_res at 1,000 rows 146 / 195 us, 2,048 rows 170 / 216,
+// 4,000 rows 219 / 235, 5,324 rows 256 / 235, 6,912 rows 310 / 253.
+#define CLUSTER_MAX_ROWS 4096
 // Lanes per row of the resident solvers: 4, 2 or 1, as many as give every row of `rows` its
 // lanes in one round of the grid; 0: too many rows.
 static int resLanes(int rows, int grid) {
@@ -2296,6 +2555,18 @@ int ppeSolvePersistent(const Dev& d, const PpeBuffers& B, int mixed, double tol,
     double t = tol, eta2 = 1e-6 * 1e-6;
     int mi = maxIter;
     void* args[6] = {&dd, &bb, &t, &mi, &eta2, nullptr};
+    if (!mixed && !B.ownOff && B.cluster && d.N0 <= CLUSTER_MAX_ROWS) {
+        int T = 0, cap = 0;
+        const size_t dyn = clusterShape(B, d.N0, &T, &cap);
+        if (dyn) {
+            if (pr) prof->begin(PROF_PPE_SOLVE, s);
+            const cudaError_t e = launchCluster(d, B, tol, maxIter, T, cap, dyn, s);
+            if (pr) prof->end(s);
+            if (e != cudaSuccess) return MPSGPU_ERR_CUDA;
+            countLaunch(1);
+            return finishPersistent(B, s, iters, refinements, relres, relres0);
+        }
+    }
     const int lanes = B.matfree == 0 && !B.ownOff && B.pgridRes > 0 ? resLanes(d.N0, B.pgridRes) : 0;
     if (lanes) {
         // at most one row per thread: the matrix stays in shared memory.  The rows are spread
