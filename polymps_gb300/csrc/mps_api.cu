@@ -632,6 +632,15 @@ static void fromRef(mpsgpu_t h, int kind, void* p, int n) {
     countLaunch(1);
 }
 
+// rows [r0, r1) of the neighbour list in reference order and indices, row r at off[r] - base
+__global__ void k_csr_rows(Dev d, const int* off, int r0, int r1, int base, int* out) {
+    const int r = r0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= r1) return;
+    const int i = d.slotOf[r], c = d.nbrCount[i];
+    int* const o = out + (off[r] - base);
+    for (int k = 0; k < c; k++) o[k] = d.orig[d.nbr[(size_t)k * d.N0 + i]];
+}
+
 // ------------------------------------------------------------------ binary .vtu output
 // Arrays of the appended block in the reference's particle order (slotOf maps a reference
 // index to its storage slot), converted as the ASCII writer converts them ((float) casts).
@@ -1352,26 +1361,34 @@ int mpsgpu_get_neighbors(mpsgpu_t h, int* counts, int* nbr, long long cap) {
     if (e) return e;
     int n = 0;
     if ((e = mpsgpu_num_particles(h, &n))) return e;
-    // rows and entries in reference indices (storage is in bucket order)
-    std::vector<int> cnt(n), orig(h->N0), slot(h->N0);
-    CK(cudaMemcpyAsync(cnt.data(), h->d.nbrCount, sizeof(int) * n, cudaMemcpyDeviceToHost, h->s));
-    CK(cudaMemcpyAsync(orig.data(), h->d.orig, sizeof(int) * h->N0, cudaMemcpyDeviceToHost, h->s));
-    CK(cudaMemcpyAsync(slot.data(), h->d.slotOf, sizeof(int) * h->N0, cudaMemcpyDeviceToHost, h->s));
+    // rows and entries in reference indices (storage is in bucket order), laid out on the GPU:
+    // counts, their scan, then the rows one after the other through the reorder scratch, as
+    // many at a time as it holds (any row fits).  Copying the whole ELL array and reordering it on
+    // the host took 9.6 ms at 108k particles, mostly host loops.
+    int* const cnt = reinterpret_cast<int*>(h->d.cellRec);   // free between two bucket builds
+    int* const off = static_cast<int*>(h->permScratch);
+    int* const out = off + (n + 1);
+    const long long room = 8ll * h->N0 - (n + 1);
+    k_to_ref<int><<<gridFor(n, 256), 256, 0, h->s>>>(h->d.nbrCount, cnt, h->d.slotOf, n);
+    CK(cudaMemcpyAsync(counts, cnt, sizeof(int) * n, cudaMemcpyDeviceToHost, h->s));
+    if (nbr) scanExclusive(cnt, off, n, h->scanScratch, h->s);
     CK(cudaStreamSynchronize(h->s));
-    for (int r = 0; r < n; r++) counts[r] = cnt[slot[r]];
-    if (!nbr) return 0;
-    std::vector<int> ell((size_t)h->d.K * h->N0);
-    CK(cudaMemcpyAsync(ell.data(), h->d.nbr, sizeof(int) * ell.size(), cudaMemcpyDeviceToHost, h->s));
-    CK(cudaStreamSynchronize(h->s));
+    countLaunch(nbr ? 3 : 1);
     long long k = 0;
-    for (int r = 0; r < n; r++) {
-        int i = slot[r];
-        for (int c = 0; c < counts[r]; c++) {
-            if (k >= cap) return MPSGPU_ERR_CAPACITY;
-            nbr[k++] = orig[ell[(size_t)c * h->N0 + i]];
-        }
+    for (int r0 = 0; nbr && r0 < n;) {
+        int r1 = r0;
+        long long m = 0;
+        while (r1 < n && m + counts[r1] <= room) m += counts[r1++];
+        k_csr_rows<<<gridFor(r1 - r0, 128), 128, 0, h->s>>>(h->d, off, r0, r1, (int)k, out);
+        countLaunch(1);
+        const long long take = std::min(m, cap - k);
+        if (take > 0) CK(cudaMemcpyAsync(nbr + k, out, sizeof(int) * take, cudaMemcpyDeviceToHost, h->s));
+        CK(cudaStreamSynchronize(h->s));
+        if (take < m) return MPSGPU_ERR_CAPACITY;
+        k += m;
+        r0 = r1;
     }
-    return 0;
+    return launchStatus();
 }
 
 int mpsgpu_get_ppe(mpsgpu_t h, long long* nnz_out, long long* rowptr, int* col, double* val, double* rhs) {
