@@ -35,6 +35,10 @@ struct MlpState {
     float* lossAcc = nullptr;      // device loss accumulator
     int adamStep = 0;
     bool recording = false;
+    bool hostTables = false;       // kernels may read pageable host memory (host page tables)
+    void* hostBuf = nullptr;       // device memory of the calls with host arrays
+    size_t hostBytes = 0;
+    float* hostPinned = nullptr;   // page-locked gradient and loss
     int* tcErr = nullptr;          // set by the tensor-core forward when a completion wait ran out
 };
 
