@@ -66,7 +66,8 @@ __global__ void k_cell_key(Dev d) {
         dvec4 p = d.pos[i];
         // x - min once: the key's first operation and the FP32 copies' argument
         const double dx = xsub(p.x, P.domainMin[0]), dy = xsub(p.y, P.domainMin[1]), dzz = xsub(p.z, P.domainMin[2]);
-        const float4 hi = make_float4(d2fRN(dx), d2fRN(dy), d2fRN(dzz), 0.f);
+        const df fx = dfD(dx), fy = dfD(dy), fz = dfD(dzz);
+        const float4 hi = make_float4(fx.h, fy.h, fz.h, 0.f);
         const bool two = (int)P.dim == 2;
         int ix = bucketKeyCoord(hi.x, dx, d.invSidef, d.epsf, P.invBucketSide, P.epsilonZero, two);
         int iy = bucketKeyCoord(hi.y, dy, d.invSidef, d.epsf, P.invBucketSide, P.epsilonZero, two);
@@ -80,7 +81,7 @@ __global__ void k_cell_key(Dev d) {
         }
         // FP32 copy of the start-of-step positions for the prefiltered scans (hi, lo parts)
         d.posf[i] = hi;
-        d.posLo[i] = make_float4(d2fRN(dx - f2dExact(hi.x)), d2fRN(dy - f2dExact(hi.y)), d2fRN(dzz - f2dExact(hi.z)), 0.f);
+        d.posLo[i] = make_float4(fx.l, fy.l, fz.l, 0.f);
     }
     warpGroupAdd(d.cellCount, key, key >= 0);
     if (i < d.N0) d.cellOf[i] = key;
@@ -288,11 +289,10 @@ void launchBuckets(const Dev& d, int* scanScratch, cudaStream_t s, int* perm, vo
 __global__ void k_posf(Dev d) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.N0) return;   // every slot: stale bucket entries may name removed particles
-    dvec4 p = d.pos[i];
-    float4 hi = make_float4(d2fRN(p.x - d.P.domainMin[0]), d2fRN(p.y - d.P.domainMin[1]),
-                            d2fRN(p.z - d.P.domainMin[2]), 0.f);
+    float4 hi, lo;
+    splitPos(d.pos[i], d.P, hi, lo);
     d.posf[i] = hi;
-    d.posLo[i] = posLoOf(p, hi, d.P);
+    d.posLo[i] = lo;
 }
 
 // ------------------------------------------------------------------ neighbour list

@@ -18,9 +18,9 @@ __global__ void k_df_vel(Dev d) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.N0) return;
     dvec4 v = d.vel[i];
-    float4 h = make_float4(d2fRN(v.x), d2fRN(v.y), d2fRN(v.z), 0.f);
-    d.velHi[i] = h;
-    d.velLo[i] = make_float4(d2fRN(v.x - f2dExact(h.x)), d2fRN(v.y - f2dExact(h.y)), d2fRN(v.z - f2dExact(h.z)), 0.f);
+    const df x = dfD(v.x), y = dfD(v.y), z = dfD(v.z);
+    d.velHi[i] = make_float4(x.h, y.h, z.h, 0.f);
+    d.velLo[i] = make_float4(x.l, y.l, z.l, 0.f);
 }
 __global__ void k_df_press(Dev d) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -38,7 +38,8 @@ __device__ __forceinline__ df loadDF(const float2* p, int j) {
 }
 
 template <int L>
-__device__ __forceinline__ df laneSumDF(df v) {
+__device__ __forceinline__ df laneSumDF(df v) {   // of accumulators (normalised here)
+    v = normDF(v);
 #pragma unroll
     for (int o = 1; o < L; o <<= 1) {
         const df q = {__shfl_xor_sync(laneGroup<L>(), v.h, o), __shfl_xor_sync(laneGroup<L>(), v.l, o)};
@@ -111,9 +112,9 @@ __global__ void __launch_bounds__(VBLK) k_visc_df(Dev d) {
             WeightDF w = weightDF(q.d2, RL, P.weightType);
             df c = w.w * ((d.type[j] == P.wall) ? neuW : neuF);
             float4 vhj = d.velHi[j], vlj = d.velLo[j];
-            ax += diffDF(vhj.x, vlj.x, vh.x, vl.x) * c;
-            ay += diffDF(vhj.y, vlj.y, vh.y, vl.y) * c;
-            az += diffDF(vhj.z, vlj.z, vh.z, vl.z) * c;
+            mac(ax, diffDF(vhj.x, vlj.x, vh.x, vl.x), c);
+            mac(ay, diffDF(vhj.y, vlj.y, vh.y, vl.y), c);
+            mac(az, diffDF(vhj.z, vlj.z, vh.z, vl.z), c);
         }
     }
     double cv = P.coeffViscMultiphase;
@@ -189,9 +190,7 @@ struct MirrorDF {
 };
 __device__ __forceinline__ MirrorDF mirrorDF(const Dev& d, dvec4 m) {
     MirrorDF o;
-    const MpsParams& P = d.P;
-    o.mh = make_float4(d2fRN(m.x - P.domainMin[0]), d2fRN(m.y - P.domainMin[1]), d2fRN(m.z - P.domainMin[2]), 0.f);
-    o.ml = posLoOf(m, o.mh, P);
+    splitPos(m, d.P, o.mh, o.ml);
     return o;
 }
 // MpsPndNeigh::calcWallNPCD, src/MpsPndNeigh.cpp:105-195
@@ -205,7 +204,7 @@ __global__ void __launch_bounds__(WALL_BLK) k_wall_npcd_df(Dev d) {
         forBitsShared<WALL_L>(d.nbr + i, d.N0, d.mirrorS[i], l, [&](int j, int) {
             const PairF m = pairDF(__ldg(&d.posf[j]), __ldg(&d.posLo[j]), M.mh, M.ml);
             const df wS = weightDF(m.d2, RS, P.weightType).w;
-            sx += m.v.x * wS; sy += m.v.y * wS; sz += m.v.z * wS;
+            mac(sx, m.v.x, wS); mac(sy, m.v.y, wS); mac(sz, m.v.z, wS);
         });
         sx = laneSumDF<WALL_L>(sx); sy = laneSumDF<WALL_L>(sy); sz = laneSumDF<WALL_L>(sz);
         if (l == 0) { sm[0][g] = dD(sx); sm[1][g] = dD(sy); sm[2][g] = dD(sz); }
@@ -248,8 +247,8 @@ struct MomentsDF {
     df xx = {0.f, 0.f}, xy = {0.f, 0.f}, xz = {0.f, 0.f}, yy = {0.f, 0.f}, yz = {0.f, 0.f}, zz = {0.f, 0.f};
     __device__ __forceinline__ void add(const V3& v, df wr2) {
         const df t0 = v.x * wr2, t1 = v.y * wr2, t2 = v.z * wr2;
-        xx += t0 * v.x; xy += t0 * v.y; xz += t0 * v.z;
-        yy += t1 * v.y; yz += t1 * v.z; zz += t2 * v.z;
+        mac(xx, t0, v.x); mac(xy, t0, v.y); mac(xz, t0, v.z);
+        mac(yy, t1, v.y); mac(yz, t1, v.z); mac(zz, t2, v.z);
     }
     template <int L>
     __device__ __forceinline__ void sum() {
@@ -346,8 +345,8 @@ __global__ void __launch_bounds__(BLK, 9) k_pnd_npcd_df(Dev d) {
                      WeightDF w = weightDF(q.d2, RS, P.weightType);
                      if (CORR) M.add(q.v, w.wr2);
                      if (!CORR || maskHas(mL, k)) {
-                         ni += w.w;
-                         nx += q.v.x * w.w; ny += q.v.y * w.w; nz += q.v.z * w.w;
+                         acc(ni, w.w);
+                         mac(nx, q.v.x, w.w); mac(ny, q.v.y, w.w); mac(nz, q.v.z, w.w);
                      }
                  });
     ni = laneSumDF<L>(ni); nx = laneSumDF<L>(nx); ny = laneSumDF<L>(ny); nz = laneSumDF<L>(nz);
@@ -425,7 +424,7 @@ __global__ void __launch_bounds__(128, 9) k_ppe_assemble_df(Dev d, PpeBuffers B)
                          return;
                      }
                      df mij = wL * cP;
-                     sum -= mij;
+                     acc(sum, -mij);
                      if (n.bc != P.inner) return;
                      int at;
                      if (L > 1) at = maskRank(mm, k);
@@ -497,7 +496,7 @@ __global__ void __launch_bounds__(BLK, 8) k_press_grad_df(Dev d) {
                          double nj = d.pndi[j], Pj = d.press[j], Pid = d.press[i];
                          f = (ni > P.epsilonZero && nj > P.epsilonZero) ? dfD(ni * Pj / nj + nj * Pid / ni) * w.wr2 : w.w;
                      }
-                     ax += q.v.x * f; ay += q.v.y * f; az += q.v.z * f;
+                     mac(ax, q.v.x, f); mac(ay, q.v.y, f); mac(az, q.v.z, f);
                  });
     ax = laneSumDF<L>(ax); ay = laneSumDF<L>(ay); az = laneSumDF<L>(az);
     if (l != 0) return;
@@ -554,7 +553,7 @@ __global__ void __launch_bounds__(WALL_BLK) k_wall_press_grad_df(Dev d, bool fre
                 double nj = d.pndi[j], Pj = d.press[j];
                 f = (ni > P.epsilonZero && nj > P.epsilonZero) ? dfD(ni * Pj / nj + nj * Pid / ni) * w.wr2 : w.w;
             }
-            sx += m.v.x * f; sy += m.v.y * f; sz += m.v.z * f;
+            mac(sx, m.v.x, f); mac(sy, m.v.y, f); mac(sz, m.v.z, f);
         });
         sx = laneSumDF<WALL_L>(sx); sy = laneSumDF<WALL_L>(sy); sz = laneSumDF<WALL_L>(sz);
         if (l == 0) { sm[0][g] = dD(sx); sm[1][g] = dD(sy); sm[2][g] = dD(sz); pmn[g] = dD(pmin); }
@@ -626,9 +625,9 @@ __global__ void __launch_bounds__(WALL_BLK) k_wall_visc_df(Dev d) {
             const PairF m = pairDF(__ldg(&d.posf[j]), __ldg(&d.posLo[j]), Mi.mh, Mi.ml);
             const df c = weightDF(m.d2, RL, P.weightType).w * neuF;
             float4 vhj = d.velHi[j], vlj = d.velLo[j];
-            sx += (dfOf(vhj.x, vlj.x) - vmx) * c;
-            sy += (dfOf(vhj.y, vlj.y) - vmy) * c;
-            sz += (dfOf(vhj.z, vlj.z) - vmz) * c;
+            mac(sx, dfOf(vhj.x, vlj.x) - vmx, c);
+            mac(sy, dfOf(vhj.y, vlj.y) - vmy, c);
+            mac(sz, dfOf(vhj.z, vlj.z) - vmz, c);
         });
         sx = laneSumDF<WALL_L>(sx); sy = laneSumDF<WALL_L>(sy); sz = laneSumDF<WALL_L>(sz);
         if (l == 0) { sm[0][g] = dD(sx); sm[1][g] = dD(sy); sm[2][g] = dD(sz); }
@@ -721,9 +720,9 @@ struct ShiftVelDF {
         const RadiusDF RS = {K(d.k.reS), K(d.k.invReS)};
         df dw = dweightDF(q.d2, RS, d.P.weightType);
         float4 vhj = d.velHi[j], vlj = d.velLo[j];
-        st.ux += diffDF(vhj.x, vlj.x, st.vh.x, st.vl.x) * dw;
-        st.uy += diffDF(vhj.y, vlj.y, st.vh.y, st.vl.y) * dw;
-        st.uz += diffDF(vhj.z, vlj.z, st.vh.z, st.vl.z) * dw;
+        mac(st.ux, diffDF(vhj.x, vlj.x, st.vh.x, st.vl.x), dw);
+        mac(st.uy, diffDF(vhj.y, vlj.y, st.vh.y, st.vl.y), dw);
+        mac(st.uz, diffDF(vhj.z, vlj.z, st.vh.z, st.vl.z), dw);
     }
     __device__ void end(const Dev& d, int i, State& st, bool on) const {
         bool apply = on && d.bc[i] == d.P.inner;
@@ -736,7 +735,7 @@ struct ConcDF {
     __device__ bool begin(const Dev&, int, State& st) const { st.sum = dfF(0.f); return true; }
     __device__ void visit(const Dev& d, State& st, int, const PairF& q) const {
         const RadiusDF RS = {K(d.k.reS), K(d.k.invReS)};
-        st.sum += weightDF(q.d2, RS, d.P.weightType).w;
+        acc(st.sum, weightDF(q.d2, RS, d.P.weightType).w);
     }
     __device__ void end(const Dev& d, int i, State& st, bool) const {
         d.conc[i] = (dD(st.sum) + d.pndWall[i]) / d.P.pndSmallZero;
@@ -760,7 +759,7 @@ struct GradConcDF {
     __device__ void visit(const Dev& d, State& st, int j, const PairF& q) const {
         const RadiusDF RS = {K(d.k.reS), K(d.k.invReS)};
         df cc = (st.ci + loadDF(d.concDF, j)) * weightDF(q.d2, RS, d.P.weightType).wr2;
-        st.gx += q.v.x * cc; st.gy += q.v.y * cc; st.gz += q.v.z * cc;
+        mac(st.gx, q.v.x, cc); mac(st.gy, q.v.y, cc); mac(st.gz, q.v.z, cc);
     }
     __device__ void end(const Dev& d, int i, State& st, bool on) const {
         const MpsParams& P = d.P;
@@ -796,7 +795,7 @@ __global__ void __launch_bounds__(WALL_BLK) k_wall_grad_conc_df(Dev d, bool skin
             forWallCand(d, W, i, g, l, [&](int j) {
                 const PairF m = pairDF(__ldg(&d.posf[j]), __ldg(&d.posLo[j]), M.mh, M.ml);
                 const df cc = (ci + loadDF(d.concDF, j)) * weightDF(m.d2, RS, P.weightType).wr2;
-                sx += m.v.x * cc; sy += m.v.y * cc; sz += m.v.z * cc;
+                mac(sx, m.v.x, cc); mac(sy, m.v.y, cc); mac(sz, m.v.z, cc);
             });
             sx = laneSumDF<WALL_L>(sx); sy = laneSumDF<WALL_L>(sy); sz = laneSumDF<WALL_L>(sz);
             if (l == 0) { sm[0][g] = dD(sx); sm[1][g] = dD(sy); sm[2][g] = dD(sz); }
@@ -880,9 +879,9 @@ __global__ void __launch_bounds__(128) k_visc_list_df(Dev d) {
     auto add = [&](int, int, const Nbr& n) {
         const PairF q = pairDF(n.p.h, n.p.l, hi, li);
         const df c = weightDF(q.d2, RL, P.weightType).w * (n.type == P.wall ? K(d.k.neuW) : K(d.k.neuF));
-        ax += diffDF(n.vh.x, n.vl.x, vh.x, vl.x) * c;
-        ay += diffDF(n.vh.y, n.vl.y, vh.y, vl.y) * c;
-        az += diffDF(n.vh.z, n.vl.z, vh.z, vl.z) * c;
+        mac(ax, diffDF(n.vh.x, n.vl.x, vh.x, vl.x), c);
+        mac(ay, diffDF(n.vh.y, n.vl.y, vh.y, vl.y), c);
+        mac(az, diffDF(n.vh.z, n.vl.z, vh.z, vl.z), c);
     };
     const int c = d.nbrCount[i];
     if (c <= d.K) {
