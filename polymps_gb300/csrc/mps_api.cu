@@ -779,7 +779,7 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
         h->permScratch = sc;
     }
     A(d.cellSorted, n);
-    A(d.posfCell, n);
+    A(d.posfCell, (size_t)n + 32);   // padded: the list build reads past a range's end
     A(d.posLo, n);
     A(d.posLoCell, n);
     A(d.velHi, n);

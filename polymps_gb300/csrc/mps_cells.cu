@@ -349,36 +349,47 @@ __global__ void __launch_bounds__(128) k_build_list(Dev d) {
             const int s1 = d.cellStart[hi + 1];
 #pragma unroll 1
             for (int s0 = d.cellStart[lo]; s0 < s1; s0 += 32) {
-                const int w = s1 - s0 < 32 ? s1 - s0 : 32;
-                unsigned m = 0u;
-#pragma unroll 1
-                for (int t = l; t < w; t += 4 * L) {
-                    float4 f[4];
+                // bit b: candidate s0 + b.  Every lane's bit positions are constants and nothing is
+                // predicated: what lies past the range (the array is padded) is masked off
+                // after, like the particle itself, so a candidate costs nine instructions
+                const int w = s1 - s0;
+                const float4* const f = d.posfCell + s0 + l;
+                unsigned m = 0u, sure = 0u;
 #pragma unroll
-                    for (int u = 0; u < 4; u++)
-                        f[u] = t + u * L < w ? __ldg(&d.posfCell[s0 + t + u * L]) : make_float4(3e38f, 0.f, 0.f, 0.f);
+                for (int g = 0; g < 32 / L; g += 4) {
+                    if (g * L >= w) break;
+                    float4 h[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) h[u] = __ldg(f + (g + u) * L);
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
-                        const float d2f = dist2f(f[u], fi);
-                        bool in = t + u * L < w && s0 + t + u * L != me;
-                        if (MODE == 0) in = in && !(d2f > d.skinR2);
-                        else {
-                            in = in && !(d2f > d.bandHi);
-                            if (in && !(d2f < d.bandLo))
-                                in = pairInsideExact(d.pos, __ldg(d.cellSorted + s0 + t + u * L), i, d.reMax2);
-                        }
-                        if (in) m |= 1u << (t + u * L);
+                        const float d2f = dist2f(h[u], fi);
+                        if (!(d2f > (MODE == 0 ? d.skinR2 : d.bandHi))) m |= 1u << ((g + u) * L);
+                        if (MODE != 0 && d2f < d.bandLo) sure |= 1u << ((g + u) * L);
                     }
                 }
-                unsigned all = m;
+                if (L > 1) { m <<= l; sure <<= l; }
+                if (w < 32) m &= (1u << w) - 1u;
+                if ((unsigned)(me - s0) < 32u) m &= ~(1u << (me - s0));
+                if (MODE != 0)
+                    for (unsigned r = m & ~sure; r; r &= r - 1u) {   // inside the band: FP64 decides
+                        const int b = __ffs((int)r) - 1;
+                        if (!pairInsideExact(d.pos, __ldg(d.cellSorted + s0 + b), i, d.reMax2)) m &= ~(1u << b);
+                    }
+                if (L == 1) {
+                    for (; m; m &= m - 1u, cnt++)
+                        if (cnt < d.K) d.nbr[(size_t)cnt * N0 + i] = __ldg(d.cellSorted + s0 + __ffs((int)m) - 1);
+                } else {
+                    unsigned all = m;
 #pragma unroll
-                for (int o = 1; o < L; o <<= 1) all |= __shfl_xor_sync(laneGroup<L>(), all, o);
-                for (unsigned r = m; r; r &= r - 1u) {
-                    const int b = __ffs((int)r) - 1;
-                    const int k = cnt + __popc(all & ((1u << b) - 1u));
-                    if (k < d.K) d.nbr[(size_t)k * N0 + i] = __ldg(d.cellSorted + s0 + b);
+                    for (int o = 1; o < L; o <<= 1) all |= __shfl_xor_sync(laneGroup<L>(), all, o);
+                    for (; m; m &= m - 1u) {
+                        const int b = __ffs((int)m) - 1;
+                        const int k = cnt + __popc(all & ((1u << b) - 1u));
+                        if (k < d.K) d.nbr[(size_t)k * N0 + i] = __ldg(d.cellSorted + s0 + b);
+                    }
+                    cnt += __popc(all);
                 }
-                cnt += __popc(all);
             }
         }
     if (MODE == 0) {
