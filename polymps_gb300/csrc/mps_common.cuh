@@ -410,6 +410,8 @@ __device__ __forceinline__ void forNbrsPosf(const Dev& d, int i, F&& f) {
 template <class T, bool RO>
 __device__ __forceinline__ T ellRow(const T* diag, const T* val, const int* col, const T* x, int i, int len, size_t base,
                                     size_t stride) {
+    // FP64 takes four sums, not eight: each further one is an addition per row on its pipe
+    constexpr int NA = sizeof(T) == 8 ? 4 : ELL_U;
     T acc[ELL_U];
 #pragma unroll
     for (int u = 0; u < ELL_U; u++) acc[u] = T(0);
@@ -433,10 +435,11 @@ __device__ __forceinline__ T ellRow(const T* diag, const T* val, const int* col,
             vv[u] = ok ? ldStream(v + (size_t)(k + u) * stride) : T(0);
         }
 #pragma unroll
-        for (int u = 0; u < ELL_U; u++) acc[u] += vv[u] * (RO ? __ldg(x + cc[u]) : x[cc[u]]);
+        for (int u = 0; u < ELL_U; u++) acc[u % NA] += vv[u] * (RO ? __ldg(x + cc[u]) : x[cc[u]]);
     }
     T xi = RO ? __ldg(x + i) : x[i];
-    return __ldg(diag + i) * xi + (((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7])));
+    const T lo = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    return __ldg(diag + i) * xi + (NA == 4 ? lo : lo + ((acc[4] + acc[5]) + (acc[6] + acc[7])));
 }
 
 // f(j, e, k) for the entries k of the mask (e = k N0 + i, the entry's ELL index).

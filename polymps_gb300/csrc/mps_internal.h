@@ -146,6 +146,7 @@ struct PpeBuffers {
     // grid (one block per SM; 0: unavailable), the row slots per block, and 1 to keep every
     // vector in global memory instead
     int pgridOwn, ownCap, ownOff;
+    int ownVec;              // how many of the mixed solve's four vectors are there (2 to 4)
     int pgridOwn64, ownCap64;
     int cluster;             // 1: the one-cluster solver of small systems is available
     int pgridRes;            // blocks of the solvers with resident matrices at most (0: unavailable)
@@ -173,9 +174,9 @@ int ppeSolveMixed(const Dev& d, const PpeBuffers& B, double tol, int maxIter, cu
 int ppeSolvePersistent(const Dev& d, const PpeBuffers& B, int mixed, double tol, int maxIter, cudaStream_t s,
                        int* iters, int* refinements, double* relres, double* relres0, Prof* prof);
 int ppePersistentGrid(int mixed);
-// row slots per block of the shared-memory solvers at most (a multiple of their block sizes,
-// 1024 mixed, 768 plain FP64)
-#define OWN_CAP_ROWS 13312
+// shared memory of the mixed solve's vectors at most, and row slots per block of the plain FP64
+// one's (a multiple of its block size, 768)
+#define OWN_SMEM (224 * 1024)
 #define OWN64_CAP_ROWS 8448
 // BiCGSTAB (solver_type 1) in one cooperative launch
 int ppeSolveBicgstab(const Dev& d, const PpeBuffers& B, double tol, int maxIter, cudaStream_t s, int* iters,

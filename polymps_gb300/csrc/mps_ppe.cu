@@ -1134,15 +1134,15 @@ __global__ void __launch_bounds__(OP == 3 ? QB : QBX, OP == 3 ? 4 : 1) k_mx_solv
 }
 
 // ------------------------------------------------------------------ shared-memory vectors
-// The mixed solver with the FP32 inner-CG vectors of each block's rows (x, r, p, Ap: 16
-// bytes per row) in shared memory from the first inner iteration to the last; only z, the
+// The mixed solver with the FP32 inner-CG vectors of each block's rows (Ap, p, r, x: 16
+// bytes per row, fewer of them above 1.7M rows) in shared memory from the first inner iteration
+// to the last; only z, the
 // vector every block gathers through the matrix columns, goes through global memory.  A
 // block's rows are those of the grid-stride rounds (RowSet: at any moment all blocks
 // stream adjacent slices of the column-major ELL arrays, which measured 28% faster than one
 // contiguous range per block), and the m-th row of thread t sits at slot m BS + t of the
 // block's vectors.  The vector pass of an iteration is then shared-memory work plus one
 // coalesced store of z.
-#define OWN_CAPMAX OWN_CAP_ROWS   // slots per block: 4 x 13312 x 4 B = 208 KB of shared memory
 
 // The thread's rows of a RowSet with their shared-memory slot l = m BS + t (m-th row of the
 // thread), f(l, i, len) with the next row's length prefetched; forOwnL without the length.
@@ -1237,17 +1237,24 @@ __device__ __forceinline__ bool mxSetup(const PpeBuffers& B, const RowSet& rs, Q
     return true;
 }
 
-template <bool LEARNED>
+// NV of the four inner vectors are in shared memory: Ap, p, r, x in this order (the ones an
+// iteration touches most first), the others in B.rf and B.xf.  The step scalars are formed in
+// float-float from the float-float sums (FP64 divisions on one thread between two grid sums:
+// 864k rows 8.31 ms for four solves, now 7.94).
+template <bool LEARNED, int NV>
 __global__ void __launch_bounds__(QBX, 1) k_mx_own(Dev d, PpeBuffers B, double tol, int maxIter, double eta2, int cap) {
     __shared__ QLocal qL;   // this block's copy of the solver scalars and flags
+    __shared__ df rz, stop2;   // inner solve: r.z, and the squared residual norm that ends it
     qInit(qL);
     double* const qS = qL.scal;
     int* const qF = qL.flag;
     extern __shared__ __align__(128) unsigned char dynSmem[];
-    float* const sx = reinterpret_cast<float*>(dynSmem);   // inner correction x_f
-    float* const sr = sx + cap;                             // inner residual
-    float* const sp = sr + cap;                             // search direction
-    float* const sap = sp + cap;                            // A p
+    float* const sap = reinterpret_cast<float*>(dynSmem);   // A p
+    float* const sp = sap + cap;                             // search direction
+    float* const sr = sp + cap;                              // inner residual
+    float* const sx = sr + cap;                              // inner correction x_f
+    auto R = [&](int l, int i) -> float& { return NV >= 3 ? sr[l] : B.rf[i]; };
+    auto X = [&](int l, int i) -> float& { return NV >= 4 ? sx[l] : B.xf[i]; };
     const int n = liveN(d);
     const RowSet rs = rowSet(n, QBX);   // this thread's rows (rowCount(rs) * QBX <= cap)
     QCtl c = {0u};
@@ -1260,12 +1267,16 @@ __global__ void __launch_bounds__(QBX, 1) k_mx_own(Dev d, PpeBuffers B, double t
             forOwnL(rs, [&](int l, int i) {
                 const float r = (float)(B.r[i] * inv);
                 const float z = r * __ldg(B.diagInvf + i);
-                sr[l] = r; sx[l] = 0.f;
+                R(l, i) = r; X(l, i) = 0.f;
                 B.zf[i] = z;
                 a[0] += prod2(r, z);
                 a[1] += prod2(r, r);
             });
-            if (!qSumDF<2>(a, B, c, [&](const double* t) { qS[S_RZ] = t[0]; qS[S_RR0] = t[1]; qF[3] = 0; }))
+            if (!qSumF2<2>(a, B, c, [&](const df* t) {
+                    rz = t[0];
+                    stop2 = t[1] * dfD(qS[S_ETA2]);
+                    qF[3] = 0;
+                }))
                 return;
         }
         int inner = 0;
@@ -1281,44 +1292,40 @@ __global__ void __launch_bounds__(QBX, 1) k_mx_own(Dev d, PpeBuffers B, double t
                     sap[l] = ap; sp[l] = p;
                     a[0] += prod2(p, ap);
                 });
-                if (!qSumDF<1>(a, B, c, [&](const double* t) {
-                        qS[S_PAP] = t[0];
-                        qS[S_ALPHA] = qS[S_RZ] / t[0];
-                        qL.scalf[SF_ALPHA] = d2fRN(qS[S_ALPHA]);
-                    }))
-                    return;
+                if (!qSumF2<1>(a, B, c, [&](const df* t) { qL.scalf[SF_ALPHA] = divDF(rz, t[0]).h; })) return;
             }
             {   // x_f += alpha p, r -= alpha Ap, z = M^-1 r; r.z, r.r
                 const float alpha = vf(qL.scalf + SF_ALPHA);
                 df a[2] = {dfF(0.f), dfF(0.f)};
                 const int cnt = rowCount(rs);
                 for (int m0 = 0; m0 < cnt; m0 += 4) {
-                    float mi[4];
+                    float mi[4], ro[4], xo[4];
                     int ii[4];
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         ii[u] = (m0 + u < cnt) ? rowAt(rs, m0 + u) : -1;
                         mi[u] = (ii[u] >= 0) ? __ldg(B.diagInvf + ii[u]) : 0.f;
+                        if (NV < 3) ro[u] = (ii[u] >= 0) ? B.rf[ii[u]] : 0.f;
+                        if (NV < 4) xo[u] = (ii[u] >= 0) ? B.xf[ii[u]] : 0.f;
                     }
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         if (ii[u] < 0) continue;
                         const int l = (m0 + u) * (int)blockDim.x + (int)threadIdx.x;
-                        const float r = sr[l] - alpha * sap[l];
+                        const float r = (NV < 3 ? ro[u] : sr[l]) - alpha * sap[l];
                         const float z = r * mi[u];
-                        sx[l] += alpha * sp[l];
-                        sr[l] = r;
+                        X(l, ii[u]) = (NV < 4 ? xo[u] : sx[l]) + alpha * sp[l];
+                        R(l, ii[u]) = r;
                         B.zf[ii[u]] = z;
                         a[0] += prod2(r, z);
                         a[1] += prod2(r, r);
                     }
                 }
-                if (!qSumDF<2>(a, B, c, [&](const double* t) {
+                if (!qSumF2<2>(a, B, c, [&](const df* t) {
                         qF[1] += 1;
-                        qS[S_BETA] = t[0] / qS[S_RZ];
-                        qL.scalf[SF_BETA] = d2fRN(qS[S_BETA]);
-                        qS[S_RZ] = t[0];
-                        if (t[1] < qS[S_ETA2] * qS[S_RR0] || !(t[1] == t[1])) qF[3] = 1;
+                        qL.scalf[SF_BETA] = divDF(t[0], rz).h;
+                        rz = t[0];
+                        if (t[1] < stop2 || !(t[1].h == t[1].h)) qF[3] = 1;
                     }))
                     return;
             }
@@ -1328,7 +1335,7 @@ __global__ void __launch_bounds__(QBX, 1) k_mx_own(Dev d, PpeBuffers B, double t
         total += inner;
         {   // x += ||r|| x_f (FP64)
             const double sc = vd(qS + S_SQRT);
-            forOwnL(rs, [&](int l, int i) { B.x[i] += sc * (double)sx[l]; });
+            forOwnL(rs, [&](int l, int i) { B.x[i] += sc * (double)X(l, i); });
             if (!qBarrier(B, c)) return;
         }
         {   // FP64 residual r = b - A x
@@ -1352,6 +1359,11 @@ __global__ void __launch_bounds__(QBX, 1) k_mx_own(Dev d, PpeBuffers B, double t
         refine++;
     }
     qStore(B, qL);
+}
+// Kernel and shared memory of the mixed solve with nv vectors there
+static const void* ownKernel(bool learned, int nv) {
+    if (learned) return nv >= 4 ? (const void*)k_mx_own<true, 4> : nv == 3 ? (const void*)k_mx_own<true, 3> : (const void*)k_mx_own<true, 2>;
+    return nv >= 4 ? (const void*)k_mx_own<false, 4> : nv == 3 ? (const void*)k_mx_own<false, 3> : (const void*)k_mx_own<false, 2>;
 }
 
 // FP64 residual row of the refinement without a pass in between: x_j + d_j is formed from
@@ -2439,11 +2451,11 @@ int ppePersistentGrid(int kind) {
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     if (!coop) return 0;
     if (kind == 7) {
-        const int dyn = OWN_CAPMAX * 16;
-        if (cudaFuncSetAttribute(k_mx_own<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
-            cudaFuncSetAttribute(k_mx_own<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
-            return 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mx_own<true>, QBX, dyn) != cudaSuccess || per <= 0) return 0;
+        for (int k = 0; k < 6; k++) {
+            const void* f = ownKernel(k & 1, 2 + k / 2);
+            if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, OWN_SMEM) != cudaSuccess) return 0;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, QBX, OWN_SMEM) != cudaSuccess || per <= 0) return 0;
+        }
         return sms;   // one block per SM: the ranges are sized for it
     }
     if (kind == 8) {
@@ -2601,8 +2613,8 @@ int ppeSolvePersistent(const Dev& d, const PpeBuffers& B, int mixed, double tol,
         int cap = B.ownCap;
         args[5] = &cap;
         if (pr) prof->begin(PROF_PPE_SOLVE, s);
-        const void* fn = B.cdir ? (const void*)k_mx_own<true> : (const void*)k_mx_own<false>;
-        cudaError_t e = cudaLaunchCooperativeKernel(fn, B.pgridOwn, QBX, args, (size_t)cap * 16, s);
+        cudaError_t e = cudaLaunchCooperativeKernel(ownKernel(B.cdir != nullptr, B.ownVec), B.pgridOwn, QBX, args,
+                                                    (size_t)cap * 4 * B.ownVec, s);
         if (pr) prof->end(s);
         if (e != cudaSuccess) return MPSGPU_ERR_CUDA;
         countLaunch(1);
