@@ -647,6 +647,14 @@ __device__ __forceinline__ bool qSumD(double (&v)[NV], const PpeBuffers& B, QCtl
     return qSumDF<NV>(a, B, c, fin);
 }
 
+template <int NV, class Fin>
+__device__ __forceinline__ bool qSumDF2(double (&v)[NV], const PpeBuffers& B, QCtl& c, Fin fin) {   // fin takes the pairs
+    df a[NV];
+#pragma unroll
+    for (int q = 0; q < NV; q++) a[q] = dfD(v[q]);
+    return qSumF2<NV>(a, B, c, fin);
+}
+
 // Rows inside the persistent kernels: matrix arrays are read-only for the launch, the
 // gathered vector is written by other blocks during it (plain loads, made visible by the
 // barrier's fences).  forRows walks a thread's rows with the next row's length prefetched.
@@ -1830,9 +1838,22 @@ __device__ __forceinline__ void resLoad(const ResRow& r, int* sc, T* sv, int cap
     }
 }
 
-// Plain FP64 Jacobi-PCG: method, stopping rule and reports of k_cg_own.
+// a / b to the last bits of the pair: the quotient of divDF corrected by its remainder
+__device__ __forceinline__ df divDF2(df a, df b) {
+    const df q = divDF(a, b);
+    return q + divDF(a - b * q, b);
+}
+// Plain FP64 Jacobi-PCG with one reduction an iteration (Chronopoulos and Gear, s-step methods,
+// J. Comput. Appl. Math. 25, 1989): with q = A z,
+//   gamma = r.z, delta = z.q, rho = r.r;  beta = gamma / gamma_old,
+//   alpha = gamma / (delta - gamma^2 / (gamma_old alpha_old)),
+//   p = z + beta p,  Ap = q + beta Ap,  x += alpha p,  r -= alpha Ap,  z = M^-1 r,
+// the vectors of k_cg_own, whose p.Ap comes by linearity too; the second synchronisation of an
+// iteration is then a barrier (z is complete) without a sum.  The step scalars are formed in
+// float-float like the sums they come from.  Stopping rule and reports of k_cg_own.
 __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double tol, int maxIter, int L, int cap) {
     __shared__ QLocal qL;
+    __shared__ struct { double alpha, beta; df gamma, step, stop2; int stop; } S;   // step: gamma alpha
     qInit(qL);
     double* const qS = qL.scal;
     int* const qF = qL.flag;
@@ -1845,7 +1866,7 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
     resLoad(R, sc, sv, cap, B.col, B.val);
     double x = 0.0, r = 0.0, z = 0.0, p = 0.0, ap = 0.0, di = 0.0, dg = 0.0;
     {
-        double v[3] = {0.0, 0.0, 0.0};
+        double v[2] = {0.0, 0.0};
         if (R.any) {
             const double q = resDot<double>(R, sc, sv, cap, B.col, B.val, B.x);
             if (R.i >= 0) {
@@ -1857,59 +1878,57 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
                 z = r * di;
                 if (own) {
                     B.z[R.i] = z;
-                    v[0] = r * z; v[1] = r * r; v[2] = bi * bi;
+                    v[0] = r * r; v[1] = bi * bi;
                 }
             }
         }
-        if (!qSum<3>(v, B, c, [&](const double* t) {
-                qS[S_RZ] = t[0]; qS[S_RR] = t[1]; qS[S_BB] = t[2];
-                double thr = tol * tol * t[2];
+        if (!qSum<2>(v, B, c, [&](const double* t) {   // and z is complete
+                qS[S_RR] = t[0]; qS[S_BB] = t[1];
+                double thr = tol * tol * t[1];
                 if (thr < 2.2250738585072014e-308) thr = 2.2250738585072014e-308;
                 qS[S_THR] = thr;
-                qS[S_SCALE] = sqrt(t[1] / (t[2] > 0 ? t[2] : 1.0));
-                qF[0] = (t[2] == 0.0 || t[1] < thr) ? 1 : 0;
+                qS[S_SCALE] = sqrt(t[0] / (t[1] > 0 ? t[1] : 1.0));
+                qF[0] = (t[1] == 0.0 || t[0] < thr) ? 1 : 0;
                 qF[1] = 0;
-                if (!(t[0] == t[0]) || !(t[1] == t[1])) { qF[0] = 1; qF[2] = 1; }
+                if (!(t[0] == t[0])) { qF[0] = 1; qF[2] = 1; }
+                S.stop2 = dfD(thr);
+                S.stop = qF[0] || maxIter <= 0;
             }))
             return;
     }
-    int it = 0;
-    while (!vi(qF) && it < maxIter) {
-        {   // Ap = A z + beta Ap, p = z + beta p, p.Ap
-            double v[1] = {0.0};
-            if (R.any) {
-                const double beta = it ? vd(qS + S_BETA) : 0.0;
-                const double q = dg * z + resDot<double>(R, sc, sv, cap, B.col, B.val, B.z);
-                ap = it ? q + beta * ap : q;
-                p = it ? z + beta * p : z;
-                if (own) v[0] = p * ap;
-            }
-            if (!qSumD<1>(v, B, c, [&](const double* t) { qS[S_PAP] = t[0]; qS[S_ALPHA] = qS[S_RZ] / t[0]; }))
-                return;
+    while (!*(volatile int*)&S.stop) {
+        double v[3] = {0.0, 0.0, 0.0}, q = 0.0;
+        if (R.any) {
+            q = dg * z + resDot<double>(R, sc, sv, cap, B.col, B.val, B.z);
+            if (own) { v[0] = r * z; v[1] = z * q; v[2] = r * r; }
         }
-        {   // x += alpha p, r -= alpha Ap, z = M^-1 r; r.z, r.r
-            double v[2] = {0.0, 0.0};
-            if (R.any) {
-                const double alpha = vd(qS + S_ALPHA);
-                x += alpha * p;
-                r -= alpha * ap;
-                z = r * di;
-                if (own) {
-                    B.z[R.i] = z;
-                    v[0] = r * z; v[1] = r * r;
-                }
-            }
-            if (!qSumD<2>(v, B, c, [&](const double* t) {
-                    qF[1] += 1;
-                    qS[S_RR] = t[1];
-                    qS[S_BETA] = t[0] / qS[S_RZ];
-                    qS[S_RZ] = t[0];
-                    if (t[1] < qS[S_THR]) qF[0] = 1;
-                    if (!(t[1] == t[1])) { qF[0] = 1; qF[2] = 1; }
-                }))
-                return;
+        if (!qSumDF2<3>(v, B, c, [&](const df* t) {
+                const bool first = qF[1] == 0;
+                const df gamma = t[0];
+                qS[S_RR] = dD(t[2]);
+                if (t[2] < S.stop2) qF[0] = 1;
+                if (!(t[2].h == t[2].h) || !(gamma.h == gamma.h)) { qF[0] = 1; qF[2] = 1; }
+                S.stop = qF[0] || qF[1] >= maxIter;
+                if (S.stop) return;
+                const df alpha = divDF2(gamma, first ? t[1] : t[1] - divDF2(gamma * gamma, S.step));
+                S.beta = first ? 0.0 : dD(divDF2(gamma, S.gamma));
+                S.alpha = dD(alpha);
+                S.gamma = gamma;
+                S.step = gamma * alpha;
+                qF[1] += 1;
+            }))
+            return;
+        if (*(volatile int*)&S.stop) break;
+        if (R.any) {
+            const double alpha = vd(&S.alpha), beta = vd(&S.beta);
+            p = z + beta * p;
+            ap = q + beta * ap;
+            x += alpha * p;
+            r -= alpha * ap;
+            z = r * di;
+            if (own) B.z[R.i] = z;
         }
-        it++;
+        if (!qBarrier(B, c)) return;
     }
     if (own) B.x[R.i] = x;
     if (!qBarrier(B, c)) return;
@@ -1994,11 +2013,6 @@ __device__ __forceinline__ void clSum(const double (&v)[NV], ClShared& S, unsign
             for (int o = 16; o > 0; o >>= 1) a[q] += shflXorDF(a[q], o);
         if (lane == 0) fin(a);
     }
-}
-// a / b to the last bits of the pair: the quotient of divDF corrected by its remainder
-__device__ __forceinline__ df divDF2(df a, df b) {
-    const df q = divDF(a, b);
-    return q + divDF(a - b * q, b);
 }
 __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffers B, double tol, int maxIter, int cap) {
     __shared__ QLocal qL;
