@@ -27,6 +27,9 @@ struct mpsgpu_s {
     int* scanScratch = nullptr;
     int* outFlags = nullptr;
     int* outCounter = nullptr;
+    int* nearNext = nullptr;      // the near-wall counter not in use (zero)
+    double* velNext = nullptr;    // the maximum-speed slot not in use (zero)
+    bool fuseBC = false;          // inside a step: the PND sweep writes the boundary condition
     int* perm = nullptr;          // storage renumbering: permutation and gather scratch
     void* permScratch = nullptr;
     int renumberEvery = 20;       // bucket rebuilds between storage renumberings (0: never)
@@ -115,7 +118,7 @@ static int opLaunches(int op, const MpsParams& P, bool x) {
     switch (op) {
         case MPS_OP_UPDATE_BUCKETS: return 5;   // key, 2 scan, scatter, rank (small grids: 1 scan)
         case MPS_OP_VISCOSITY: return x ? 3 : 1;   // (DF32: velocity copy) + sweep (+ unlisted particles)
-        case MPS_OP_OUT_OF_DOMAIN: return 2;
+        case MPS_OP_OUT_OF_DOMAIN: return 1;
         case MPS_OP_COLLISION: return P.collisionType == 1 ? 2 : (x ? 3 : 2);
         case MPS_OP_WALL_DISTANCE: case MPS_OP_WALL_NPCD: return P.wallType == 1 ? 1 : 0;
         case MPS_OP_WALL_PRESS_GRADIENT: case MPS_OP_WALL_VISCOSITY: return P.wallType == 1 ? (x ? 2 : 1) : 0;
@@ -180,8 +183,8 @@ static void ensureList(mpsgpu_t h) {
     if (h->listValid) return;
     if (h->prof.on) h->prof.begin(PROF_NEIGHBOR_LIST, h->s);
     if (h->skinValid) {
-        launchNeighborFilter(h->d, h->s, !df32(h));
-        countLaunch(5);   // FP32 copies (2), skin check, filter, scan of the particles it left
+        launchNeighborFilter(h->d, h->s, !df32(h), false);
+        countLaunch(3);   // FP32 copies and skin check, filter, scan of the particles it left
     } else {
         launchNeighborList(h->d, h->s, !df32(h));
         countLaunch(3);   // FP32 copies (2), list build
@@ -203,12 +206,16 @@ static void ensureCache(mpsgpu_t h) {
     countLaunch(1);
     h->cacheValid = true;
 }
+static void sideMasks(mpsgpu_t h) {
+    std::swap(h->d.nearCount, h->nearNext);
+    launchSideMasks(h->d, h->nearNext, h->s);
+}
 // Entry masks depend on the list and on the mirror positions of the wall pass.
 static void ensureMasks(mpsgpu_t h) {
     ensureList(h);
     if (h->masksValid) return;
     if (h->prof.on) h->prof.begin(PROF_NEIGHBOR_LIST, h->s);
-    launchSideMasks(h->d, h->s);
+    sideMasks(h);
     if (h->prof.on) h->prof.end(h->s);
     countLaunch(1);
     h->masksValid = true;
@@ -278,9 +285,7 @@ static int calcPress(mpsgpu_t h) {
         countLaunch(ownSolve ? 6 : 9);
         if (e) return e;
         if (ownSolve) { h->B.cdir = h->mlp.cdir; h->B.cq = h->mlp.re; }
-    } else if (h->warm == MPSGPU_WARM_PREVIOUS) {
-        cudaMemcpyAsync(h->B.x, h->d.pressPPE, sizeof(double) * h->N0, cudaMemcpyDeviceToDevice, h->s);
-    }
+    }   // the previous solution: written by the assembly
     int iters = 0, refine = 0;
     double rr = 0, rr0 = 0;
     int maxIt = h->maxIter > 0 ? h->maxIter : 2 * h->N0;
@@ -445,7 +450,7 @@ static int runOpBody(mpsgpu_t h, int op) {
             // the correction matrix of the step (read after the pressure solve, positions and
             // masks unchanged in between) is formed in the same pass
             bool corr = P.gradientCorrection && P.pndType != 2;
-            if (x) launchPndNeighNpcdDF(d, s, corr); else launchPndNeighNpcd(d, s, corr);
+            if (x) launchPndNeighNpcdDF(d, s, corr, h->fuseBC); else launchPndNeighNpcd(d, s, corr, h->fuseBC);
             h->corrFresh = corr;
             break;
         }
@@ -470,15 +475,15 @@ static int runOpBody(mpsgpu_t h, int op) {
             break;
         }
         case MPS_OP_WALL_VISCOSITY: ensureMasks(h); if (x) launchWallViscosityDF(d, s); else launchWallViscosity(d, s); break;
-        case MPS_OP_CORRECT: launchCorrect(d, s); invalidate(); break;
+        case MPS_OP_CORRECT: launchCorrect(d, h->velNext, s); std::swap(d.velMax, h->velNext); invalidate(); break;
         case MPS_OP_SHIFTING:
             if (x && h->skinShift && (P.shiftingType == 1 || P.shiftingType == 2)) {
                 // the list of the post-corrector positions filtered from the skin list (a
                 // particle that moved out of its skin or scan window, or any particle after a
                 // removal, scans the buckets), its masks, then list sweeps
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(PROF_NEIGHBOR_LIST, s, false); }
-                launchNeighborFilter(d, s, false);
-                launchSideMasks(d, s);
+                launchNeighborFilter(d, s, false, true);
+                sideMasks(h);
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(MPS_OP_SHIFTING, s, false); }
                 launchShiftingListDF(d, s);
                 invalidate();
@@ -488,8 +493,8 @@ static int runOpBody(mpsgpu_t h, int op) {
             } else if (!x && h->skinShift && (P.shiftingType == 1 || P.shiftingType == 2)) {
                 // FP64: the same list, with its weights (type 2), and the operators' sweeps over it
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(PROF_NEIGHBOR_LIST, s, false); }
-                launchNeighborFilter(d, s, P.shiftingType == 2);
-                launchSideMasks(d, s);
+                launchNeighborFilter(d, s, P.shiftingType == 2, true);
+                sideMasks(h);
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(MPS_OP_SHIFTING, s, false); }
                 launchShifting(d, s, true);
                 invalidate();
@@ -514,9 +519,16 @@ static int stepImpl(mpsgpu_t h) {
 #define RUN(op) do { if ((e = runOpImpl(h, op))) return e; } while (0)
     RUN(MPS_OP_UPDATE_BUCKETS);
     RUN(MPS_OP_VISCOSITY);
-    RUN(MPS_OP_ADD_GRAVITY);
-    if (P.relaxPress < 1.0) RUN(MPS_OP_PREDICT_PRESS_GRADIENT);
-    RUN(MPS_OP_PREDICT);
+    if (P.relaxPress < 1.0 || h->prof.on) {
+        RUN(MPS_OP_ADD_GRAVITY);
+        if (P.relaxPress < 1.0) RUN(MPS_OP_PREDICT_PRESS_GRADIENT);
+        RUN(MPS_OP_PREDICT);
+    } else {   // both operators in one pass (the profiler keeps them apart)
+        launchGravityPredict(h->d, h->s);
+        countLaunch(1);
+        h->listValid = h->masksValid = h->cacheValid = h->corrFresh = h->pAuxFresh = false;
+        if ((e = launchStatus())) return e;
+    }
     RUN(MPS_OP_OUT_OF_DOMAIN);
     // The wall distance reads the positions left by the out-of-domain removal and writes only
     // the wall fields (squared distance, wall point, mirror, normal, near-wall flag, wall PND
@@ -554,10 +566,16 @@ static int stepImpl(mpsgpu_t h) {
     // PND and the velocity divergence of the PND + div u source; otherwise the second call
     // (src/main.cpp:375-377, same positions) overwrites it.
     if (P.gradientCorrection && (P.pndType == 2 || P.mpsType == 3)) RUN(MPS_OP_CORRECTION_MATRIX);
-    RUN(MPS_OP_PND_NEIGH_NPCD);
+    // the boundary condition follows from the PND sweep's own sums where nothing changes the PND
+    // in between and the free surface is not judged by arcs
+    h->fuseBC = P.pndType != 1 && P.pndType != 2 && P.freeSurfType != 2 && !h->prof.on;
+    e = runOpImpl(h, MPS_OP_PND_NEIGH_NPCD);
+    const bool bcDone = h->fuseBC;
+    h->fuseBC = false;
+    if (e) return e;
     if (P.pndType == 2) RUN(MPS_OP_PND_DIFFUSIVE);
     else if (P.pndType == 1) RUN(MPS_OP_PND_MEAN);
-    RUN(MPS_OP_UPDATE_BC);
+    if (!bcDone) RUN(MPS_OP_UPDATE_BC);
     RUN(MPS_OP_CALC_PRESS);
     if (P.wallType == 0) RUN(MPS_OP_EXTRAPOLATE_PRESS);
     if (P.gradientCorrection) RUN(MPS_OP_CORRECTION_MATRIX);
@@ -813,13 +831,15 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
     A(d.pAux, n);
     A(d.nearList, n);
     A(d.nearCount, 1);
+    A(h->nearNext, 1);
     A(d.velMax, 1);
+    A(h->velNext, 1);
     A(d.err, 1);
     A(d.counters, 4);
     A(h->scanScratch, scanScratchInts(std::max(d.nB + 1, n)));
     A(h->outFlags, n);
     cudaMemsetAsync(h->outFlags, 0, sizeof(int) * n, h->s);
-    A(h->outCounter, 1);
+    A(h->outCounter, 2);
     // FP32 prefilter band (see k_build_nbr): |d2f - d2| <= 3.47 delta re + 3 delta^2 + 3.1 u re^2
     {
         double X = 0;
@@ -967,7 +987,8 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
                                    std::max(std::max(B.pgridCg, std::max(ppePersistentGrid(5), ppePersistentGrid(6))),
                                             std::max(B.pgridMx, ppePersistentGrid(2)))));
         A(B.counter, 1);
-        A(B.flag, 8);
+        A(B.flag, PPE_CTL_FLAGS + 96);   // flags, then three 128-byte lines of barrier words
+        B.bar = reinterpret_cast<unsigned int*>(B.flag + PPE_CTL_FLAGS);
         A(B.dinv, n);
         A(B.mfMask, n);
         B.pgridMf = ppePersistentGrid(2);
@@ -982,7 +1003,6 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
         A(B.sclf, n);
         A(B.sgs, n);
         A(B.wideRow, n);
-        A(B.bar, 96);   // three 128-byte lines of barrier words
         // solver vectors in shared memory: a block's rows are its grid-stride rounds, at
         // most n / (G BS) + 1 of them per thread (the remainder is split over the blocks)
         B.pgridOwn = ppePersistentGrid(7);

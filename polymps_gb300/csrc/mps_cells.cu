@@ -103,8 +103,10 @@ __global__ void k_cell_scatter(Dev d) {
 // copies below (one thread sorting each bucket by insertion walked dependent loads: 28 and 52
 // us, and two more launches).  place: also the inverse list and the FP32 copies in
 // bucket order (the renumbering, which moves the slots, writes them after it).
+// The counters and cursors are cleared for the next build.
 __global__ void k_cell_rank(Dev d, bool place) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int k = p; k < 2 * (d.nB + 2); k += gridDim.x * blockDim.x) d.cellCount[k] = 0;
     if (p >= d.cellStart[d.nB + 1]) return;
     const int2 me = d.cellRec[p];
     const int c = d.cellOf[me.y];
@@ -273,7 +275,6 @@ __global__ void k_cell_pos(Dev d) {
 }
 
 void launchBuckets(const Dev& d, int* scanScratch, cudaStream_t s, int* perm, void* permScratch) {
-    cudaMemsetAsync(d.cellCount, 0, sizeof(int) * 2 * (d.nB + 2), s);   // counters and cursors
     k_cell_key<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
     scanExclusive(d.cellCount, d.cellStart, d.nB + 1, scanScratch, s);
     k_cell_scatter<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
@@ -294,6 +295,20 @@ __global__ void k_posf(Dev d) {
     d.posf[i] = hi;
     d.posLo[i] = lo;
 }
+
+// The copies and, for the list filter that follows, the skin list's validity (k_skin_check) and
+// the filter's cleared counters, in one pass.
+__global__ void k_posf_check(Dev d) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) { *d.rescan = 0; d.counters[0] = 0ull; }
+    if (i >= d.N0) return;
+    float4 hi, lo;
+    splitPos(d.pos[i], d.P, hi, lo);
+    d.posf[i] = hi;
+    d.posLo[i] = lo;
+    if (i < liveN(d) && !(dist2f(hi, d.posSkin[i]) <= d.skinMove2)) d.skinFlag[0] = 1;
+}
+void launchPosfCheck(const Dev& d, cudaStream_t s) { k_posf_check<<<gridFor(d.N0, 256), 256, 0, s>>>(d); }
 
 // ------------------------------------------------------------------ neighbour list
 // FP32 copy of the positions in bucket order, refreshed whenever positions change.
@@ -393,6 +408,7 @@ __global__ void __launch_bounds__(128) k_build_list(Dev d) {
             }
         }
     if (MODE == 0) {
+        if (i == 0 && l == 0) d.skinFlag[0] = 0;
         if (l == 0) {
             d.nbrCount[i] = cnt > d.K ? d.K + 1 : cnt;   // K + 1: the row overflowed, rescanned where read
             d.posSkin[i] = fi;
@@ -444,7 +460,6 @@ void launchNeighborList(const Dev& d, cudaStream_t s, bool weights) {
     else launchBuild<1>(d, s);
 }
 void launchSkinList(const Dev& d, cudaStream_t s) {
-    cudaMemsetAsync(d.skinFlag, 0, sizeof(int), s);
     launchBuild<0>(d, s);
 }
 
@@ -457,8 +472,9 @@ void launchSkinList(const Dev& d, cudaStream_t s) {
 // their mirror entries and are appended to nearList for the wall-only sweeps, which walk the
 // masks instead of testing the list again.
 template <int L>
-__global__ void __launch_bounds__(128) k_side_masks(Dev d) {
+__global__ void __launch_bounds__(128) k_side_masks(Dev d, int* oldCount) {
     const int i = laneRow<L>(), l = laneOf<L>();
+    if (i == 0 && l == 0) *oldCount = 0;   // the next call's counter
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
     const int c = d.nbrCount[i];
@@ -512,9 +528,8 @@ __global__ void __launch_bounds__(128) k_side_masks(Dev d) {
     }
 }
 
-void launchSideMasks(const Dev& d, cudaStream_t s) {
-    cudaMemsetAsync(d.nearCount, 0, sizeof(int), s);
-#define LAUNCH(L) k_side_masks<L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d)
+void launchSideMasks(const Dev& d, int* oldCount, cudaStream_t s) {
+#define LAUNCH(L) k_side_masks<L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d, oldCount)
     MPS_FOR_LANES(d.N0, LAUNCH);
 #undef LAUNCH
 }

@@ -284,6 +284,16 @@ __device__ __forceinline__ double ppeSource(const Dev& d, int i, double rho) {
     return -P.coeffPPESource * rho * (d.pndSmall[i] - P.pndSmallZero);
 }
 
+// Free-surface flag of a particle, types 0 and 1 (src/MpsBoundaryCondition.cpp:173-204)
+__device__ __forceinline__ int boundaryCondition(const Dev& d, int i, double ps, int numNeigh, double npcd2) {
+    const MpsParams& P = d.P;
+    if (d.type[i] == P.dummyWall) return P.other;
+    int bc = (ps < P.betaPnd) ? P.surface : P.inner;
+    if (P.freeSurfType == 0) bc = (ps < P.betaPnd && numNeigh < P.betaNeigh) ? P.surface : P.inner;
+    else if (P.freeSurfType == 1 && bc == P.surface && numNeigh > 4 && npcd2 < P.delta2) bc = P.inner;
+    return bc;
+}
+
 // ------------------------------------------------------------------ weights
 // MpsParticle::weight / delWeight, src/MpsParticle.cpp:57-108
 __device__ __forceinline__ double wfun(double dst, double re, int t) {

@@ -41,7 +41,8 @@ void launchNeighborList(const Dev& d, cudaStream_t s, bool weights);   // weight
 void launchSkinList(const Dev& d, cudaStream_t s);
 void launchPosf(const Dev& d, cudaStream_t s);       // FP32 copy, then its bucket-ordered copy
 void launchPosfCell(const Dev& d, cudaStream_t s);   // bucket-ordered copy only
-void launchSideMasks(const Dev& d, cudaStream_t s);   // also nearList and the mirror masks
+// also nearList and the mirror masks; nearCount is zero, oldCount (the one used before) is cleared
+void launchSideMasks(const Dev& d, int* oldCount, cudaStream_t s);
 void launchNearList(const Dev& d, cudaStream_t s);
 void launchFillCache(const Dev& d, cudaStream_t s);
 
@@ -50,16 +51,20 @@ void launchViscosity(const Dev& d, cudaStream_t s);
 // over the start-of-step skin list (built by launchSkinList): the FP64 viscosity sweep, and
 // the list of the current positions filtered from it (weights: the FP64 tier's cache)
 void launchViscosityList(const Dev& d, cudaStream_t s);
-void launchNeighborFilter(const Dev& d, cudaStream_t s, bool weights);
+// cells: refresh the bucket-ordered FP32 copies too
+void launchNeighborFilter(const Dev& d, cudaStream_t s, bool weights, bool cells);
+void launchPosfCheck(const Dev& d, cudaStream_t s);   // FP32 copies and skin check in one pass
 void launchAddGravity(const Dev& d, cudaStream_t s);
 void launchPredict(const Dev& d, cudaStream_t s);
+void launchGravityPredict(const Dev& d, cudaStream_t s);   // both operators in one pass
 void launchOutOfDomain(const Dev& d, int* flags, int* counter, cudaStream_t s);
 void launchCollision(const Dev& d, cudaStream_t s);
 void launchCollisionApply(const Dev& d, cudaStream_t s);
 void launchWallNpcd(const Dev& d, cudaStream_t s);
 void launchCorrectionMatrix(const Dev& d, cudaStream_t s);
 // withCorrection: also the correction matrix of the same positions and masks
-void launchPndNeighNpcd(const Dev& d, cudaStream_t s, bool withCorrection);
+// withBC: the boundary condition too (free-surface types 0 and 1)
+void launchPndNeighNpcd(const Dev& d, cudaStream_t s, bool withCorrection, bool withBC);
 void launchPndDiffusive(const Dev& d, cudaStream_t s);
 void launchPndMean(const Dev& d, cudaStream_t s);
 void launchInitPnd(const Dev& d, cudaStream_t s);
@@ -71,7 +76,8 @@ void launchPressGradient(const Dev& d, cudaStream_t s);
 void launchWallPressGradient(const Dev& d, cudaStream_t s, bool fresh);
 void launchPredictPressGradient(const Dev& d, bool skin, cudaStream_t s);   // relax_fact < 1, before PREDICT
 void launchWallViscosity(const Dev& d, cudaStream_t s);
-void launchCorrect(const Dev& d, cudaStream_t s);
+// next: the slot of the new maximum speed (zero); the one in use is cleared
+void launchCorrect(const Dev& d, double* next, cudaStream_t s);
 void launchShifting(const Dev& d, cudaStream_t s, bool list);   // list: filter and masks of these positions are built
 void launchDummyVelocity(const Dev& d, cudaStream_t s);
 
@@ -81,7 +87,7 @@ void launchCollisionDF(const Dev& d, cudaStream_t s);
 void launchWallNpcdDF(const Dev& d, cudaStream_t s);
 void launchCorrectionMatrixDF(const Dev& d, cudaStream_t s);
 void launchCorrDF(const Dev& d, cudaStream_t s);
-void launchPndNeighNpcdDF(const Dev& d, cudaStream_t s, bool withCorrection = false);
+void launchPndNeighNpcdDF(const Dev& d, cudaStream_t s, bool withCorrection, bool withBC);
 void launchPressGradientDF(const Dev& d, cudaStream_t s);
 void launchWallPressGradientDF(const Dev& d, cudaStream_t s, bool fresh);
 void launchWallViscosityDF(const Dev& d, cudaStream_t s);
@@ -97,7 +103,8 @@ void launchVelDivergence(const Dev& d, cudaStream_t s);
 // DF32 viscosity over the start-of-step list
 void launchViscosityListDF(const Dev& d, cudaStream_t s);
 // the skin list's validity flag for the current positions (moved more than half the skin)
-void launchSkinCheck(const Dev& d, cudaStream_t s);
+// clear: also the counters of the list filter that follows
+void launchSkinCheck(const Dev& d, cudaStream_t s, bool clear);
 void launchShiftVelApply(const Dev& d, cudaStream_t s);
 void launchApplyShift(const Dev& d, cudaStream_t s);
 void launchApplyShiftNear(const Dev& d, cudaStream_t s);   // the particles of nearList
@@ -119,6 +126,8 @@ struct PpeBuffers {
     float *valf, *diagf, *diagInvf, *rf, *zf, *pf, *Apf, *xf;  // mixed-precision copies
     double* partials;
     unsigned int* counter;
+    // flag and bar lie in one allocation, bar after PPE_CTL_FLAGS words
+#define PPE_CTL_FLAGS 32
     int* flag;       // [0] done, [1] iterations, [2] breakdown, [3] inner done, [4] refinements
     int nblocks;
     double* dinv;            // FP64 inverse diagonal (persistent plain solver)

@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(128) k_rescan(Dev d) {
 #pragma unroll
         for (int r = 0; r < 9; r++) {
             const int s0 = __shfl_sync(0xffffffffu, a, r), s1 = __shfl_sync(0xffffffffu, b, r);
-            if (s0 + lane < s1) f[r] = __ldg(&d.posfCell[s0 + lane]);
+            if (s0 + lane < s1) f[r] = __ldg(&d.posf[__ldg(d.cellSorted + s0 + lane)]);
         }
         int cnt = 0;
 #pragma unroll
@@ -168,9 +168,9 @@ __global__ void __launch_bounds__(128) k_rescan(Dev d) {
                 int j = i;
                 bool in = false;
                 if (s < s1) {
-                    const float d2f = dist2f(t == s0 ? f[r] : __ldg(&d.posfCell[s]), fi);
+                    j = __ldg(d.cellSorted + s);
+                    const float d2f = dist2f(t == s0 ? f[r] : __ldg(&d.posf[j]), fi);
                     if (!(d2f > d.bandHi)) {
-                        j = __ldg(d.cellSorted + s);
                         in = j != i && insideF(d, d2f, d.bandLo, d.bandHi, d.reMax2, i, j);
                     }
                 }
@@ -194,10 +194,13 @@ __global__ void __launch_bounds__(128) k_rescan(Dev d) {
         }
     }
 }
-void launchNeighborFilter(const Dev& d, cudaStream_t s, bool weights) {
-    cudaMemsetAsync(d.counters, 0, sizeof(unsigned long long), s);
-    launchPosf(d, s);
-    launchSkinCheck(d, s);   // also clears the rescan count
+void launchNeighborFilter(const Dev& d, cudaStream_t s, bool weights, bool cells) {
+    if (cells) {
+        launchPosf(d, s);
+        launchSkinCheck(d, s, true);
+    } else {
+        launchPosfCheck(d, s);
+    }
 #define LAUNCH(L)                                                                        \
     if (weights) k_filter_nbr<true, L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d);        \
     else k_filter_nbr<false, L><<<gridFor(d.N0 * L, 128), 128, 0, s>>>(d)
@@ -220,13 +223,12 @@ __global__ void k_add_gravity(Dev d) {
 }
 void launchAddGravity(const Dev& d, cudaStream_t s) { k_add_gravity<<<gridFor(d.N0, 256), 256, 0, s>>>(d); }
 
-// MpsParticleVelPos::predictionVelocityPosition, src/MpsParticleVelPos.cpp:20-50
-__global__ void k_predict(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= liveN(d)) return;
+// MpsParticleVelPos::predictionVelocityPosition, src/MpsParticleVelPos.cpp:20-50, with the
+// acceleration a of particle i
+__device__ __forceinline__ void predictParticle(const Dev& d, int i, dvec4 a) {
     const MpsParams& P = d.P;
     if (d.type[i] == P.fluid) {
-        dvec4 v = d.vel[i], a = d.acc[i], x = d.pos[i];
+        dvec4 v = d.vel[i], x = d.pos[i];
         v.x += a.x * P.timeStep; v.y += a.y * P.timeStep; v.z += a.z * P.timeStep;
         x.x += v.x * P.timeStep; x.y += v.y * P.timeStep; x.z += v.z * P.timeStep;
         d.vel[i] = v; d.pos[i] = x;
@@ -239,7 +241,21 @@ __global__ void k_predict(Dev d) {
     d.riw2[i] = big;
     if (P.wallType == 1) d.mirror[i] = make_dvec4(big, big, big, 0.0);
 }
+__global__ void k_predict(Dev d) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < liveN(d)) predictParticle(d, i, d.acc[i]);
+}
 void launchPredict(const Dev& d, cudaStream_t s) { k_predict<<<gridFor(d.N0, 256), 256, 0, s>>>(d); }
+// both operators in one pass (a step without the prediction's pressure gradient between them)
+__global__ void k_gravity_predict(Dev d) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= liveN(d)) return;
+    dvec4 a = d.acc[i];
+    a.x += d.P.gravity[0]; a.y += d.P.gravity[1]; a.z += d.P.gravity[2];
+    d.accStar[i] = a;
+    predictParticle(d, i, a);
+}
+void launchGravityPredict(const Dev& d, cudaStream_t s) { k_gravity_predict<<<gridFor(d.N0, 256), 256, 0, s>>>(d); }
 
 // ------------------------------------------------------------------ out of domain
 // MpsParticle::checkParticleOutDomain, src/MpsParticle.cpp:270-396.  A parallel pass flags
@@ -253,17 +269,6 @@ void launchPredict(const Dev& d, cudaStream_t s) { k_predict<<<gridFor(d.N0, 256
 __device__ __forceinline__ bool outside(const Dev& d, dvec4 p) {
     return p.x > d.oodHi[0] || p.x < d.oodLo[0] || p.y > d.oodHi[1] || p.y < d.oodLo[1] ||
            (d.dz3 && (p.z > d.oodHi[2] || p.z < d.oodLo[2]));
-}
-// flags (by reference index) are zero between calls: only flagged particles write theirs,
-// and the serial pass clears what it read
-__global__ void k_out_flag(Dev d, int* flags, int* counter) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    int n = liveN(d);
-    if (s >= n) return;
-    if (d.type[s] == d.P.fluid && outside(d, d.pos[s])) {
-        flags[d.orig[s]] = 1;
-        atomicAdd(counter, 1);
-    }
 }
 template <class T> __device__ __forceinline__ void mv(T* a, int i, int L) { a[i] = a[L]; }
 template <class T> __device__ __forceinline__ void sw(T* a, int i, int j) { T t = a[i]; a[i] = a[j]; a[j] = t; }
@@ -286,9 +291,7 @@ __device__ void swapSlots(const Dev& d, int a, int b) {
     if (pb >= 0) d.cellSorted[pb] = a;
     d.cellPos[a] = pb; d.cellPos[b] = pa;
 }
-__global__ void k_out_serial(Dev d, int* flags, int* counter) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (*counter == 0) return;
+__device__ void outSerial(const Dev& d, int* flags) {
     const MpsParams& P = d.P;
     const int oldN = *d.nLive;
     int newN = oldN;
@@ -317,14 +320,29 @@ __global__ void k_out_serial(Dev d, int* flags, int* counter) {
         removed++;
     }
     *d.nLive = newN;
-    *counter = removed;
     if (removed) d.skinFlag[0] = 1;   // indices moved: the start-of-step list is stale
     for (int r = 0; r < oldN; r++) flags[r] = 0;
 }
+// flags (by reference index) and the counters (flagged particles, blocks done) are zero between
+// calls: only flagged particles write theirs, the serial pass clears what it read, and the last
+// block to finish, which runs it, clears the counters.
+__global__ void k_out_of_domain(Dev d, int* flags, int* counter) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < liveN(d) && d.type[s] == d.P.fluid && outside(d, d.pos[s])) {
+        flags[d.orig[s]] = 1;
+        atomicAdd(counter, 1);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (atomicAdd(counter + 1, 1) != (int)gridDim.x - 1) return;
+    __threadfence();
+    if (*(volatile int*)counter) outSerial(d, flags);
+    counter[0] = 0;
+    counter[1] = 0;
+}
 void launchOutOfDomain(const Dev& d, int* flags, int* counter, cudaStream_t s) {
-    cudaMemsetAsync(counter, 0, sizeof(int), s);
-    k_out_flag<<<gridFor(d.N0, 256), 256, 0, s>>>(d, flags, counter);
-    k_out_serial<<<1, 32, 0, s>>>(d, flags, counter);
+    k_out_of_domain<<<gridFor(d.N0, 256), 256, 0, s>>>(d, flags, counter);
 }
 
 // ------------------------------------------------------------------ collision
@@ -627,8 +645,10 @@ void launchCorrectionMatrix(const Dev& d, cudaStream_t s) {
 // the entries, their gathers and their pair vectors), into the staging arrays that the
 // correction-matrix operator publishes.  FP64-pipe bound: 864k particles 951 us (463 for the
 // PND sums and 1,003 for the matrix when each had its own pass).
+// bc: the boundary condition follows from these sums alone and is written too (the step's next
+// operator).
 template <int INIT, bool CORR, int L>
-__global__ void __launch_bounds__(BLK) k_pnd_npcd(Dev d) {
+__global__ void __launch_bounds__(BLK) k_pnd_npcd(Dev d, bool bc) {
     const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
@@ -675,17 +695,18 @@ __global__ void __launch_bounds__(BLK) k_pnd_npcd(Dev d) {
     d.npcd2[i] = np.x * np.x + np.y * np.y + np.z * np.z;
     dvec4 nw = d.polyNormal[i];
     d.devDot[i] = (np.x * nw.x + np.y * nw.y + np.z * nw.z < 0.0) ? 1.0 : -1.0;
+    if (bc) d.bc[i] = boundaryCondition(d, i, pndSmall, nn, np.x * np.x + np.y * np.y + np.z * np.z);
     if (CORR) M.store(d, i, nn, d.c1n, d.c2n, d.c3n);
 }
 template <int INIT, bool CORR>
-static void launchPndNpcd(const Dev& d, cudaStream_t s) {
-#define LAUNCH(L) k_pnd_npcd<INIT, CORR, L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d)
+static void launchPndNpcd(const Dev& d, bool bc, cudaStream_t s) {
+#define LAUNCH(L) k_pnd_npcd<INIT, CORR, L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d, bc)
     MPS_FOR_LANES(d.N0, LAUNCH);
 #undef LAUNCH
 }
-void launchPndNeighNpcd(const Dev& d, cudaStream_t s, bool withCorrection) {
-    if (withCorrection) launchPndNpcd<0, true>(d, s);
-    else launchPndNpcd<0, false>(d, s);
+void launchPndNeighNpcd(const Dev& d, cudaStream_t s, bool withCorrection, bool withBC) {
+    if (withCorrection) launchPndNpcd<0, true>(d, withBC, s);
+    else launchPndNpcd<0, false>(d, withBC, s);
 }
 
 // ------------------------------------------------------------------ diffusive PND (pnd type 2)
@@ -899,7 +920,7 @@ void launchPndMean(const Dev& d, cudaStream_t s) {
 }
 // step-0 sequence, src/main.cpp:158-166
 void launchInitPnd(const Dev& d, cudaStream_t s) {
-    launchPndNpcd<1, false>(d, s);
+    launchPndNpcd<1, false>(d, false, s);
     launchPndMean(d, s);
     k_mean_neigh_fluid_pnd<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
 }
@@ -909,19 +930,7 @@ void launchInitPnd(const Dev& d, cudaStream_t s) {
 __global__ void k_update_bc(Dev d) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= liveN(d)) return;
-    const MpsParams& P = d.P;
-    int bc;
-    if (d.type[i] == P.dummyWall) bc = P.other;
-    else {
-        double ps = d.pndSmall[i];
-        bc = (ps < P.betaPnd) ? P.surface : P.inner;
-        if (P.freeSurfType == 0) {
-            bc = (ps < P.betaPnd && d.numNeigh[i] < P.betaNeigh) ? P.surface : P.inner;
-        } else if (P.freeSurfType == 1) {
-            if (bc == P.surface && d.numNeigh[i] > 4 && d.npcd2[i] < P.delta2) bc = P.inner;
-        }
-    }
-    d.bc[i] = bc;
+    d.bc[i] = boundaryCondition(d, i, d.pndSmall[i], d.numNeigh[i], d.npcd2[i]);
 }
 void launchUpdateBC(const Dev& d, cudaStream_t s) { k_update_bc<<<gridFor(d.N0, 256), 256, 0, s>>>(d); }
 
@@ -1435,8 +1444,9 @@ void launchWallViscosity(const Dev& d, cudaStream_t s) {
 // ------------------------------------------------------------------ corrector
 // MpsParticleVelPos::correctionVelocityPosition, src/MpsParticleVelPos.cpp:53-97, with the
 // maximum fluid speed reduced on the device (max is order independent).
-__global__ void k_correct(Dev d) {
+__global__ void k_correct(Dev d, double* next) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *d.velMax = 0.0;   // the last step's value, read before; the next call's slot
     const MpsParams& P = d.P;
     double v = 0.0;
     if (i < liveN(d) && d.type[i] == P.fluid) {
@@ -1459,12 +1469,11 @@ __global__ void k_correct(Dev d) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
         if (lane == 0 && v > 0.0)
-            atomicMax((unsigned long long*)d.velMax, (unsigned long long)__double_as_longlong(v));
+            atomicMax((unsigned long long*)next, (unsigned long long)__double_as_longlong(v));
     }
 }
-void launchCorrect(const Dev& d, cudaStream_t s) {
-    cudaMemsetAsync(d.velMax, 0, sizeof(double), s);
-    k_correct<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
+void launchCorrect(const Dev& d, double* next, cudaStream_t s) {
+    k_correct<<<gridFor(d.N0, 256), 256, 0, s>>>(d, next);
 }
 
 // ------------------------------------------------------------------ shifting
@@ -1681,7 +1690,7 @@ void launchShifting(const Dev& d, cudaStream_t s, bool list) {
         }
         k_apply_shift<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
         if (P.wallType == 1) {   // the wall sweep sees the shifted positions
-            if (list) launchSkinCheck(d, s);
+            if (list) launchSkinCheck(d, s, false);
             else launchNearList(d, s);
             k_wall_grad_conc<<<wallGrid(d.N0), WALL_BLK, 0, s>>>(d, list);
             launchApplyShiftNear(d, s);

@@ -330,7 +330,7 @@ void launchCorrectionMatrixDF(const Dev& d, cudaStream_t s) {
 // pair evaluation serves both; the PND sums take the entries also inside reL, in the same
 // ascending order as the plain sweep, so both results equal the separate kernels').
 template <bool CORR, int L>
-__global__ void __launch_bounds__(BLK, 9) k_pnd_npcd_df(Dev d) {
+__global__ void __launch_bounds__(BLK, 9) k_pnd_npcd_df(Dev d, bool bc) {
     const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
@@ -368,14 +368,15 @@ __global__ void __launch_bounds__(BLK, 9) k_pnd_npcd_df(Dev d) {
     d.npcd2[i] = np.x * np.x + np.y * np.y + np.z * np.z;
     dvec4 nw = d.polyNormal[i];
     d.devDot[i] = (np.x * nw.x + np.y * nw.y + np.z * nw.z < 0.0) ? 1.0 : -1.0;
+    if (bc) d.bc[i] = boundaryCondition(d, i, pndSmall, nn, np.x * np.x + np.y * np.y + np.z * np.z);
     // into the staging arrays: the correction-matrix operator publishes them (the reference
     // writes the matrix there, not in this sweep)
     if (CORR) corrFinish(d, i, nn, M.xx, M.xy, M.xz, M.yy, M.yz, M.zz, d.c1n, d.c2n, d.c3n, d.corrDFn);
 }
-void launchPndNeighNpcdDF(const Dev& d, cudaStream_t s, bool withCorrection) {
+void launchPndNeighNpcdDF(const Dev& d, cudaStream_t s, bool withCorrection, bool withBC) {
 #define LAUNCH(L)                                                                            \
-    if (withCorrection) k_pnd_npcd_df<true, L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d);    \
-    else k_pnd_npcd_df<false, L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d)
+    if (withCorrection) k_pnd_npcd_df<true, L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d, withBC);    \
+    else k_pnd_npcd_df<false, L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d, withBC)
     MPS_FOR_LANES(d.N0, LAUNCH);
 #undef LAUNCH
 }
@@ -388,6 +389,7 @@ __global__ void __launch_bounds__(128, 9) k_ppe_assemble_df(Dev d, PpeBuffers B)
     const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
+    if (l == 0) B.x[i] = d.pressPPE[i];   // the start of a solve from the previous solution
     int bci = d.bc[i];
     if (bci == P.other || bci == P.surface) {
         if (l == 0) {
@@ -807,7 +809,7 @@ __global__ void __launch_bounds__(WALL_BLK) k_wall_grad_conc_df(Dev d, bool skin
     }
 }
 static void launchWallGradConcDF(const Dev& d, cudaStream_t s, bool list) {
-    if (list) launchSkinCheck(d, s);
+    if (list) launchSkinCheck(d, s, false);
     else launchNearList(d, s);
     k_wall_grad_conc_df<<<wallGrid(d.N0), WALL_BLK, 0, s>>>(d, list);
     launchApplyShiftNear(d, s);
@@ -916,14 +918,14 @@ void launchViscosityListDF(const Dev& d, cudaStream_t s) {
 
 // The skin list covers the list of the current positions while every particle is within
 // half the skin of its start position (FP32 test with margin).
-__global__ void k_skin_check(Dev d) {
+__global__ void k_skin_check(Dev d, bool clear) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) *d.rescan = 0;   // read by the filter that follows
+    if (clear && i == 0) { *d.rescan = 0; d.counters[0] = 0ull; }
     if (i >= liveN(d)) return;
     float4 a = d.posf[i], b = d.posSkin[i];
     float ex = a.x - b.x, ey = a.y - b.y, ez = a.z - b.z;
     if (!(ex * ex + ey * ey + ez * ez <= d.skinMove2)) d.skinFlag[0] = 1;
 }
-void launchSkinCheck(const Dev& d, cudaStream_t s) {
-    k_skin_check<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
+void launchSkinCheck(const Dev& d, cudaStream_t s, bool clear) {
+    k_skin_check<<<gridFor(d.N0, 256), 256, 0, s>>>(d, clear);
 }

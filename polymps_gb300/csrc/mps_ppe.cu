@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(128) k_ppe_assemble(Dev d, PpeBuffers B) {
     const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
+    if (l == 0) B.x[i] = d.pressPPE[i];   // the start of a solve from the previous solution
     const int bci = d.bc[i];
     if (bci == P.other || bci == P.surface) {
         if (l == 0) { B.diag[i] = 1.0; B.rowLen[i] = 0; B.b[i] = 0.0; B.mfMask[i] = maskNone(); }
@@ -2526,12 +2527,16 @@ static int finishPersistent(const PpeBuffers& B, cudaStream_t s, int* iters, int
     return 0;
 }
 
+// flags and barrier words (adjacent: PPE_CTL_FLAGS words of flags first)
+static void qClear(const PpeBuffers& B, cudaStream_t s) {
+    cudaMemsetAsync(B.flag, 0, (PPE_CTL_FLAGS + QB_WORDS) * sizeof(int), s);
+}
+
 int ppeSolveBicgstab(const Dev& d, const PpeBuffers& B, double tol, int maxIter, cudaStream_t s, int* iters,
                      double* relres, double* relres0, Prof* prof) {
     if (B.pgridBi <= 0) return MPSGPU_ERR_UNSUPPORTED;
     bool pr = prof && prof->on;
-    cudaMemsetAsync(B.flag, 0, 8 * sizeof(int), s);
-    cudaMemsetAsync(B.bar, 0, QB_WORDS * sizeof(unsigned int), s);
+    qClear(B, s);
     Dev dd = d;
     PpeBuffers bb = B;
     double t = tol;
@@ -2565,8 +2570,7 @@ int ppeSolvePersistent(const Dev& d, const PpeBuffers& B, int mixed, double tol,
                                                           : (B.matfree == 2 ? B.pgridH16 : (B.matfree ? B.pgridMf : B.pgridMx))));
     if (grid <= 0) return MPSGPU_ERR_UNSUPPORTED;
     bool pr = prof && prof->on;
-    cudaMemsetAsync(B.flag, 0, 5 * sizeof(int), s);
-    cudaMemsetAsync(B.bar, 0, QB_WORDS * sizeof(unsigned int), s);
+    qClear(B, s);
     if (mixed && !B.prepared) {
         if (pr) prof->begin(PROF_PPE_OTHER, s);
         k_mixed_prepare<<<gridFor(d.N0, 256), 256, 0, s>>>(d, B);
