@@ -30,8 +30,7 @@ struct mpsgpu_s {
     int* nearNext = nullptr;      // the near-wall counter not in use (zero)
     double* velNext = nullptr;    // the maximum-speed slot not in use (zero)
     bool fuseBC = false;          // inside a step: the PND sweep writes the boundary condition
-    int* perm = nullptr;          // storage renumbering: permutation and gather scratch
-    void* permScratch = nullptr;
+    void* permScratch = nullptr;  // field transfers: reorder scratch, 32 bytes per particle
     int renumberEvery = 20;       // bucket rebuilds between storage renumberings (0: never)
     int renumberCountdown = 0;    // 0: renumber at the next bucket rebuild
     // solver controls
@@ -283,6 +282,7 @@ static int calcPress(mpsgpu_t h) {
         // x_e, its FP64 residual, features, scale, forward, A c; or x_e copy, residual,
         // features, scale, forward, correction, step dot products, step, apply
         countLaunch(ownSolve ? 6 : 9);
+        if (!e) e = mlpTcQueue(h->mlp, h->s);   // read after the solve
         if (e) return e;
         if (ownSolve) { h->B.cdir = h->mlp.cdir; h->B.cq = h->mlp.re; }
     }   // the previous solution: written by the assembly
@@ -314,7 +314,8 @@ static int calcPress(mpsgpu_t h) {
     } else {
         e = ppeSolvePlain(h->d, h->B, h->tol, maxIt, h->s, &iters, &rr, &rr0, &h->prof);
     }
-    if (h->warm == MPSGPU_WARM_MLP && !e && (e = mlpTcStatus(h->mlp, h->s)))
+    // (every solver above has waited for the stream)
+    if (h->warm == MPSGPU_WARM_MLP && !e && (e = mlpTcResult(h->mlp)))
         g_lastError = "learned warm start: a tensor-core completion wait ran out";
     // the final FP64 residual judges the fast solvers: a mixed solve that missed the
     // tolerance is redone by the plain FP64 CG from the previous unclamped solution
@@ -382,7 +383,7 @@ static int runOpBody(mpsgpu_t h, int op) {
     switch (op) {
         case MPS_OP_UPDATE_BUCKETS: {
             bool rn = h->renumberEvery > 0 && h->renumberCountdown <= 0;
-            launchBuckets(d, h->scanScratch, s, rn ? h->perm : nullptr, h->permScratch);
+            launchBuckets(d, h->scanScratch, s, rn);
             if (rn) { h->renumberCountdown = h->renumberEvery; countLaunch(renumberLaunches()); }
             h->renumberCountdown--;
             invalidate();
@@ -790,7 +791,6 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
     A(d.slotOf, n);
     A(d.cellRec, n);
     A(d.cellPos, n);
-    A(h->perm, n);
     {
         double* sc = nullptr;   // 32 bytes per particle: the widest per-particle element
         A(sc, (size_t)4 * n);
@@ -982,13 +982,19 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
         A(B.xalt, n);
         B.pgridCg = ppePersistentGrid(0);
         B.pgridMx = ppePersistentGrid(1);
-        A(B.scal, 32);
             A(B.partials, 8 * std::max(std::max(std::max(B.nblocks, ppePersistentGrid(4)), ppePersistentGrid(3)),
                                    std::max(std::max(B.pgridCg, std::max(ppePersistentGrid(5), ppePersistentGrid(6))),
                                             std::max(B.pgridMx, ppePersistentGrid(2)))));
         A(B.counter, 1);
-        A(B.flag, PPE_CTL_FLAGS + 96);   // flags, then three 128-byte lines of barrier words
+        A(B.scal, PPE_CTL_BYTES / 8);   // scalars, flags, then three 128-byte lines of barrier words
+        B.flag = reinterpret_cast<int*>(B.scal + 32);
         B.bar = reinterpret_cast<unsigned int*>(B.flag + PPE_CTL_FLAGS);
+        if (cudaMallocHost(&B.hostCtl, PPE_CTL_BYTES) != cudaSuccess) {
+            B.hostCtl = nullptr;
+            g_lastError = "page-locked solver report";
+            mpsgpu_destroy(h);
+            return MPSGPU_ERR_NOMEM;
+        }
         A(B.dinv, n);
         A(B.mfMask, n);
         B.pgridMf = ppePersistentGrid(2);
@@ -1064,6 +1070,7 @@ int mpsgpu_destroy(mpsgpu_t h) {
     for (void* p : h->allocs) cudaFree(p);
     if (h->vtuDev) cudaFree(h->vtuDev);
     if (h->vtuHost) cudaFreeHost(h->vtuHost);
+    if (h->B.hostCtl) cudaFreeHost(h->B.hostCtl);
     for (cudaEvent_t ev : {h->e0, h->e1, h->ea0, h->ea1, h->es0, h->es1, h->evFork, h->evJoin}) if (ev) cudaEventDestroy(ev);
     if (h->s2) cudaStreamDestroy(h->s2);
     if (h->s) cudaStreamDestroy(h->s);

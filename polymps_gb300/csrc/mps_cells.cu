@@ -226,64 +226,95 @@ int scanScratchInts(int n) { return 2 * ((n + SCAN_TILE - 1) / SCAN_TILE) + 4; }
 // per-particle array is gathered through a scratch buffer, the reference-index maps follow,
 // and the list becomes the identity.  Neighbours are then stored next to each other, which
 // is what the gathers of every sweep and the coalescing of the bucket-order scans want.
-__global__ void k_perm_build(Dev d, int* perm) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= d.N0) return;
-    perm[s] = (s < *d.nLive) ? d.cellSorted[s] : s;
+// Two launches: all arrays gathered into the weight cache of the list (K doubles per particle,
+// twice; the bucket rebuild has just made the list stale), then copied back, with the maps, the
+// inverse list and the bucket-ordered copies of the new order.  (A launch and a copy per array were
+// 84 launches of 2 to 30 us.)
+#define PERM_V 16
+#define PERM_S 18
+#define PERM_I 6
+struct PermArrays {
+    dvec4* v[PERM_V];
+    double* s[PERM_S];
+    int* i[PERM_I];
+};
+static PermArrays permArrays(const Dev& d) {
+    return {{d.pos, d.vel, d.acc, d.accStar, d.mirror, d.wallPos, d.polyNormal, d.normal, d.npcd, d.gradC, d.forceWall, d.c1,
+             d.c2, d.c3, d.dvel, d.shift},
+            {d.press, d.pressPPE, d.pressPPEprev, d.pressPPEprev2, d.pndi, d.pndki, d.pndski, d.pndSmall, d.npcd2, d.conc,
+             d.velDiv, d.diffTerm, d.pndWall, d.riw2, d.devDot, d.source, d.aux1, d.aux2},
+            {d.type, d.bc, d.numNeigh, d.nNeighWall, d.nearWall, d.cellOf}};
 }
-template <class T>
-__global__ void k_gather(const T* src, T* dst, const int* perm, int n) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n) dst[s] = src[perm[s]];
+// scratch: vectors in cw (32 PERM_V = 512 bytes a particle), the rest in cwd
+struct PermScratch {
+    dvec4* v;
+    float4 *hi, *lo;
+    double* s;
+    int* i;
+};
+__host__ __device__ __forceinline__ PermScratch permScratch(const Dev& d) {
+    const size_t n = d.N0;
+    PermScratch t;
+    t.v = reinterpret_cast<dvec4*>(d.cw);
+    t.hi = reinterpret_cast<float4*>(d.cwd);
+    t.lo = t.hi + n;
+    t.s = reinterpret_cast<double*>(t.lo + n);
+    t.i = reinterpret_cast<int*>(t.s + PERM_S * n);
+    return t;
 }
-__global__ void k_perm_maps(Dev d, const int* perm, const int* origOld) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_perm_gather(Dev d, PermArrays a) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= d.N0) return;
-    int r = origOld[perm[s]];
+    const size_t n = d.N0;
+    const int p = (s < *d.nLive) ? d.cellSorted[s] : s;
+    const PermScratch t = permScratch(d);
+#pragma unroll
+    for (int k = 0; k < PERM_V; k++) t.v[k * n + s] = a.v[k][p];
+    t.hi[s] = d.posf[p];
+    t.lo[s] = d.posLo[p];
+#pragma unroll
+    for (int k = 0; k < PERM_S; k++) t.s[k * n + s] = a.s[k][p];
+#pragma unroll
+    for (int k = 0; k < PERM_I; k++) t.i[k * n + s] = a.i[k][p];
+    t.i[PERM_I * n + s] = d.orig[p];
+}
+__global__ void k_perm_place(Dev d, PermArrays a) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= d.N0) return;
+    const size_t n = d.N0;
+    const PermScratch t = permScratch(d);
+#pragma unroll
+    for (int k = 0; k < PERM_V; k++) a.v[k][s] = t.v[k * n + s];
+    const float4 hi = t.hi[s], lo = t.lo[s];
+    d.posf[s] = hi;
+    d.posLo[s] = lo;
+#pragma unroll
+    for (int k = 0; k < PERM_S; k++) a.s[k][s] = t.s[k * n + s];
+#pragma unroll
+    for (int k = 0; k < PERM_I; k++) a.i[k][s] = t.i[k * n + s];
+    const int r = t.i[PERM_I * n + s];
     d.orig[s] = r;
     d.slotOf[r] = s;
     if (s < *d.nLive) d.cellSorted[s] = s;
+    d.cellPos[s] = s < d.cellStart[d.nB + 1] ? s : -1;
+    if (s < d.cellStart[d.nB]) {
+        d.posfCell[s] = hi;
+        d.posLoCell[s] = lo;
+    }
 }
-template <class T>
-static void permute(T* a, const int* perm, void* scratch, int n, cudaStream_t s) {
-    if (!a) return;
-    k_gather<T><<<gridFor(n, 256), 256, 0, s>>>(a, (T*)scratch, perm, n);
-    cudaMemcpyAsync(a, scratch, sizeof(T) * n, cudaMemcpyDeviceToDevice, s);
-}
-int renumberLaunches() { return 1 + (15 + 17 + 5 + 3) + 1 + 2; }
-static void launchRenumber(const Dev& d, int* perm, void* scratch, cudaStream_t s) {
-    const int n = d.N0;
-    k_perm_build<<<gridFor(n, 256), 256, 0, s>>>(d, perm);
-    for (dvec4* v : {d.pos, d.vel, d.acc, d.accStar, d.mirror, d.wallPos, d.polyNormal, d.normal, d.npcd, d.gradC,
-                     d.forceWall, d.c1, d.c2, d.c3, d.dvel, d.shift})
-        permute(v, perm, scratch, n, s);
-    for (double* v : {d.press, d.pressPPE, d.pressPPEprev, d.pressPPEprev2, d.pndi, d.pndki, d.pndski, d.pndSmall, d.npcd2, d.conc,
-                      d.velDiv, d.diffTerm, d.pndWall, d.riw2, d.devDot, d.source, d.aux1, d.aux2})
-        permute(v, perm, scratch, n, s);
-    for (int* v : {d.type, d.bc, d.numNeigh, d.nNeighWall, d.nearWall}) permute(v, perm, scratch, n, s);
-    permute(d.posf, perm, scratch, n, s);
-    permute(d.posLo, perm, scratch, n, s);
-    permute(d.cellOf, perm, scratch, n, s);
-    // maps: the old orig goes through the scratch (the gather reads it while writing orig)
-    cudaMemcpyAsync(scratch, d.orig, sizeof(int) * n, cudaMemcpyDeviceToDevice, s);
-    k_perm_maps<<<gridFor(n, 256), 256, 0, s>>>(d, perm, (const int*)scratch);
+int renumberLaunches() { return 2; }
+static void launchRenumber(const Dev& d, cudaStream_t s) {
+    const PermArrays a = permArrays(d);
+    k_perm_gather<<<gridFor(d.N0, 256), 256, 0, s>>>(d, a);
+    k_perm_place<<<gridFor(d.N0, 256), 256, 0, s>>>(d, a);
 }
 
-__global__ void k_cell_pos(Dev d) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < d.cellStart[d.nB + 1]) d.cellPos[d.cellSorted[p]] = p;
-}
-
-void launchBuckets(const Dev& d, int* scanScratch, cudaStream_t s, int* perm, void* permScratch) {
+void launchBuckets(const Dev& d, int* scanScratch, cudaStream_t s, bool renumber) {
     k_cell_key<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
     scanExclusive(d.cellCount, d.cellStart, d.nB + 1, scanScratch, s);
     k_cell_scatter<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
-    k_cell_rank<<<gridFor(d.N0, 256), 256, 0, s>>>(d, perm == nullptr);
-    if (!perm) return;
-    launchRenumber(d, perm, permScratch, s);
-    cudaMemsetAsync(d.cellPos, 0xff, sizeof(int) * d.N0, s);
-    k_cell_pos<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
-    k_posf_cell<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
+    k_cell_rank<<<gridFor(d.N0, 256), 256, 0, s>>>(d, !renumber);
+    if (renumber) launchRenumber(d, s);
 }
 
 // ------------------------------------------------------------------ FP32 copy

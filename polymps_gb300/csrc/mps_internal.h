@@ -33,8 +33,8 @@ struct Prof {
 // mps_cells.cu
 void scanExclusive(const int* in, int* out, int n, int* scratch, cudaStream_t s);
 int scanScratchInts(int n);
-// perm != NULL: renumber the storage into bucket order (perm: N0 ints, permScratch: 32 N0 bytes)
-void launchBuckets(const Dev& d, int* scanScratch, cudaStream_t s, int* perm, void* permScratch);
+// renumber: the storage into bucket order too (through the list's weight cache)
+void launchBuckets(const Dev& d, int* scanScratch, cudaStream_t s, bool renumber);
 int renumberLaunches();
 void launchNeighborList(const Dev& d, cudaStream_t s, bool weights);   // weights: the FP64 tier's cache
 // start-of-step list with a skin (both tiers)
@@ -126,10 +126,11 @@ struct PpeBuffers {
     float *valf, *diagf, *diagInvf, *rf, *zf, *pf, *Apf, *xf;  // mixed-precision copies
     double* partials;
     unsigned int* counter;
-    // flag and bar lie in one allocation, bar after PPE_CTL_FLAGS words
+    // scal (32), flag and bar lie in one allocation, bar after PPE_CTL_FLAGS words
 #define PPE_CTL_FLAGS 32
     int* flag;       // [0] done, [1] iterations, [2] breakdown, [3] inner done, [4] refinements
     int nblocks;
+    void* hostCtl;           // page-locked copy of scal, flag and bar (the report of a solve)
     double* dinv;            // FP64 inverse diagonal (persistent plain solver)
     unsigned int* bar;       // grid barrier of the persistent solvers: arrivals, generation, abort
     int pgridCg, pgridMx;    // co-resident grid sizes of the persistent solvers (0: unavailable)
@@ -174,6 +175,8 @@ void launchPpeAssembleDF(const Dev& d, const PpeBuffers& B, cudaStream_t s);
 void launchWarmExtrapolate(const Dev& d, const PpeBuffers& B, cudaStream_t s, bool quadratic = false);
 // FP32 copies of the assembled matrix (valf, diagf, diagInvf) for the FP64 assembly
 void launchMixedPrepare(const Dev& d, const PpeBuffers& B, cudaStream_t s);
+// hostCtl: page-locked copy of the solver's scalars, flags and barrier words (PPE_CTL_BYTES)
+#define PPE_CTL_BYTES (32 * 8 + (PPE_CTL_FLAGS + 96) * 4)
 // Returns iterations and final relative residual through host pointers (synchronises).
 int ppeSolvePlain(const Dev& d, const PpeBuffers& B, double tol, int maxIter, cudaStream_t s,
                   int* iters, double* relres, double* relres0, Prof* prof);

@@ -449,6 +449,7 @@ void mlpFree(MlpState& m) {
                     (void*)m.re, (void*)m.cdir, (void*)m.part, (void*)m.sig, (void*)m.xe32, (void*)m.tcErr, m.hostBuf})
         if (p) cudaFree(p);
     if (m.hostPinned) cudaFreeHost(m.hostPinned);
+    if (m.hostTc) cudaFreeHost(m.hostTc);
     m = MlpState();
 }
 
@@ -810,13 +811,17 @@ int mlpTrain(MlpState& m, int iters, int batch, float lr, unsigned long long see
 
 // ------------------------------------------------------------------ checks
 // Network outputs for host-supplied raw features (inference check against a CPU model).
-int mlpTcStatus(MlpState& m, cudaStream_t s) {
-    int h = 0;
-    if (cudaMemcpyAsync(&h, m.tcErr, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemsetAsync(m.tcErr, 0, sizeof(int), s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)
-        return MPSGPU_ERR_CUDA;
-    return h ? MPSGPU_ERR_CUDA : 0;
+int mlpTcQueue(MlpState& m, cudaStream_t s) {
+    if (!m.hostTc && cudaMallocHost((void**)&m.hostTc, sizeof(int)) != cudaSuccess) {
+        m.hostTc = nullptr;
+        return MPSGPU_ERR_NOMEM;
+    }
+    return cudaMemcpyAsync(m.hostTc, m.tcErr, sizeof(int), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+                   cudaMemsetAsync(m.tcErr, 0, sizeof(int), s) == cudaSuccess
+               ? 0
+               : MPSGPU_ERR_CUDA;
 }
+int mlpTcResult(const MlpState& m) { return m.hostTc && *m.hostTc ? MPSGPU_ERR_CUDA : 0; }
 
 // Device memory of a call with host arrays: kept between calls up to HOST_KEEP bytes (an
 // allocation and its release took 100 to 220 us, and the release waits for the device), freed
@@ -857,14 +862,13 @@ int mlpForwardHost(MlpState& m, const float* hfeat, int n, float* hout, cudaStre
         if (cudaMemcpyAsync((void*)df, hfeat, sizeof(float) * NF * n, cudaMemcpyHostToDevice, s) != cudaSuccess) e = MPSGPU_ERR_CUDA;
     }
     if (!e) e = mlpForwardTc(m, df, n, nullptr, nullptr, 0, nullptr, dout, s);
-    int tc = 0;
     if (!e) {
         for (size_t k = 0; k < (size_t)n; k += 1024) ((volatile float*)hout)[k] = 0.f;   // 4 KB pages
         if (cudaMemcpyAsync(hout, dout, sizeof(float) * n, cudaMemcpyDeviceToHost, s) != cudaSuccess) e = MPSGPU_ERR_CUDA;
     }
-    if (cudaMemcpyAsync(&tc, m.tcErr, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemsetAsync(m.tcErr, 0, sizeof(int), s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess || tc)
-        e = MPSGPU_ERR_CUDA;
+    const int q = mlpTcQueue(m, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess) e = MPSGPU_ERR_CUDA;
+    if (!e) e = q ? q : mlpTcResult(m);
     if (!kept) cudaFree(w);
     return e;
 }

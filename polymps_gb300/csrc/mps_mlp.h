@@ -39,6 +39,7 @@ struct MlpState {
     void* hostBuf = nullptr;       // device memory of the calls with host arrays
     size_t hostBytes = 0;
     float* hostPinned = nullptr;   // page-locked gradient and loss
+    int* hostTc = nullptr;         // page-locked copy of tcErr
     int* tcErr = nullptr;          // set by the tensor-core forward when a completion wait ran out
 };
 
@@ -48,9 +49,11 @@ int mlpInit(MlpState& m, int n0, cudaStream_t s);
 // others (sig: the system scale of the raw features, nullptr for normalised inputs as given).
 int mlpForwardTc(const MlpState& m, const float* feat, int n, const int* nLive, const int* bc, int inner,
                  const double* sig, float* out, cudaStream_t s);
-// 0, or MPSGPU_ERR_CUDA when a tensor-core forward since the last call reported a
-// completion wait that ran out (clears the word; synchronises the stream)
-int mlpTcStatus(MlpState& m, cudaStream_t s);
+// Queues the copy of the tensor-core forward's error word to the host and its clearing; once the
+// stream has been waited for, mlpTcResult is 0, or MPSGPU_ERR_CUDA when a forward before the
+// queueing reported a completion wait that ran out
+int mlpTcQueue(MlpState& m, cudaStream_t s);
+int mlpTcResult(const MlpState& m);
 void mlpFree(MlpState& m);
 int mlpSetWeights(MlpState& m, const float* params, const float* norm32, cudaStream_t s);
 int mlpGetWeights(MlpState& m, float* params, float* norm32, cudaStream_t s);

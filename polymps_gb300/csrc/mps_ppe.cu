@@ -2509,14 +2509,12 @@ int ppePersistentGrid(int kind) {
 
 static int finishPersistent(const PpeBuffers& B, cudaStream_t s, int* iters, int* refinements, double* relres,
                             double* relres0) {
-    int f[5];
-    unsigned int abortWord = 0;
-    double sc[S_COUNT];
-    if (cudaMemcpyAsync(f, B.flag, sizeof(f), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MPSGPU_ERR_CUDA;
-    if (cudaMemcpyAsync(&abortWord, B.bar + QB_ABT, sizeof(unsigned int), cudaMemcpyDeviceToHost, s) != cudaSuccess)
-        return MPSGPU_ERR_CUDA;
-    if (cudaMemcpyAsync(sc, B.scal, sizeof(sc), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MPSGPU_ERR_CUDA;
+    // one copy into page-locked memory (three into pageable variables waited for the stream three times)
+    if (cudaMemcpyAsync(B.hostCtl, B.scal, PPE_CTL_BYTES, cudaMemcpyDeviceToHost, s) != cudaSuccess) return MPSGPU_ERR_CUDA;
     if (cudaStreamSynchronize(s) != cudaSuccess) return MPSGPU_ERR_CUDA;
+    const double* sc = static_cast<const double*>(B.hostCtl);
+    const int* f = reinterpret_cast<const int*>(sc + 32);
+    const unsigned int abortWord = *reinterpret_cast<const unsigned int*>(f + PPE_CTL_FLAGS + QB_ABT);
     if (abortWord) return MPSGPU_ERR_CUDA;   // a grid-barrier wait ran out (reported by the caller)
     *iters = f[1];
     if (refinements) *refinements = f[4];
