@@ -131,7 +131,7 @@ static int opLaunches(int op, const MpsParams& P, bool x) {
         case MPS_OP_SHIFTING:   // FP32 copies (2) + scans + apply kernels (DF32: two scans per sweep + copies)
             if (x) return P.shiftingType == 1 ? 6 : (P.shiftingType == 2 ? (P.wallType == 1 ? 11 : 8) : 0);
             return P.shiftingType == 1 ? 4 : (P.shiftingType == 2 ? (P.wallType == 1 ? 8 : 5) : 0);
-        case MPS_OP_DUMMY_VELOCITY: return P.wallType == 0 ? 3 : 0;
+        case MPS_OP_DUMMY_VELOCITY: return P.wallType == 0 ? 2 : 0;
         case MPS_OP_UPDATE_BC: return P.freeSurfType == 2 ? (P.wallType == 1 ? 3 : 2) : 1;   // (normals) + flags
         default: return 1;
     }

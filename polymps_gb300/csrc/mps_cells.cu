@@ -353,6 +353,7 @@ __global__ void k_posf_cell(Dev d) {
 void launchPosfCell(const Dev& d, cudaStream_t s) {
     k_posf_cell<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
 }
+void launchPosfOnly(const Dev& d, cudaStream_t s) { k_posf<<<gridFor(d.N0, 256), 256, 0, s>>>(d); }
 void launchPosf(const Dev& d, cudaStream_t s) {
     k_posf<<<gridFor(d.N0, 256), 256, 0, s>>>(d);
     launchPosfCell(d, s);

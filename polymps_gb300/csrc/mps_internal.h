@@ -40,6 +40,7 @@ void launchNeighborList(const Dev& d, cudaStream_t s, bool weights);   // weight
 // start-of-step list with a skin (both tiers)
 void launchSkinList(const Dev& d, cudaStream_t s);
 void launchPosf(const Dev& d, cudaStream_t s);       // FP32 copy, then its bucket-ordered copy
+void launchPosfOnly(const Dev& d, cudaStream_t s);   // FP32 copy only
 void launchPosfCell(const Dev& d, cudaStream_t s);   // bucket-ordered copy only
 // also nearList and the mirror masks; nearCount is zero, oldCount (the one used before) is cleared
 void launchSideMasks(const Dev& d, int* oldCount, cudaStream_t s);

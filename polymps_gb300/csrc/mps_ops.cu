@@ -1702,23 +1702,47 @@ void launchShifting(const Dev& d, cudaStream_t s, bool list) {
 
 // ------------------------------------------------------------------ dummy velocity
 // MpsParticleVelPos::updateVelocityParticlesWallDummy, src/MpsParticleVelPos.cpp:100-158
-// (dummy particles read fluid velocities only, so the update is race free in place)
+// (dummy particles read fluid velocities only, so the update is race free in place).  L lanes per
+// particle test a bucket row's candidates by their FP32 copies and sum those inside.
+template <int L>
 __global__ void __launch_bounds__(BLK) k_dummy_vel(Dev d) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = laneRow<L>(), l = laneOf<L>();
     if (i >= liveN(d)) return;
     const MpsParams& P = d.P;
     if (d.type[i] != P.dummyWall) return;
-    dvec4 pi = d.pos[i];
+    const dvec4 pi = d.pos[i];
+    const float4 fi = d.posf[i];
     double ni = 0.0, ux = 0, uy = 0, uz = 0;
-    forCellsNear(d, pi, d.posf[i], d.bandHiL, [&](int j, dvec4 pj, PairG q) {
-        if (q.d2 < P.reL2 && j != i && d.type[j] == P.fluid) {
-            double wL, wd;
-            weightR(q.d2, P.reL, P.weightType, wL, wd);
-            dvec4 vj = d.vel[j];
-            ni += wL;
-            ux += vj.x * wL; uy += vj.y * wL; uz += vj.z * wL;
+    int ix, iy, iz;
+    bucketCoordsHi(d, pi, fi, ix, iy, iz);
+    const int minZ = (iz - 1) * d.dz3, maxZ = (iz + 1) * d.dz3;
+    for (int jz = minZ; jz <= maxZ; jz++)
+        for (int jy = iy - 1; jy <= iy + 1; jy++) {
+            const long long jb = (long long)jz * P.numBucketsXY + (long long)jy * P.numBucketsX + ix;
+            const long long lo = jb - 1 > 0 ? jb - 1 : 0, hi = jb + 1 < d.nB - 1 ? jb + 1 : d.nB - 1;
+            if (lo > hi) continue;
+            const int s1 = d.cellStart[hi + 1];
+            for (int s0 = d.cellStart[lo]; s0 < s1; s0 += 32) {
+                unsigned m = 0u;
+#pragma unroll 4
+                for (int t = l; t < 32; t += L) {
+                    if (s0 + t >= s1) break;
+                    const int j = __ldg(d.cellSorted + s0 + t);
+                    if (d.type[j] != P.fluid || j == i) continue;
+                    if (insideF(d, dist2f(__ldg(&d.posf[j]), fi), d.bandLoL, d.bandHiL, P.reL2, i, j)) m |= 1u << t;
+                }
+                for (; m; m &= m - 1u) {
+                    const int j = __ldg(d.cellSorted + s0 + __ffs((int)m) - 1);
+                    double wL, wd;
+                    weightR(pairSum(d.pos[j], pi).d2, P.reL, P.weightType, wL, wd);
+                    const dvec4 vj = d.vel[j];
+                    ni += wL;
+                    ux += vj.x * wL; uy += vj.y * wL; uz += vj.z * wL;
+                }
+            }
         }
-    });
+    ni = laneSum<L>(ni); ux = laneSum<L>(ux); uy = laneSum<L>(uy); uz = laneSum<L>(uz);
+    if (l != 0) return;
     dvec4 v;
     if (ni > P.epsilonZero) v = make_dvec4(2.0 * 0.0 - ux / ni, 2.0 * 0.0 - uy / ni, 2.0 * 0.0 - uz / ni, 0.0);
     else v = make_dvec4(2.0 * 0.0 - ux, 2.0 * 0.0 - uy, 2.0 * 0.0 - uz, 0.0);
@@ -1726,6 +1750,8 @@ __global__ void __launch_bounds__(BLK) k_dummy_vel(Dev d) {
 }
 void launchDummyVelocity(const Dev& d, cudaStream_t s) {
     if (d.P.wallType != 0) return;
-    launchPosf(d, s);
-    k_dummy_vel<<<gridFor(d.N0, BLK), BLK, 0, s>>>(d);
+    launchPosfOnly(d, s);
+#define LAUNCH(L) k_dummy_vel<L><<<gridFor(d.N0 * L, BLK), BLK, 0, s>>>(d)
+    MPS_FOR_LANES(d.N0, LAUNCH);
+#undef LAUNCH
 }

@@ -600,13 +600,15 @@ __device__ __forceinline__ df shflXorDF(df a, int o) {
     return {__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)};
 }
 template <int NV, class Fin>
-__device__ __forceinline__ bool qSumF2(df (&a)[NV], const PpeBuffers& B, QCtl& c, Fin fin) {
+__device__ __forceinline__ bool qSumF2(df (&a)[NV], const PpeBuffers& B, QCtl& c, Fin fin, bool any = true) {
     __shared__ float2 sm[NV * 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
     for (int q = 0; q < NV; q++) {
+        if (any) {   // a warp without rows keeps its zeros: its trees would take the others' issue slots
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a[q] += shflXorDF(a[q], o);
+            for (int o = 16; o > 0; o >>= 1) a[q] += shflXorDF(a[q], o);
+        }
         if (lane == 0) sm[q * 32 + w] = make_float2(a[q].h, a[q].l);
     }
     __syncthreads();
@@ -649,11 +651,11 @@ __device__ __forceinline__ bool qSumD(double (&v)[NV], const PpeBuffers& B, QCtl
 }
 
 template <int NV, class Fin>
-__device__ __forceinline__ bool qSumDF2(double (&v)[NV], const PpeBuffers& B, QCtl& c, Fin fin) {   // fin takes the pairs
+__device__ __forceinline__ bool qSumDF2(double (&v)[NV], const PpeBuffers& B, QCtl& c, Fin fin, bool any) {   // fin takes the pairs
     df a[NV];
 #pragma unroll
     for (int q = 0; q < NV; q++) a[q] = dfD(v[q]);
-    return qSumF2<NV>(a, B, c, fin);
+    return qSumF2<NV>(a, B, c, fin, any);
 }
 
 // Rows inside the persistent kernels: matrix arrays are read-only for the launch, the
@@ -1917,7 +1919,7 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
                 S.gamma = gamma;
                 S.step = gamma * alpha;
                 qF[1] += 1;
-            }))
+            }, R.any))
             return;
         if (*(volatile int*)&S.stop) break;
         if (R.any) {
@@ -2278,7 +2280,7 @@ __global__ void __launch_bounds__(RBS, 1) k_mx_res(Dev d, PpeBuffers B, double t
                     pf = inner ? zf + beta * pf : zf;
                     if (own) a[0] = prod2(pf, apf);
                 }
-                if (!qSumF2<1>(a, B, c, [&](const df* t) { qL.scalf[SF_ALPHA] = divDF(rz, t[0]).h; })) return;
+                if (!qSumF2<1>(a, B, c, [&](const df* t) { qL.scalf[SF_ALPHA] = divDF(rz, t[0]).h; }, R.any)) return;
             }
             {   // x_f += alpha p, r -= alpha Ap, z = M^-1 r; r.z, r.r
                 const float alpha = vf(qL.scalf + SF_ALPHA);
@@ -2296,7 +2298,7 @@ __global__ void __launch_bounds__(RBS, 1) k_mx_res(Dev d, PpeBuffers B, double t
                         qL.scalf[SF_BETA] = divDF(t[0], rz).h;
                         rz = t[0];
                         if (t[1] < stop2 || !(t[1].h == t[1].h)) qF[3] = 1;
-                    }))
+                    }, R.any))
                     return;
             }
             inner++;
