@@ -1962,10 +1962,16 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
 //   p = z + beta p,  Ap = q + beta Ap,  x += alpha p,  r -= alpha Ap,  z = M^-1 r,
 // the same vectors as k_cg_res, whose p.Ap it forms by linearity too.  The first warp has no
 // rows: it sums the warps' partials and forms the step scalars.
+// Bound by latency: at 2,916 rows an iteration takes ~7,000 cycles, the product 1,650, delta and
+// its barrier 1,700, collecting the partials 660.  Only delta waits for the product, so z is
+// published as soon as it is known, and the x update and the trees of the next iteration's r.z
+// and r.r run between arrival and wait of its barrier (three sums after the product, all in one
+// exchange: 603 us for the three solves named at CLUSTER_MAX_ROWS, now 510).
 #define CLB 16                 // blocks of the cluster
 #define CL_ROWS 256            // rows of a block at most
 struct ClShared {
-    float2 part[3][CL_ROWS / 32][CLB];   // the warps' partials (every warp writes its own into all blocks)
+    // the warps' partials (every warp writes its own into all blocks), two sets in turn
+    float2 part[2][3][CL_ROWS / 32][CLB];
     double alpha, beta;
     int stop;
 };
@@ -1982,40 +1988,39 @@ __device__ __forceinline__ void clStore(const void* p, unsigned rank, double v) 
 __device__ __forceinline__ void clStore(const void* p, unsigned rank, float2 v) {
     asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(clAddr(p, rank)), "f"(v.x), "f"(v.y) : "memory");
 }
-// The cluster's sums of NV values per thread, in float-float from the warp level on (as qSumD):
-// every warp writes its partials into all blocks, the first warp of each sums them in the same
-// order; fin(totals) on its thread 0; the caller synchronises the block before reading what it
-// wrote.  One cluster barrier.
-template <int NV, class Fin>
-__device__ __forceinline__ void clSum(const double (&v)[NV], ClShared& S, unsigned rank, Fin&& fin) {
-    const int lane = threadIdx.x & 31, w = (int)threadIdx.x >> 5, nw = ((int)blockDim.x >> 5) - 1;
-    if (w > 0) {
+// Sums over the cluster, in float-float from the warp level on (as qSumD): every warp with rows
+// writes its partial of value q into set `set` of all blocks (clPush); after a cluster barrier the
+// first warp of each block sums the partials in the same order (clTotal, in every lane).
+// NV values, v[k] as value q0 + k dq; their trees run side by side.
+template <int NV>
+__device__ __forceinline__ void clPush(const double (&v)[NV], int q0, int dq, int set, ClShared& S, unsigned rank) {
+    const int lane = threadIdx.x & 31, w = ((int)threadIdx.x >> 5) - 1;
+    df a[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) a[k] = dfD(v[k]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < NV; k++) a[k] += shflXorDF(a[k], o);
+    if (lane < CLB)
+#pragma unroll
+        for (int k = 0; k < NV; k++) clStore(&S.part[set][q0 + k * dq][w][rank], lane, make_float2(a[k].h, a[k].l));
+}
+template <int NV>
+__device__ __forceinline__ void clTotal(int set, const ClShared& S, df (&a)[NV]) {
+    const int lane = threadIdx.x & 31, nw = ((int)blockDim.x >> 5) - 1;
+#pragma unroll
+    for (int q = 0; q < NV; q++) a[q] = dfF(0.f);
+    for (int m = lane; m < nw * CLB; m += 32)
 #pragma unroll
         for (int q = 0; q < NV; q++) {
-            df a = dfD(v[q]);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a += shflXorDF(a, o);
-            if (lane < CLB) clStore(&S.part[q][w - 1][rank], lane, make_float2(a.h, a.l));
+            const float2 x = S.part[set][q][0][m];
+            a[q] += df{x.x, x.y};
         }
-    }
-    clArrive();
-    clWait();
-    if (w == 0) {
-        df a[NV];
 #pragma unroll
-        for (int q = 0; q < NV; q++) a[q] = dfF(0.f);
-        for (int m = lane; m < nw * CLB; m += 32)
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-            for (int q = 0; q < NV; q++) {
-                const float2 x = S.part[q][0][m];
-                a[q] += df{x.x, x.y};
-            }
-#pragma unroll
-        for (int q = 0; q < NV; q++)
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a[q] += shflXorDF(a[q], o);
-        if (lane == 0) fin(a);
-    }
+        for (int q = 0; q < NV; q++) a[q] += shflXorDF(a[q], o);
 }
 __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffers B, double tol, int maxIter, int cap) {
     __shared__ QLocal qL;
@@ -2036,8 +2041,9 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
     const int len = own ? __ldg(B.rowLen + i) : 0;
     const int most = __reduce_max_sync(0xffffffffu, len);
     const size_t base = own ? ellBase(B, i) : 0;
-    const int held = min((most + 3) & ~3, cap);   // cap is a multiple of 4
+    const int held = min(most, cap);
     if (t >= 0)
+#pragma unroll 8
         for (int e = 0; e < held; e++) {
             const bool ok = e < len;
             sc[e * T + t] = ok ? (unsigned short)ldStream(B.col + base + (size_t)e * B.ellStride) : (unsigned short)0;
@@ -2048,17 +2054,19 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
     double dg = 1.0, x = 0.0, r = 0.0, z = 0.0, p = 0.0, ap = 0.0, di = 1.0, bi = 0.0;
     // (A v)_i of the vector in zc, v its own element
     auto product = [&](double v) {
-        double a[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int e = 0; e < held; e += 4) {
+        double a[2] = {dg * v, 0.0};   // (an FP64 operation of a warp takes 64 issue slots: few sums, no padding)
+        int e = 0;
+        for (; e + 4 <= held; e += 4) {
             double g[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) g[u] = zc[sc[(e + u) * T + t]];
 #pragma unroll
-            for (int u = 0; u < 4; u++) a[u] += sv[(e + u) * T + t] * g[u];
+            for (int u = 0; u < 4; u++) a[u & 1] += sv[(e + u) * T + t] * g[u];
         }
-        for (int e = held; e < len; e++)
+        for (; e < held; e++) a[e & 1] += sv[e * T + t] * zc[sc[e * T + t]];
+        for (; e < len; e++)
             a[0] += ldStream(B.val + base + (size_t)e * B.ellStride) * zc[ldStream(B.col + base + (size_t)e * B.ellStride)];
-        return dg * v + ((a[0] + a[1]) + (a[2] + a[3]));
+        return a[0] + a[1];
     };
     auto publish = [&](double v) {   // into every block's copy
 #pragma unroll
@@ -2072,68 +2080,87 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
         r = bi - product(x);
         z = r * di;
     }
-    {
+    if (t >= 0) {
         const double v[2] = {bi * bi, r * r};
-        clSum<2>(v, S, rank, [&](const df* sums) {   // its barrier also ends every block's reads of x
-            const double s[2] = {dD(sums[0]), dD(sums[1])};
-            qS[S_BB] = s[0];
-            double thr = tol * tol * s[0];
+        clPush<2>(v, 0, 1, 0, S, rank);
+    }
+    clArrive();
+    clWait();   // also ends every block's reads of x
+    if (threadIdx.x < 32) {
+        df a[2];
+        clTotal<2>(0, S, a);
+        if (threadIdx.x == 0) {
+            const double bb = dD(a[0]), rr = dD(a[1]);
+            qS[S_BB] = bb;
+            double thr = tol * tol * bb;
             if (thr < 2.2250738585072014e-308) thr = 2.2250738585072014e-308;
             qS[S_THR] = thr;
-            qS[S_RR] = s[1];
-            qS[S_SCALE] = sqrt(s[1] / (s[0] > 0 ? s[0] : 1.0));
-            qF[0] = (s[0] == 0.0 || s[1] < thr) ? 1 : 0;
+            qS[S_RR] = rr;
+            qS[S_SCALE] = sqrt(rr / (bb > 0 ? bb : 1.0));
+            qF[0] = (bb == 0.0 || rr < thr) ? 1 : 0;
             qF[1] = 0;
-            if (!(s[1] == s[1])) { qF[0] = 1; qF[2] = 1; }
+            if (!(rr == rr)) { qF[0] = 1; qF[2] = 1; }
             S.stop = qF[0] || maxIter <= 0;
-        });
+        }
     }
     if (own) publish(z);
+    if (t >= 0) {   // gamma and rho of the first iteration
+        const double v[2] = {r * z, r * r};
+        clPush<2>(v, 0, 2, 1, S, rank);
+    }
     clArrive();
     clWait();
-    // thread 0: gamma_old and gamma_old alpha_old, and the squared residual norm that ends it
-    df gammaOld = dfF(0.f), step = dfF(0.f);
-    const df stop2 = dfD(qS[S_THR]);
+    // thread 0: 1 / gamma_old and 1 / alpha_old, and the squared residual norm that ends it
+    df invGamma = dfF(0.f), invAlpha = dfF(0.f);
+    const df stop2 = dfD(qS[S_THR]), one = dfF(1.f);
     __syncthreads();
-    while (!S.stop) {
-        double v[3] = {0.0, 0.0, 0.0}, q = 0.0;
-        if (own) {
-            q = product(z);
-            v[0] = r * z; v[1] = z * q; v[2] = r * r;
+    for (int set = 1; !S.stop; set ^= 1) {
+        double q = 0.0;
+        if (own) q = product(z);
+        if (t >= 0) {
+            const double v[1] = {own ? z * q : 0.0};
+            clPush<1>(v, 1, 0, set, S, rank);
         }
-        df gamma = dfF(0.f), rr = dfF(0.f), alpha2 = dfF(0.f);
-        clSum<3>(v, S, rank, [&](const df* s) {
-            // (step scalars in float-float like the sums they come from: a chain of FP64
-            // divisions on one thread would be a third of the iteration)
-            const bool first = qF[1] == 0;
-            gamma = s[0];
-            rr = s[2];
-            if (rr < stop2) qF[0] = 1;
-            if (!(rr.h == rr.h) || !(gamma.h == gamma.h)) { qF[0] = 1; qF[2] = 1; }
-            S.stop = qF[0] || qF[1] >= maxIter;
-            S.beta = first ? 0.0 : dD(divDF2(gamma, gammaOld));
-            alpha2 = divDF2(gamma, first ? s[1] : s[1] - divDF2(gamma * gamma, step));
-            S.alpha = dD(alpha2);
-        });
+        clArrive();
+        clWait();
+        df gamma = dfF(0.f), alpha2 = dfF(0.f);
+        if (threadIdx.x < 32) {
+            df a[3];
+            clTotal<3>(set, S, a);
+            if (threadIdx.x == 0) {
+                // step scalars in float-float like the sums they come from (a chain of FP64
+                // divisions on one thread would be a third of the iteration)
+                gamma = a[0];
+                const df beta = gamma * invGamma;                      // 0 in the first iteration
+                alpha2 = divDF2(gamma, a[1] - gamma * (beta * invAlpha));
+                S.alpha = dD(alpha2);
+                S.beta = dD(beta);
+                if (a[2] < stop2) qF[0] = 1;
+                if (!(a[2].h == a[2].h) || !(gamma.h == gamma.h)) { qF[0] = 1; qF[2] = 1; }
+                S.stop = qF[0] || qF[1] >= maxIter;
+                if (S.stop) qS[S_RR] = dD(a[2]);
+            }
+        }
         __syncthreads();
-        if (S.stop) {
-            if (threadIdx.x == 0) qS[S_RR] = dD(rr);
-            break;
-        }
+        if (S.stop) break;
         if (own) {
             const double alpha = S.alpha, beta = S.beta;
             p = z + beta * p;
             ap = q + beta * ap;
-            x += alpha * p;
             r -= alpha * ap;
             z = r * di;
             publish(z);
         }
-        clArrive();
+        clArrive();   // z is published; the rest runs while the other blocks arrive
+        if (own) x += S.alpha * p;
+        if (t >= 0) {
+            const double v[2] = {own ? r * z : 0.0, own ? r * r : 0.0};
+            clPush<2>(v, 0, 2, set ^ 1, S, rank);
+        }
         if (threadIdx.x == 0) {
             qF[1] += 1;
-            gammaOld = gamma;
-            step = gamma * alpha2;
+            invGamma = divDF2(one, gamma);
+            invAlpha = divDF2(one, alpha2);
         }
         clWait();
     }
@@ -2143,13 +2170,17 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
     if (own) { B.x[i] = x; publish(x); }
     clArrive();
     clWait();
-    {
-        double v[1] = {0.0};
-        if (own) {
-            const double e = bi - product(x);
-            v[0] = e * e;
-        }
-        clSum<1>(v, S, rank, [&](const df* s) { qS[S_RR] = dD(s[0]); });
+    if (t >= 0) {
+        const double e = own ? bi - product(x) : 0.0;
+        const double v[1] = {e * e};
+        clPush<1>(v, 0, 0, 0, S, rank);
+    }
+    clArrive();
+    clWait();
+    if (threadIdx.x < 32) {
+        df a[1];
+        clTotal<1>(0, S, a);
+        if (threadIdx.x == 0) qS[S_RR] = dD(a[0]);
     }
     __syncthreads();
     if (rank == 0) qStore(B, qL);
@@ -2550,9 +2581,10 @@ int ppeSolveBicgstab(const Dev& d, const PpeBuffers& B, double tol, int maxIter,
     return finishPersistent(B, s, iters, nullptr, relres, relres0);
 }
 
-// Rows up to which one cluster takes the plain FP64 solve (its 16 SMs' FP64 pipes bound it above):
-// whole solves by k_cg_cluster and k_cg_res at 1,000 rows 146 / 195 us, 2,048 rows 170 / 216,
-// 4,000 rows 219 / 235, 5,324 rows 256 / 235, 6,912 rows 310 / 253.
+// Rows up to which one cluster takes the plain FP64 solve, all that its blocks hold at one row per
+// thread.  Three first solves of a run (64 to 76 iterations, set-up included) by k_cg_cluster and
+// k_cg_res at 1,000 rows 417 / 563 us, 2,048 rows 488 / 618, 2,916 rows 510 / 639, 4,000 rows
+// 594 / 665: the gain shrinks as the 16 SMs' FP64 pipes fill.
 #define CLUSTER_MAX_ROWS 4096
 // Lanes per row of the resident solvers: 4, 2 or 1, as many as give every row of `rows` its
 // lanes in one round of the grid; 0: too many rows.
