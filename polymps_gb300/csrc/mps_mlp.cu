@@ -849,7 +849,10 @@ static void* hostWork(MlpState& m, size_t bytes, bool* kept) {
 // cost 310 us of faults).  Whole call: 864,000 rows 749 -> 429 us, 100,000 256 -> 112, 1,000 57 ->
 // 46.
 int mlpForwardHost(MlpState& m, const float* hfeat, int n, float* hout, cudaStream_t s) {
-    const bool direct = m.hostTables && (reinterpret_cast<uintptr_t>(hfeat) & 15u) == 0;   // float4 loads
+    // float4 loads; an output in the features' own memory is written only after they are read
+    const uintptr_t f0 = reinterpret_cast<uintptr_t>(hfeat), o0 = reinterpret_cast<uintptr_t>(hout);
+    const bool apart = o0 + sizeof(float) * (size_t)n <= f0 || f0 + sizeof(float) * NF * (size_t)n <= o0;
+    const bool direct = m.hostTables && (f0 & 15u) == 0 && apart;
     const size_t outBytes = (sizeof(float) * (size_t)n + 255) / 256 * 256;
     bool kept = false;
     char* const w = (char*)hostWork(m, outBytes + (direct ? 0 : sizeof(float) * NF * (size_t)n), &kept);
@@ -863,7 +866,8 @@ int mlpForwardHost(MlpState& m, const float* hfeat, int n, float* hout, cudaStre
     }
     if (!e) e = mlpForwardTc(m, df, n, nullptr, nullptr, 0, nullptr, dout, s);
     if (!e) {
-        for (size_t k = 0; k < (size_t)n; k += 1024) ((volatile float*)hout)[k] = 0.f;   // 4 KB pages
+        if (apart)
+            for (size_t k = 0; k < (size_t)n; k += 1024) ((volatile float*)hout)[k] = 0.f;   // 4 KB pages
         if (cudaMemcpyAsync(hout, dout, sizeof(float) * n, cudaMemcpyDeviceToHost, s) != cudaSuccess) e = MPSGPU_ERR_CUDA;
     }
     const int q = mlpTcQueue(m, s);

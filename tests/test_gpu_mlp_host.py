@@ -41,6 +41,18 @@ def test_forward_alignment(net, n):
     assert np.any(a) and np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("n", [1, 129, 70001])
+def test_forward_output_in_the_features_memory(net, n):
+    from polymps_gb300 import mps
+    f = np.random.default_rng(n).standard_normal((n, abi.MLP_NFEAT)).astype(np.float32)
+    want = net.mlp_forward(f)
+    for first in (0, (abi.MLP_NFEAT - 1) * n):   # the outputs over the first or the last n features
+        buf = _place(f, 0).reshape(-1)
+        out = buf[first:first + n]
+        assert mps.lib().mpsgpu_mlp_forward(net.h, abi.fptr(buf), n, abi.fptr(out)) == 0
+        assert np.array_equal(out, want)
+
+
 @pytest.mark.parametrize("n", [64, 128, 65536 + 64, 2097152, 64])
 def test_gradient_alignment(net, n):
     rng = np.random.default_rng(n)
