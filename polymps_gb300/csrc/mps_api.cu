@@ -840,7 +840,7 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
     A(h->outFlags, n);
     cudaMemsetAsync(h->outFlags, 0, sizeof(int) * n, h->s);
     A(h->outCounter, 2);
-    // FP32 prefilter band (see k_build_nbr): |d2f - d2| <= 3.47 delta re + 3 delta^2 + 3.1 u re^2
+    // FP32 prefilter band (see k_build_list): |d2f - d2| <= 3.47 delta re + 3 delta^2 + 3.1 u re^2
     {
         double X = 0;
         for (int k = 0; k < 3; k++) X = std::max(X, p->domainMax[k] - p->domainMin[k]);

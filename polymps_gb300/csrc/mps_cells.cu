@@ -470,7 +470,7 @@ static void launchBuild(const Dev& d, cudaStream_t s) {
 }
 
 // Per-entry weights of the current list for the FP64 sweeps, when the list was built by
-// the DF32 tier (which stores none); the same expressions as k_build_nbr.
+// the DF32 tier (which stores none); the same expressions as k_build_list.
 __global__ void __launch_bounds__(128) k_fill_cache(Dev d) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= liveN(d)) return;

@@ -70,12 +70,6 @@ __device__ __forceinline__ int maskRank(const Mask& m, int k) {
     return __popcll(m.lo) + __popcll(m.hi & ((1ull << (k - 64)) - 1ull));
 }
 
-// a < b for non-negative doubles by their bits (NaN compares false, as in FP64): two integer
-// comparisons instead of one on the FP64 pipe.
-__device__ __forceinline__ bool lessPos(double a, double b) {
-    return (unsigned long long)__double_as_longlong(a) < (unsigned long long)__double_as_longlong(b);
-}
-
 // The reference's FP64 decisions, out of line: inlined, the compiler predicates them into every
 // entry and their FP64 operations then run for all of them.
 static __device__ __noinline__ bool pairInsideExact(const dvec4* pos, int j, int i, double R2) {

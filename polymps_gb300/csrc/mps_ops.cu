@@ -1,11 +1,13 @@
 // mps_ops.cu — the per-particle operators of the PolyMPS step on sm_103a.
 //
-// One thread per particle i.  Sweeps at the post-prediction positions walk the ELL
-// neighbour row of i (built once per position epoch through the stale bucket list, in
-// the reference's scan order); the start-of-step viscosity and the post-correction
-// shifting/dummy sweeps, which see their positions once, walk the 27 buckets directly.
-// Every sweep applies the reference's own radius and mirror-side tests to each entry,
-// with the distance comparisons evaluated in exact FP64 (see mps_common.cuh).
+// One thread per particle i, or 8 or 4 lanes in small systems (lanesFor).  Sweeps at the
+// post-prediction positions walk the ELL neighbour row of i (built once per position epoch
+// through the stale bucket list, in the reference's scan order); the start-of-step viscosity and
+// the post-correction shifting read the start-of-step skin list and its filter.  With the skin
+// list off both walk the 27 buckets, as the dummy velocities do.
+// Membership (the reference's own radius and mirror-side tests) is decided first, from the FP32
+// copies outside their rounding band and in exact FP64 inside it (see mps_common.cuh); the FP64
+// sums then run over the members only.
 #include "mps_df.cuh"
 #include "mps_internal.h"
 #include "mps_lanes.cuh"
@@ -91,7 +93,7 @@ void launchViscosityList(const Dev& d, cudaStream_t s) {
 }
 
 // List of the current positions filtered from the skin list: the set, order and (WEIGHTS, the
-// FP64 tier) per-entry weights of k_build_nbr, L lanes per particle.  Membership (d^2 <
+// FP64 tier) per-entry weights of k_build_list, L lanes per particle.  Membership (d^2 <
 // reMax^2) comes from the FP32 copies outside their rounding band; the weights, the FP64
 // part, are then formed over the members only (864k particles: 1,699 -> 992 us; decided and
 // formed entry by entry, every warp issued the weights for 56 entries instead of 33).  A
@@ -131,7 +133,7 @@ __global__ void __launch_bounds__(128) k_filter_nbr(Dev d) {
     }
     warpCount(d.counters, l == 0 ? (unsigned)cnt : 0u);
 }
-// The particles the filter left: the 27-bucket scan of k_build_nbr by one warp each.  The
+// The particles the filter left: the 27-bucket scan of k_build_list by one warp each.  The
 // window's nine rows of three buckets are ranges of the bucket order of about 28 particles, one
 // pass of the warp's lanes each; their bounds are loaded by nine lanes at once.
 template <bool WEIGHTS>
