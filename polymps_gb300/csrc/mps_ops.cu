@@ -327,12 +327,18 @@ __device__ void outSerial(const Dev& d, int* flags) {
 }
 // flags (by reference index) and the counters (flagged particles, blocks done) are zero between
 // calls: only flagged particles write theirs, the serial pass clears what it read, and the last
-// block to finish, which runs it, clears the counters.
+// block to finish, which runs it, clears the counters.  Every block adds one to the same word, so
+// the grid is at most four blocks per SM that stride over the particles: at 864k particles, cold
+// cache, 15.7 us against 20.1 with a block per 256 particles and 17.5 with eight blocks per SM.
+#define OUT_BLOCKS 608
 __global__ void k_out_of_domain(Dev d, int* flags, int* counter) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < liveN(d) && d.type[s] == d.P.fluid && outside(d, d.pos[s])) {
-        flags[d.orig[s]] = 1;
-        atomicAdd(counter, 1);
+    const int n = liveN(d);
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        const dvec4 p = d.pos[s];
+        if (d.type[s] == d.P.fluid && outside(d, p)) {
+            flags[d.orig[s]] = 1;
+            atomicAdd(counter, 1);
+        }
     }
     __threadfence();
     __syncthreads();
@@ -344,7 +350,8 @@ __global__ void k_out_of_domain(Dev d, int* flags, int* counter) {
     counter[1] = 0;
 }
 void launchOutOfDomain(const Dev& d, int* flags, int* counter, cudaStream_t s) {
-    k_out_of_domain<<<gridFor(d.N0, 256), 256, 0, s>>>(d, flags, counter);
+    const int grid = gridFor(d.N0, 256) < OUT_BLOCKS ? gridFor(d.N0, 256) : OUT_BLOCKS;
+    k_out_of_domain<<<grid, 256, 0, s>>>(d, flags, counter);
 }
 
 // ------------------------------------------------------------------ collision
