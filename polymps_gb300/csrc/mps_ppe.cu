@@ -2032,6 +2032,9 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
     unsigned short* const sc = reinterpret_cast<unsigned short*>(sv + (size_t)cap * T);
     unsigned rank;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    // a block's shared memory may be written by another only once it has started: arrive here, wait
+    // before the first push, the matrix loads between the two
+    clArrive();
     qInit(qL);
     double* const qS = qL.scal;
     int* const qF = qL.flag;
@@ -2080,6 +2083,7 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
         r = bi - product(x);
         z = r * di;
     }
+    clWait();   // every block of the cluster has started
     if (t >= 0) {
         const double v[2] = {bi * bi, r * r};
         clPush<2>(v, 0, 1, 0, S, rank);
