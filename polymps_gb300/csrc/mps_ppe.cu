@@ -629,13 +629,13 @@ __device__ __forceinline__ bool qSumF2(df (&a)[NV], const PpeBuffers& B, QCtl& c
 }
 // ... with the totals in FP64 for fin
 template <int NV, class Fin>
-__device__ __forceinline__ bool qSumDF(df (&a)[NV], const PpeBuffers& B, QCtl& c, Fin fin) {
+__device__ __forceinline__ bool qSumDF(df (&a)[NV], const PpeBuffers& B, QCtl& c, Fin fin, bool any = true) {
     return qSumF2<NV>(a, B, c, [&](const df* t) {
         double tot[NV];
 #pragma unroll
         for (int q = 0; q < NV; q++) tot[q] = dD(t[q]);
         fin(tot);
-    });
+    }, any);
 }
 
 // FP64 per-thread partials summed as float-float from the warp level on (each partial split
@@ -643,19 +643,11 @@ __device__ __forceinline__ bool qSumDF(df (&a)[NV], const PpeBuffers& B, QCtl& c
 // trees off the FP64 pipe.  A tree of float-float sums over the 864k row terms rounds less
 // than the sequential FP64 dot product of the reference's solver.
 template <int NV, class Fin>
-__device__ __forceinline__ bool qSumD(double (&v)[NV], const PpeBuffers& B, QCtl& c, Fin fin) {
+__device__ __forceinline__ bool qSumD(double (&v)[NV], const PpeBuffers& B, QCtl& c, Fin fin, bool any = true) {
     df a[NV];
 #pragma unroll
     for (int q = 0; q < NV; q++) a[q] = dfD(v[q]);
-    return qSumDF<NV>(a, B, c, fin);
-}
-
-template <int NV, class Fin>
-__device__ __forceinline__ bool qSumDF2(double (&v)[NV], const PpeBuffers& B, QCtl& c, Fin fin, bool any) {   // fin takes the pairs
-    df a[NV];
-#pragma unroll
-    for (int q = 0; q < NV; q++) a[q] = dfD(v[q]);
-    return qSumF2<NV>(a, B, c, fin, any);
+    return qSumDF<NV>(a, B, c, fin, any);
 }
 
 // Rows inside the persistent kernels: matrix arrays are read-only for the launch, the
@@ -1849,14 +1841,15 @@ __device__ __forceinline__ df divDF2(df a, df b) {
 // Plain FP64 Jacobi-PCG with one reduction an iteration (Chronopoulos and Gear, s-step methods,
 // J. Comput. Appl. Math. 25, 1989): with q = A z,
 //   gamma = r.z, delta = z.q, rho = r.r;  beta = gamma / gamma_old,
-//   alpha = gamma / (delta - gamma^2 / (gamma_old alpha_old)),
+//   p.Ap = delta - beta^2 (p.Ap)_old,  alpha = gamma / p.Ap,
 //   p = z + beta p,  Ap = q + beta Ap,  x += alpha p,  r -= alpha Ap,  z = M^-1 r,
 // the vectors of k_cg_own, whose p.Ap comes by linearity too; the second synchronisation of an
-// iteration is then a barrier (z is complete) without a sum.  The step scalars are formed in
-// float-float like the sums they come from.  Stopping rule and reports of k_cg_own.
+// iteration is then a barrier (z is complete) without a sum.  The sums and the FP64 step scalars
+// are k_cg_own's: no product of two sums is formed, so the right-hand side may have any scale
+// that the sums themselves hold.  Stopping rule and reports of k_cg_own.
 __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double tol, int maxIter, int L, int cap) {
     __shared__ QLocal qL;
-    __shared__ struct { double alpha, beta; df gamma, step, stop2; int stop; } S;   // step: gamma alpha
+    __shared__ struct { double alpha, beta, gamma, pap; int stop; } S;
     qInit(qL);
     double* const qS = qL.scal;
     int* const qF = qL.flag;
@@ -1894,7 +1887,6 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
                 qF[0] = (t[1] == 0.0 || t[0] < thr) ? 1 : 0;
                 qF[1] = 0;
                 if (!(t[0] == t[0])) { qF[0] = 1; qF[2] = 1; }
-                S.stop2 = dfD(thr);
                 S.stop = qF[0] || maxIter <= 0;
             }))
             return;
@@ -1905,19 +1897,17 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
             q = dg * z + resDot<double>(R, sc, sv, cap, B.col, B.val, B.z);
             if (own) { v[0] = r * z; v[1] = z * q; v[2] = r * r; }
         }
-        if (!qSumDF2<3>(v, B, c, [&](const df* t) {
-                const bool first = qF[1] == 0;
-                const df gamma = t[0];
-                qS[S_RR] = dD(t[2]);
-                if (t[2] < S.stop2) qF[0] = 1;
-                if (!(t[2].h == t[2].h) || !(gamma.h == gamma.h)) { qF[0] = 1; qF[2] = 1; }
+        if (!qSumD<3>(v, B, c, [&](const double* t) {
+                const double gamma = t[0];
+                qS[S_RR] = t[2];
+                if (t[2] < qS[S_THR]) qF[0] = 1;
+                if (!(t[2] == t[2]) || !(gamma == gamma)) { qF[0] = 1; qF[2] = 1; }
                 S.stop = qF[0] || qF[1] >= maxIter;
                 if (S.stop) return;
-                const df alpha = divDF2(gamma, first ? t[1] : t[1] - divDF2(gamma * gamma, S.step));
-                S.beta = first ? 0.0 : dD(divDF2(gamma, S.gamma));
-                S.alpha = dD(alpha);
+                S.beta = qF[1] ? gamma / S.gamma : 0.0;
+                S.pap = qF[1] ? t[1] - S.beta * (S.beta * S.pap) : t[1];
+                S.alpha = gamma / S.pap;
                 S.gamma = gamma;
-                S.step = gamma * alpha;
                 qF[1] += 1;
             }, R.any))
             return;
