@@ -45,6 +45,7 @@ struct mpsgpu_s {
     int nHost = -1;            // live count known on the host (-1: read it from the device)
     int *nbrAlt = nullptr, *cntAlt = nullptr;   // second list arrays (the skin list keeps its own)
     int skinOn = 1;            // viscosity and the post-prediction list from the start-of-step skin list
+    bool copiesFresh = false;  // the FP32 copies, by particle and by bucket, are those of the positions
     bool corrFresh = false;    // the correction matrix of the current positions and masks is written
     bool pAuxFresh = false;    // the last operator was the pressure gradient: its p_min still stand
     bool opSkipped = false;    // the last operator had nothing left to launch
@@ -178,6 +179,15 @@ static int launchStatus() {
 }
 
 static bool df32(mpsgpu_t h) { return h->d.prec == MPSGPU_PRECISION_DF32; }
+// The FP32 copies for an operator that reads them without a list of its own (the start-of-step
+// sweeps).  In a step the bucket build has just made them; an operator on its own may follow one
+// that moved the particles, and the list filter refreshes the copy by particle only.
+static void ensureCopies(mpsgpu_t h) {
+    if (h->copiesFresh) return;
+    launchPosf(h->d, h->s);
+    countLaunch(2);
+    h->copiesFresh = true;
+}
 static void ensureList(mpsgpu_t h) {
     if (h->listValid) return;
     if (h->prof.on) h->prof.begin(PROF_NEIGHBOR_LIST, h->s);
@@ -186,6 +196,7 @@ static void ensureList(mpsgpu_t h) {
         countLaunch(3);   // FP32 copies and skin check, filter, scan of the particles it left
     } else {
         launchNeighborList(h->d, h->s, !df32(h));
+        h->copiesFresh = true;
         countLaunch(3);   // FP32 copies (2), list build
     }
     h->skinValid = false;
@@ -387,15 +398,17 @@ static int runOpBody(mpsgpu_t h, int op) {
             if (rn) { h->renumberCountdown = h->renumberEvery; countLaunch(renumberLaunches()); }
             h->renumberCountdown--;
             invalidate();
+            h->copiesFresh = true;
             h->skinValid = false;
             h->skinShift = false;
             break;
         }
         case MPS_OP_VISCOSITY:
+            ensureCopies(h);
             if (h->skinOn) {
                 // start-of-step list with a skin: the viscosity sweep reads it, and the list of
-                // the predicted positions is filtered from it (ensureList); in the FP64 tier
-                // the sweep and the filter keep the bucket scan's FP64 arithmetic and order
+                // the predicted positions is filtered from it (ensureList); its members are those
+                // of the bucket scan, in its order
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(PROF_NEIGHBOR_LIST, s, false); }
                 launchSkinList(d, s);
                 if (h->prof.on) { h->prof.end(s); h->prof.begin(MPS_OP_VISCOSITY, s, false); }
@@ -417,12 +430,17 @@ static int runOpBody(mpsgpu_t h, int op) {
         case MPS_OP_PREDICT_PRESS_GRADIENT:
             // FP64 in both tiers, over the start-of-step skin list while it is built for
             // these positions (else the bucket scan)
-            if (P.relaxPress < 1.0) launchPredictPressGradient(d, h->skinValid, s);
+            if (P.relaxPress < 1.0) {
+                const bool skin = h->skinValid && h->copiesFresh;
+                ensureCopies(h);
+                launchPredictPressGradient(d, skin, s);
+            }
             break;
-        case MPS_OP_PREDICT: launchPredict(d, s); invalidate(); break;
+        case MPS_OP_PREDICT: launchPredict(d, s); invalidate(); h->copiesFresh = false; break;
         case MPS_OP_OUT_OF_DOMAIN:
             launchOutOfDomain(d, h->outFlags, h->outCounter, s);
             invalidate();
+            h->copiesFresh = false;
             h->nHost = -1;   // removals change the live count on the device
             break;
         case MPS_OP_COLLISION:
@@ -430,6 +448,7 @@ static int runOpBody(mpsgpu_t h, int op) {
             if (P.collisionType == 1) {   // DPC moves the positions: every list is stale
                 launchCollisionDPC(d, s);
                 invalidate();
+                h->copiesFresh = false;
             } else if (x) launchCollisionDF(d, s);
             else launchCollision(d, s);
             break;
@@ -476,7 +495,7 @@ static int runOpBody(mpsgpu_t h, int op) {
             break;
         }
         case MPS_OP_WALL_VISCOSITY: ensureMasks(h); if (x) launchWallViscosityDF(d, s); else launchWallViscosity(d, s); break;
-        case MPS_OP_CORRECT: launchCorrect(d, h->velNext, s); std::swap(d.velMax, h->velNext); invalidate(); break;
+        case MPS_OP_CORRECT: launchCorrect(d, h->velNext, s); std::swap(d.velMax, h->velNext); invalidate(); h->copiesFresh = false; break;
         case MPS_OP_SHIFTING:
             if (x && h->skinShift && (P.shiftingType == 1 || P.shiftingType == 2)) {
                 // the list of the post-corrector positions filtered from the skin list (a
@@ -506,6 +525,7 @@ static int runOpBody(mpsgpu_t h, int op) {
                 if (x) launchShiftingDF(d, s); else launchShifting(d, s, false);
                 if (P.shiftingType == 2) invalidate();
             }
+            h->copiesFresh = false;
             break;
         case MPS_OP_DUMMY_VELOCITY: launchDummyVelocity(d, s); break;
         case MPS_OP_INIT_PND: ensureMasks(h); ensureCache(h); launchInitPnd(d, s); break;
@@ -527,7 +547,7 @@ static int stepImpl(mpsgpu_t h) {
     } else {   // both operators in one pass (the profiler keeps them apart)
         launchGravityPredict(h->d, h->s);
         countLaunch(1);
-        h->listValid = h->masksValid = h->cacheValid = h->corrFresh = h->pAuxFresh = false;
+        h->listValid = h->masksValid = h->cacheValid = h->corrFresh = h->pAuxFresh = h->copiesFresh = false;
         if ((e = launchStatus())) return e;
     }
     RUN(MPS_OP_OUT_OF_DOMAIN);
@@ -1381,7 +1401,7 @@ int mpsgpu_set_field(mpsgpu_t h, int f, const void* host) {
     h->pAuxFresh = false;
     h->masksValid = false;
     h->cacheValid = false;
-    if (f == MPS_F_POS) launchPosf(h->d, h->s);
+    if (f == MPS_F_POS) { launchPosf(h->d, h->s); h->copiesFresh = true; }
     if (f == MPS_F_CORR1 || f == MPS_F_CORR2 || f == MPS_F_CORR3) launchCorrDF(h->d, h->s);
     CK(cudaStreamSynchronize(h->s));
     return 0;
