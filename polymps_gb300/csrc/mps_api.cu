@@ -1414,6 +1414,7 @@ int mpsgpu_get_neighbors(mpsgpu_t h, int* counts, int* nbr, long long cap) {
     if (e) return e;
     int n = 0;
     if ((e = mpsgpu_num_particles(h, &n))) return e;
+    if (n == 0) return 0;   // every particle has been removed
     // rows and entries in reference indices (storage is in bucket order), laid out on the GPU:
     // counts, their scan, then the rows one after the other through the reorder scratch, as
     // many at a time as it holds (any row fits).  Copying the whole ELL array and reordering it on
