@@ -89,9 +89,10 @@ __device__ __forceinline__ df divDF(df a, df b) {
 __device__ __forceinline__ bool operator<(df a, df b) { return a.h < b.h || (a.h == b.h && a.l < b.l); }
 __device__ __forceinline__ bool operator>(df a, df b) { return b < a; }
 
-// conversions (per particle and per stored value).  dfD: the significand's upper 24 bits and its
-// lower 29 bits as two floats, normalised by a fast two-sum, without an FP64 operation; values
-// outside the normal range of FP32 are rounded and subtracted in FP64.
+// conversions (per particle and per stored value).  dfD: h = fl32(x), l = fl32(x - h), within
+// 2^-49 of x, without an FP64 operation: the significand's upper 24 bits rounded to nearest by the
+// lower 29, and what the rounding left, a 29-bit signed integer, as the second float.  Values outside
+// the range in which that float is exact to its last bit are rounded and subtracted in FP64.
 static __device__ __noinline__ df dfWide(double x) {
     const float h = d2fRN(x);
     return {h, d2fRN(x - f2dExact(h))};
@@ -99,10 +100,11 @@ static __device__ __noinline__ df dfWide(double x) {
 __device__ __forceinline__ df dfD(double x) {
     const unsigned xh = (unsigned)__double2hiint(x), xl = (unsigned)__double2loint(x);
     const unsigned s = xh & 0x80000000u, e = (xh >> 20) & 0x7ffu;
-    if (e - 897u >= 253u) return (x == 0.0) ? df{(float)0.f, 0.f} : dfWide(x);
-    const float h = __uint_as_float(s | __funnelshift_l(xl, (xh & 0x7fffffffu) - 0x38000000u, 3));
-    const float l = (float)(xl & 0x1fffffffu) * 0x1p-52f * __uint_as_float(s | ((e - 896u) << 23));
-    return quick2(h, l);
+    if (e - 926u >= 224u) return (x == 0.0) ? df{(float)0.f, 0.f} : dfWide(x);   // below 2^-97 or from 2^127 up
+    const unsigned t = __funnelshift_l(xl, (xh & 0x7fffffffu) - 0x38000000u, 3), low = xl & 0x1fffffffu;
+    const unsigned up = (low + 0x0fffffffu + (t & 1u)) >> 29;
+    const int r = (int)(low - (up << 29));
+    return {__uint_as_float(s | (t + up)), (float)r * 0x1p-52f * __uint_as_float(s | ((e - 896u) << 23))};
 }
 // one FP64 addition
 __device__ __forceinline__ double dD(df a) { return f2dExact(a.h) + f2dExact(a.l); }
