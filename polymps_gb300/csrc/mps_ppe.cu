@@ -1833,11 +1833,6 @@ __device__ __forceinline__ void resLoad(const ResRow& r, int* sc, T* sv, int cap
     }
 }
 
-// a / b to the last bits of the pair: the quotient of divDF corrected by its remainder
-__device__ __forceinline__ df divDF2(df a, df b) {
-    const df q = divDF(a, b);
-    return q + divDF(a - b * q, b);
-}
 // Plain FP64 Jacobi-PCG with one reduction an iteration (Chronopoulos and Gear, s-step methods,
 // J. Comput. Appl. Math. 25, 1989): with q = A z,
 //   gamma = r.z, delta = z.q, rho = r.r;  beta = gamma / gamma_old,
@@ -1948,9 +1943,10 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
 // columns.  One reduction an iteration (Chronopoulos and Gear, s-step methods, J. Comput. Appl.
 // Math. 25, 1989): with q = A z,
 //   gamma = r.z, delta = z.q, rho = r.r;  beta = gamma / gamma_old,
-//   alpha = gamma / (delta - gamma^2 / (gamma_old alpha_old)),
+//   p.Ap = delta - beta^2 (p.Ap)_old,  alpha = gamma / p.Ap,
 //   p = z + beta p,  Ap = q + beta Ap,  x += alpha p,  r -= alpha Ap,  z = M^-1 r,
-// the same vectors as k_cg_res, whose p.Ap it forms by linearity too.  The first warp has no
+// the same vectors as k_cg_res, whose p.Ap it forms by linearity too, and like there the set-up's
+// sums, the step scalars and the residual of the result are FP64.  The first warp has no
 // rows: it sums the warps' partials and forms the step scalars.
 // Bound by latency: at 2,916 rows an iteration takes ~7,000 cycles, the product 1,650, delta and
 // its barrier 1,700, collecting the partials 660.  Only delta waits for the product, so z is
@@ -1995,6 +1991,31 @@ __device__ __forceinline__ void clPush(const double (&v)[NV], int q0, int dq, in
     if (lane < CLB)
 #pragma unroll
         for (int k = 0; k < NV; k++) clStore(&S.part[set][q0 + k * dq][w][rank], lane, make_float2(a[k].h, a[k].l));
+}
+// The same in FP64, for the sums of the set-up and of the result.
+template <int NV>
+__device__ __forceinline__ void clPushD(double (&v)[NV], int set, ClShared& S, unsigned rank) {
+    const int lane = threadIdx.x & 31, w = ((int)threadIdx.x >> 5) - 1;
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+        if (lane < CLB) clStore(&S.part[set][q][w][rank], lane, v[q]);
+    }
+}
+template <int NV>
+__device__ __forceinline__ void clTotalD(int set, const ClShared& S, double (&a)[NV]) {
+    const int lane = threadIdx.x & 31, nw = ((int)blockDim.x >> 5) - 1;
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+        a[q] = 0.0;
+        for (int m = lane; m < nw * CLB; m += 32) {
+            const float2 x = S.part[set][q][0][m];   // an FP64 value's two words
+            a[q] += __hiloint2double(__float_as_int(x.y), __float_as_int(x.x));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a[q] += __shfl_xor_sync(0xffffffffu, a[q], o);
+    }
 }
 template <int NV>
 __device__ __forceinline__ void clTotal(int set, const ClShared& S, df (&a)[NV]) {
@@ -2075,16 +2096,16 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
     }
     clWait();   // every block of the cluster has started
     if (t >= 0) {
-        const double v[2] = {bi * bi, r * r};
-        clPush<2>(v, 0, 1, 0, S, rank);
+        double v[2] = {bi * bi, r * r};
+        clPushD<2>(v, 0, S, rank);
     }
     clArrive();
     clWait();   // also ends every block's reads of x
     if (threadIdx.x < 32) {
-        df a[2];
-        clTotal<2>(0, S, a);
+        double a[2];
+        clTotalD<2>(0, S, a);
         if (threadIdx.x == 0) {
-            const double bb = dD(a[0]), rr = dD(a[1]);
+            const double bb = a[0], rr = a[1];
             qS[S_BB] = bb;
             double thr = tol * tol * bb;
             if (thr < 2.2250738585072014e-308) thr = 2.2250738585072014e-308;
@@ -2104,10 +2125,7 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
     }
     clArrive();
     clWait();
-    // thread 0: 1 / gamma_old and 1 / alpha_old, and the squared residual norm that ends it
-    df invGamma = dfF(0.f), invAlpha = dfF(0.f);
-    const df stop2 = dfD(qS[S_THR]), one = dfF(1.f);
-    __syncthreads();
+    double gamma = 0.0, pap = 0.0, invGamma = 0.0;   // thread 0 (invGamma: 1 / gamma, 0 before the first iteration)
     for (int set = 1; !S.stop; set ^= 1) {
         double q = 0.0;
         if (own) q = product(z);
@@ -2117,22 +2135,23 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
         }
         clArrive();
         clWait();
-        df gamma = dfF(0.f), alpha2 = dfF(0.f);
         if (threadIdx.x < 32) {
             df a[3];
             clTotal<3>(set, S, a);
             if (threadIdx.x == 0) {
-                // step scalars in float-float like the sums they come from (a chain of FP64
-                // divisions on one thread would be a third of the iteration)
-                gamma = a[0];
-                const df beta = gamma * invGamma;                      // 0 in the first iteration
-                alpha2 = divDF2(gamma, a[1] - gamma * (beta * invAlpha));
-                S.alpha = dD(alpha2);
-                S.beta = dD(beta);
-                if (a[2] < stop2) qF[0] = 1;
-                if (!(a[2].h == a[2].h) || !(gamma.h == gamma.h)) { qF[0] = 1; qF[2] = 1; }
+                const double g = dD(a[0]), rr = dD(a[2]);
+                // g / gamma by the reciprocal taken while the other blocks arrived, and its remainder (a
+                // division here would be a tenth of the iteration)
+                double beta = g * invGamma;
+                beta = fma(fma(-beta, gamma, g), invGamma, beta);
+                pap = dD(a[1]) - beta * (beta * pap);
+                gamma = g;
+                S.alpha = g / pap;
+                S.beta = beta;
+                if (rr < qS[S_THR]) qF[0] = 1;
+                if (!(rr == rr) || !(g == g)) { qF[0] = 1; qF[2] = 1; }
                 S.stop = qF[0] || qF[1] >= maxIter;
-                if (S.stop) qS[S_RR] = dD(a[2]);
+                if (S.stop) qS[S_RR] = rr;
             }
         }
         __syncthreads();
@@ -2153,8 +2172,7 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
         }
         if (threadIdx.x == 0) {
             qF[1] += 1;
-            invGamma = divDF2(one, gamma);
-            invAlpha = divDF2(one, alpha2);
+            invGamma = 1.0 / gamma;
         }
         clWait();
     }
@@ -2166,15 +2184,15 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
     clWait();
     if (t >= 0) {
         const double e = own ? bi - product(x) : 0.0;
-        const double v[1] = {e * e};
-        clPush<1>(v, 0, 0, 0, S, rank);
+        double v[1] = {e * e};
+        clPushD<1>(v, 0, S, rank);
     }
     clArrive();
     clWait();
     if (threadIdx.x < 32) {
-        df a[1];
-        clTotal<1>(0, S, a);
-        if (threadIdx.x == 0) qS[S_RR] = dD(a[0]);
+        double a[1];
+        clTotalD<1>(0, S, a);
+        if (threadIdx.x == 0) qS[S_RR] = a[0];
     }
     __syncthreads();
     if (rank == 0) qStore(B, qL);
