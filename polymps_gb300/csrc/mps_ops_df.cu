@@ -38,8 +38,7 @@ __device__ __forceinline__ df loadDF(const float2* p, int j) {
 }
 
 template <int L>
-__device__ __forceinline__ df laneSumDF(df v) {   // of accumulators (normalised here)
-    v = normDF(v);
+__device__ __forceinline__ df laneSumDF(df v) {
 #pragma unroll
     for (int o = 1; o < L; o <<= 1) {
         const df q = {__shfl_xor_sync(laneGroup<L>(), v.h, o), __shfl_xor_sync(laneGroup<L>(), v.l, o)};
