@@ -67,11 +67,19 @@ __device__ __forceinline__ df& operator-=(df& a, df b) { a = a - b; return a; }
 // for 2^-48.3, of 128 terms 2^-45.6 for 2^-47.2, at most 1.5% of a step's time.
 __device__ __forceinline__ void mac(df& s, df a, df b) { s += a * b; }
 __device__ __forceinline__ void acc(df& s, df b) { s += b; }
-// a / b: the FP32 quotient and one correction of the remainder (about 2^-45 relative)
-__device__ __forceinline__ df divDF(df a, df b) {
+// a / b rounded to FP32, the bits of the FP64 quotient so rounded: the FP32 quotient and one
+// correction of its remainder are within 2^-44, which settles the rounding unless the quotient
+// lies within 2^-41 of a tie, or a value near the ends of FP32's range; those are divided in FP64.
+static __device__ __noinline__ float divWide(df a, df b) {
+    return d2fRN((f2dExact(a.h) + f2dExact(a.l)) / (f2dExact(b.h) + f2dExact(b.l)));
+}
+__device__ __forceinline__ bool midRange(float x) { return ((__float_as_uint(x) >> 23) & 0xffu) - 27u <= 200u; }   // 2^-100 .. 2^100
+__device__ __forceinline__ float divF(df a, df b) {
     const float y = 1.0f / b.h, q = fM(a.h, y);
     const df r = a - b * q;
-    return quick2(q, fM(r.h, y));
+    const df t = quick2(q, fM(r.h, y));
+    const bool sure = fA(t.h, fM(t.l, 1.0f + 0x1p-16f)) == t.h;
+    return sure && midRange(a.h) && midRange(b.h) && midRange(t.h) ? t.h : divWide(a, b);
 }
 // ordering of normalised values (|l| <= ulp(h)/2)
 __device__ __forceinline__ bool operator<(df a, df b) { return a.h < b.h || (a.h == b.h && a.l < b.l); }

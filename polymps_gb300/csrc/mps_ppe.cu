@@ -1241,9 +1241,9 @@ __device__ __forceinline__ bool mxSetup(const PpeBuffers& B, const RowSet& rs, Q
 }
 
 // NV of the four inner vectors are in shared memory: Ap, p, r, x in this order (the ones an
-// iteration touches most first), the others in B.rf and B.xf.  The step scalars are formed in
-// float-float from the float-float sums (FP64 divisions on one thread between two grid sums:
-// 864k rows 8.31 ms for four solves, now 7.94).
+// iteration touches most first), the others in B.rf and B.xf.  The FP32 step scalars
+// are the bits of the FP64 quotients of the sums, without an FP64 division on one thread between
+// two grid sums (108k learned start 4.76 ms with them, 4.63 without; 864k steps 19.17 / 18.94).
 template <bool LEARNED, int NV>
 __global__ void __launch_bounds__(QBX, 1) k_mx_own(Dev d, PpeBuffers B, double tol, int maxIter, double eta2, int cap) {
     __shared__ QLocal qL;   // this block's copy of the solver scalars and flags
@@ -1277,7 +1277,7 @@ __global__ void __launch_bounds__(QBX, 1) k_mx_own(Dev d, PpeBuffers B, double t
             });
             if (!qSumF2<2>(a, B, c, [&](const df* t) {
                     rz = t[0];
-                    stop2 = t[1] * dfD(qS[S_ETA2]);
+                    stop2 = dfD(dD(t[1]) * qS[S_ETA2]);
                     qF[3] = 0;
                 }))
                 return;
@@ -1295,7 +1295,7 @@ __global__ void __launch_bounds__(QBX, 1) k_mx_own(Dev d, PpeBuffers B, double t
                     sap[l] = ap; sp[l] = p;
                     a[0] += prod2(p, ap);
                 });
-                if (!qSumF2<1>(a, B, c, [&](const df* t) { qL.scalf[SF_ALPHA] = divDF(rz, t[0]).h; })) return;
+                if (!qSumF2<1>(a, B, c, [&](const df* t) { qL.scalf[SF_ALPHA] = divF(rz, t[0]); })) return;
             }
             {   // x_f += alpha p, r -= alpha Ap, z = M^-1 r; r.z, r.r
                 const float alpha = vf(qL.scalf + SF_ALPHA);
@@ -1326,7 +1326,7 @@ __global__ void __launch_bounds__(QBX, 1) k_mx_own(Dev d, PpeBuffers B, double t
                 }
                 if (!qSumF2<2>(a, B, c, [&](const df* t) {
                         qF[1] += 1;
-                        qL.scalf[SF_BETA] = divDF(t[0], rz).h;
+                        qL.scalf[SF_BETA] = divF(t[0], rz);
                         rz = t[0];
                         if (t[1] < stop2 || !(t[1].h == t[1].h)) qF[3] = 1;
                     }))
@@ -2307,7 +2307,7 @@ __global__ void __launch_bounds__(RBS, 1) k_mx_res(Dev d, PpeBuffers B, double t
             }
             if (!qSumF2<2>(a, B, c, [&](const df* t) {
                     rz = t[0];
-                    stop2 = t[1] * dfD(qS[S_ETA2]);
+                    stop2 = dfD(dD(t[1]) * qS[S_ETA2]);
                     qF[3] = 0;
                 }))
                 return;
@@ -2323,7 +2323,7 @@ __global__ void __launch_bounds__(RBS, 1) k_mx_res(Dev d, PpeBuffers B, double t
                     pf = inner ? zf + beta * pf : zf;
                     if (own) a[0] = prod2(pf, apf);
                 }
-                if (!qSumF2<1>(a, B, c, [&](const df* t) { qL.scalf[SF_ALPHA] = divDF(rz, t[0]).h; }, R.any)) return;
+                if (!qSumF2<1>(a, B, c, [&](const df* t) { qL.scalf[SF_ALPHA] = divF(rz, t[0]); }, R.any)) return;
             }
             {   // x_f += alpha p, r -= alpha Ap, z = M^-1 r; r.z, r.r
                 const float alpha = vf(qL.scalf + SF_ALPHA);
@@ -2338,7 +2338,7 @@ __global__ void __launch_bounds__(RBS, 1) k_mx_res(Dev d, PpeBuffers B, double t
                 }
                 if (!qSumF2<2>(a, B, c, [&](const df* t) {
                         qF[1] += 1;
-                        qL.scalf[SF_BETA] = divDF(t[0], rz).h;
+                        qL.scalf[SF_BETA] = divF(t[0], rz);
                         rz = t[0];
                         if (t[1] < stop2 || !(t[1].h == t[1].h)) qF[3] = 1;
                     }, R.any))
