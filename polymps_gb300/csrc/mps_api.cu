@@ -458,7 +458,7 @@ static int runOpBody(mpsgpu_t h, int op) {
             ensureMasks(h);
             if (h->corrFresh && h->masksValid) {   // formed by the PND sweep: publish it
                 std::swap(d.c1, d.c1n); std::swap(d.c2, d.c2n); std::swap(d.c3, d.c3n);
-                std::swap(d.corrDF, d.corrDFn);
+                if (x) std::swap(d.corrDF, d.corrDFn);   // the FP64 sweep writes no float-float copy
                 h->corrFresh = false;
                 h->opSkipped = true;
                 break;
