@@ -1270,6 +1270,7 @@ __global__ void __launch_bounds__(WALL_BLK) k_wall_press_grad(Dev d, bool fresh)
             const PairG m = pairSum(pi, mi);
             double wS, wd;
             weightR(m.d2, P.reS, P.weightType, wS, wd);
+            if (!(m.d2 > 0.0)) wS = wfun(0.0, P.reS, P.weightType);   // on the wall: 1 / r does not give w
             const double f = phi(i, i, Pi, ni, pmn[g], wS, wd);
             ax += m.v0 * f; ay += m.v1 * f; az += m.v2 * f;
         }
