@@ -789,7 +789,7 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
         d.oodHi[k] = p->domainMax[k] - p->bucketSide;
     }
     d.nB = p->numBucketsXYZ;
-    d.K = ((int)p->dim == 3) ? 128 : 64;   // entries per neighbour row (compressed flows reach ~2x the rest count)
+    d.K = ((int)p->dim == 3) ? NBR_CAP_3D : NBR_CAP_2D;
     int e = 0;
 #define A(ptr, cnt) do { if ((e = dalloc(h, &(ptr), (cnt)))) { mpsgpu_destroy(h); return e; } } while (0)
     A(d.nLive, 1);

@@ -245,7 +245,10 @@ static PermArrays permArrays(const Dev& d) {
              d.velDiv, d.diffTerm, d.pndWall, d.riw2, d.devDot, d.source, d.aux1, d.aux2},
             {d.type, d.bc, d.numNeigh, d.nNeighWall, d.nearWall, d.cellOf}};
 }
-// scratch: vectors in cw (32 PERM_V = 512 bytes a particle), the rest in cwd
+// scratch: vectors in cw, the rest in cwd (each K doubles a particle)
+static_assert(PERM_V * sizeof(dvec4) <= NBR_CAP_2D * sizeof(double) && NBR_CAP_2D <= NBR_CAP_3D, "cw holds the vectors");
+static_assert(2 * sizeof(float4) + PERM_S * sizeof(double) + (PERM_I + 1) * sizeof(int) <= NBR_CAP_2D * sizeof(double),
+              "cwd holds the FP32 copies, the scalars, the integers and the reference index");
 struct PermScratch {
     dvec4* v;
     float4 *hi, *lo;

@@ -30,6 +30,10 @@ struct Prof {
     void destroy();
 };
 
+// entries per neighbour row (compressed flows reach about twice the rest count)
+#define NBR_CAP_2D 64
+#define NBR_CAP_3D 128
+
 // mps_cells.cu
 void scanExclusive(const int* in, int* out, int n, int* scratch, cudaStream_t s);
 int scanScratchInts(int n);
