@@ -866,8 +866,10 @@ int mlpForwardHost(MlpState& m, const float* hfeat, int n, float* hout, cudaStre
     }
     if (!e) e = mlpForwardTc(m, df, n, nullptr, nullptr, 0, nullptr, dout, s);
     if (!e) {
+        // touched by adding nothing: work queued on the stream before may still read the array
         if (apart)
-            for (size_t k = 0; k < (size_t)n; k += 1024) ((volatile float*)hout)[k] = 0.f;   // 4 KB pages
+            for (size_t k = 0; k < sizeof(float) * (size_t)n; k += 4096)
+                __atomic_fetch_add(reinterpret_cast<unsigned char*>(hout) + k, 0, __ATOMIC_RELAXED);
         if (cudaMemcpyAsync(hout, dout, sizeof(float) * n, cudaMemcpyDeviceToHost, s) != cudaSuccess) e = MPSGPU_ERR_CUDA;
     }
     const int q = mlpTcQueue(m, s);
