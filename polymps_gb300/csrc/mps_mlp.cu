@@ -887,7 +887,9 @@ int mlpForwardHost(MlpState& m, const float* hfeat, int n, float* hout, cudaStre
 int mlpGradient(MlpState& m, const float* hfeat, const float* htarget, int n, float* hgrad, float* hloss,
                 cudaStream_t s) {
     if (n < 64 || (n % 64)) return MPSGPU_ERR_ARG;
-    const bool direct = m.hostTables && (reinterpret_cast<uintptr_t>(hfeat) & 15u) == 0;
+    // float4 and float loads
+    const bool direct = m.hostTables && (reinterpret_cast<uintptr_t>(hfeat) & 15u) == 0 &&
+                        (reinterpret_cast<uintptr_t>(htarget) & 3u) == 0;
     const size_t gradWords = (NPARAM + 1 + 63) / 64 * 64;
     bool kept = false;
     float* const grad = (float*)hostWork(m, sizeof(float) * (gradWords + (direct ? 0 : (size_t)(NF + 1) * n)), &kept);
