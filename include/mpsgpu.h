@@ -384,9 +384,9 @@ int mpsgpu_launch_count(long long* n);
  *    turns;
  *  - the first call on a device looks the array's address up with that device
  *    current; make it before any stream capture begins.
- * The call synchronises `stream` (cudaStream_t as void*, may be NULL) to poll
- * convergence.  iters / relres (may be NULL) receive the iteration count and the true
- * relative residual |b - Ax| / |b|.  mpsgpu_pcg_static_error() gives the last message. */
+ * The call waits for `stream` (cudaStream_t as void*, may be NULL) once, at its end.
+ * iters / relres (may be NULL) receive the iteration count and the true relative residual
+ * |b - Ax| / |b|.  mpsgpu_pcg_static_error() gives the last message. */
 #define MPSGPU_STATIC_MAX_ROWS (1 << 17)
 int mpsgpu_pcg_solve_static(int n, const int* rowptr, const int* col, const double* val,
                             const double* b, double* x, double tol, int max_iter, void* stream,

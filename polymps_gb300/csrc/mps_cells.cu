@@ -11,8 +11,6 @@
 #include "mps_internal.h"
 #include "mps_lanes.cuh"
 
-__global__ void k_posf_cell(Dev d);
-
 static std::atomic<long long> g_launches{0};
 void countLaunch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long long launchCount() { return g_launches.load(std::memory_order_relaxed); }

@@ -60,7 +60,8 @@ __device__ __forceinline__ Mask laneOr(Mask m) {
 template <int L>
 __device__ __forceinline__ Mask laneShare(Mask m, int l) {
     if (L == 1) return m;
-    const unsigned long long p = (L == 2 ? 0x5555555555555555ull : L == 4 ? 0x1111111111111111ull : 0x0101010101010101ull) << l;
+    static_assert(L == 1 || L == 4 || L == 8, "the lane counts of lanesFor");
+    const unsigned long long p = (L == 4 ? 0x1111111111111111ull : 0x0101010101010101ull) << l;
     m.lo &= p; m.hi &= p;
     return m;
 }

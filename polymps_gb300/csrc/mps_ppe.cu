@@ -1739,7 +1739,7 @@ __global__ void __launch_bounds__(QBC, 1) k_cg_own(Dev d, PpeBuffers B, double t
 
 // ------------------------------------------------------------------ resident matrices
 // The solvers of systems with at most one row per thread of the grid (152 x RBS = 116,736
-// rows): L lanes (1, 2, 4 or 8: as many as fit) share a row, lane l holding the entries l,
+// rows): L lanes (4, 2 or 1: as many as fit) share a row, lane l holding the entries l,
 // l + L, ..., and the first `cap` entries of every lane stay in the block's shared memory from the
 // first iteration to the last (slot e RBS + thread), the others, if any, are streamed.  A
 // row's vector elements are registers of its lanes.  An iteration then reads nothing but z, in
