@@ -1857,7 +1857,7 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
     resLoad(R, sc, sv, cap, B.col, B.val);
     double x = 0.0, r = 0.0, z = 0.0, p = 0.0, ap = 0.0, di = 0.0, dg = 0.0;
     {
-        double v[2] = {0.0, 0.0};
+        double v[3] = {0.0, 0.0, 0.0};
         if (R.any) {
             const double q = resDot<double>(R, sc, sv, cap, B.col, B.val, B.x);
             if (R.i >= 0) {
@@ -1869,11 +1869,11 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
                 z = r * di;
                 if (own) {
                     B.z[R.i] = z;
-                    v[0] = r * r; v[1] = bi * bi;
+                    v[0] = r * r; v[1] = bi * bi; v[2] = r * z;
                 }
             }
         }
-        if (!qSum<2>(v, B, c, [&](const double* t) {   // and z is complete
+        if (!qSum<3>(v, B, c, [&](const double* t) {   // and z is complete
                 qS[S_RR] = t[0]; qS[S_BB] = t[1];
                 double thr = tol * tol * t[1];
                 if (thr < 2.2250738585072014e-308) thr = 2.2250738585072014e-308;
@@ -1882,6 +1882,7 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
                 qF[0] = (t[1] == 0.0 || t[0] < thr) ? 1 : 0;
                 qF[1] = 0;
                 if (!(t[0] == t[0])) { qF[0] = 1; qF[2] = 1; }
+                S.gamma = t[2];
                 S.stop = qF[0] || maxIter <= 0;
             }))
             return;
@@ -1893,10 +1894,10 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
             if (own) { v[0] = r * z; v[1] = z * q; v[2] = r * r; }
         }
         if (!qSumD<3>(v, B, c, [&](const double* t) {
-                const double gamma = t[0];
-                qS[S_RR] = t[2];
-                if (t[2] < qS[S_THR]) qF[0] = 1;
-                if (!(t[2] == t[2]) || !(gamma == gamma)) { qF[0] = 1; qF[2] = 1; }
+                const double gamma = qF[1] ? t[0] : S.gamma, rr = qF[1] ? t[2] : qS[S_RR];   // first: of the set-up
+                qS[S_RR] = rr;
+                if (rr < qS[S_THR]) qF[0] = 1;
+                if (!(rr == rr) || !(gamma == gamma)) { qF[0] = 1; qF[2] = 1; }
                 S.stop = qF[0] || qF[1] >= maxIter;
                 if (S.stop) return;
                 S.beta = qF[1] ? gamma / S.gamma : 0.0;
@@ -2096,16 +2097,18 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
     }
     clWait();   // every block of the cluster has started
     if (t >= 0) {
-        double v[2] = {bi * bi, r * r};
-        clPushD<2>(v, 0, S, rank);
+        double v[3] = {bi * bi, r * r, r * z};
+        clPushD<3>(v, 0, S, rank);
     }
     clArrive();
     clWait();   // also ends every block's reads of x
+    double gamma = 0.0, pap = 0.0, invGamma = 0.0;   // thread 0 (invGamma: 1 / gamma, 0 before the first iteration)
     if (threadIdx.x < 32) {
-        double a[2];
-        clTotalD<2>(0, S, a);
+        double a[3];
+        clTotalD<3>(0, S, a);
         if (threadIdx.x == 0) {
             const double bb = a[0], rr = a[1];
+            gamma = a[2];
             qS[S_BB] = bb;
             double thr = tol * tol * bb;
             if (thr < 2.2250738585072014e-308) thr = 2.2250738585072014e-308;
@@ -2125,7 +2128,6 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
     }
     clArrive();
     clWait();
-    double gamma = 0.0, pap = 0.0, invGamma = 0.0;   // thread 0 (invGamma: 1 / gamma, 0 before the first iteration)
     for (int set = 1; !S.stop; set ^= 1) {
         double q = 0.0;
         if (own) q = product(z);
@@ -2139,7 +2141,7 @@ __global__ void __launch_bounds__(CL_ROWS + 32, 1) k_cg_cluster(Dev d, PpeBuffer
             df a[3];
             clTotal<3>(set, S, a);
             if (threadIdx.x == 0) {
-                const double g = dD(a[0]), rr = dD(a[2]);
+                const double g = qF[1] ? dD(a[0]) : gamma, rr = qF[1] ? dD(a[2]) : qS[S_RR];   // first: of the set-up
                 // g / gamma by the reciprocal taken while the other blocks arrived, and its remainder (a
                 // division here would be a tenth of the iteration)
                 double beta = g * invGamma;
