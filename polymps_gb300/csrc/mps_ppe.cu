@@ -1949,11 +1949,12 @@ __global__ void __launch_bounds__(RBS, 1) k_cg_res(Dev d, PpeBuffers B, double t
 // the same vectors as k_cg_res, whose p.Ap it forms by linearity too, and like there the set-up's
 // sums, the step scalars and the residual of the result are FP64.  The first warp has no
 // rows: it sums the warps' partials and forms the step scalars.
-// Bound by latency: at 2,916 rows an iteration takes ~7,000 cycles, the product 1,650, delta and
-// its barrier 1,700, collecting the partials 660.  Only delta waits for the product, so z is
+// Bound by latency: at the 2-D dam's 2,916 rows an iteration takes ~9,600 cycles, the product 1,700,
+// delta and its barrier 1,900, collecting the partials 750, the FP64 scalars 2,000, the update
+// with the next sums 2,500.  Only delta waits for the product, so z is
 // published as soon as it is known, and the x update and the trees of the next iteration's r.z
 // and r.r run between arrival and wait of its barrier (three sums after the product, all in one
-// exchange: 603 us for the three solves named at CLUSTER_MAX_ROWS, now 510).
+// exchange, took 18% longer).
 #define CLB 16                 // blocks of the cluster
 #define CL_ROWS 256            // rows of a block at most
 struct ClShared {
@@ -2596,9 +2597,9 @@ int ppeSolveBicgstab(const Dev& d, const PpeBuffers& B, double tol, int maxIter,
 }
 
 // Rows up to which one cluster takes the plain FP64 solve, all that its blocks hold at one row per
-// thread.  Three first solves of a run (64 to 76 iterations, set-up included) by k_cg_cluster and
-// k_cg_res at 1,000 rows 417 / 563 us, 2,048 rows 488 / 618, 2,916 rows 510 / 639, 4,000 rows
-// 594 / 665: the gain shrinks as the 16 SMs' FP64 pipes fill.
+// thread.  Three first solves of a run (65 to 76 iterations, set-up included) by k_cg_cluster and
+// k_cg_res at 1,000 rows 463 / 599 us, 2,048 rows 535 / 658, 2,916 rows 567 / 682, 4,000 rows
+// 650 / 713: the gain shrinks as the 16 SMs' FP64 pipes fill.
 #define CLUSTER_MAX_ROWS 4096
 // Lanes per row of the resident solvers: 4, 2 or 1, as many as give every row of `rows` its
 // lanes in one round of the grid; 0: too many rows.
