@@ -11,6 +11,7 @@
 #include <algorithm>
 #include "mps_common.cuh"
 #include "mps_internal.h"
+#include "mps_lanes.cuh"
 #include "mps_host.h"
 #include "mps_mlp.h"
 
@@ -44,7 +45,7 @@ struct mpsgpu_s {
     bool skinShift = false;    // ... and still intact for the shifting sweeps of the step
     int nHost = -1;            // live count known on the host (-1: read it from the device)
     int *nbrAlt = nullptr, *cntAlt = nullptr;   // second list arrays (the skin list keeps its own)
-    int skinOn = 1;            // viscosity and the post-prediction list from the start-of-step skin list
+    bool skinOn = true;        // viscosity and the post-prediction list from the start-of-step skin list
     bool copiesFresh = false;  // the FP32 copies, by particle and by bucket, are those of the positions
     bool corrFresh = false;    // the correction matrix of the current positions and masks is written
     bool pAuxFresh = false;    // the last operator was the pressure gradient: its p_min still stand
@@ -229,6 +230,12 @@ static void ensureMasks(mpsgpu_t h) {
     if (h->prof.on) h->prof.end(h->s);
     countLaunch(1);
     h->masksValid = true;
+}
+
+// Particles in the ball (2D: the disc) of radius r of a filled neighbourhood.
+static double filledBall(const MpsParams& P, double r) {
+    const double x = r / P.partDist;
+    return (int)P.dim == 2 ? M_PI * x * x : 4.0 / 3.0 * M_PI * x * x * x;
 }
 
 // Switches of the reference outside the implemented path, each with the reason.
@@ -886,6 +893,14 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
         {
             double skin = 0.15 * p->partDist;
             double rs = std::sqrt(d.reMax2) + skin;
+            // where filled neighbourhoods do not fit the rows (radii above 2.92 l0 in 3D), they overflow
+            // and every such particle scans the buckets again after the list was built for it: the
+            // buckets are scanned at once instead.  A step of 384k incompressible particles, float-float
+            // / FP64, with a radius of 2.9 l0 (119 particles in the list's ball) 3.27 / 5.6 ms with
+            // the list and 4.17 / 11.4 without, 3.0 l0 (131) 7.17 / 15.9 and 5.06 / 12.9, 3.1 l0 8.35 / 17.5
+            // and 5.54 / 14.2; 97k 2.71 / 5.35 and 2.18 / 4.88.  Small systems, whose lanes share a
+            // particle, keep the list (8,000 particles, 3.1 l0: 0.83 / 1.40 and 0.97 / 1.31).
+            h->skinOn = lanesFor(n) > 1 || filledBall(*p, rs) <= 0.95 * d.K;
             d.skinR2 = (float)(rs * rs + band(rs * rs));
             double mv = 0.5 * skin - 8.0 * std::ldexp(1.0, -24) * X;   // FP32 hi-part error of both copies
             d.skinMove2 = (float)(mv > 0.0 ? mv * mv : 0.0);
