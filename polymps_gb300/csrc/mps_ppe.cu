@@ -1750,7 +1750,8 @@ __global__ void __launch_bounds__(QBC, 1) k_cg_own(Dev d, PpeBuffers B, double t
 // Whole solves per step, k_cg_own / k_mx_own before and now: plain FP64 CG at 2,000 rows (27
 // iterations) 0.355 -> 0.242 ms, at 6,912 (25) 0.391 -> 0.252 ms, mixed solver to 1e-10 at
 // 108,000 rows (39 iterations, 1.75 refinements) 0.65 -> 0.38 ms.  Above one row per
-// thread the matrix of a block no longer fits: k_cg_own and k_mx_own stream it.
+// thread, or with long rows (resLanes), the matrix of a block no longer fits: k_cg_own and
+// k_mx_own stream it.
 #define RBS 768
 #define RES_CAP32 36   // entries per lane: 36 x 768 x 8 B = 216 KB
 #define RES_CAP64 24   // 24 x 768 x 12 B = 216 KB
@@ -2602,10 +2603,17 @@ int ppeSolveBicgstab(const Dev& d, const PpeBuffers& B, double tol, int maxIter,
 // 650 / 713: the gain shrinks as the 16 SMs' FP64 pipes fill.
 #define CLUSTER_MAX_ROWS 4096
 // Lanes per row of the resident solvers: 4, 2 or 1, as many as give every row of `rows` its
-// lanes in one round of the grid; 0: too many rows.
-static int resLanes(int rows, int grid) {
+// lanes in one round of the grid; 0: too many rows, or too many entries (`filled` a row in a filled
+// neighbourhood, `cap` of each lane held) are left to be streamed in every product, which the
+// solvers without a resident matrix do eight at a time.  Whole solves, resident / k_cg_own and
+// resident / k_mx_own: 97k rows of 92 entries (6.6M and 5.4M streamed) 0.561 / 0.591 and 0.533 / 0.549 ms,
+// 115k of 80 (6.5M, 5.1M) 0.670 / 0.652 and 0.509 / 0.561, 115k of 92 (7.8M, 6.5M) 0.710 / 0.646 and
+// 0.603 / 0.589, 61k of 122 (6.0M, 5.2M) 0.600 / 0.597 and 0.560 / 0.570, 97k of 122 (9.5M, 8.4M) 0.698 /
+// 0.657 and 0.755 / 0.627.
+#define RES_STREAMED 6e6
+static int resLanes(int rows, int grid, double filled, int cap) {
     for (int L = 4; L; L >>= 1)
-        if (rows <= grid * (RBS / L)) return L;
+        if (rows <= grid * (RBS / L)) return rows * (filled - (double)(L * cap)) <= RES_STREAMED ? L : 0;
     return 0;
 }
 
@@ -2644,7 +2652,9 @@ int ppeSolvePersistent(const Dev& d, const PpeBuffers& B, int mixed, double tol,
             return finishPersistent(B, s, iters, refinements, relres, relres0);
         }
     }
-    const int lanes = B.matfree == 0 && !B.ownOff && B.pgridRes > 0 ? resLanes(d.N0, B.pgridRes) : 0;
+    const int lanes = B.matfree == 0 && !B.ownOff && B.pgridRes > 0
+                          ? resLanes(d.N0, B.pgridRes, d.P.numNeighZero, mixed ? RES_CAP32 : RES_CAP64)
+                          : 0;
     if (lanes) {
         // at most one row per thread: the matrix stays in shared memory.  The rows are spread
         // over all SMs (the FP64 pipe and the latencies are per SM), 16 to a block at least
