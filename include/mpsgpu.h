@@ -261,7 +261,7 @@ int mpsgpu_set_solver(mpsgpu_t h, int solver, int warm_start, double tol, int ma
  * convergence every few iterations; 1 (default) the whole solve in one cooperative launch
  * with device-side grid barriers (the mixed solver with every block owning one contiguous,
  * work-balanced range of rows and keeping its FP32 inner-CG vectors in shared memory, where
- * they fit: all four up to 11,264 rows per SM, two of them up to 28,672; up to one row per thread of
+ * they fit: all four up to 11,264 rows per SM, two of them up to 24,576; up to one row per thread of
  * the grid, 116,736 rows, both solvers also keep the matrix in shared memory, as far as its
  * rows are not too long for that); 2 as 1, with the mixed solver's FP32 matrix
  * streamed through shared memory by bulk copies (measured slower than 1 at 864k rows: the

@@ -1051,7 +1051,9 @@ int mpsgpu_create(const MpsParams* p, int n, const int* type, const double* pos3
             const long long slots = ((long long)n / ((long long)B.pgridOwn * 1024) + 1) * 1024;
             // shared memory for the vectors is taken from the L1 cache of the z gathers.  Solves
             // with 4, 3 and 2 vectors there: 864k rows 7.94 / 8.07 / 8.10 ms, 1.5M 8.14 / 8.31 / 8.47,
-            // 2.0M 11.00 / 10.67 / 10.77; 2.8M rows with 2 (more do not fit) 14.6, none 15.4.
+            // 2.0M 11.00 / 10.67 / 10.77; 2.8M rows with 2 (more do not fit) 14.6, none 15.4.  One solve of
+            // 3.72M rows of 32 / 80 entries with 2 takes 4.09 / 7.44 ms, with none 4.25 / 7.67; of 3.84M,
+            // where 2 would leave less L1 (OWN_SMEM), 4.54 / 8.26 and 4.40 / 7.89.
             // MPSGPU_OWN_VECTORS sets the number (2 to 4).
             B.ownVec = slots <= 11264 ? 4 : (slots <= 13312 ? 3 : 2);
             if (const char* env = std::getenv("MPSGPU_OWN_VECTORS")) B.ownVec = std::max(2, std::min(4, std::atoi(env)));

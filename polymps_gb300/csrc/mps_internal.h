@@ -191,9 +191,10 @@ int ppeSolveMixed(const Dev& d, const PpeBuffers& B, double tol, int maxIter, cu
 int ppeSolvePersistent(const Dev& d, const PpeBuffers& B, int mixed, double tol, int maxIter, cudaStream_t s,
                        int* iters, int* refinements, double* relres, double* relres0, Prof* prof);
 int ppePersistentGrid(int mixed);
-// shared memory of the mixed solve's vectors at most, and row slots per block of the plain FP64
-// one's (a multiple of its block size, 768)
-#define OWN_SMEM (224 * 1024)
+// shared memory of the mixed solve's vectors at most (with it a block stays within the 196 KB
+// configuration, which leaves the L1 cache 60 KB; the next one leaves 28), and row slots per block
+// of the plain FP64 one's (a multiple of its block size, 768)
+#define OWN_SMEM (192 * 1024)
 #define OWN64_CAP_ROWS 8448
 // BiCGSTAB (solver_type 1) in one cooperative launch
 int ppeSolveBicgstab(const Dev& d, const PpeBuffers& B, double tol, int maxIter, cudaStream_t s, int* iters,
