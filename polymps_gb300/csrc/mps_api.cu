@@ -31,6 +31,7 @@ struct mpsgpu_s {
     int* nearNext = nullptr;      // the near-wall counter not in use (zero)
     double* velNext = nullptr;    // the maximum-speed slot not in use (zero)
     bool fuseBC = false;          // inside a step: the PND sweep writes the boundary condition
+    bool fuseCorr = false;        // ... and the FP64 one forms the correction matrix, which the step reads later
     void* permScratch = nullptr;  // field transfers: reorder scratch, 32 bytes per particle
     int renumberEvery = 20;       // bucket rebuilds between storage renumberings (0: never)
     int renumberCountdown = 0;    // 0: renumber at the next bucket rebuild
@@ -476,7 +477,8 @@ static int runOpBody(mpsgpu_t h, int op) {
             ensureMasks(h);
             // the correction matrix of the step (read after the pressure solve, positions and
             // masks unchanged in between) is formed in the same pass
-            bool corr = P.gradientCorrection && P.pndType != 2;
+            // (called alone, the FP64 sweep would take twice its time for it)
+            const bool corr = P.gradientCorrection && P.pndType != 2 && (x || h->fuseCorr);
             if (x) launchPndNeighNpcdDF(d, s, corr, h->fuseBC); else launchPndNeighNpcd(d, s, corr, h->fuseBC);
             h->corrFresh = corr;
             break;
@@ -597,9 +599,10 @@ static int stepImpl(mpsgpu_t h) {
     // the boundary condition follows from the PND sweep's own sums where nothing changes the PND
     // in between and the free surface is not judged by arcs
     h->fuseBC = P.pndType != 1 && P.pndType != 2 && P.freeSurfType != 2 && !h->prof.on;
+    h->fuseCorr = true;
     e = runOpImpl(h, MPS_OP_PND_NEIGH_NPCD);
     const bool bcDone = h->fuseBC;
-    h->fuseBC = false;
+    h->fuseBC = h->fuseCorr = false;
     if (e) return e;
     if (P.pndType == 2) RUN(MPS_OP_PND_DIFFUSIVE);
     else if (P.pndType == 1) RUN(MPS_OP_PND_MEAN);

@@ -46,3 +46,31 @@ def test_float_float_matrix_across_tiers(oracle_mod, mps_lib):
     assert relerr(g.get(abi.F_ACC), o.get(abi.F_ACC)) <= 1e-8
     g.close()
     o.close()
+
+
+@pytest.mark.parametrize("alone", [True, False])
+def test_fp64_matrix_of_its_own_operator_and_of_a_step(oracle_mod, mps_lib, alone):
+    """The FP64 PND operator called alone leaves the matrix to the matrix operator; a step forms both
+    in one sweep.  The published matrix is the oracle's either way."""
+    import ctypes as C
+    from polymps_gb300 import mps
+    o, g = _pair(oracle_mod, mps, abi.PRECISION_FP64)
+    sync(o, g)
+    if alone:
+        ops = step_ops(o.params)
+        for op in ops[: ops.index("CORRECTION_MATRIX")]:
+            o.run_op(op)
+            g.run_op(op)
+        n = [C.c_longlong(), C.c_longlong()]
+        mps.lib().mpsgpu_launch_count(C.byref(n[0]))
+        o.run_op("CORRECTION_MATRIX")
+        g.run_op("CORRECTION_MATRIX")
+        mps.lib().mpsgpu_launch_count(C.byref(n[1]))
+        assert n[1].value - n[0].value == 1   # 0: published from what the PND sweep formed
+    else:
+        o.step()
+        g.step()
+    for f in (abi.F_CORR1, abi.F_CORR2, abi.F_CORR3):
+        assert relerr(g.get(f), o.get(f)) <= 1e-10
+    g.close()
+    o.close()
