@@ -337,8 +337,9 @@ __device__ __forceinline__ PairM pairMirror(dvec4 pj, dvec4 mi) {
 
 // Per-particle context for the "j is not on the mirror side" test of every sweep
 // (dstij2 < dstimj2 || wallType == PARTICLE, e.g. src/MpsPndNeigh.cpp:249).  When the
-// mirror of i lies farther than 2.2 reL from i, every j within reL of i satisfies
-// |x_j - m_i| >= |x_i - m_i| - r_ij > r_ij + 0.2 reL, so the test is skipped exactly.
+// mirror of i lies farther than 2.2 reMax from i (the larger of the two radii), every j within
+// reMax of i satisfies |x_j - m_i| >= |x_i - m_i| - r_ij > r_ij + 0.2 reMax, so the test is
+// skipped exactly.
 struct SideCtx {
     dvec4 mi;
     bool check;
@@ -348,8 +349,7 @@ __device__ __forceinline__ SideCtx sideCtx(const Dev& d, int i, dvec4 pi) {
     s.mi = d.mirror[i];
     if (d.P.wallType == 0) { s.check = false; return s; }
     double a = pi.x - s.mi.x, b = pi.y - s.mi.y, c = pi.z - s.mi.z;
-    double lim = 2.2 * d.P.reL;
-    s.check = (a * a + b * b + c * c) <= lim * lim;
+    s.check = (a * a + b * b + c * c) <= 4.84 * d.reMax2;
     return s;
 }
 __device__ __forceinline__ bool sideOK(const SideCtx& s, dvec4 pj, double d2) {

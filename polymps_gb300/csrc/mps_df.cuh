@@ -198,8 +198,7 @@ __device__ __forceinline__ SideDF sideDF(const Dev& d, int i, dvec4 pi) {
     if (d.P.wallType == 0) return s;
     dvec4 m = d.mirror[i];
     double a = pi.x - m.x, b = pi.y - m.y, c = pi.z - m.z;
-    double lim = 2.2 * d.P.reL;
-    s.check = (a * a + b * b + c * c) <= lim * lim;
+    s.check = (a * a + b * b + c * c) <= 4.84 * d.reMax2;
     if (s.check) {
         const MpsParams& P = d.P;
         splitPos(m, P, s.mh, s.ml);
