@@ -1185,6 +1185,11 @@ int mpsgpu_set_precision(mpsgpu_t h, int precision) {
         h->corrFresh = false;
         h->masksValid = false;
         h->cacheValid = false;
+        if (precision == MPSGPU_PRECISION_DF32) {   // the matrix that the FP64 tier has formed
+            launchCorrDF(h->d, h->s);
+            countLaunch(1);
+            return launchStatus();
+        }
     }
     return 0;
 }

@@ -74,3 +74,23 @@ def test_fp64_matrix_of_its_own_operator_and_of_a_step(oracle_mod, mps_lib, alon
         assert relerr(g.get(f), o.get(f)) <= 1e-10
     g.close()
     o.close()
+
+
+def test_matrix_of_the_fp64_tier_in_the_float_float_one(oracle_mod, mps_lib):
+    """A float-float pressure gradient after a change of tier reads the matrix the FP64 one formed."""
+    from polymps_gb300 import mps
+    o, g = _pair(oracle_mod, mps, abi.PRECISION_FP64)
+    sync(o, g)
+    ops = step_ops(o.params)
+    for op in ops[: ops.index("CORRECTION_MATRIX") + 1]:
+        o.run_op(op)
+        g.run_op(op)
+    g.set_precision(abi.PRECISION_DF32)
+    # the same pressures on both sides, without the field interface (it would copy the matrix)
+    o.set(abi.F_PRESS, g.get(abi.F_PRESS))
+    o.run_op("PRESS_GRADIENT")
+    g.run_op("PRESS_GRADIENT")
+    assert np.any(o.get(abi.F_ACC))
+    assert relerr(g.get(abi.F_ACC), o.get(abi.F_ACC)) <= 1e-8
+    g.close()
+    o.close()
